@@ -1,4 +1,5 @@
-"""ctypes binding of ``libnvfp4_b200.so`` (the C ABI declared in ``include/nvfp4_b200.h``)."""
+"""Bindings: ``native()`` is the operators' host path (``_native.so``, csrc/host/native.cpp), ``lib()``
+the ctypes view of ``libnvfp4_b200.so`` (the C ABI declared in ``include/nvfp4_b200.h``)."""
 
 from __future__ import annotations
 
@@ -96,6 +97,23 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The native host path of the operators; like the CUDA library it has no fallback."""
+    global _native
+    if _native is None:
+        lib()                                # a missing or stale CUDA library is reported first
+        try:
+            from . import _native as ext
+        except ImportError as exc:
+            raise RuntimeError("sageattention_b200/_native.so is missing or unusable: build it with "
+                               f"`python -m sageattention_b200.build` ({exc})") from exc
+        _native = ext
+    return _native
+
+
 def check(rc: int, what: str = "nvfp4") -> None:
     if rc != 0:
         msg = lib().nvfp4_last_error().decode("utf-8", "replace")
@@ -168,17 +186,10 @@ def stream_ptr(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
-_status_words: dict = {}
-
-
 def status_word(device) -> torch.Tensor:
     """Per-device int32 the kernels write when one of their bounded waits expires."""
-    key = torch.device(device).index
-    w = _status_words.get(key)
-    if w is None:
-        w = torch.zeros(1, dtype=torch.int32, device=device)
-        _status_words[key] = w
-    return w
+    index = torch.device(device).index
+    return native().status_word(torch.cuda.current_device() if index is None else index)
 
 
 def read_status(device) -> int:

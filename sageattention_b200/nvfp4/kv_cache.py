@@ -23,7 +23,6 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from . import flash as _flash
 from .flash import _next_mult, _pack_into
 
 
@@ -31,66 +30,13 @@ def append_token(key_new, value_new, knv, ksc, vnv, vsc, v_partial, rk, rv, pos:
     """One decode token ([Z, Hk, 1, D] or [Z*Hk, D]) into the cache buffers at position ``pos``: one
     kernel launch (K row pack, V stash and re-pack of the open 16-key V^T group, ring write when
     ``rk`` / ``rv`` are given).  The buffer-level form of ``NVFP4KVCache.append``."""
-    zhk, _, half = knv.shape
-    d = half * 2
-    dtype = v_partial.dtype
-    _lib.require_cuda(key_new, "key_new")
-    kn = key_new.reshape(zhk, d)
-    vn = value_new.reshape(zhk, d)
-    if kn.dtype != dtype or kn.stride(1) != 1:
-        kn = kn.to(dtype).contiguous()
-    if vn.dtype != dtype or vn.stride(1) != 1:
-        vn = vn.to(dtype).contiguous()
-    if kn.stride(0) != vn.stride(0):
-        kn, vn = kn.contiguous(), vn.contiguous()
-    ring = rk is not None
-    dev = knv.device
-    _lib.call("nvfp4_kv_append", _lib.same_device(kn, vn, knv),
-              kn.data_ptr(), vn.data_ptr(), _lib.dtype_code(dtype), kn.stride(0), zhk, d, int(pos),
-              knv.data_ptr(), knv.stride(0), ksc.data_ptr(), ksc.stride(0),
-              vnv.data_ptr(), vnv.stride(0), vnv.stride(1), vsc.data_ptr(), vsc.stride(0), vsc.stride(1),
-              v_partial.data_ptr(), rk.data_ptr() if ring else None, rv.data_ptr() if ring else None,
-              rk.shape[2] if ring else 0, _lib.stream_ptr(dev))
+    _lib.native().append_token(key_new, value_new, knv, ksc, vnv, vsc, v_partial, rk, rv, int(pos))
 
 
 def hybrid_decode_buffers(query, knv, ksc, vnv, vsc, rk, rv, length: int, recent_window: int, scaling: float,
                           g: int, block_n: int = 128) -> torch.Tensor:
     """``NVFP4KVCache.hybrid_decode`` on the raw buffers of a cache holding ``length`` tokens."""
-    z, h, _, d = query.shape
-    hk, ring_cap, dtype = rk.shape[1], rk.shape[2], rk.dtype
-    s = int(length)
-    cut = (max(0, s - recent_window) // 16) * 16
-    w = s - cut
-    _lib.require_cuda(query, "query")
-    qv = query if query.stride(-1) == 1 else query.contiguous()
-    if qv.dtype != dtype:
-        qv = qv.to(dtype)
-    dev = query.device
-    if cut == 0:
-        # everything is still inside the window: exact attention over the ring alone
-        out_rec = torch.empty(z, h, d, dtype=torch.float32, device=dev)
-        lse_rec = torch.empty(z, h, dtype=torch.float32, device=dev)
-        _lib.call("nvfp4_window_attention", _lib.same_device(qv, rk),
-                  qv.data_ptr(), _lib.dtype_code(qv.dtype), qv.stride(0), qv.stride(1), rk.data_ptr(),
-                  rv.data_ptr(), z, hk, g, d, ring_cap, cut, w, float(scaling),
-                  out_rec.data_ptr(), lse_rec.data_ptr(), _lib.stream_ptr(dev))
-        return out_rec.reshape(z, h, 1, d).to(query.dtype)
-    # The window is cut into a few key ranges per (batch, kv head); each block stages its rows in
-    # shared memory and writes an un-normalised split-K partial behind the FP4 decode's own, and the
-    # decode's combine merges prefix and window in one pass (two launches + the combine; no
-    # intermediate outputs, no copy of the query).  Pieces of at most 144 keys.
-    pieces = max(1, min(64, -(-w // 144)))
-
-    def fill(ws, total_slots, extra_base):
-        _lib.call("nvfp4_window_partials", _lib.same_device(qv, rk, ws),
-                  qv.data_ptr(), _lib.dtype_code(qv.dtype), qv.stride(0), qv.stride(1), rk.data_ptr(),
-                  rv.data_ptr(), z, hk, g, d, ring_cap, cut, w, float(scaling), pieces,
-                  ws.data_ptr(), total_slots, extra_base, _lib.stream_ptr(dev))
-
-    s_pad = _next_mult(cut, block_n)
-    packed = (knv[:, :cut], ksc[:, :cut], vnv[:, :, : s_pad // 2], vsc[:, :, : s_pad // 16], cut, s_pad)
-    out, _ = _flash._decode_core(qv, packed, scaling, g, want_lse=False, extra=(pieces, fill))
-    return out.to(query.dtype)
+    return _lib.native().hybrid_decode(query, knv, ksc, vnv, vsc, rk, rv, int(length), int(recent_window), scaling, g)
 
 
 class NVFP4KVCache:
@@ -184,8 +130,7 @@ class NVFP4KVCache:
         if _check:
             assert cut % self.GROUP == 0, "cut must be a multiple of 16"
         s_pad = _next_mult(cut, self.block_n)
-        return (self.knv[:, :cut], self.ksc[:, :cut], self.vnv[:, :, : s_pad // 2],
-                self.vsc[:, :, : s_pad // 16], cut, s_pad)
+        return (*_lib.native().packed_views(self.knv, self.ksc, self.vnv, self.vsc, cut, s_pad), cut, s_pad)
 
     # ------------------------------------------------------------------ hybrid decode
     @torch.no_grad()
