@@ -159,6 +159,22 @@ int nvfp4_kv_append(const void* k_new, const void* v_new, int dtype, int64_t s_n
                     int64_t ring_cap, nvfp4_stream_t stream);
 
 /*
+ * A prompt's keys and values into an NVFP4 KV cache, one launch.  Replaces NVFP4KVCache.prefill
+ * (sageattention/nvfp4/kv_cache.py:187-224): packs K [zhk, s, d] along D and V along the keys (the
+ * open 16-key group zero-padded) straight into the cache buffers, stores the V tokens of the open
+ * group in `partial` (rows behind the prompt zeroed) and the last min(s, ring_cap) tokens in the
+ * recent-window rings (slot = position % ring_cap; NULL without a window).  Element strides skb /
+ * svb between units, skr / svr between tokens, unit stride along D; cache strides as for
+ * nvfp4_kv_append; partial and rings in the dtype of k and v.
+ */
+int nvfp4_kv_prefill(const void* k, const void* v, int dtype, int64_t zhk, int64_t s, int d,
+                     int64_t skb, int64_t skr, int64_t svb, int64_t svr, uint8_t* knv,
+                     int64_t knv_unit, uint8_t* ksc, int64_t ksc_unit, uint8_t* vnv,
+                     int64_t vnv_unit, int64_t vnv_row, uint8_t* vsc, int64_t vsc_unit,
+                     int64_t vsc_row, void* partial, void* ring_k, void* ring_v, int64_t ring_cap,
+                     nvfp4_stream_t stream);
+
+/*
  * Split-K decode plan for a cache of s_kv keys and zhk (batch x kv-head) units: how many
  * splits the decode kernel will use, keys per split (a multiple of 128) and the scratch bytes it
  * needs.  Replaces the heuristic of `_decode_compute` (flash.py:3255-3266), sized for the

@@ -37,6 +37,9 @@ SIGNATURES = {
                                 c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int64,
                                 c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_int64,
                                 c_void_p]),
+    "nvfp4_kv_prefill": (c_int, [c_void_p, c_void_p, c_int, c_int64, c_int64, c_int, c_int64, c_int64, c_int64, c_int64,
+                                 c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int64,
+                                 c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_void_p]),
     "nvfp4_decode_plan": (c_int, [c_int64, c_int64, c_int, c_int, POINTER(c_int), POINTER(c_int64),
                                   POINTER(c_size_t)]),
     "nvfp4_decode": (c_int, [c_void_p, c_int, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64,

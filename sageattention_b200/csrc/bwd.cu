@@ -26,6 +26,7 @@
 // wait is bounded.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
+#include "common/launch.cuh"
 #include "common/sm100.cuh"
 #include "common/tma_host.cuh"
 #include "common/bwd_util.cuh"
@@ -65,6 +66,8 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const T* __restrict__ x, 
                                                        int64_t rows, __nv_bfloat16* __restrict__ xc,
                                                        float* __restrict__ delta, float* __restrict__ amax,
                                                        int aligned) {
+  griddep_launch();
+  griddep_wait();
   const int lane = threadIdx.x & 31, l16 = lane & 15;
   float vmax = 0.0f;   // largest |x| this thread has seen (non-negative floats order like their bit patterns)
   // 32-bit divisions (the host keeps rows below 2^31): a 64-bit divide costs more instructions than
@@ -297,17 +300,6 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
   const int n0 = jt * 128;
   const int shift = p.s_kv - p.s_q;
   const bool varlen = p.seq_start != nullptr;
-  // 64-query steps that can see a key of this tile
-  int q_lo = 0, q_hi = p.s_q;
-  if (p.causal) q_lo = max(0, n0 - shift);
-  if (varlen) {
-    q_lo = max(q_lo, (int)p.seq_start[min(n0, p.s_kv - 1)]);
-    q_hi = min(q_hi, (int)p.seq_end[min(n0 + 127, p.s_kv - 1)]);
-  }
-  const int i_lo = q_lo / 64, i_hi = (q_hi + 63) / 64;
-  const int n_i = max(i_hi - i_lo, 0);
-  const int nstep = n_i * p.g;
-
   if (tid == 0) {
     err = 0;
     for (int i = 0; i < L::NSTAGE; ++i) {
@@ -327,9 +319,21 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&tmem_base_s, 512);
+  griddep_wait();
+  // 64-query steps that can see a key of this tile
+  int q_lo = 0, q_hi = p.s_q;
+  if (p.causal) q_lo = max(0, n0 - shift);
+  if (varlen) {
+    q_lo = max(q_lo, (int)p.seq_start[min(n0, p.s_kv - 1)]);
+    q_hi = min(q_hi, (int)p.seq_end[min(n0 + 127, p.s_kv - 1)]);
+  }
+  const int i_lo = q_lo / 64, i_hi = (q_hi + 63) / 64;
+  const int n_i = max(i_hi - i_lo, 0);
+  const int nstep = n_i * p.g;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  griddep_launch();
   const uint32_t tmem = tmem_base_s;
   constexpr uint32_t T_DV = 0, T_DK = 128, T_ST = 256, T_DPT = 384, T_SFK = 448, T_SFQ = T_SFK + L::KB * 4;
   constexpr uint32_t SFQ_SLOT = L::KB * 4;
@@ -628,15 +632,6 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
   const int m0 = mblk * 128;
   const int shift = p.s_kv - p.s_q;
   const bool varlen = p.seq_start != nullptr;
-  int k_lo = 0, k_hi = p.s_kv;
-  if (p.causal) k_hi = max(0, min(p.s_kv, m0 + 128 + shift));
-  if (varlen) {
-    k_lo = p.seq_start[min(m0, p.s_q - 1)];
-    k_hi = min(k_hi, (int)p.seq_end[min(m0 + 127, p.s_q - 1)]);
-  }
-  const int j_lo = k_lo / 64;
-  const int nstep = max((k_hi + 63) / 64 - j_lo, 0);
-
   if (tid == 0) {
     err = 0;
     for (int i = 0; i < L::NSTAGE; ++i) {
@@ -656,9 +651,19 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&tmem_base_s, 512);
+  griddep_wait();
+  int k_lo = 0, k_hi = p.s_kv;
+  if (p.causal) k_hi = max(0, min(p.s_kv, m0 + 128 + shift));
+  if (varlen) {
+    k_lo = p.seq_start[min(m0, p.s_q - 1)];
+    k_hi = min(k_hi, (int)p.seq_end[min(m0 + 127, p.s_q - 1)]);
+  }
+  const int j_lo = k_lo / 64;
+  const int nstep = max((k_hi + 63) / 64 - j_lo, 0);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  griddep_launch();
   const uint32_t tmem = tmem_base_s;
   constexpr uint32_t T_DQ = 0, T_S = 128, T_DP = 256, T_SFQ = 320, T_SFK = T_SFQ + L::KB * 4;
   constexpr uint32_t SFK_SLOT = L::KB * 4;
@@ -889,10 +894,8 @@ int prep_launch(const void* x, int64_t sxb1, int64_t sxb2, int64_t sxs, int64_t 
   const int64_t per_block = aligned ? 16 * kPrepRows : 16;
   const int64_t blocks = (rows + per_block - 1) / per_block;
   const unsigned grid = (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16);
-  bwd_prep_kernel<T><<<grid, 256, 0, st>>>(static_cast<const T*>(x), sxb1, sxb2, sxs, (int)nb2,
-                                           static_cast<const T*>(y), syb1, syb2, sys, S, D, rows, xc, delta, amax,
-                                           aligned);
-  return launch_result("nvfp4_bwd_prep");
+  return launch("nvfp4_bwd_prep", bwd_prep_kernel<T>, dim3(grid), 256, 0, st, static_cast<const T*>(x), sxb1, sxb2, sxs,
+                (int)nb2, static_cast<const T*>(y), syb1, syb2, sys, S, D, rows, xc, delta, amax, aligned);
 }
 
 }  // namespace nvfp4
@@ -962,17 +965,14 @@ extern "C" int nvfp4_bwd_hp(const uint8_t* qnv, const uint8_t* qsc, const uint8_
   p.scaling = scaling; p.causal = (flags & NVFP4_FWD_CAUSAL) ? 1 : 0; p.status = status;
   const unsigned halves = (unsigned)(d / 128);
   auto launch = [&](auto kdkdv, auto kdq, int smem_dkdv, int smem_dq) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kdkdv, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dkdv);
-    if (e != cudaSuccess) return fail((int)e, "nvfp4_bwd_hp: smem attribute: %s", cudaGetErrorString(e));
-    e = cudaFuncSetAttribute(kdq, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dq);
-    if (e != cudaSuccess) return fail((int)e, "nvfp4_bwd_hp: smem attribute: %s", cudaGetErrorString(e));
+    if (int r0 = allow_smem("nvfp4_bwd_hp", reinterpret_cast<const void*>(kdkdv), smem_dkdv)) return r0;
+    if (int r0 = allow_smem("nvfp4_bwd_hp", reinterpret_cast<const void*>(kdq), smem_dq)) return r0;
     dim3 g1((unsigned)zhk, (unsigned)((s_kv + 127) / 128), halves);
-    kdkdv<<<g1, kBwdThreads, smem_dkdv, st>>>(t_kp128, t_qp64, t_v128, t_do64, t_q64, p);
-    int r1 = launch_result("nvfp4_bwd_hp(dkdv)");
-    if (r1) return r1;
+    if (int r1 = nvfp4::launch("nvfp4_bwd_hp(dkdv)", kdkdv, g1, kBwdThreads, smem_dkdv, st, t_kp128, t_qp64, t_v128, t_do64,
+                               t_q64, p))
+      return r1;
     dim3 g2((unsigned)zh, (unsigned)((s_q + 127) / 128), halves);
-    kdq<<<g2, kBwdThreads, smem_dq, st>>>(t_qp128, t_kp64, t_do128, t_v64, t_k64, p);
-    return launch_result("nvfp4_bwd_hp(dq)");
+    return nvfp4::launch("nvfp4_bwd_hp(dq)", kdq, g2, kBwdThreads, smem_dq, st, t_qp128, t_kp64, t_do128, t_v64, t_k64, p);
   };
 #define NVFP4_BWD_LAUNCH(DD, TT) \
   launch(bwd_dkdv_kernel<DD, TT>, bwd_dq_kernel<DD, TT>, DkdvSmem<DD>::TOTAL, DqSmem<DD>::TOTAL)

@@ -35,6 +35,7 @@
 // is bounded.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
+#include "common/launch.cuh"
 #include "common/sm100.cuh"
 #include "common/tma_host.cuh"
 #include "common/bwd_util.cuh"
@@ -222,6 +223,30 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   const int shift = p.s_kv - p.s_q;
   const bool varlen = p.seq_start != nullptr;
 
+  if (tid == 0) {
+    err = 0;
+    for (int i = 0; i < C::NSTAGE; ++i) {
+      mbar_init(&full_tma[i], 1);
+      mbar_init(&full_aux[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(&x_full, 1);
+    mbar_init(&xsf_full, 1);
+    mbar_init(&g_full, 1);
+    mbar_init(&g_free, 4 * C::NP);
+    mbar_init(&acc_done, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&s_full[b], 1);
+      mbar_init(&s_free[b], 4 * C::NP);
+      mbar_init(&a_full[b], 4 * C::NP);
+      mbar_init(&a_free[b], 1);
+    }
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(&tmem_base_s, 512);
+  griddep_wait();
+  if (tid == 0) gs_s = pow2_ceil(p.amax != nullptr ? *p.amax : 1.0f);
+
   // ---- rows of this CTA, and the range of 128-column stages it has to visit
   int rb, row0, zi, kh = 0, cb0;     // row batch entry, first row, batch index, kv head, first column batch entry
   int R, Ccols;                      // row / column extents
@@ -255,31 +280,10 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   const int nstage = (kDkdv ? p.g : 1) * n_i;
   const int nstep = 2 * nstage;
 
-  if (tid == 0) {
-    err = 0;
-    for (int i = 0; i < C::NSTAGE; ++i) {
-      mbar_init(&full_tma[i], 1);
-      mbar_init(&full_aux[i], 1);
-      mbar_init(&empty[i], 1);
-    }
-    mbar_init(&x_full, 1);
-    mbar_init(&xsf_full, 1);
-    mbar_init(&g_full, 1);
-    mbar_init(&g_free, 4 * C::NP);
-    mbar_init(&acc_done, 1);
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&s_full[b], 1);
-      mbar_init(&s_free[b], 4 * C::NP);
-      mbar_init(&a_full[b], 4 * C::NP);
-      mbar_init(&a_free[b], 1);
-    }
-    mbar_fence_init();
-    gs_s = pow2_ceil(p.amax != nullptr ? *p.amax : 1.0f);
-  }
-  if (warp == 1) tmem_alloc(&tmem_base_s, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  griddep_launch();
   const uint32_t tmem = tmem_base_s;
   const float gs = gs_s;
 
@@ -814,27 +818,23 @@ extern "C" int nvfp4_bwd_fp4(const uint8_t* qnv, const uint8_t* qsc, const uint8
   p.seed = seed; p.sr_p = 0; p.sr_ds = 0;
   const unsigned halves = (unsigned)(d / 128);
   auto launch = [&](auto kdkdv, auto kdq, int smem, int threads) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kdkdv, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail((int)e, "nvfp4_bwd_fp4: smem attribute: %s", cudaGetErrorString(e));
-    e = cudaFuncSetAttribute(kdq, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail((int)e, "nvfp4_bwd_fp4: smem attribute: %s", cudaGetErrorString(e));
+    if (int r0 = allow_smem("nvfp4_bwd_fp4", reinterpret_cast<const void*>(kdkdv), smem)) return r0;
+    if (int r0 = allow_smem("nvfp4_bwd_fp4", reinterpret_cast<const void*>(kdq), smem)) return r0;
     // dK / dV: rows = keys (K, V packs), columns = queries (Q, dO' packs; dO'^T, Q^T transposed packs)
     B4Params a = p;
     a.x1sc = ksc; a.x2sc = vdsc; a.y1sc = qsc; a.y2sc = dosc; a.t1sc = dotsc; a.t2sc = qtsc;
     a.out1 = dv; a.out2 = dk; a.c_pad = (int)sq_pad;
     a.sr_p = (flags & NVFP4_BWD_SR_P_DV) ? 1 : 0; a.sr_ds = (flags & NVFP4_BWD_SR_DS_DK) ? 1 : 0;
     dim3 g1((unsigned)zhk, (unsigned)((s_kv + 127) / 128), halves);
-    kdkdv<<<g1, threads, smem, st>>>(t_k, t_vd, t_q, t_do, t_dot, t_qt, a);
-    int r1 = launch_result("nvfp4_bwd_fp4(dkdv)");
-    if (r1) return r1;
+    if (int r1 = nvfp4::launch("nvfp4_bwd_fp4(dkdv)", kdkdv, g1, threads, smem, st, t_k, t_vd, t_q, t_do, t_dot, t_qt, a))
+      return r1;
     // dQ: rows = queries (Q, dO' packs), columns = keys (K, V packs; K^T transposed pack)
     B4Params b = p;
     b.x1sc = qsc; b.x2sc = dosc; b.y1sc = ksc; b.y2sc = vdsc; b.t1sc = nullptr; b.t2sc = ktsc;
     b.out1 = nullptr; b.out2 = dq; b.c_pad = (int)skv_pad;
     b.sr_ds = (flags & NVFP4_BWD_SR_DS_DQ) ? 1 : 0;
     dim3 g2((unsigned)zh, (unsigned)((s_q + 127) / 128), halves);
-    kdq<<<g2, threads, smem, st>>>(t_q, t_do, t_k, t_vd, t_kt, t_kt, b);
-    return launch_result("nvfp4_bwd_fp4(dq)");
+    return nvfp4::launch("nvfp4_bwd_fp4(dq)", kdq, g2, threads, smem, st, t_q, t_do, t_k, t_vd, t_kt, t_kt, b);
   };
   const bool any_sr = (flags & (NVFP4_BWD_SR_DS_DK | NVFP4_BWD_SR_P_DV | NVFP4_BWD_SR_DS_DQ)) != 0;
 #define NVFP4_B4_LAUNCH(DD, TT)                                                                                   \

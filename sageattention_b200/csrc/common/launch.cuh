@@ -1,0 +1,68 @@
+// Kernel launches with programmatic stream serialisation, and the shared-memory opt-in done once.
+//
+// Every kernel of the library is launched so that its CTAs may start while the kernel before it on the
+// stream drains: barrier initialisation, tensor-memory allocation and descriptor fetches then overlap
+// the predecessor's tail instead of following it.  The rules that make this safe:
+//   * every thread executes griddep_wait() before its first access to global memory (L2 prefetch hints
+//     excepted: L2 is the point of coherence); it returns when all earlier work of the stream is
+//     complete and visible, and since no kernel finishes without it, completion is transitive;
+//   * a kernel that allocates tensor memory calls griddep_launch() only after its allocation, so a
+//     dependent that starts on the same SM cannot take columns its predecessor still waits for.
+#pragma once
+#include <cuda_runtime.h>
+#include <atomic>
+#include <stdint.h>
+#include "abi.cuh"
+
+namespace nvfp4 {
+
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per kernel and device: a fixed open-addressing
+// table of kernel addresses (the library has fewer kernels than slots), lock-free, so that a launch
+// pays a look-up (~20 ns) instead of the driver call.  `bytes` must be the same in every call for a kernel.
+inline int allow_smem(const char* what, const void* kern, int bytes) {
+  constexpr int kSlots = 512;
+  static std::atomic<const void*> keys[kSlots];
+  static std::atomic<uint64_t> devices[kSlots];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return fail((int)e, "%s: cudaGetDevice: %s", what, cudaGetErrorString(e));
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  uint32_t i = (uint32_t)((reinterpret_cast<uintptr_t>(kern) >> 4) * 2654435761u) % kSlots;
+  for (int probe = 0; probe < kSlots; ++probe, i = (i + 1) % kSlots) {
+    const void* k = keys[i].load(std::memory_order_acquire);
+    if (k == nullptr && keys[i].compare_exchange_strong(k, kern, std::memory_order_acq_rel)) k = kern;
+    if (k != kern) continue;
+    if (devices[i].load(std::memory_order_acquire) & bit) return 0;
+    break;
+  }
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return fail((int)e, "%s: smem attribute: %s", what, cudaGetErrorString(e));
+  if (keys[i].load(std::memory_order_acquire) == kern) devices[i].fetch_or(bit, std::memory_order_acq_rel);
+  return 0;
+}
+
+// Launch with programmatic stream serialisation.
+template <typename... P, typename... A>
+int launch(const char* what, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, P(args)...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();          // the failure is reported here; leave no sticky code behind
+    return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
+  }
+  return 0;
+}
+
+}  // namespace nvfp4

@@ -17,6 +17,7 @@
 // wait is bounded.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
+#include "common/launch.cuh"
 #include "common/sm100.cuh"
 #include "common/tma_host.cuh"
 
@@ -192,6 +193,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     mbar_fence_init();
   }
   __syncthreads();
+  griddep_wait();
   // The TMA producer (warp 0) and the scale loader (warp 2) need nothing but the barriers and the
   // stage buffers: they start streaming now, while the other warps allocate TMEM and clear the
   // operand buffers behind a barrier of their own.
@@ -207,6 +209,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     tc_fence_before();
     named_bar_sync(5, kDecodeThreads - 64);
     tc_fence_after();
+    griddep_launch();
     tmem = tmem_base_s;
   }
 
@@ -724,6 +727,8 @@ __global__ void decode_combine_kernel(const float* __restrict__ ws_acc,
                                       const float* __restrict__ ws_l, int nsplit, int64_t extra_base,
                                       int n_extra, int hk, int g, int d,
                                       TQ* __restrict__ out, float* __restrict__ lse) {
+  griddep_launch();
+  griddep_wait();
   const int unit = blockIdx.x / g, qi = blockIdx.x % g;
   const int t = threadIdx.x;
   float gm = -INFINITY;
@@ -754,6 +759,8 @@ __global__ void decode_combine_balanced_kernel(const float* __restrict__ ws_acc,
                                                int ntiles, int nctas, int maxseg, int64_t extra_base,
                                                int n_extra, int hk, int g, int d,
                                                TQ* __restrict__ out, float* __restrict__ lse) {
+  griddep_launch();
+  griddep_wait();
   const int unit = blockIdx.x / g, qi = blockIdx.x % g;
   const int t = threadIdx.x;
   const int64_t x0 = (int64_t)unit * ntiles, x1 = x0 + ntiles;
@@ -813,11 +820,8 @@ int decode_launch(const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtens
     decode_balanced_geometry(zhk, p.ntiles, sm_count, &grid, &ms);
   }
   auto launch = [&](auto kern) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         C::SMEM_BYTES);
-    if (e != cudaSuccess) return fail((int)e, "nvfp4_decode: smem attribute: %s", cudaGetErrorString(e));
-    kern<<<grid, kDecodeThreads, C::SMEM_BYTES, st>>>(tm_k, tm_v, tm_vpf, tm_vpf4, p);
-    return launch_result("nvfp4_decode");
+    if (int rc = allow_smem("nvfp4_decode", reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return rc;
+    return nvfp4::launch("nvfp4_decode", kern, dim3(grid), kDecodeThreads, C::SMEM_BYTES, st, tm_k, tm_v, tm_vpf, tm_vpf4, p);
   };
   int rc;
   if (p.g <= 4) rc = launch(decode_kernel<D, TQ, 4>);
@@ -825,13 +829,11 @@ int decode_launch(const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtens
   else rc = launch(decode_kernel<D, TQ, 16>);
   if (rc) return rc;
   if (p.balanced)
-    decode_combine_balanced_kernel<TQ><<<(unsigned)(zhk * p.g), D, 0, st>>>(
-        p.ws_acc, p.ws_m, p.ws_l, p.total_tiles, p.ntiles, grid, p.maxseg, p.extra_base, p.n_extra, p.hk, p.g, D,
+    return nvfp4::launch(
+        "nvfp4_decode(combine)", decode_combine_balanced_kernel<TQ>, dim3((unsigned)(zhk * p.g)), D, 0, st, p.ws_acc, p.ws_m, p.ws_l, p.total_tiles, p.ntiles, grid, p.maxseg, p.extra_base, p.n_extra, p.hk, p.g, D,
         static_cast<TQ*>(out), lse);
-  else
-    decode_combine_kernel<TQ><<<(unsigned)(zhk * p.g), D, 0, st>>>(
-        p.ws_acc, p.ws_m, p.ws_l, p.nsplit, p.extra_base, p.n_extra, p.hk, p.g, D, static_cast<TQ*>(out), lse);
-  return launch_result("nvfp4_decode(combine)");
+  return nvfp4::launch("nvfp4_decode(combine)", decode_combine_kernel<TQ>, dim3((unsigned)(zhk * p.g)), D, 0, st, p.ws_acc,
+                       p.ws_m, p.ws_l, p.nsplit, p.extra_base, p.n_extra, p.hk, p.g, D, static_cast<TQ*>(out), lse);
 }
 
 }  // namespace nvfp4

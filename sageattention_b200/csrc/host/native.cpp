@@ -609,6 +609,27 @@ void append_token(const Tensor& key_new, const Tensor& value_new, const Tensor& 
          "nvfp4_kv_append");
 }
 
+// A prompt into the cache buffers in one launch; false when the operands need the general path (another
+// dtype than the cache's, or rows that are not contiguous along D).
+bool kv_prefill(const Tensor& key, const Tensor& value, const Tensor& knv, const Tensor& ksc, const Tensor& vnv,
+                const Tensor& vsc, const Tensor& v_partial, const OptTensor& rk, const OptTensor& rv) {
+  require_cuda(key, "key");
+  Call c(knv);
+  c.same(key);
+  c.same(value);
+  const auto t = v_partial.scalar_type();
+  if (key.scalar_type() != t || value.scalar_type() != t) return false;
+  const Rows k = rows_of(key), v = rows_of(value);
+  if (k.sk != 1 || v.sk != 1) return false;
+  require(k.b == knv.size(0) && v.b == k.b && v.r == k.r && v.k == k.k, "key and value must be [Z, Hk, S, D] of the cache");
+  require(k.r <= knv.size(1), "prefill exceeds capacity");
+  c.done(nvfp4_kv_prefill(k.p, v.p, dtype_code(t), k.b, k.r, (int)k.k, k.sb, k.sr, v.sb, v.sr, u8(knv), knv.stride(0), u8(ksc),
+                          ksc.stride(0), u8(vnv), vnv.stride(0), vnv.stride(1), u8(vsc), vsc.stride(0), vsc.stride(1),
+                          v_partial.data_ptr(), opt_ptr<>(rk), opt_ptr<>(rv), rk.has_value() ? rk->size(2) : 0, c.stream),
+         "nvfp4_kv_prefill");
+  return true;
+}
+
 // ---------------------------------------------------------------- backward
 struct Prep {
   OptTensor copy, delta, amax;
@@ -806,6 +827,7 @@ PYBIND11_MODULE(_native, m) {
   m.def("hybrid_decode", &hybrid_decode, nogil());
   m.def("packed_views", &packed_views, nogil());
   m.def("append_token", &append_token, nogil());
+  m.def("kv_prefill", &kv_prefill, nogil());
   m.def("bwd_prep", &bwd_prep, nogil());
   m.def("bf16_rows", &bf16_rows, nogil());
   m.def("bwd_hp", &bwd_hp, nogil());

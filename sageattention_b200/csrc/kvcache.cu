@@ -2,6 +2,7 @@
 // decode, and the log-sum-exp merge of two attention regions.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
+#include "common/launch.cuh"
 
 namespace nvfp4 {
 
@@ -18,6 +19,8 @@ __global__ void kv_append_kernel(const T* __restrict__ k_new, const T* __restric
                                  uint8_t* __restrict__ vsc, int64_t vsc_unit, int64_t vsc_row,
                                  T* __restrict__ partial, T* __restrict__ ring_k,
                                  T* __restrict__ ring_v, int64_t ring_cap) {
+  griddep_launch();
+  griddep_wait();
   const int64_t u = blockIdx.x;
   const int t = threadIdx.x;
   const T* kr = k_new + u * s_new;
@@ -77,6 +80,8 @@ __global__ void __launch_bounds__(512) window_attention_kernel(
     int count_all, int chunk, float scaling, float* __restrict__ out, float* __restrict__ lse,
     float* __restrict__ ws_acc, float* __restrict__ ws_m, float* __restrict__ ws_l, int64_t extra_base) {
   extern __shared__ __align__(16) float sm[];
+  griddep_launch();
+  griddep_wait();
   const bool partial = ws_acc != nullptr;
   const int k0 = partial ? (int)blockIdx.y * chunk : 0;
   const int count = partial ? min(chunk, count_all - k0) : count_all;
@@ -277,6 +282,7 @@ __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], uint32_t saddr) 
 }
 
 constexpr int kWinThreads = 256;
+constexpr int kWinMaxSmem = 200 * 1024;      // of both window kernels
 // bytes of dynamic shared memory for a piece of `keys` (multiple of 16) keys
 __host__ __device__ constexpr size_t win_mma_smem(int d, int keys) {
   return (size_t)16 * d * 2            // Q rows (16-bit), swizzled
@@ -294,6 +300,8 @@ __global__ void __launch_bounds__(kWinThreads, D == 128 ? 2 : 1) window_mma_kern
   constexpr int kRowB = D * 2;            // bytes of a row
   constexpr int kChunks = D / 8;          // 16-byte chunks of a row
   extern __shared__ __align__(128) uint8_t wsm[];
+  griddep_launch();
+  griddep_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int k0 = (int)blockIdx.y * chunk;
   const int count = min(chunk, count_all - k0);
@@ -450,6 +458,8 @@ template <typename T>
 __global__ void lse_merge_kernel(const T* __restrict__ o1, const float* __restrict__ l1,
                                  const T* __restrict__ o2, const float* __restrict__ l2,
                                  T* __restrict__ out, float* __restrict__ lse_out, int64_t rows, int d) {
+  griddep_launch();
+  griddep_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= rows * d) return;
   const int64_t r = i / d;
@@ -474,11 +484,10 @@ int append_launch(const void* k_new, const void* v_new, int64_t s_new, int64_t z
                   uint8_t* vnv, int64_t vnv_unit, int64_t vnv_row, uint8_t* vsc, int64_t vsc_unit,
                   int64_t vsc_row, void* partial, void* ring_k, void* ring_v, int64_t ring_cap,
                   cudaStream_t st) {
-  kv_append_kernel<T><<<(unsigned)zhk, d, 0, st>>>(
-      static_cast<const T*>(k_new), static_cast<const T*>(v_new), s_new, d, pos, knv, knv_unit, ksc,
+  return launch(
+      "nvfp4_kv_append", kv_append_kernel<T>, dim3((unsigned)zhk), d, 0, st, static_cast<const T*>(k_new), static_cast<const T*>(v_new), s_new, d, pos, knv, knv_unit, ksc,
       ksc_unit, vnv, vnv_unit, vnv_row, vsc, vsc_unit, vsc_row, static_cast<T*>(partial),
       static_cast<T*>(ring_k), static_cast<T*>(ring_v), ring_cap);
-  return launch_result("nvfp4_kv_append");
 }
 
 }  // namespace nvfp4
@@ -524,22 +533,15 @@ extern "C" int nvfp4_window_attention(const void* q, int dtype, int64_t s_qz, in
   NVFP4_REQUIRE(z * hk * g < (1LL << 31), "nvfp4_window_attention: too many heads");
   const size_t smem = (size_t)(5 * g * d + g * count + 4) * sizeof(float);
   NVFP4_REQUIRE(g >= 1 && g <= 16, "nvfp4_window_attention: GQA group %d must be <= 16", g);
-  NVFP4_REQUIRE(smem <= 200 * 1024, "nvfp4_window_attention: window too long (%lld keys)", (long long)count);
+  NVFP4_REQUIRE(smem <= kWinMaxSmem, "nvfp4_window_attention: window too long (%lld keys)", (long long)count);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned grid = (unsigned)(z * hk);
 #define NVFP4_WIN(T)                                                                              \
-  if (smem > 48 * 1024) {                                                                         \
-    cudaError_t e = cudaFuncSetAttribute(window_attention_kernel<T>,                              \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    if (e != cudaSuccess) return fail((int)e, "nvfp4_window_attention: smem attribute: %s", cudaGetErrorString(e)); \
-  }                                                                                               \
-  window_attention_kernel<T><<<grid, 512, smem, st>>>(static_cast<const T*>(q), s_qz, s_qh,       \
-                                                      static_cast<const T*>(rk),                  \
-                                                      static_cast<const T*>(rv), (int)hk, g, d,   \
-                                                      ring_cap, first_pos, (int)count, (int)count, \
-                                                      scaling, out, lse, nullptr, nullptr,        \
-                                                      nullptr, 0);                                \
-  return launch_result("nvfp4_window_attention")
+  if (int rc = allow_smem("nvfp4_window_attention", reinterpret_cast<const void*>(window_attention_kernel<T>), kWinMaxSmem)) \
+    return rc;                                                                                    \
+  return launch("nvfp4_window_attention", window_attention_kernel<T>, dim3(grid), 512, smem, st,  \
+                static_cast<const T*>(q), s_qz, s_qh, static_cast<const T*>(rk), static_cast<const T*>(rv), (int)hk, g, d, \
+                ring_cap, first_pos, (int)count, (int)count, scaling, out, lse, nullptr, nullptr, nullptr, 0)
   switch (dtype) {
     case NVFP4_DT_BF16: NVFP4_WIN(__nv_bfloat16);
     case NVFP4_DT_FP16: NVFP4_WIN(__half);
@@ -574,16 +576,14 @@ extern "C" int nvfp4_window_partials(const void* q, int dtype, int64_t s_qz, int
     const bool aligned = ((uintptr_t)q % 16) == 0 && ((uintptr_t)rk % 16) == 0 && ((uintptr_t)rv % 16) == 0 &&
                          s_qz % 8 == 0 && s_qh % 8 == 0;
     if ((dtype == NVFP4_DT_BF16 || dtype == NVFP4_DT_FP16) && (d == 128 || d == 256) && aligned &&
-        smem16 <= 200 * 1024) {
+        smem16 <= kWinMaxSmem) {
 #define NVFP4_WINM(T, DD)                                                                             \
   {                                                                                                   \
-    cudaError_t e = cudaFuncSetAttribute(window_mma_kernel<T, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                         (int)smem16);                                                \
-    if (e != cudaSuccess) return fail((int)e, "nvfp4_window_partials: smem attribute: %s", cudaGetErrorString(e)); \
-    window_mma_kernel<T, DD><<<grid, kWinThreads, smem16, st>>>(                                      \
-        static_cast<const T*>(q), s_qz, s_qh, static_cast<const T*>(rk), static_cast<const T*>(rv), (int)hk, g, \
+    if (int rc = allow_smem("nvfp4_window_partials", reinterpret_cast<const void*>(window_mma_kernel<T, DD>), kWinMaxSmem)) \
+      return rc;                                                                                      \
+    return launch(                                                                                    \
+        "nvfp4_window_partials", window_mma_kernel<T, DD>, grid, kWinThreads, smem16, st, static_cast<const T*>(q), s_qz, s_qh, static_cast<const T*>(rk), static_cast<const T*>(rv), (int)hk, g, \
         ring_cap, first_pos, (int)count, chunk16, scaling, ws_acc, ws_m, ws_l, extra_base);           \
-    return launch_result("nvfp4_window_partials");                                                    \
   }
       if (dtype == NVFP4_DT_BF16) {
         if (d == 128) NVFP4_WINM(__nv_bfloat16, 128) else NVFP4_WINM(__nv_bfloat16, 256)
@@ -595,18 +595,14 @@ extern "C" int nvfp4_window_partials(const void* q, int dtype, int64_t s_qz, int
   }
   const int chunk = (int)(((count + pieces - 1) / pieces + 3) / 4 * 4);
   const size_t smem = (size_t)(5 * g * d + g * chunk + 4) * sizeof(float);
-  NVFP4_REQUIRE(smem <= 200 * 1024, "nvfp4_window_partials: window piece too long (%d keys)", chunk);
+  NVFP4_REQUIRE(smem <= kWinMaxSmem, "nvfp4_window_partials: window piece too long (%d keys)", chunk);
 #define NVFP4_WINP(T)                                                                               \
   {                                                                                                 \
-    if (smem > 48 * 1024) {                                                                         \
-      cudaError_t e = cudaFuncSetAttribute(window_attention_kernel<T>,                              \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-      if (e != cudaSuccess) return fail((int)e, "nvfp4_window_partials: smem attribute: %s", cudaGetErrorString(e)); \
-    }                                                                                               \
-    window_attention_kernel<T><<<grid, 512, smem, st>>>(                                            \
-        static_cast<const T*>(q), s_qz, s_qh, static_cast<const T*>(rk), static_cast<const T*>(rv), (int)hk, g, d, \
+    if (int rc = allow_smem("nvfp4_window_partials", reinterpret_cast<const void*>(window_attention_kernel<T>), kWinMaxSmem)) \
+      return rc;                                                                                    \
+    return launch(                                                                                  \
+        "nvfp4_window_partials", window_attention_kernel<T>, grid, 512, smem, st, static_cast<const T*>(q), s_qz, s_qh, static_cast<const T*>(rk), static_cast<const T*>(rv), (int)hk, g, d, \
         ring_cap, first_pos, (int)count, chunk, scaling, nullptr, nullptr, ws_acc, ws_m, ws_l, extra_base); \
-    return launch_result("nvfp4_window_partials");                                                  \
   }
   switch (dtype) {
     case NVFP4_DT_BF16: NVFP4_WINP(__nv_bfloat16)
@@ -626,10 +622,8 @@ extern "C" int nvfp4_lse_merge(const void* o1, const float* lse1, const void* o2
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned grid = (unsigned)((rows * d + 255) / 256);
 #define NVFP4_MERGE(T)                                                                           \
-  lse_merge_kernel<T><<<grid, 256, 0, st>>>(static_cast<const T*>(o1), lse1,                     \
-                                            static_cast<const T*>(o2), lse2, static_cast<T*>(out), \
-                                            lse_out, rows, d);                                   \
-  return launch_result("nvfp4_lse_merge")
+  return launch("nvfp4_lse_merge", lse_merge_kernel<T>, dim3(grid), 256, 0, st, static_cast<const T*>(o1), lse1, \
+                static_cast<const T*>(o2), lse2, static_cast<T*>(out), lse_out, rows, d)
   switch (dtype) {
     case NVFP4_DT_BF16: NVFP4_MERGE(__nv_bfloat16);
     case NVFP4_DT_FP16: NVFP4_MERGE(__half);

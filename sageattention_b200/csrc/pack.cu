@@ -15,6 +15,7 @@
 // A scalar kernel covers any other stride combination.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
+#include "common/launch.cuh"
 #include "common/bwd_util.cuh"
 
 namespace nvfp4 {
@@ -141,6 +142,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) pack_rows_quad_kernel(
     const T* __restrict__ x, int ng_log2, int64_t per_batch, int64_t sxb, int64_t sxr,
     uint8_t* __restrict__ nib, int64_t snb, int64_t snr, uint8_t* __restrict__ sc, int64_t ssb, int64_t ssr) {
+  griddep_launch();
+  griddep_wait();
   const int64_t first = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * 128;
   if (first >= per_batch) return;
   pack_rows_quad<T>(x, ng_log2, per_batch, sxb, sxr, nib, snb, snr, sc, ssb, ssr, first, blockIdx.y);
@@ -151,6 +154,8 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(
     const T* __restrict__ x, int64_t R, int64_t k_read, int64_t ngroups, int ngroups_log2,
     int64_t per_batch, int64_t sxb, int64_t sxr, uint8_t* __restrict__ nib, int64_t snb,
     int64_t snr, uint8_t* __restrict__ sc, int64_t ssb, int64_t ssr, int vec_in) {
+  griddep_launch();
+  griddep_wait();
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= per_batch) return;
   pack_rows_group<T>(x, k_read, ngroups, ngroups_log2, sxb, sxr, nib, snb, snr, sc, ssb, ssr, vec_in, gid,
@@ -168,6 +173,8 @@ __global__ void __launch_bounds__(256) rope_pack_rows_kernel(
     int64_t sxr, const float* __restrict__ cs, const float* __restrict__ sn,
     const int32_t* __restrict__ positions, int64_t pos0, uint8_t* __restrict__ nib, int64_t snb,
     int64_t snr, uint8_t* __restrict__ sc, int64_t ssb, int64_t ssr, int vec_in) {
+  griddep_launch();
+  griddep_wait();
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= per_batch) return;
   const int64_t b = blockIdx.y;
@@ -460,6 +467,8 @@ __global__ void __launch_bounds__(256, 3) pack_cols_kernel(
     uint8_t* __restrict__ dsc, int64_t dsb, int64_t dsr, const float* __restrict__ prescale_amax,
     int sr_flags, uint32_t seed) {
   __shared__ ColsSmem<T> sm;
+  griddep_launch();
+  griddep_wait();
   const int64_t tx = (k_pad + kColsKeys - 1) / kColsKeys, bx = (int64_t)blockIdx.x * kColsRun;
   pack_cols_tile<T, kDual>(sm, x, R, k_read, k_pad, sxb, sxk, nib, snb, snr, sc, ssb, ssr, vec_in, bx,
                            (int)(tx - bx < kColsRun ? tx - bx : kColsRun), blockIdx.y, blockIdx.z, dnib, dnb, dnr,
@@ -476,6 +485,8 @@ __global__ void __launch_bounds__(256) pack_mx8_cols_kernel(
     const T* __restrict__ x, int64_t R, int64_t k_read, int64_t k_pad, int64_t sxb, int64_t sxk,
     uint8_t* __restrict__ out, uint8_t* __restrict__ sc, int vec_in, const float* __restrict__ prescale_amax) {
   __shared__ float tile[kColsKeys][kColsRows + 1];
+  griddep_launch();
+  griddep_wait();
   const float pre = prescale_amax != nullptr ? __frcp_rn(pow2_ceil(*prescale_amax)) : 1.0f;
   const int tid = threadIdx.x;
   const int64_t k0 = (int64_t)blockIdx.x * kColsKeys, r0 = (int64_t)blockIdx.y * kColsRows, b = blockIdx.z;
@@ -562,6 +573,8 @@ struct QkvArgs {
 template <typename T>
 __global__ void __launch_bounds__(256, 3) pack_qkv_kernel(const QkvArgs a) {
   __shared__ ColsSmem<T> sm;
+  griddep_launch();
+  griddep_wait();
   const int64_t v = blockIdx.x;
   const int ngroups = a.d >> 4;
   if (v < a.nbq + a.nbk) {
@@ -603,12 +616,103 @@ __global__ void __launch_bounds__(256, 3) pack_qkv_kernel(const QkvArgs a) {
                            nullptr, 0, 0, nullptr, 0, 0, nullptr);
 }
 
+// ---------------------------------------------------------------- prompt into a KV cache, one launch
+// A flat grid like pack_qkv_kernel's: K row blocks (into the cache's [unit][token] rows), the V -> V^T
+// tiles (into its [unit][d] rows), and copy blocks for what the cache keeps in high precision: the
+// open 16-key V group (zero-filled behind the prompt) and the recent-window rings.
+// As separate steps this was two packs, a zero fill, a strided copy, a third pack and six index
+// kernels -- eleven launches, 26 us of GPU time for a prompt of 777 tokens that has 1.2 MB to move.
+struct PrefillArgs {
+  const void *k, *v;
+  int64_t s, zhk;
+  int d, ngroups_log2, vec_v, vec_k, vec_c, quad_k;
+  int64_t skb, skr, svb, svr;       // element strides of k / v: unit, token
+  uint8_t *knv, *ksc, *vnv, *vsc;
+  int64_t knv_unit, ksc_unit, vnv_unit, vnv_row, vsc_unit, vsc_row;
+  void *partial, *rk, *rv;          // [unit][16][d]; rings [unit][ring_cap][d] or null
+  int64_t ring_cap, ring_n;         // the last ring_n tokens go to the rings
+  int64_t bpk, nbk, s_pad, tx, ty, nbv, bpc;
+};
+
+constexpr int kPrefillCopyIters = 8;   // 16-byte pieces per thread of a copy block
+
+template <typename T>
+__global__ void __launch_bounds__(256, 3) kv_prefill_kernel(const PrefillArgs a) {
+  __shared__ ColsSmem<T> sm;
+  griddep_launch();
+  griddep_wait();
+  const int64_t blk = blockIdx.x;
+  const int ngroups = a.d >> 4;
+  if (blk < a.nbk) {
+    const int64_t b = blk / a.bpk, w = blk - b * a.bpk;
+    const int64_t per = a.s * ngroups;
+    if (a.quad_k) {
+      const int64_t first = (w * 8 + (threadIdx.x >> 5)) * 128;
+      if (first < per)
+        pack_rows_quad<T>(static_cast<const T*>(a.k), a.ngroups_log2, per, a.skb, a.skr, a.knv, a.knv_unit, a.d / 2, a.ksc,
+                          a.ksc_unit, ngroups, first, b);
+    } else {
+      const int64_t gid = w * 256 + threadIdx.x;
+      if (gid < per)
+        pack_rows_group<T>(static_cast<const T*>(a.k), a.d, ngroups, a.ngroups_log2, a.skb, a.skr, a.knv, a.knv_unit,
+                           a.d / 2, a.ksc, a.ksc_unit, ngroups, a.vec_k, gid, b);
+    }
+    return;
+  }
+  if (blk < a.nbk + a.nbv) {
+    const int64_t w = blk - a.nbk;
+    const int64_t runs = (a.tx + kColsRun - 1) / kColsRun, per = runs * a.ty;
+    const int64_t b = w / per, rem = w - b * per;
+    const int64_t by = rem / runs, bx = (rem - by * runs) * kColsRun;
+    pack_cols_tile<T, false>(sm, static_cast<const T*>(a.v), a.d, a.s, a.s_pad, a.svb, a.svr, a.vnv, a.vnv_unit, a.vnv_row,
+                             a.vsc, a.vsc_unit, a.vsc_row, a.vec_v, bx, (int)(a.tx - bx < kColsRun ? a.tx - bx : kColsRun),
+                             by, b, nullptr, 0, 0, nullptr, 0, 0, nullptr);
+    return;
+  }
+  // copies: pieces of kE elements; per unit 16 open-group rows, then ring_n rows of K and of V
+  constexpr int kE = 16 / sizeof(T);
+  const int64_t w = blk - a.nbk - a.nbv;
+  const int64_t u = w / a.bpc;
+  const int pr = a.d / kE;                              // pieces per row
+  const int64_t n_part = 16 * pr, n_ring = a.rk != nullptr ? a.ring_n * pr : 0;
+  const int64_t open0 = a.s / 16 * 16;
+  const T* k = static_cast<const T*>(a.k) + u * a.skb;
+  const T* v = static_cast<const T*>(a.v) + u * a.svb;
+#pragma unroll 1
+  for (int i = 0; i < kPrefillCopyIters; ++i) {
+    const int64_t idx = ((w - u * a.bpc) * kPrefillCopyIters + i) * 256 + threadIdx.x;
+    if (idx >= n_part + 2 * n_ring) return;
+    const T* src = nullptr;                             // null: zeros
+    T* dst;
+    if (idx < n_part) {
+      const int64_t r = idx / pr, e = (idx - r * pr) * kE;
+      if (open0 + r < a.s) src = v + (open0 + r) * a.svr + e;
+      dst = static_cast<T*>(a.partial) + (u * 16 + r) * a.d + e;
+    } else {
+      const bool is_v = idx >= n_part + n_ring;
+      const int64_t j = idx - n_part - (is_v ? n_ring : 0);
+      const int64_t r = j / pr, e = (j - r * pr) * kE;
+      const int64_t pos = a.s - a.ring_n + r;
+      src = is_v ? v + pos * a.svr + e : k + pos * a.skr + e;
+      dst = static_cast<T*>(is_v ? a.rv : a.rk) + (u * a.ring_cap + pos % a.ring_cap) * a.d + e;
+    }
+    if (a.vec_c) {
+      *reinterpret_cast<uint4*>(dst) = src ? *reinterpret_cast<const uint4*>(src) : make_uint4(0u, 0u, 0u, 0u);
+    } else {
+#pragma unroll
+      for (int e = 0; e < kE; ++e) dst[e] = src ? src[e] : from_f32<T>(0.0f);
+    }
+  }
+}
+
 // ---------------------------------------------------------------- any strides (scalar)
 template <typename T>
 __global__ void __launch_bounds__(256) pack_generic_kernel(
     const T* __restrict__ x, int64_t R, int64_t k_read, int64_t ngroups, int64_t total, int64_t sxb,
     int64_t sxr, int64_t sxk, uint8_t* __restrict__ nib, int64_t snb, int64_t snr,
     uint8_t* __restrict__ sc, int64_t ssb, int64_t ssr) {
+  griddep_launch();
+  griddep_wait();
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= total) return;
   const int64_t g = gid % ngroups;
@@ -649,27 +753,24 @@ int pack_dispatch(const T* x, int64_t B, int64_t R, int64_t k_read, int64_t k_pa
     if (lg >= 0 && k_read >= k_pad && (reinterpret_cast<uintptr_t>(x) & 31) == 0 && sxb % kVec32 == 0 &&
         sxr % kVec32 == 0 && (reinterpret_cast<uintptr_t>(nib) & 7) == 0 && snb % 8 == 0 && snr % 8 == 0) {
       dim3 qgrid((unsigned)((per_batch + 1023) / 1024), (unsigned)B);
-      pack_rows_quad_kernel<T><<<qgrid, 256, 0, st>>>(x, lg, per_batch, sxb, sxr, nib, snb, snr, sc, ssb, ssr);
-      return launch_result("nvfp4_pack(rows)");
+      return launch("nvfp4_pack(rows)", pack_rows_quad_kernel<T>, qgrid, 256, 0, st, x, lg, per_batch, sxb, sxr, nib, snb,
+                    snr, sc, ssb, ssr);
     }
     dim3 grid((unsigned)blocks, (unsigned)B);
-    pack_rows_kernel<T><<<grid, 256, 0, st>>>(x, R, k_read, ngroups, lg, per_batch, sxb, sxr, nib, snb,
-                                              snr, sc, ssb, ssr, vec);
-    return launch_result("nvfp4_pack(rows)");
+    return launch("nvfp4_pack(rows)", pack_rows_kernel<T>, grid, 256, 0, st, x, R, k_read, ngroups, lg, per_batch, sxb, sxr,
+                  nib, snb, snr, sc, ssb, ssr, vec);
   }
   if (sxr == 1 && B < 65536 && (R + kColsRows - 1) / kColsRows < 65536) {
     const int vec = base_ok && sxb % kVecElems == 0 && sxk % kVecElems == 0;
     dim3 grid((unsigned)((k_pad + kColsKeys * kColsRun - 1) / (kColsKeys * kColsRun)),
               (unsigned)((R + kColsRows - 1) / kColsRows), (unsigned)B);
-    pack_cols_kernel<T, false><<<grid, 256, 0, st>>>(x, R, k_read, k_pad, sxb, sxk, nib, snb, snr, sc,
-                                                     ssb, ssr, vec, nullptr, 0, 0, nullptr, 0, 0, nullptr, 0, 0u);
-    return launch_result("nvfp4_pack(cols)");
+    return launch("nvfp4_pack(cols)", pack_cols_kernel<T, false>, grid, 256, 0, st, x, R, k_read, k_pad, sxb, sxk, nib, snb,
+                  snr, sc, ssb, ssr, vec, nullptr, 0, 0, nullptr, 0, 0, nullptr, 0, 0u);
   }
   const int64_t blocks = (total + 255) / 256;
   NVFP4_REQUIRE(blocks < (1LL << 31), "nvfp4_pack: tensor too large");
-  pack_generic_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(x, R, k_read, ngroups, total, sxb, sxr,
-                                                         sxk, nib, snb, snr, sc, ssb, ssr);
-  return launch_result("nvfp4_pack(generic)");
+  return launch("nvfp4_pack(generic)", pack_generic_kernel<T>, dim3((unsigned)blocks), 256, 0, st, x, R, k_read, ngroups,
+                total, sxb, sxr, sxk, nib, snb, snr, sc, ssb, ssr);
 }
 
 }  // namespace nvfp4
@@ -710,11 +811,10 @@ int pack_dual_launch(const void* x, int64_t B, int64_t S, int d, int64_t s_pad, 
   const int vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && sxb % kVecElems == 0 && sxs % kVecElems == 0;
   dim3 grid((unsigned)((s_pad + kColsKeys * kColsRun - 1) / (kColsKeys * kColsRun)),
             (unsigned)((d + kColsRows - 1) / kColsRows), (unsigned)B);
-  pack_cols_kernel<T, true><<<grid, 256, 0, st>>>(
-      static_cast<const T*>(x), d, S, s_pad, sxb, sxs, tnib, (int64_t)d * (s_pad / 2), s_pad / 2, tsc,
+  return launch(
+      "nvfp4_pack_dual", pack_cols_kernel<T, true>, grid, 256, 0, st, static_cast<const T*>(x), d, S, s_pad, sxb, sxs, tnib, (int64_t)d * (s_pad / 2), s_pad / 2, tsc,
       (int64_t)d * (s_pad / 16), s_pad / 16, vec, dnib, S * (int64_t)(d / 2), d / 2, dsc, S * (int64_t)(d / 16),
       d / 16, prescale_amax, sr_flags, seed);
-  return launch_result("nvfp4_pack_dual");
 }
 
 template <typename T>
@@ -740,11 +840,64 @@ int pack_qkv_launch(QkvArgs a, cudaStream_t st) {
   a.nbk = a.bpk * a.bk;
   const int64_t total = a.nbq + a.nbk + a.bk * ((a.tx + kColsRun - 1) / kColsRun) * a.ty;
   NVFP4_REQUIRE(total < (1LL << 31), "nvfp4_pack_qkv: tensors too large");
-  pack_qkv_kernel<T><<<(unsigned)total, 256, 0, st>>>(a);
-  return launch_result("nvfp4_pack_qkv");
+  return launch("nvfp4_pack_qkv", pack_qkv_kernel<T>, dim3((unsigned)total), 256, 0, st, a);
+}
+
+template <typename T>
+int kv_prefill_launch(PrefillArgs a, cudaStream_t st) {
+  constexpr int64_t kVecElems = 16 / sizeof(T), kVec32 = 32 / sizeof(T);
+  auto mult = [](const void* p, int64_t bytes, int64_t s0, int64_t s1, int64_t elems) {
+    return (int)((reinterpret_cast<uintptr_t>(p) % bytes) == 0 && s0 % elems == 0 && s1 % elems == 0);
+  };
+  a.vec_v = mult(a.v, 16, a.svb, a.svr, kVecElems);
+  a.vec_k = mult(a.k, 16, a.skb, a.skr, kVecElems);
+  a.vec_c = a.vec_v && a.vec_k && mult(a.partial, 16, 0, 0, 1) && mult(a.rk, 16, 0, 0, 1) &&
+            mult(a.rv, 16, 0, 0, 1);
+  a.quad_k = mult(a.k, 32, a.skb, a.skr, kVec32);
+  const int64_t ng = a.d / 16;
+  a.bpk = (a.s * ng + (a.quad_k ? 1023 : 255)) / (a.quad_k ? 1024 : 256);
+  a.nbk = a.bpk * a.zhk;
+  a.tx = (a.s_pad + kColsKeys - 1) / kColsKeys;
+  a.ty = (a.d + kColsRows - 1) / kColsRows;
+  a.nbv = a.zhk * ((a.tx + kColsRun - 1) / kColsRun) * a.ty;
+  const int64_t pieces = (16 + (a.rk != nullptr ? 2 * a.ring_n : 0)) * (a.d / kVecElems);
+  a.bpc = (pieces + 256 * kPrefillCopyIters - 1) / (256 * kPrefillCopyIters);
+  const int64_t total = a.nbk + a.nbv + a.bpc * a.zhk;
+  NVFP4_REQUIRE(total < (1LL << 31), "nvfp4_kv_prefill: tensors too large");
+  return launch("nvfp4_kv_prefill", kv_prefill_kernel<T>, dim3((unsigned)total), 256, 0, st, a);
 }
 
 }  // namespace nvfp4
+
+extern "C" int nvfp4_kv_prefill(const void* k, const void* v, int dtype, int64_t zhk, int64_t s, int d, int64_t skb,
+                                int64_t skr, int64_t svb, int64_t svr, uint8_t* knv, int64_t knv_unit, uint8_t* ksc,
+                                int64_t ksc_unit, uint8_t* vnv, int64_t vnv_unit, int64_t vnv_row, uint8_t* vsc,
+                                int64_t vsc_unit, int64_t vsc_row, void* partial, void* ring_k, void* ring_v,
+                                int64_t ring_cap, nvfp4_stream_t stream) {
+  using namespace nvfp4;
+  NVFP4_REQUIRE(d == 128 || d == 256, "nvfp4_kv_prefill: D must be 128 or 256");
+  NVFP4_REQUIRE(zhk > 0 && s >= 0, "nvfp4_kv_prefill: bad extent");
+  NVFP4_REQUIRE((s == 0 || (k && v)) && knv && ksc && vnv && vsc && partial, "nvfp4_kv_prefill: null pointer");
+  NVFP4_REQUIRE((ring_k == nullptr) == (ring_v == nullptr) && (ring_k == nullptr || ring_cap > 0),
+                "nvfp4_kv_prefill: ring_k/ring_v/ring_cap inconsistent");
+  NVFP4_REQUIRE(((uintptr_t)knv % 8) == 0 && knv_unit % 8 == 0, "nvfp4_kv_prefill: K nibble rows must be 8-byte aligned");
+  PrefillArgs a;
+  a.k = k; a.v = v; a.s = s; a.zhk = zhk; a.d = d; a.ngroups_log2 = d == 128 ? 3 : 4;
+  a.skb = skb; a.skr = skr; a.svb = svb; a.svr = svr;
+  a.knv = knv; a.ksc = ksc; a.vnv = vnv; a.vsc = vsc;
+  a.knv_unit = knv_unit; a.ksc_unit = ksc_unit; a.vnv_unit = vnv_unit; a.vnv_row = vnv_row;
+  a.vsc_unit = vsc_unit; a.vsc_row = vsc_row;
+  a.partial = partial; a.rk = ring_k; a.rv = ring_v; a.ring_cap = ring_cap;
+  a.ring_n = ring_k != nullptr ? (s < ring_cap ? s : ring_cap) : 0;
+  a.s_pad = (s + 15) / 16 * 16;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  switch (dtype) {
+    case NVFP4_DT_BF16: return kv_prefill_launch<__nv_bfloat16>(a, st);
+    case NVFP4_DT_FP16: return kv_prefill_launch<__half>(a, st);
+    case NVFP4_DT_FP32: return kv_prefill_launch<float>(a, st);
+    default: return fail(-1, "nvfp4_kv_prefill: unknown dtype %d", dtype);
+  }
+}
 
 extern "C" int nvfp4_pack_dual(const void* x, int dtype, int64_t B, int64_t S, int d, int64_t s_pad,
                                int64_t sxb, int64_t sxs, const float* prescale_amax, int sr_flags,
@@ -781,9 +934,8 @@ extern "C" int nvfp4_pack_mx8_t(const void* x, int dtype, int64_t B, int64_t S, 
   {                                                                                                     \
     constexpr int64_t kVecElems = 16 / sizeof(T);                                                       \
     const int vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && sxb % kVecElems == 0 && sxs % kVecElems == 0; \
-    pack_mx8_cols_kernel<T><<<grid, 256, 0, st>>>(static_cast<const T*>(x), d, S, s_pad, sxb, sxs, out, sc, vec, \
-                                                  prescale_amax);                                       \
-    return launch_result("nvfp4_pack_mx8_t");                                                           \
+    return launch("nvfp4_pack_mx8_t", pack_mx8_cols_kernel<T>, grid, 256, 0, st, static_cast<const T*>(x), d, S, s_pad, \
+                  sxb, sxs, out, sc, vec, prescale_amax);                                               \
   }
   switch (dtype) {
     case NVFP4_DT_BF16: NVFP4_MX8(__nv_bfloat16)
@@ -851,10 +1003,8 @@ extern "C" int nvfp4_rope_pack(const void* x, int dtype, int64_t B, int64_t R, i
   const int es = dtype == NVFP4_DT_FP32 ? 4 : 2;
   const int vec = ((uintptr_t)x % 16 == 0) && (sxb * es) % 16 == 0 && (sxr * es) % 16 == 0;
 #define NVFP4_ROPE(T)                                                                              \
-  rope_pack_rows_kernel<T><<<grid, 256, 0, st>>>(static_cast<const T*>(x), R, d, lg, per_batch, sxb, \
-                                                 sxr, cos_tab, sin_tab, positions, pos0, nib, snb,  \
-                                                 snr, sc, ssb, ssr, vec);                           \
-  return launch_result("nvfp4_rope_pack")
+  return launch("nvfp4_rope_pack", rope_pack_rows_kernel<T>, grid, 256, 0, st, static_cast<const T*>(x), R, d, lg, \
+                per_batch, sxb, sxr, cos_tab, sin_tab, positions, pos0, nib, snb, snr, sc, ssb, ssr, vec)
   switch (dtype) {
     case NVFP4_DT_BF16: NVFP4_ROPE(__nv_bfloat16);
     case NVFP4_DT_FP16: NVFP4_ROPE(__half);

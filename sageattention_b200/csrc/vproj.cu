@@ -13,6 +13,7 @@
 // 128 TMEM columns.  Warps: 0 TMA producer, 1 MMA issuer, 2-5 epilogue.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
+#include "common/launch.cuh"
 #include "common/sm100.cuh"
 #include "common/tma_host.cuh"
 #include "common/bwd_util.cuh"
@@ -60,6 +61,8 @@ vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  griddep_launch();
+  griddep_wait();
   const uint32_t tmem = tmem_base_s;
 
   if (warp == 0) {
@@ -170,10 +173,8 @@ extern "C" int nvfp4_vproj_pack(const void* x, const void* w, const void* bias, 
   dim3 grid((unsigned)((features + 127) / 128), (unsigned)((s_pad + 127) / 128), (unsigned)z);
 #define NVFP4_VP(T)                                                                                       \
   {                                                                                                       \
-    cudaError_t e = cudaFuncSetAttribute(vproj_pack_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
-    if (e != cudaSuccess) return fail((int)e, "nvfp4_vproj_pack: smem attribute: %s", cudaGetErrorString(e)); \
-    vproj_pack_kernel<T><<<grid, kVpThreads, smem, st>>>(t_w, t_x, p);                                    \
-    return launch_result("nvfp4_vproj_pack");                                                             \
+    if ((rc = allow_smem("nvfp4_vproj_pack", reinterpret_cast<const void*>(vproj_pack_kernel<T>), smem))) return rc; \
+    return launch("nvfp4_vproj_pack", vproj_pack_kernel<T>, grid, kVpThreads, smem, st, t_w, t_x, p);     \
   }
   if (dtype == NVFP4_DT_BF16) NVFP4_VP(__nv_bfloat16)
   NVFP4_VP(__half)

@@ -7,8 +7,8 @@ through the C ABI:
 * ``append`` is ONE launch (``nvfp4_kv_append``): K row pack, partial-group V store, re-pack of
   the current 16-key V^T group and the optional ring write, with no host synchronisation
   (the reference issues two Triton launches and about six small torch ops per token);
-* ``prefill`` packs K and the full V groups straight into the cache buffers through the strided
-  packer (no temporaries), then stashes the trailing < 16 tokens;
+* ``prefill`` is ONE launch (``nvfp4_kv_prefill``): K and V^T packed straight into the cache buffers,
+  the trailing < 16 tokens and the recent window stored as they are;
 * ``hybrid_decode`` runs the split-K FP4 decode over the old prefix, an exact window-attention
   kernel over the bf16 ring, and merges the two on the device by their log-sum-exps.
 
@@ -82,6 +82,15 @@ class NVFP4KVCache:
         z, hk, s, d = key.shape
         assert (z, hk, d) == (self.z, self.hk, self.d)
         assert s <= self.max_seq_len, "prefill exceeds capacity"
+        rings = (self.rk, self.rv) if self.recent_window > 0 else (None, None)
+        if not _lib.native().kv_prefill(key, value, self.knv, self.ksc, self.vnv, self.vsc, self.v_partial_bf16, *rings):
+            self._prefill_converting(key, value)
+        self.length, self.partial_len = s, s % self.GROUP
+
+    def _prefill_converting(self, key, value):
+        """Operands of another dtype than the cache's (or strided along D): packed as they are, while the
+        open V group and the rings hold them rounded to the cache's dtype."""
+        s, d = key.shape[2:]
         k2 = key.reshape(self.zhk, s, d)
         v2 = value.reshape(self.zhk, s, d)
         _pack_into(k2, self.knv[:, :s], self.ksc[:, :s])
@@ -90,7 +99,6 @@ class NVFP4KVCache:
             _pack_into(v2[:, :full], self.vnv[:, :, : full // 2], self.vsc[:, :, : full // 16],
                        transpose=True)
         rem = s - full
-        self.partial_len = rem
         self.v_partial_bf16.zero_()
         if rem:
             self.v_partial_bf16[:, :rem] = v2[:, full:]
@@ -103,7 +111,6 @@ class NVFP4KVCache:
             slots = pos % self.ring_cap
             self.rk[:, :, slots] = key[:, :, s - w :].to(self.dtype)
             self.rv[:, :, slots] = value[:, :, s - w :].to(self.dtype)
-        self.length = s
 
     # ------------------------------------------------------------------ append
     @torch.no_grad()
