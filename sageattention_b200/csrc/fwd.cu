@@ -5,35 +5,50 @@
 //     P             = exp(S*scale - m) packed to NVFP4 per 16 keys (same scale rule as the packer)
 //     O[128 x D]   += P . V_tile               same MMA kind, V held as V^T (packed along keys)
 // Q/K/V^T nibble tiles arrive by TMA straight from the packed tensors; scale bytes are re-laid
-// into the 32x16-byte form tcgen05.cp expects by two loader warps; S and O live in TMEM.  One
-// thread owns a slice of one query row (one TMEM lane, 32 or 64 key columns), so the
-// per-16-key P pack needs no cross-thread traffic.  The running maximum is exact (O is rescaled in TMEM whenever a row's maximum moves),
-// which keeps the P quantisation decisions those of a plain 128-key tile walk.
+// into the 32x16-byte form tcgen05.cp expects by a loader warp; S and O live in TMEM.  The running
+// maximum is exact (O is rescaled in TMEM whenever a row's maximum moves), which keeps the P
+// quantisation decisions those of a plain 128-key tile walk.
 //
-// Warp roles (640 threads): 0 TMA producer, 1 QK^T issuer, 2 scale loader (+bias, +sample
-// ids), 3 PV issuer, 4-19 softmax / correction / epilogue.  At D=128 the sixteen softmax warps
-// form two groups that alternate key tiles; at D=256 (one S buffer) they share each tile.
-// Every barrier wait is bounded.
+// Warps (608 threads): 0 TMA producer + scale loader (+bias, +sample ids), 1 QK^T issuer, 2 PV
+// issuer, 3-18 softmax / correction / epilogue in two groups of eight that alternate key tiles.
+// Within a group two threads share a query row, 64 key columns each, so the per-16-key P pack needs
+// no cross-thread traffic.  Every barrier wait is bounded.
+//
+// What bounds it: the floor is one ex2 per score (16 lanes per clock and SM, 1024 clocks per tile at
+// D = 128); a softmax warp's tile is a chain -- wait, read, maxima, exchange, exponentials and pack,
+// rescale of O -- that is about four times its share of that, and two groups hide half of it.  What the
+// layout does about the chain: the running maximum is not handed from tile to tile; every thread
+// publishes the maximum of its 64 columns and forms the exact running maximum itself from its group's
+// last one, the two of the tile in between and the other half's (one 64-thread barrier with the warp
+// that holds it); reciprocal scales come from a table in shared memory, not from the pipe that ex2
+// needs; P leaves in 16-byte stores.  Measured on a B200, causal bf16: Z4 H32 Hk8 S8192 D128
+// 2228 -> 2045 us (1.08 PFLOP/s), H16 Hk4 S8192 D256 441 -> 352 us, S1024 D256 26.0 -> 17.9 us.
+// Registers decide here (96 per thread at nineteen warps): variants that spilled even a few hundred
+// bytes took up to three times as long.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
+#include "common/launch.cuh"
 #include "common/sm100.cuh"
 #include "common/tma_host.cuh"
 
 namespace nvfp4 {
 
-#ifndef NVFP4_FWD_NP
-#define NVFP4_FWD_NP 4
-#endif
-constexpr int kFwdNP = NVFP4_FWD_NP;               // softmax threads per query row (D = 256 path)
-constexpr int kFwdThreads = 128 + 128 * kFwdNP;
+constexpr int kFwdRoleWarps = 3;
+constexpr int kFwdThreads = 32 * (kFwdRoleWarps + 16);
 constexpr float kFwdLog2e = 1.4426950408889634f;
+// Tiles whose row maxima are kept for exchange.  A slot may be rewritten six tiles later at the earliest:
+// a thread that publishes tile i has waited for tile i - 3 of the other group, which by then has read i - 6.
+constexpr int kFwdMaxSlots = 8;
 
 template <int D>
 struct FwdCfg {
   static constexpr int KSUB = D / 128;  // 64-byte-wide sub-tiles of a Q/K row
   static constexpr int KB = D / 64;     // K=64 MMAs per QK tile
   static constexpr int NT = D / 128;    // 128-row pieces of the V^T tile (N of the PV MMA = D)
-  static constexpr int NSBUF = (D == 128) ? 2 : 1;  // S / P buffers
+  static constexpr int NSBUF = (D == 128) ? 2 : 1;  // S buffers
+  // D = 256: the one S buffer is emptied into registers at once; D = 128 reads it twice in 32-column
+  // chunks instead (maxima, then exponentials), which keeps the loop free of spills
+  static constexpr bool kOneRead = NSBUF == 1;
   static constexpr int NSTAGE = (D == 128) ? 4 : 3;
   static constexpr int Q_BYTES = KSUB * 8192;
   static constexpr int K_BYTES = KSUB * 8192;
@@ -45,8 +60,7 @@ struct FwdCfg {
   static constexpr int QSF_BYTES = KB * 512;
   static constexpr int P_BYTES = 8192;
   static constexpr int PSF_BYTES = 1024;
-  static constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + Q_BYTES + QSF_BYTES +
-                                    NSBUF * (P_BYTES + PSF_BYTES) + 1024;
+  static constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + Q_BYTES + QSF_BYTES + 2 * (P_BYTES + PSF_BYTES) + 1024;
   // TMEM columns
   static constexpr int T_S = 0;                       // NSBUF x 128
   static constexpr int T_O = NSBUF * 128;             // D
@@ -87,10 +101,12 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+__device__ __forceinline__ void fwd_sts_v4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
 // kVarlen: packed rows with per-token sample ids (a separate instantiation keeps the dense kernel
 // free of the sample tests).
-// sample-id test: a compile-time yes in the varlen instantiation, the run-time test otherwise
-#define FWD_HAS_SEQ (kVarlen || p.seq_id != nullptr)
 template <int D, typename TO, bool kVarlen>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -101,19 +117,20 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* s_stage = smem;
   uint8_t* s_q = s_stage + C::NSTAGE * C::STAGE_BYTES;
-  uint8_t* s_qsf = s_q + C::Q_BYTES;
-  uint8_t* s_p = s_qsf + C::QSF_BYTES;
-  uint8_t* s_psf = s_p + C::NSBUF * C::P_BYTES;
+  uint8_t* s_p = s_q + C::Q_BYTES;
+  uint8_t* s_psf = s_p + 2 * C::P_BYTES;
+  uint8_t* s_qsf = s_psf + 2 * C::PSF_BYTES;
 
   __shared__ uint64_t full_kv[C::NSTAGE], full_sf[C::NSTAGE], empty[C::NSTAGE];
   __shared__ uint64_t s_full[2], s_free[2], p_full[2], pv_done[2], q_full, qsf_full;
+  __shared__ uint64_t mx_ready[kFwdMaxSlots][4];     // row maxima of a tile, one barrier per 32-row quadrant
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
   __shared__ int s_lo_tile;
-  __shared__ float xmax[2][kFwdNP][128];
-  __shared__ float xl[kFwdNP][128];
-  __shared__ float m_row[2][128];
-  __shared__ uint64_t m_ready[2];
+  __shared__ float xmax[kFwdMaxSlots][2][128];       // [tile % slots][key half][row]
+  __shared__ float xl[4][128];
+  __shared__ float xm[2][128];
+  __shared__ float inv_tab[128];                     // reciprocal of every (non-negative) e4m3 byte
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // grid = (heads, query tiles): all heads of the heaviest (last) query tile are scheduled first,
@@ -140,52 +157,56 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
-      mbar_init(&s_free[i], C::NSBUF == 2 ? 256 : 128 * kFwdNP);
-      mbar_init(&p_full[i], C::NSBUF == 2 ? 8 : 4 * kFwdNP);
+      mbar_init(&s_free[i], 8);
+      mbar_init(&p_full[i], 8);
       mbar_init(&pv_done[i], 1);
-      mbar_init(&m_ready[i], 128);
     }
+    for (int i = 0; i < kFwdMaxSlots; ++i)
+      for (int q = 0; q < 4; ++q) mbar_init(&mx_ready[i][q], 2);
     mbar_init(&q_full, 1);
     mbar_init(&qsf_full, 4);
     mbar_fence_init();
-    int lo = 0;
-    if (FWD_HAS_SEQ) lo = (p.seq_start[min(m0, p.s_q - 1)] / 128) * 128;
-    s_lo_tile = lo / 128;
+  }
+  if (tid >= 128 && tid < 256) {
+    float inv;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(e4m3_to_f32((uint8_t)(tid - 128))));
+    inv_tab[tid - 128] = inv;
   }
   if (warp == 1) tmem_alloc(&tmem_base_s, 512);
+  griddep_wait();
+  if (tid == 0) s_lo_tile = kVarlen ? p.seq_start[min(m0, p.s_q - 1)] / 128 : 0;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  griddep_launch();
   const uint32_t tmem = tmem_base_s;
   // varlen: rows of a tile are sorted by sample, so the first row has the earliest start
   const int t_lo = s_lo_tile;
   const int ntile = max(t_hi - t_lo, 0);
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (elect_one() && ntile > 0) {
-      mbar_expect_tx(&q_full, C::Q_BYTES);
-#pragma unroll
-      for (int ks = 0; ks < C::KSUB; ++ks) tma_load_3d(s_q + ks * 8192, &tm_q, &q_full, ks * 64, m0, zh);
-      for (int i = 0; i < ntile; ++i) {
-        const int s = i % C::NSTAGE, t = t_lo + i;
-        if (i >= C::NSTAGE) mbar_wait(&empty[s], ((i / C::NSTAGE) & 1) ^ 1, &err, 1);
-        uint8_t* st = s_stage + s * C::STAGE_BYTES;
-        mbar_expect_tx(&full_kv[s], C::K_BYTES + C::V_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < C::KSUB; ++ks)
-          tma_load_3d(st + ks * 8192, &tm_k, &full_kv[s], ks * 64, t * 128, unit);
-#pragma unroll
-        for (int nt = 0; nt < C::NT; ++nt)
-          tma_load_3d(st + C::K_BYTES + nt * 8192, &tm_v, &full_kv[s], t * 64, nt * 128, unit);
-      }
-    }
-    __syncwarp();
-  } else if (warp == 2) {
-    // ------------------------------------------------------------------ scale loader
+    // ------------------------------------------------------------------ TMA producer, scale loader
     // K scales (+ key bias, sample ids) and V^T scales of a tile, re-laid into the 32 x 16-byte
     // atoms tcgen05.cp copies.  The next tile's bytes are fetched into registers one tile
     // ahead, so per tile the warp pays a shared-memory store, not a trip to L2.
+    const bool leader = elect_one();
+    auto load_tile = [&](int i) {
+      const int s = i % C::NSTAGE, t = t_lo + i;
+      uint8_t* st = s_stage + s * C::STAGE_BYTES;
+      mbar_expect_tx(&full_kv[s], C::K_BYTES + C::V_BYTES);
+#pragma unroll
+      for (int ks = 0; ks < C::KSUB; ++ks) tma_load_3d(st + ks * 8192, &tm_k, &full_kv[s], ks * 64, t * 128, unit);
+#pragma unroll
+      for (int nt = 0; nt < C::NT; ++nt)
+        tma_load_3d(st + C::K_BYTES + nt * 8192, &tm_v, &full_kv[s], t * 64, nt * 128, unit);
+    };
+    if (leader && ntile > 0) {
+      mbar_expect_tx(&q_full, C::Q_BYTES);
+#pragma unroll
+      for (int ks = 0; ks < C::KSUB; ++ks) tma_load_3d(s_q + ks * 8192, &tm_q, &q_full, ks * 64, m0, zh);
+      for (int i = 0; i < min(ntile, C::NSTAGE); ++i) load_tile(i);
+    }
+    __syncwarp();
     const uint8_t* ksrc = p.ksc + (int64_t)unit * p.s_kv * (D / 16);
     const uint8_t* vsrc = p.vsc + (int64_t)unit * D * (p.s_pad / 16);
     uint32_t kx[4][C::KB];
@@ -205,7 +226,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll
           for (int k = 0; k < C::KB; ++k) kx[j][k] = __ldg(gsrc + k);
           if (p.bias != nullptr) nb[j] = __ldg(p.bias + (int64_t)zi * p.s_kv + key);
-          if (FWD_HAS_SEQ) ns[j] = __ldg(p.seq_id + key);
+          if (kVarlen) ns[j] = __ldg(p.seq_id + key);
         }
       }
 #pragma unroll
@@ -215,18 +236,19 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     if (ntile > 0) fetch(t_lo);
     for (int i = 0; i < ntile; ++i) {
       const int s = i % C::NSTAGE;
-      if (i >= C::NSTAGE) mbar_wait(&empty[s], ((i / C::NSTAGE) & 1) ^ 1, &err, 2);
+      if (i >= C::NSTAGE) {
+        mbar_wait(&empty[s], ((i / C::NSTAGE) & 1) ^ 1, &err, 1);
+        if (leader) load_tile(i);
+      }
       uint8_t* st = s_stage + s * C::STAGE_BYTES + C::K_BYTES + C::V_BYTES;
-      float* aux_bias = reinterpret_cast<float*>(st + C::KSF_BYTES + C::VSF_BYTES);
-      int32_t* aux_seq = reinterpret_cast<int32_t*>(st + C::KSF_BYTES + C::VSF_BYTES + 512);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int r = lane + 32 * j;
 #pragma unroll
         for (int k = 0; k < C::KB; ++k)
           *reinterpret_cast<uint32_t*>(st + k * 512 + sf_atom_offset(r, 0)) = kx[j][k];
-        aux_bias[r] = nb[j];
-        aux_seq[r] = ns[j];
+        if (p.bias != nullptr) reinterpret_cast<float*>(st + C::KSF_BYTES + C::VSF_BYTES)[r] = nb[j];
+        if (kVarlen) reinterpret_cast<int32_t*>(st + C::KSF_BYTES + C::VSF_BYTES + 512)[r] = ns[j];
       }
       uint8_t* dst = st + C::KSF_BYTES;
 #pragma unroll
@@ -256,7 +278,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         const uint32_t ph = (j / C::NSTAGE) & 1;
         mbar_wait(&full_kv[s], ph, &err, 5);
         mbar_wait(&full_sf[s], ph, &err, 6);
-        if (j >= C::NSBUF) mbar_spin_wait(&s_free[b], ((j / C::NSBUF) & 1) ^ 1, &err, 7);
+        if (j >= C::NSBUF) {      // the S buffer's last tile has been read into registers
+          const int u = j - C::NSBUF;
+          mbar_spin_wait(&s_free[u & 1], (u >> 1) & 1, &err, 7);
+        }
         tc_fence_after();
         uint8_t* st = s_stage + s * C::STAGE_BYTES;
         const uint32_t sfk = tmem + C::T_SFK + (j & 1) * C::KB * 4;
@@ -270,26 +295,26 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           umma_nvfp4(tmem + C::T_S + b * 128, ad, bd, idesc_qk, tmem + C::T_SFQ + k * 4, sfk + k * 4,
                      k > 0);
         }
-        umma_commit(&s_full[b]);
+        umma_commit(&s_full[j & 1]);     // by tile parity: each group waits for its own tiles
       }
     }
     __syncwarp();
-  } else if (warp == 3) {
+  } else if (warp == 2) {
     // ------------------------------------------------------------------ PV issuer
     // A thread of its own, so a QK^T for tile i+2 is never queued behind the wait for P(i).
     if (elect_one() && ntile > 0) {
       const uint32_t idesc_pv = make_idesc_nvfp4(128, D);
       for (int i = 0; i < ntile; ++i) {
-        const int s = i % C::NSTAGE, b = i % C::NSBUF;
+        const int s = i % C::NSTAGE, b = i & 1;
         // the V tile and V scales of stage s landed before this tile's QK^T was issued, but this
         // thread has to observe them itself; it does so while P is still being written
         mbar_wait(&full_kv[s], (i / C::NSTAGE) & 1, &err, 15);
         mbar_wait(&full_sf[s], (i / C::NSTAGE) & 1, &err, 16);
-        mbar_spin_wait(&p_full[b], (i / C::NSBUF) & 1, &err, 8);
+        mbar_spin_wait(&p_full[b], (i >> 1) & 1, &err, 8);
         tc_fence_after();
         uint8_t* st = s_stage + s * C::STAGE_BYTES;
-        const uint32_t sfp = tmem + C::T_SFP + (i & 1) * 8;
-        const uint32_t sfv = tmem + C::T_SFV + (i & 1) * (2 * C::NT * 4);
+        const uint32_t sfp = tmem + C::T_SFP + b * 8;
+        const uint32_t sfv = tmem + C::T_SFV + b * (2 * C::NT * 4);
 #pragma unroll
         for (int k = 0; k < 2; ++k)
           tmem_cp_32x128b_warpx4(sfp + k * 4, smem_u32(s_psf + b * C::PSF_BYTES + k * 512));
@@ -309,18 +334,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       }
     }
     __syncwarp();
-  } else if (C::NSBUF == 2) {
-    // ------------------------------------------------------------------ softmax / epilogue (D = 128)
-    // Two groups of eight warps alternate key tiles (group g owns tiles g, g+2, ...), so while
-    // one group sits in its exp/pack phase the other does its TMEM loads, row maxima,
-    // barrier and O rescale: the phases of consecutive tiles overlap instead of adding up.
-    // Within a group two threads share a query row (64 key columns each, handled as two
-    // 32-column chunks to stay inside the register budget of a 640-thread CTA).  The running
-    // maximum is handed from tile to tile through shared memory (m_row / m_ready), so it is
-    // still the exact maximum of a sequential 128-key tile walk.
-    const int sw = warp - 4;
+  } else {
+    // ------------------------------------------------------------------ softmax / correction / epilogue
+    const int sw = warp - kFwdRoleWarps;
     const int grp = sw >> 3;             // which tiles (parity)
-    const int wq = sw & 3;               // TMEM lane quadrant
+    const int wq = warp & 3;             // TMEM lane quadrant
     const int half = (sw >> 2) & 1;      // which 64 key columns
     const int part = grp * 2 + half;     // 0..3: slice of O this thread stores in the epilogue
     const int row_in = wq * 32 + lane;
@@ -345,197 +363,190 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       __syncwarp();
       if (lane == 0) mbar_arrive(&qsf_full);
     }
-    const int my_seq = FWD_HAS_SEQ ? p.seq_id[min(row, p.s_q - 1)] : 0;
+    const int my_seq = kVarlen ? p.seq_id[min(row, p.s_q - 1)] : 0;
     // packed rows: when all 128 rows of this tile belong to one sample, key tiles that lie wholly
     // inside that sample need no per-element sample test
     const bool q_one_sample =
-        FWD_HAS_SEQ && (p.seq_id[min(m0, p.s_q - 1)] == p.seq_id[min(m0 + 127, p.s_q - 1)]);
-    const int my_limit = p.causal ? (row + shift) : (p.s_kv - 1);
+        kVarlen && (p.seq_id[min(m0, p.s_q - 1)] == p.seq_id[min(m0 + 127, p.s_q - 1)]);
+    // last visible key of this row, relative to this thread's first column of the first tile
+    const int lim0 = min(p.causal ? (row + shift) : (p.s_kv - 1), p.s_kv - 1) - t_lo * 128 - half * 64;
+    // tiles from i_mask on need a test per score: the causal diagonal, the ragged end, a key bias
+    const int last_full = min(p.causal ? m0 + shift + 1 : p.s_kv, p.s_kv);     // keys below it are visible to every row
+    const int i_mask = p.bias != nullptr ? 0 : max(last_full, 0) / 128 - t_lo;
     const float c2 = p.scaling * kFwdLog2e;
-    const float inv_scaling = 1.0f / p.scaling;
     float m_own = -INFINITY, l_run = 0.0f;   // running max (log2 units) after this group's last tile
-    const uint32_t xmax_s = smem_u32(&xmax[0][0][0]);
-    const uint32_t mrow_s = smem_u32(&m_row[0][0]);
+    const uint32_t xmax_s = smem_u32(&xmax[0][0][0]) + (uint32_t)row_in * 4u;
+    const uint32_t inv_s = smem_u32(inv_tab);
+    const uint32_t pt = smem_u32(s_p + grp * C::P_BYTES) + sw64_offset(row_in, half * 32);   // the next 16 bytes: ^ 16
+    const uint32_t psf = smem_u32(s_psf + grp * C::PSF_BYTES) + half * 512 + sf_atom_offset(row_in, 0);
+    const uint32_t s_base = tmem + lane_addr + C::T_S + half * 64;
+
+    // scores of N columns from column c of this thread's 64, masked where the tile needs it
+    auto load_scores = [&](int i, int c, bool tile_masked, auto& sv) {
+      constexpr int N = sizeof(sv) / sizeof(float);
+      uint32_t r[N / 32][32];
+      const uint32_t addr = s_base + (C::NSBUF == 2 ? grp * 128 : 0) + c;
+#pragma unroll
+      for (int k = 0; k < N / 32; ++k) tmem_ld32(addr + 32 * k, r[k]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int e = 0; e < N; ++e) sv[e] = __uint_as_float(r[e >> 5][e & 31]);
+      if (tile_masked) {
+        const uint8_t* aux = s_stage + (i % C::NSTAGE) * C::STAGE_BYTES + C::K_BYTES + C::V_BYTES + C::KSF_BYTES + C::VSF_BYTES;
+        const int col0 = half * 64 + c;
+        if (p.bias != nullptr) {
+          const float inv_scaling = 1.0f / p.scaling;
+          const float* bp = reinterpret_cast<const float*>(aux) + col0;
+#pragma unroll
+          for (int e = 0; e < N; ++e) sv[e] += bp[e] * inv_scaling;
+        }
+        if constexpr (kVarlen) {
+          const int32_t* ids = reinterpret_cast<const int32_t*>(aux + 512) + col0;
+#pragma unroll
+          for (int e = 0; e < N; ++e) sv[e] = (ids[e] == my_seq) ? sv[e] : -INFINITY;
+        }
+        const int lim = lim0 - i * 128 - c;     // last visible column of these
+#pragma unroll
+        for (int e = 0; e < N; ++e) sv[e] = (e <= lim) ? sv[e] : -INFINITY;
+      }
+    };
+    auto free_scores = [&]() {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_free[grp]);
+    };
 
     for (int i = grp; i < ntile; i += 2) {
-      const int b = i & 1, s = i % C::NSTAGE, t = t_lo + i;
-      const int n0 = t * 128 + half * 64;
-      const uint32_t s_addr = tmem + lane_addr + C::T_S + b * 128 + half * 64;
-      bool tile_masked = (t * 128 + 127 > m0 + shift && p.causal) || (t * 128 + 128 > p.s_kv) ||
-                         (p.bias != nullptr) || (!kVarlen && p.seq_id != nullptr);   // varlen: completed below
-      const uint8_t* aux = s_stage + s * C::STAGE_BYTES + C::K_BYTES + C::V_BYTES + C::KSF_BYTES +
-                           C::VSF_BYTES;
-      const float* aux_bias0 = reinterpret_cast<const float*>(aux);
-      const int32_t* aux_seq0 = reinterpret_cast<const int32_t*>(aux + 512);
-      // visible keys of this row inside the tile: columns [0, lim128] (causal + tail)
-      const int lim128 = min(my_limit, p.s_kv - 1) - t * 128;
-      auto mask_cols = [&](int col0, float (&sv)[32]) {   // col0: first key column inside the tile
-        if (tile_masked) {
-          if (p.bias != nullptr) {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) sv[e] += aux_bias0[col0 + e] * inv_scaling;
-          }
-          if (FWD_HAS_SEQ) {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) sv[e] = (aux_seq0[col0 + e] == my_seq) ? sv[e] : -INFINITY;
-          }
-#pragma unroll
-          for (int e = 0; e < 32; ++e) sv[e] = (col0 + e <= lim128) ? sv[e] : -INFINITY;
-        }
-      };
-      auto mask_chunk = [&](int c, float (&sv)[32]) { mask_cols(half * 64 + c * 32, sv); };
-      auto load_chunk = [&](int c, float (&sv)[32]) {
-        uint32_t r[32];
-        tmem_ld32(s_addr + c * 32, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int e = 0; e < 32; ++e) sv[e] = __uint_as_float(r[e]);
-        mask_chunk(c, sv);
-      };
-      mbar_wait(&s_full[b], (i >> 1) & 1, &err, 9);
+      const int slot = i % kFwdMaxSlots;
+      mbar_wait(&s_full[grp], (i >> 1) & 1, &err, 9);
       tc_fence_after();
-      if constexpr (kVarlen)   // keys are sorted by sample: first and last id equal => all equal
-        tile_masked = tile_masked || !(q_one_sample && aux_seq0[0] == my_seq && aux_seq0[127] == my_seq);
-      // ---- pass 1: maxima of the four 16-key groups of this thread's 64 columns, and their maximum
-      float mx = -INFINITY;
+      bool tile_masked = i >= i_mask;
+      if constexpr (kVarlen) {  // keys are sorted by sample: first and last id equal => all equal
+        const int32_t* ids = reinterpret_cast<const int32_t*>(s_stage + (i % C::NSTAGE) * C::STAGE_BYTES + C::K_BYTES +
+                                                              C::V_BYTES + C::KSF_BYTES + C::VSF_BYTES + 512);
+        tile_masked = tile_masked || !(q_one_sample && ids[0] == my_seq && ids[127] == my_seq);
+      }
+      // ---- maxima of the four 16-key groups and of the 64 columns; the latter goes to the exchange
       float gm[4];
-      auto group_max = [&](int c, const float (&sv)[32]) {
+      float sv1[C::kOneRead ? 64 : 32];
+      auto group_max = [&](int g, const float* v16) {
+        float v = fmax3(v16[0], v16[1], v16[2]);
 #pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2) {
-          float v = fmax3(sv[h2 * 16], sv[h2 * 16 + 1], sv[h2 * 16 + 2]);
-#pragma unroll
-          for (int e = 3; e < 15; e += 2) v = fmax3(v, sv[h2 * 16 + e], sv[h2 * 16 + e + 1]);
-          gm[c * 2 + h2] = fmaxf(v, sv[h2 * 16 + 15]);
-        }
-        mx = fmax3(mx, gm[c * 2], gm[c * 2 + 1]);
+        for (int e = 3; e < 15; e += 2) v = fmax3(v, v16[e], v16[e + 1]);
+        gm[g] = fmaxf(v, v16[15]);
       };
+      if constexpr (C::kOneRead) {
+        load_scores(i, 0, tile_masked, sv1);
+        free_scores();
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        float sv[32];
-        load_chunk(c, sv);
-        group_max(c, sv);
+        for (int g = 0; g < 4; ++g) group_max(g, sv1 + 16 * g);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          load_scores(i, 32 * c, tile_masked, sv1);
+          group_max(2 * c, sv1);
+          group_max(2 * c + 1, sv1 + 16);
+        }
       }
-      const uint32_t xb = (uint32_t)(((i >> 1) & 1) * 4 + grp * 2);
-      sts_f32(xmax_s + ((xb + half) * 128 + row_in) * 4u, mx);
-      named_bar_sync(1 + grp, 256);
-      mx = fmaxf(mx, lds_f32(xmax_s + ((xb + (half ^ 1)) * 128 + row_in) * 4u));
-      // ---- running maximum handed over from the tile before (owned by the other group)
-      float m_prev = -INFINITY;
+      const float mx = fmaxf(fmax3(gm[0], gm[1], gm[2]), gm[3]) * c2;      // c2 > 0: the scaled maximum
+      sts_f32(xmax_s + (uint32_t)(slot * 2 + half) * 512u, mx);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&mx_ready[slot][wq]);
+      // ---- the exact running maximum: own group's last tile, the tile in between, this tile's other half
+      float m_prev = m_own;
       if (i > 0) {
-        mbar_wait(&m_ready[b ^ 1], ((i - 1) >> 1) & 1, &err, 13);
-        m_prev = lds_f32(mrow_s + (uint32_t)((b ^ 1) * 128 + row_in) * 4u);
+        const int ps = (i - 1) % kFwdMaxSlots;
+        mbar_wait(&mx_ready[ps][wq], ((i - 1) / kFwdMaxSlots) & 1, &err, 13);
+        m_prev = fmax3(m_prev, lds_f32(xmax_s + (uint32_t)(ps * 2) * 512u), lds_f32(xmax_s + (uint32_t)(ps * 2 + 1) * 512u));
       }
-      const float m_new = fmaxf(m_prev, mx * c2);
-      if (half == 0) {
-        sts_f32(mrow_s + (uint32_t)(b * 128 + row_in) * 4u, m_new);
-        mbar_arrive(&m_ready[b]);
-      }
+      named_bar_sync(1 + grp * 4 + wq, 64);
+      const float m_new = fmax3(m_prev, mx, lds_f32(xmax_s + (uint32_t)(slot * 2 + (half ^ 1)) * 512u));
       const float m_sf = (m_new == -INFINITY) ? 0.0f : m_new;
-      const float alpha = ex2_approx(m_prev - m_sf);
-      const bool changed = (m_new > m_prev) && (i > 0);
-      l_run *= ex2_approx(m_own - m_sf);
-      m_own = m_new;
-
-      // Block scales of P ahead of the exponentials: ex2 is monotonic, so the largest probability
-      // of a 16-key group is ex2 of its largest score -- the same bits as the maximum over the
-      // sixteen results -- and the scale chain (e4m3 round, decode, reciprocal) leaves the
-      // dependent path of the pack.
       uint32_t scw = 0u;
       float inv_g[4];
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
-        const float am = ex2_approx(fmaf(gm[g], c2, -m_sf));
-        const float s32 = fminf(fmaxf(am * 0.16666667f, kScaleFloor), kScaleMax);
+        const float a = ex2_approx(fmaf(gm[g], c2, -m_sf));
+        const float s32 = fminf(fmaxf(a * 0.16666667f, kScaleFloor), kScaleMax);
         uint16_t sb16;
         asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(sb16) : "f"(0.0f), "f"(s32));
         const uint32_t sb = sb16 & 0xFFu;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv_g[g]) : "f"(e4m3_to_f32((uint8_t)sb)));
+        inv_g[g] = lds_f32(inv_s + sb * 4u);
         scw |= sb << (8 * g);
       }
-      // P buffer b must have been consumed by the PV of tile i - 2
-      if (i >= 2) mbar_wait(&pv_done[b], ((i >> 1) & 1) ^ 1, &err, 10);
-      const uint32_t pt = smem_u32(s_p + b * C::P_BYTES);
-      const uint32_t psf = smem_u32(s_psf + b * C::PSF_BYTES);
-      const float2 c22 = make_float2(c2, c2);
-      const float2 nm2 = make_float2(-m_sf, -m_sf);
-      float2 lsum4[4];
+      // P buffer of this group must have been consumed by the PV of tile i - 2
+      if (i >= 2) mbar_wait(&pv_done[grp], ((i >> 1) & 1) ^ 1, &err, 10);
+      float2 ls0 = make_float2(0.0f, 0.0f), ls1 = ls0;
+      const float2 c22 = make_float2(c2, c2), nm2 = make_float2(-m_sf, -m_sf);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) lsum4[c] = make_float2(0.0f, 0.0f);
-      // ---- pass 2: exp, row sum, NVFP4 pack of P (two 32-column chunks = four 16-key groups)
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        const int c = cc;
-        float sv[32];
-        load_chunk(c, sv);
-        if (c == 1) {
-          tc_fence_before();
-          mbar_arrive(&s_free[b]);
+      for (int g2 = 0; g2 < 2; ++g2) {
+        if constexpr (!C::kOneRead) {
+          load_scores(i, 32 * g2, tile_masked, sv1);
+          if (g2 == 1) free_scores();
         }
+        const float* sv = sv1 + (C::kOneRead ? 32 * g2 : 0);
+        uint32_t w[4];
 #pragma unroll
-        for (int g2 = 0; g2 < 2; ++g2) {
-          const int g = c * 2 + g2;
+        for (int h2 = 0; h2 < 2; ++h2) {
+          const int g = g2 * 2 + h2;
           const float2 inv2 = make_float2(inv_g[g], inv_g[g]);
           float2 y[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            const float2 t2 = __ffma2_rn(make_float2(sv[g2 * 16 + 2 * e], sv[g2 * 16 + 2 * e + 1]), c22, nm2);
+            const float2 t2 = __ffma2_rn(make_float2(sv[h2 * 16 + 2 * e], sv[h2 * 16 + 2 * e + 1]), c22, nm2);
             const float2 pe = make_float2(ex2_approx(t2.x), ex2_approx(t2.y));
-            lsum4[g] = __fadd2_rn(lsum4[g], pe);
+            if (e & 1) ls1 = __fadd2_rn(ls1, pe);
+            else ls0 = __fadd2_rn(ls0, pe);
             y[e] = __fmul2_rn(pe, inv2);
           }
-          const uint32_t lo = e2m1x8(y[0].x, y[0].y, y[1].x, y[1].y, y[2].x, y[2].y, y[3].x, y[3].y);
-          const uint32_t hi2 = e2m1x8(y[4].x, y[4].y, y[5].x, y[5].y, y[6].x, y[6].y, y[7].x, y[7].y);
-          sts_v2(pt + sw64_offset(row_in, (half * 4 + g) * 8), lo, hi2);
+          w[2 * h2] = e2m1x8(y[0].x, y[0].y, y[1].x, y[1].y, y[2].x, y[2].y, y[3].x, y[3].y);
+          w[2 * h2 + 1] = e2m1x8(y[4].x, y[4].y, y[5].x, y[5].y, y[6].x, y[6].y, y[7].x, y[7].y);
         }
+        fwd_sts_v4(pt ^ (16u * g2), w[0], w[1], w[2], w[3]);
       }
-      sts_b32(psf + half * 512 + sf_atom_offset(row_in, 0), scw);
-      {
-        const float2 t01 = __fadd2_rn(lsum4[0], lsum4[1]), t23 = __fadd2_rn(lsum4[2], lsum4[3]);
-        const float2 tt = __fadd2_rn(t01, t23);
-        l_run += tt.x + tt.y;
-      }
+      ls0 = __fadd2_rn(ls0, ls1);
+      sts_b32(psf, scw);
+      const float alpha = ex2_approx(m_prev - m_sf);
+      const bool changed = (m_new > m_prev) && (i > 0);
+      l_run = fmaf(l_run, ex2_approx(m_own - m_sf), ls0.x + ls0.y);
+      m_own = m_new;
       if (__any_sync(0xffffffffu, changed)) {
         // O is rescaled (this thread: half of its row) once the PV of tile i - 1 has landed
-        mbar_wait(&pv_done[b ^ 1], ((i - 1) >> 1) & 1, &err, 11);
+        mbar_wait(&pv_done[grp ^ 1], ((i - 1) >> 1) & 1, &err, 11);
         tc_fence_after();
         const float a = changed ? alpha : 1.0f;
         const float2 a2 = make_float2(a, a);
-        {
 #pragma unroll
-          for (int c = 0; c < RC / 32; ++c) {
-            uint32_t r[32];
-            tmem_ld32(tmem + lane_addr + C::T_O + half * RC + c * 32, r);
-            tmem_ld_wait();
+        for (int c = 0; c < RC / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld32(tmem + lane_addr + C::T_O + half * RC + c * 32, r);
+          tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 32; e += 2) {
-              const float2 v = __fmul2_rn(make_float2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), a2);
-              r[e] = __float_as_uint(v.x);
-              r[e + 1] = __float_as_uint(v.y);
-            }
-            tmem_st32(tmem + lane_addr + C::T_O + half * RC + c * 32, r);
+          for (int e = 0; e < 32; e += 2) {
+            const float2 v = __fmul2_rn(make_float2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), a2);
+            r[e] = __float_as_uint(v.x);
+            r[e + 1] = __float_as_uint(v.y);
           }
+          tmem_st32(tmem + lane_addr + C::T_O + half * RC + c * 32, r);
         }
         tmem_st_wait();
         tc_fence_before();
       }
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[b]);
+      if (lane == 0) mbar_arrive(&p_full[grp]);
     }
 
     // ---- epilogue: bring the four partial row sums to the final maximum, O / l -> out, LSE
-    float m_fin = -INFINITY;
-    if (ntile > 0) {
-      const int last = ntile - 1;
-      mbar_wait(&m_ready[last & 1], (last >> 1) & 1, &err, 14);
-      m_fin = lds_f32(mrow_s + (uint32_t)((last & 1) * 128 + row_in) * 4u);
-    }
+    xl[part][row_in] = l_run;
+    if (half == 0) xm[grp][row_in] = m_own;
+    named_bar_sync(9, 512);
+    const float ma = xm[0][row_in], mb = xm[1][row_in];
+    const float m_fin = fmaxf(ma, mb);
     {
       const float m_sf = (m_fin == -INFINITY) ? 0.0f : m_fin;
-      xl[part][row_in] = l_run * ex2_approx(m_own - m_sf);
+      l_run = (xl[0][row_in] + xl[1][row_in]) * ex2_approx(ma - m_sf) + (xl[2][row_in] + xl[3][row_in]) * ex2_approx(mb - m_sf);
     }
-    named_bar_sync(3, 512);
-    l_run = xl[0][row_in] + xl[1][row_in] + xl[2][row_in] + xl[3][row_in];
     TO* orow = nullptr;
     if (row < p.s_q)
       orow = static_cast<TO*>(p.out) + (int64_t)zi * p.so_z + (int64_t)hi * p.so_h +
@@ -582,246 +593,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       const float m_f = (m_fin == -INFINITY) ? 0.0f : m_fin;
       p.lse[(int64_t)zh * p.s_q + row] = m_f * 0.6931471805599453f + logf(l_safe);
     }
-  } else {
-    // ------------------------------------------------------------------ softmax / epilogue
-    // (D = 256: one S buffer.)  All sixteen softmax warps share each tile: NP threads per query
-    // row, each owning 128/NP key columns; a row's threads exchange their partial maxima
-    // through shared memory once per tile and rescale / store their own slice of O.
-    const int sw = warp - 4;
-    const int wq = sw & 3;               // TMEM lane quadrant
-    const int half = sw >> 2;            // which slice of the tile's key columns (0 .. NP-1)
-    constexpr int NP = kFwdNP;
-    constexpr int CW = 128 / NP;         // key columns per thread
-    constexpr int NG = CW / 16;          // 16-key groups per thread
-    const int row_in = wq * 32 + lane;   // row within the query tile
-    const int row = m0 + row_in;         // query index
-    const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
-    constexpr int OC = D / kFwdNP;       // O columns owned by this thread
-    if (half == 0) {
-      // Q scale bytes -> A-operand scale atoms
-      uint32_t wds[C::KB];
-#pragma unroll
-      for (int k = 0; k < C::KB; ++k) wds[k] = 0u;
-      if (row < p.s_q) {
-        const uint32_t* gsrc =
-            reinterpret_cast<const uint32_t*>(p.qsc + ((int64_t)zh * p.s_q + row) * (D / 16));
-#pragma unroll
-        for (int k = 0; k < C::KB; ++k) wds[k] = __ldg(gsrc + k);
-      }
-#pragma unroll
-      for (int k = 0; k < C::KB; ++k)
-        *reinterpret_cast<uint32_t*>(s_qsf + k * 512 + sf_atom_offset(row_in, 0)) = wds[k];
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&qsf_full);
-    }
-    const int my_seq = FWD_HAS_SEQ ? p.seq_id[min(row, p.s_q - 1)] : 0;
-    const bool q_one_sample =
-        FWD_HAS_SEQ && (p.seq_id[min(m0, p.s_q - 1)] == p.seq_id[min(m0 + 127, p.s_q - 1)]);
-    const int my_limit = p.causal ? (row + shift) : (p.s_kv - 1);  // last visible key index
-    const float c2 = p.scaling * kFwdLog2e;
-    const float inv_scaling = 1.0f / p.scaling;
-    float m_run = -INFINITY, l_run = 0.0f;   // m_run in log2 units
-    const uint32_t xmax_s = smem_u32(&xmax[0][0][0]);
-
-    for (int i = 0; i < ntile; ++i) {
-      const int b = i % C::NSBUF, s = i % C::NSTAGE, t = t_lo + i;
-      const int n0 = t * 128 + half * CW;
-      mbar_wait(&s_full[b], (i / C::NSBUF) & 1, &err, 9);
-      tc_fence_after();
-      float sv[CW];
-      {
-        uint32_t r0[CW / 32][32];
-#pragma unroll
-        for (int c = 0; c < CW / 32; ++c) tmem_ld32(tmem + lane_addr + C::T_S + b * 128 + half * CW + c * 32, r0[c]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int c = 0; c < CW / 32; ++c)
-#pragma unroll
-          for (int e = 0; e < 32; ++e) sv[c * 32 + e] = __uint_as_float(r0[c][e]);
-      }
-      tc_fence_before();
-      mbar_arrive(&s_free[b]);
-
-      bool tile_masked = (t * 128 + 127 > m0 + shift && p.causal) || (t * 128 + 128 > p.s_kv) ||
-                         (p.bias != nullptr) || (!kVarlen && p.seq_id != nullptr);
-      {
-        const int32_t* aux_seq0 = reinterpret_cast<const int32_t*>(
-            s_stage + s * C::STAGE_BYTES + C::K_BYTES + C::V_BYTES + C::KSF_BYTES + C::VSF_BYTES + 512);
-        if constexpr (kVarlen)   // keys are sorted by sample: first and last id equal => all equal
-          tile_masked = tile_masked || !(q_one_sample && aux_seq0[0] == my_seq && aux_seq0[127] == my_seq);
-      }
-      if (tile_masked) {
-        const uint8_t* aux = s_stage + s * C::STAGE_BYTES + C::K_BYTES + C::V_BYTES + C::KSF_BYTES +
-                             C::VSF_BYTES;
-        const float* aux_bias = reinterpret_cast<const float*>(aux) + half * CW;
-        const int32_t* aux_seq = reinterpret_cast<const int32_t*>(aux + 512) + half * CW;
-#pragma unroll
-        for (int e = 0; e < CW; ++e) {
-          float v = sv[e];
-          if (p.bias != nullptr) v += aux_bias[e] * inv_scaling;
-          const int key = n0 + e;
-          bool ok = key <= my_limit && key < p.s_kv;
-          if (FWD_HAS_SEQ) ok = ok && (aux_seq[e] == my_seq);
-          sv[e] = ok ? v : -INFINITY;
-        }
-      }
-      float mx;
-      float m4[NG];                     // maxima of the thread's 16-key groups
-      {
-#pragma unroll
-        for (int c = 0; c < NG; ++c) {
-          float v = fmax3(sv[c * 16], sv[c * 16 + 1], sv[c * 16 + 2]);
-#pragma unroll
-          for (int e = 3; e < 15; e += 2) v = fmax3(v, sv[c * 16 + e], sv[c * 16 + e + 1]);
-          m4[c] = fmaxf(v, sv[c * 16 + 15]);
-        }
-        mx = m4[0];
-#pragma unroll
-        for (int c = 1; c < NG; ++c) mx = fmaxf(mx, m4[c]);
-      }
-      sts_f32(xmax_s + (uint32_t)(((i & 1) * NP + half) * 128 + row_in) * 4u, mx);
-      named_bar_sync(1, 128 * NP);
-#pragma unroll
-      for (int o = 1; o < NP; ++o)
-        mx = fmaxf(mx, lds_f32(xmax_s + (uint32_t)(((i & 1) * NP + ((half + o) % NP)) * 128 + row_in) * 4u));
-      const float m_new = fmaxf(m_run, mx * c2);
-      const float m_sf = (m_new == -INFINITY) ? 0.0f : m_new;
-      const float alpha = ex2_approx(m_run - m_sf);
-      const bool changed = (m_new > m_run) && (i > 0);
-      m_run = m_new;
-
-      // P buffer b must have been consumed by the PV of tile i - NSBUF
-      if (i >= C::NSBUF) mbar_wait(&pv_done[b], ((i / C::NSBUF) & 1) ^ 1, &err, 10);
-      const uint32_t pt = smem_u32(s_p + b * C::P_BYTES);
-      const uint32_t psf = smem_u32(s_psf + b * C::PSF_BYTES);
-      float2 lsum4[NG];
-#pragma unroll
-      for (int c = 0; c < NG; ++c) lsum4[c] = make_float2(0.0f, 0.0f);
-      uint32_t scw = 0u;
-      const float2 c22 = make_float2(c2, c2);
-      const float2 nm2 = make_float2(-m_sf, -m_sf);
-      // block scales of P ahead of the exponentials (ex2 is monotonic: the largest probability of a
-      // group is ex2 of its largest score), so the scale chain is off the dependent path of the pack
-      float inv_g[NG];
-#pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        const float am = ex2_approx(fmaf(m4[g], c2, -m_sf));
-        const float s32 = fminf(fmaxf(am * 0.16666667f, kScaleFloor), kScaleMax);
-        uint16_t sb16;
-        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(sb16) : "f"(0.0f), "f"(s32));
-        const uint32_t sb = sb16 & 0xFFu;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv_g[g]) : "f"(e4m3_to_f32((uint8_t)sb)));
-        scw |= sb << (8 * g);
-      }
-#pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        const float2 inv2 = make_float2(inv_g[g], inv_g[g]);
-        float2 y[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float2 t2 = __ffma2_rn(make_float2(sv[g * 16 + 2 * e], sv[g * 16 + 2 * e + 1]), c22, nm2);
-          const float2 pe = make_float2(ex2_approx(t2.x), ex2_approx(t2.y));
-          lsum4[g] = __fadd2_rn(lsum4[g], pe);
-          y[e] = __fmul2_rn(pe, inv2);
-        }
-        const uint32_t lo = e2m1x8(y[0].x, y[0].y, y[1].x, y[1].y, y[2].x, y[2].y, y[3].x, y[3].y);
-        const uint32_t hi2 = e2m1x8(y[4].x, y[4].y, y[5].x, y[5].y, y[6].x, y[6].y, y[7].x, y[7].y);
-        sts_v2(pt + sw64_offset(row_in, (half * NG + g) * 8), lo, hi2);
-      }
-      // this thread's NG scale bytes: groups half*NG .. of the row's 8 (4 per K=64 atom)
-      if constexpr (NG == 4) {
-        sts_b32(psf + half * 512 + sf_atom_offset(row_in, 0), scw);
-      } else {
-        asm volatile("st.shared.b16 [%0], %1;" ::"r"(psf + (half >> 1) * 512 + sf_atom_offset(row_in, (half & 1) * 2)),
-                     "h"((uint16_t)scw) : "memory");
-      }
-      {
-        float2 tt = lsum4[0];
-#pragma unroll
-        for (int c = 1; c < NG; ++c) tt = __fadd2_rn(tt, lsum4[c]);
-        l_run = l_run * alpha + (tt.x + tt.y);
-      }
-
-      if (__any_sync(0xffffffffu, changed)) {
-        // this thread's slice of O is rescaled once the previous PV has landed
-        const int pb = (i - 1) % C::NSBUF;
-        mbar_wait(&pv_done[pb], ((i - 1) / C::NSBUF) & 1, &err, 11);
-        tc_fence_after();
-        const float a = changed ? alpha : 1.0f;
-        const float2 a2 = make_float2(a, a);
-#pragma unroll
-        for (int c = 0; c < OC / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld32(tmem + lane_addr + C::T_O + half * OC + c * 32, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const float2 v = __fmul2_rn(make_float2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), a2);
-            r[e] = __float_as_uint(v.x);
-            r[e + 1] = __float_as_uint(v.y);
-          }
-          tmem_st32(tmem + lane_addr + C::T_O + half * OC + c * 32, r);
-        }
-        tmem_st_wait();
-        tc_fence_before();
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[b]);
-    }
-
-    // ---- epilogue: O / l -> out, LSE.  The row sum is the total of the NP slices.
-    xl[half][row_in] = l_run;
-    named_bar_sync(1, 128 * NP);
-#pragma unroll
-    for (int o = 1; o < NP; ++o) l_run += xl[(half + o) % NP][row_in];
-    TO* orow = nullptr;
-    if (row < p.s_q)
-      orow = static_cast<TO*>(p.out) + (int64_t)zi * p.so_z + (int64_t)hi * p.so_h +
-             (int64_t)row * p.so_s + half * OC;
-    if (ntile > 0) {
-      const int last = ntile - 1;
-      mbar_wait(&pv_done[last % C::NSBUF], (last / C::NSBUF) & 1, &err, 12);
-      tc_fence_after();
-      float inv_l;
-      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv_l) : "f"((l_run == 0.0f) ? 1.0f : l_run));
-#pragma unroll
-      for (int c = 0; c < OC / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld32(tmem + lane_addr + C::T_O + half * OC + c * 32, r);
-        tmem_ld_wait();
-        if (orow != nullptr) {
-          if constexpr (sizeof(TO) == 2) {
-            uint32_t w[16];
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const TO a0 = from_f32<TO>(__uint_as_float(r[2 * e]) * inv_l);
-              const TO a1 = from_f32<TO>(__uint_as_float(r[2 * e + 1]) * inv_l);
-              w[e] = (uint32_t)(*reinterpret_cast<const uint16_t*>(&a0)) |
-                     ((uint32_t)(*reinterpret_cast<const uint16_t*>(&a1)) << 16);
-            }
-            uint4* dst = reinterpret_cast<uint4*>(orow + c * 32);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) dst[e] = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
-          } else {
-            float4* dst = reinterpret_cast<float4*>(orow + c * 32);
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-              dst[e] = make_float4(__uint_as_float(r[4 * e]) * inv_l, __uint_as_float(r[4 * e + 1]) * inv_l,
-                                   __uint_as_float(r[4 * e + 2]) * inv_l, __uint_as_float(r[4 * e + 3]) * inv_l);
-          }
-        }
-      }
-      tc_fence_before();
-    } else if (orow != nullptr) {
-      for (int e = 0; e < OC; ++e) orow[e] = from_f32<TO>(0.0f);
-    }
-    if (p.lse != nullptr && row < p.s_q && half == 0) {
-      const float l_safe = (l_run == 0.0f) ? 1.0f : l_run;
-      const float m_fin = (m_run == -INFINITY) ? 0.0f : m_run;
-      p.lse[(int64_t)zh * p.s_q + row] = m_fin * 0.6931471805599453f + logf(l_safe);
-    }
   }
   tc_fence_before();
   __syncthreads();
@@ -829,17 +600,14 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-#undef FWD_HAS_SEQ
 template <int D, typename TO>
 int fwd_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                const FwdParams& p, int64_t zh, cudaStream_t st) {
   using C = FwdCfg<D>;
   auto kern = (p.seq_id != nullptr) ? fwd_kernel<D, TO, true> : fwd_kernel<D, TO, false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-  if (e != cudaSuccess) return fail((int)e, "nvfp4_fwd: smem attribute: %s", cudaGetErrorString(e));
+  if (int rc = allow_smem("nvfp4_fwd", reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return rc;
   dim3 grid((unsigned)zh, (unsigned)((p.s_q + 127) / 128));
-  kern<<<grid, kFwdThreads, C::SMEM_BYTES, st>>>(tq, tk, tv, p);
-  return launch_result("nvfp4_fwd");
+  return launch("nvfp4_fwd", kern, grid, kFwdThreads, C::SMEM_BYTES, st, tq, tk, tv, p);
 }
 
 }  // namespace nvfp4
