@@ -8,19 +8,19 @@
 //   dV = P^T dO',  dK = dS^T Q,  dQ = dS K     A operand packed IN THE KERNEL along the contraction
 //                                              axis, B operand = the transposed pack (dO'^T, Q^T, K^T)
 //
-// One kernel template serves both passes.  A CTA owns 128 "rows" and streams "columns" in stages
+// One kernel template serves all passes.  A CTA owns 128 "rows" and streams "columns" in stages
 // of 128 (two 64-column steps per stage):
-//   dK/dV pass  rows = keys of a (batch, kv-head) unit, columns = queries of every head of the GQA
-//               group in turn (dK / dV are reduced over the group in TMEM and written once);
+//   dV / dK passes  rows = keys of a (batch, kv-head) unit, columns = queries of every head of the GQA
+//               group in turn (dV / dK are reduced over the group in TMEM and written once); one pass
+//               for both at D = 128, one each at D = 256;
 //   dQ pass     rows = queries of a head, columns = keys.
 // Per step the issuer thread queues S (or S^T) and dP as two N=64 block-scaled MMAs each; a
 // softmax thread owns one row and 16-column chunks of the step's 64 columns, so the per-16 packs of
 // P and dS along the columns are thread-local: nibbles and scale bytes go to shared memory in the
-// operand layout and feed one M128 N128 K64 MMA per gradient.  Six FP4 MMAs per step replace the
-// twenty bf16 MMAs of the high-precision kernels.  Two teams of softmax warps alternate steps, so
-// the TMEM loads and barrier waits of one step hide behind the arithmetic of the other; at D = 128
-// two threads share a row (sixteen softmax warps, four per SM sub-partition: the per-element exp +
-// pack work is bound by how many warps a sub-partition has to interleave), at D = 256 one.
+// operand layout and feed one MMA (M128, N = head dim, K64) per gradient and step.  FP4 MMAs replace
+// the bf16 MMAs of the high-precision kernels.  Two teams of softmax warps alternate steps, so
+// the TMEM loads and barrier waits of one step hide behind the arithmetic of the other; two threads share
+// a row (the per-element exp + pack work is bound by how many warps a sub-partition has to interleave).
 //
 // Keeping the packed operands inside the e4m3 scale range (2^-9 .. 448) -- the job of the
 // reference's per-row rms normalisation, flash.py:184-228 -- is done with factors that never change
@@ -30,9 +30,8 @@
 //     full precision for P >= 6e-6 (uniform attention over 170 k keys) and flushes only below 2e-7;
 //   * the constant factors are undone on the accumulators in the epilogue.
 // Causal masking is bottom-right aligned; packed varlen is block-diagonal; an additive key bias
-// enters the recompute of P.  Head dim 128, or 256 as two 128-wide output halves per tile (both
-// halves recompute S and dP).  No atomics: results are run-to-run identical.  Every barrier wait
-// is bounded.
+// enters the recompute of P.  No atomics: results are run-to-run identical.  Every barrier wait is
+// bounded.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
 #include "common/launch.cuh"
@@ -47,37 +46,52 @@ constexpr float kB4PShift = 11.0f;   // P is packed as P * 2^11
 constexpr int kB4Prefetch = 2;       // stages prefetched into L2 ahead of the ring
 
 
+// What a CTA computes.  At D = 128 dV and dK share one pass (both accumulators fit beside S and dP in
+// tensor memory).  At D = 256 one 256-wide accumulator fills half of tensor memory, so every gradient
+// has a pass of its own over its whole head dim: dV needs S and the P pack only, dK and dQ need S, dP
+// and the dS pack.  Cutting the head dim in halves instead, each recomputing everything, ran S, dP and
+// both packs twice: the three passes of S8192 H16 Hk4 2740 -> 1483 us with the pre-pass.
+enum B4Pass { kB4DkDv = 0, kB4Dq = 1, kB4Dv = 2, kB4Dk = 3 };
+
 // kFp8: the gradient GEMMs' operands (P^T, dS^T, dS packed in the kernel; dO'^T, Q^T, K^T from the
 // pre-pass) are MXFP8 -- e4m3 bytes, e8m0 scale per 32 -- instead of NVFP4: tiles of 128-byte rows.
-template <int D, bool kFp8 = false>
+template <int D, int kPass, bool kFp8 = false>
 struct B4Cfg {
+  static constexpr bool kKeys = kPass != kB4Dq;                       // rows are keys
+  static constexpr bool kP = kPass == kB4DkDv || kPass == kB4Dv;      // the P pack feeds a gradient
+  static constexpr bool kDs = kPass != kB4Dv;                         // dP, and the dS pack
+  static_assert(kPass != kB4DkDv || D == 128, "two 256-wide accumulators do not fit");
   static constexpr int KSUB = D / 128;      // 64-byte-wide sub-tiles of a pack row
   static constexpr int KB = D / 64;         // K = 64 MMAs per product over D
+  static constexpr int NW = D / 128;        // 128-row pieces of a transposed tile (N of a gradient GEMM = D)
   static constexpr int X = KSUB * 8192;     // one pack tile: 128 rows x D/2 bytes
-  static constexpr int AT = kFp8 ? 16384 : 8192;   // an in-kernel operand tile / a transposed-pack tile
-  // resident part
-  static constexpr int O_X1 = 0, O_X2 = X, O_A1 = 2 * X, O_A2 = 2 * X + AT;
-  static constexpr int O_XSF = 2 * X + 2 * AT;            // X1 atoms [KB], X2 atoms [KB]
-  static constexpr int O_ASF = O_XSF + 2 * KB * 512;      // A1 atoms [2 parities], A2 atoms [2]
-  static constexpr int RES = ((O_ASF + 2048 + 1023) / 1024) * 1024;
+  static constexpr int AT = kFp8 ? 16384 : 8192;   // an in-kernel operand tile / a 128-row transposed-pack tile
+  static constexpr int TB = NW * AT;        // a transposed-pack tile
+  // resident part: X1, X2 (dP), the packed P and dS tiles, scale atoms
+  static constexpr int O_X1 = 0, O_X2 = X, O_A1 = O_X2 + (kDs ? X : 0), O_A2 = O_A1 + (kP ? AT : 0);
+  static constexpr int O_XSF = O_A2 + (kDs ? AT : 0);     // X1 atoms [KB], X2 atoms [KB]
+  static constexpr int O_ASF = O_XSF + 2 * KB * 512;      // P atoms [2 parities], dS atoms [2]
+  static constexpr int O_ASF2 = O_ASF + (kP ? 1024 : 0);
+  static constexpr int RES = ((O_ASF2 + (kDs ? 1024 : 0) + 1023) / 1024) * 1024;
   // one stage = 128 columns
-  static constexpr int S_Y1 = 0, S_Y2 = X, S_T1 = 2 * X, S_T2 = 2 * X + AT;
-  static constexpr int S_YSF = 2 * X + 2 * AT;            // Y1 atoms [2 steps][KB], then Y2 atoms [2][KB]
-  static constexpr int S_TSF = S_YSF + 4 * KB * 512;      // T1 atoms [2 parities], T2 atoms [2] (MXFP8: one each)
-  static constexpr int S_AUX = S_TSF + 2048;              // two float[128]
+  static constexpr int S_Y1 = 0, S_Y2 = X, S_T1 = S_Y2 + (kDs ? X : 0), S_T2 = S_T1 + (kP ? TB : 0);
+  static constexpr int S_YSF = S_T2 + (kDs ? TB : 0);     // Y1 atoms [2 steps][KB], then Y2 atoms [2][KB]
+  static constexpr int S_TSF1 = S_YSF + (kDs ? 4 : 2) * KB * 512;     // T1 atoms [2 parities][NW] (MXFP8: [NW])
+  static constexpr int S_TSF2 = S_TSF1 + (kP ? 2 * NW * 512 : 0);
+  static constexpr int S_AUX = S_TSF2 + (kDs ? 2 * NW * 512 : 0);     // two float[128]
   static constexpr int STAGE = ((S_AUX + 1024 + 1023) / 1024) * 1024;
-  static constexpr int NSTAGE = D == 128 ? 3 : 2;
-  // softmax threads per row: at D = 128 two (each owns 32 of a step's 64 columns; sixteen softmax
-  // warps, four on every SM sub-partition), at D = 256 one (eight warps: there the MMAs of a step
-  // take long enough to cover one warp per sub-partition and team)
-  static constexpr int NP = D == 128 ? 2 : 1;
+  static constexpr int NSTAGE = (RES + 3 * STAGE + 1024 <= 227 * 1024) ? 3 : 2;
+  // softmax threads per row: each owns 32 of a step's 64 columns (sixteen softmax warps, four on every SM
+  // sub-partition; one thread per row and eight warps: S8192 D256 1483 -> 1702 us for the three passes)
+  static constexpr int NP = 2;
   static constexpr int THREADS = 128 + 256 * NP;
   static constexpr int TOTAL = RES + NSTAGE * STAGE + 1024;
   // TMEM columns
-  static constexpr uint32_t T_ACC1 = 0, T_ACC2 = 128, T_S = 256, T_G = 384;
+  static constexpr uint32_t T_ACC1 = 0, T_ACC2 = kP ? 128 : 0, T_S = 256, T_G = 384;
   static constexpr uint32_t T_SFX1 = 448, T_SFX2 = T_SFX1 + KB * 4, T_SFY = T_SFX2 + KB * 4;
-  static constexpr uint32_t T_SFA1 = T_SFY + KB * 4, T_SFT1 = T_SFA1 + 4, T_SFA2 = T_SFT1 + 4, T_SFT2 = T_SFA2 + 4;
-  static_assert(T_SFT2 + 4 <= 512, "TMEM budget");
+  static constexpr uint32_t T_SFA1 = T_SFY + KB * 4, T_SFT1 = T_SFA1 + (kP ? 4 : 0);
+  static constexpr uint32_t T_SFA2 = T_SFT1 + (kP ? NW * 4 : 0), T_SFT2 = T_SFA2 + (kDs ? 4 : 0);
+  static_assert(T_SFT2 + (kDs ? NW * 4 : 0) <= 512, "TMEM budget");
   static_assert(TOTAL <= 227 * 1024, "shared memory budget");
 };
 
@@ -122,6 +136,7 @@ struct B4Params {
   int s_q, s_kv, c_pad;  // c_pad: padded column extent of the transposed packs
   float scaling;
   int causal;
+  int late_wait;         // independent of the kernel before it: wait for it at the end, not at the start
   int sr_p, sr_ds;       // stochastic rounding of the in-kernel P / dS packs (fp4_legacy mode)
   uint32_t seed;
   int* status;
@@ -195,17 +210,17 @@ __device__ __forceinline__ void sts_b16(uint32_t saddr, uint32_t a) {
   asm volatile("st.shared.b16 [%0], %1;" ::"r"(saddr), "h"((uint16_t)a) : "memory");
 }
 
-// kDkdv = true: the dK/dV pass (rows = keys), false: the dQ pass (rows = queries).
 // kMode: 0 = NVFP4 gradient operands rounded to nearest, 1 = NVFP4 with the stochastic-rounding
 // flags honoured (a kernel of its own, so the common case carries none of it), 2 = MXFP8.
-template <int D, bool kDkdv, typename TG, int kMode>
-__global__ void __launch_bounds__((B4Cfg<D, kMode == 2>::THREADS), 1)
+template <int D, int kPass, typename TG, int kMode>
+__global__ void __launch_bounds__((B4Cfg<D, kPass, kMode == 2>::THREADS), 1)
 bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ CUtensorMap tm_x2,
             const __grid_constant__ CUtensorMap tm_y1, const __grid_constant__ CUtensorMap tm_y2,
             const __grid_constant__ CUtensorMap tm_t1, const __grid_constant__ CUtensorMap tm_t2,
             const B4Params p) {
   constexpr bool kFp8 = kMode == 2, kSr = kMode == 1;
-  using C = B4Cfg<D, kFp8>;
+  using C = B4Cfg<D, kPass, kFp8>;
+  constexpr bool kKeys = C::kKeys, kP = C::kP, kDs = C::kDs;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -219,7 +234,6 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   __shared__ float gs_s;      // the power-of-two pre-scale of dO
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int half = blockIdx.z;     // 128-wide slice of the head dim owned by this CTA (D = 256)
   const int shift = p.s_kv - p.s_q;
   const bool varlen = p.seq_start != nullptr;
 
@@ -244,14 +258,14 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&tmem_base_s, 512);
-  griddep_wait();
+  if (!p.late_wait) griddep_wait();
   if (tid == 0) gs_s = pow2_ceil(p.amax != nullptr ? *p.amax : 1.0f);
 
   // ---- rows of this CTA, and the range of 128-column stages it has to visit
   int rb, row0, zi, kh = 0, cb0;     // row batch entry, first row, batch index, kv head, first column batch entry
   int R, Ccols;                      // row / column extents
   int c_lo = 0, c_hi = 0;
-  if constexpr (kDkdv) {
+  if constexpr (kKeys) {
     rb = blockIdx.x;                 // z * hk + kh
     row0 = blockIdx.y * 128;
     zi = rb / p.hk; kh = rb % p.hk;
@@ -277,7 +291,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   }
   const int i_lo = c_lo / 128;
   const int n_i = max((c_hi + 127) / 128 - i_lo, 0);
-  const int nstage = (kDkdv ? p.g : 1) * n_i;
+  const int nstage = (kKeys ? p.g : 1) * n_i;
   const int nstep = 2 * nstage;
 
   tc_fence_before();
@@ -289,7 +303,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
 
   // stage index -> (column batch entry, first column)
   auto stage_cols = [&](int sg, int& cb, int& col0) {
-    if constexpr (kDkdv) {
+    if constexpr (kKeys) {
       cb = cb0 + sg / n_i;
       col0 = (i_lo + sg % n_i) * 128;
     } else {
@@ -301,22 +315,23 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one() && nstep > 0) {
-      mbar_expect_tx(&x_full, 2 * C::X);
+      mbar_expect_tx(&x_full, (kDs ? 2 : 1) * C::X);
 #pragma unroll
       for (int c = 0; c < C::KSUB; ++c) {
         tma_load_3d(s_res + C::O_X1 + c * 8192, &tm_x1, &x_full, c * 64, row0, rb);
-        tma_load_3d(s_res + C::O_X2 + c * 8192, &tm_x2, &x_full, c * 64, row0, rb);
+        if constexpr (kDs) tma_load_3d(s_res + C::O_X2 + c * 8192, &tm_x2, &x_full, c * 64, row0, rb);
       }
       auto prefetch = [&](int sg) {
         int cb, col0;
         stage_cols(sg, cb, col0);
+        const int tc = kFp8 ? col0 : col0 / 2;
 #pragma unroll
         for (int c = 0; c < C::KSUB; ++c) {
           tma_prefetch_3d(&tm_y1, c * 64, col0, cb);
-          tma_prefetch_3d(&tm_y2, c * 64, col0, cb);
+          if constexpr (kDs) tma_prefetch_3d(&tm_y2, c * 64, col0, cb);
+          if constexpr (kP) tma_prefetch_3d(&tm_t1, tc, c * 128, cb);
+          if constexpr (kDs) tma_prefetch_3d(&tm_t2, tc, c * 128, cb);
         }
-        if constexpr (kDkdv) tma_prefetch_3d(&tm_t1, kFp8 ? col0 : col0 / 2, half * 128, cb);
-        tma_prefetch_3d(&tm_t2, kFp8 ? col0 : col0 / 2, half * 128, cb);
       };
       for (int sg = C::NSTAGE; sg < min(nstage, C::NSTAGE + kB4Prefetch); ++sg) prefetch(sg);
       for (int sg = 0; sg < nstage; ++sg) {
@@ -326,14 +341,15 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
         if (sg + C::NSTAGE + kB4Prefetch < nstage) prefetch(sg + C::NSTAGE + kB4Prefetch);
         if (sg >= C::NSTAGE) mbar_wait(&empty[s], ((sg / C::NSTAGE) & 1) ^ 1, &err, 1);
         uint8_t* sb = s_stage + s * C::STAGE;
-        mbar_expect_tx(&full_tma[s], 2 * C::X + (kDkdv ? 2 : 1) * C::AT);
+        const int tc = kFp8 ? col0 : col0 / 2;
+        mbar_expect_tx(&full_tma[s], (kDs ? 2 : 1) * C::X + ((kP ? 1 : 0) + (kDs ? 1 : 0)) * C::TB);
 #pragma unroll
         for (int c = 0; c < C::KSUB; ++c) {
           tma_load_3d(sb + C::S_Y1 + c * 8192, &tm_y1, &full_tma[s], c * 64, col0, cb);
-          tma_load_3d(sb + C::S_Y2 + c * 8192, &tm_y2, &full_tma[s], c * 64, col0, cb);
+          if constexpr (kDs) tma_load_3d(sb + C::S_Y2 + c * 8192, &tm_y2, &full_tma[s], c * 64, col0, cb);
+          if constexpr (kP) tma_load_3d(sb + C::S_T1 + c * C::AT, &tm_t1, &full_tma[s], tc, c * 128, cb);
+          if constexpr (kDs) tma_load_3d(sb + C::S_T2 + c * C::AT, &tm_t2, &full_tma[s], tc, c * 128, cb);
         }
-        if constexpr (kDkdv) tma_load_3d(sb + C::S_T1, &tm_t1, &full_tma[s], kFp8 ? col0 : col0 / 2, half * 128, cb);
-        tma_load_3d(sb + C::S_T2, &tm_t2, &full_tma[s], kFp8 ? col0 : col0 / 2, half * 128, cb);
       }
     }
     __syncwarp();
@@ -349,7 +365,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
 #pragma unroll
         for (int c = 0; c < C::KB; ++c) {
           cp_async_4(xsf + c * 512 + sf_atom_offset(r, 0), p.x1sc + gi + 4 * c, ok ? 4u : 0u);
-          cp_async_4(xsf + (C::KB + c) * 512 + sf_atom_offset(r, 0), p.x2sc + gi + 4 * c, ok ? 4u : 0u);
+          if constexpr (kDs) cp_async_4(xsf + (C::KB + c) * 512 + sf_atom_offset(r, 0), p.x2sc + gi + 4 * c, ok ? 4u : 0u);
         }
       }
       cp_async_commit();
@@ -365,7 +381,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
         stage_cols(sg, cb, col0);
         if (sg >= C::NSTAGE) mbar_wait(&empty[s], ((sg / C::NSTAGE) & 1) ^ 1, &err, 2);
         uint8_t* sb = s_stage + s * C::STAGE;
-        const uint32_t ysf = smem_u32(sb + C::S_YSF), tsf = smem_u32(sb + C::S_TSF);
+        const uint32_t ysf = smem_u32(sb + C::S_YSF), tsf1 = smem_u32(sb + C::S_TSF1), tsf2 = smem_u32(sb + C::S_TSF2);
         float* aux = reinterpret_cast<float*>(sb + C::S_AUX);
 #pragma unroll
         for (int r4 = 0; r4 < 4; ++r4) {
@@ -377,26 +393,23 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
 #pragma unroll
           for (int c = 0; c < C::KB; ++c) {
             cp_async_4(ysf + (pp * C::KB + c) * 512 + sf_atom_offset(rr, 0), p.y1sc + gi + 4 * c, ok ? 4u : 0u);
-            cp_async_4(ysf + ((2 + pp) * C::KB + c) * 512 + sf_atom_offset(rr, 0), p.y2sc + gi + 4 * c, ok ? 4u : 0u);
+            if constexpr (kDs) cp_async_4(ysf + ((2 + pp) * C::KB + c) * 512 + sf_atom_offset(rr, 0), p.y2sc + gi + 4 * c, ok ? 4u : 0u);
           }
-          // transposed packs: row = feature (this CTA's 128-wide half), 8 scale bytes = this stage's columns
-          if constexpr (kFp8) {     // one word = the four 32-column blocks of the stage
-            const int64_t ti = ((int64_t)cb * D + half * 128 + r) * csc + col0 / 32;
-            if constexpr (kDkdv) cp_async_4(tsf + sf_atom_offset(r, 0), p.t1sc + ti, 4u);
-            cp_async_4(tsf + 2 * 512 + sf_atom_offset(r, 0), p.t2sc + ti, 4u);
-          } else {
-            const int64_t ti = ((int64_t)cb * D + half * 128 + r) * csc + col0 / 16;
+          // transposed packs: row = feature, 8 (MXFP8: 4) scale bytes = this stage's columns
 #pragma unroll
-            for (int pq = 0; pq < 2; ++pq) {
-              if constexpr (kDkdv) cp_async_4(tsf + pq * 512 + sf_atom_offset(r, 0), p.t1sc + ti + 4 * pq, 4u);
-              cp_async_4(tsf + (2 + pq) * 512 + sf_atom_offset(r, 0), p.t2sc + ti + 4 * pq, 4u);
+          for (int nw = 0; nw < C::NW; ++nw) {
+            const int64_t ti = ((int64_t)cb * D + nw * 128 + r) * csc + col0 / (kFp8 ? 32 : 16);
+#pragma unroll
+            for (int pq = 0; pq < (kFp8 ? 1 : 2); ++pq) {
+              if constexpr (kP) cp_async_4(tsf1 + (pq * C::NW + nw) * 512 + sf_atom_offset(r, 0), p.t1sc + ti + 4 * pq, 4u);
+              if constexpr (kDs) cp_async_4(tsf2 + (pq * C::NW + nw) * 512 + sf_atom_offset(r, 0), p.t2sc + ti + 4 * pq, 4u);
             }
           }
-          if constexpr (kDkdv) {
+          if constexpr (kKeys) {
             // per query: -lse * log2e + 11 (exponent offset of P * 2^11) and -delta' * scaling / 4
             const int64_t qi = (int64_t)cb * p.s_q + (ok ? col : 0);
             aux[r] = ok ? fmaf(-p.lse[qi], kB4Log2e, kB4PShift) : 0.0f;
-            aux[128 + r] = ok ? -p.delta[qi] * inv_gs * (p.scaling * 0.25f) : 0.0f;
+            if constexpr (kDs) aux[128 + r] = ok ? -p.delta[qi] * inv_gs * (p.scaling * 0.25f) : 0.0f;
           } else {
             // per key: the additive bias in base-2 units
             aux[r] = (p.bias != nullptr && ok) ? p.bias[(int64_t)zi * p.s_kv + col] * kB4Log2e : 0.0f;
@@ -413,14 +426,14 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one() && nstep > 0) {
       const uint32_t id_n64 = make_idesc_nvfp4(128, 64);
-      const uint32_t id_n128 = make_idesc_nvfp4(128, 128);
+      const uint32_t id_acc = make_idesc_nvfp4(128, D);
       mbar_wait(&x_full, 0, &err, 3);
       mbar_wait(&xsf_full, 0, &err, 4);
       tc_fence_after();
 #pragma unroll
       for (int c = 0; c < C::KB; ++c) {
         tmem_cp_32x128b_warpx4(tmem + C::T_SFX1 + 4 * c, smem_u32(s_res + C::O_XSF + c * 512));
-        tmem_cp_32x128b_warpx4(tmem + C::T_SFX2 + 4 * c, smem_u32(s_res + C::O_XSF + (C::KB + c) * 512));
+        if constexpr (kDs) tmem_cp_32x128b_warpx4(tmem + C::T_SFX2 + 4 * c, smem_u32(s_res + C::O_XSF + (C::KB + c) * 512));
       }
       const uint64_t d_x1 = desc_sw64(s_res + C::O_X1, 0), d_x2 = desc_sw64(s_res + C::O_X2, 0);
       const uint64_t d_a1 = kFp8 ? desc_sw128(s_res + C::O_A1, 0) : desc_sw64(s_res + C::O_A1, 0);
@@ -428,46 +441,35 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
       const uint64_t d_y1 = desc_sw64(s_stage + C::S_Y1, 0), d_y2 = desc_sw64(s_stage + C::S_Y2, 0);
       const uint64_t d_t1 = kFp8 ? desc_sw128(s_stage + C::S_T1, 0) : desc_sw64(s_stage + C::S_T1, 0);
       const uint64_t d_t2 = kFp8 ? desc_sw128(s_stage + C::S_T2, 0) : desc_sw64(s_stage + C::S_T2, 0);
-      // acc1 += A1 T1^T, acc2 += A2 T2^T for step t (columns [64 pp, 64 pp + 64) of its stage)
+      // acc += A T^T of step pp of stage s (columns [64 pp, 64 pp + 64)), one gradient
+      auto one_grad = [&](int pp, int s, uint8_t* sb, uint32_t acc, uint32_t t_acc, uint64_t d_a, uint64_t d_t, int o_asf,
+                          int s_tsf, uint32_t t_sfa, uint32_t t_sft) {
+        tmem_cp_32x128b_warpx4(tmem + t_sfa, smem_u32(s_res + o_asf + pp * 512));
+#pragma unroll
+        for (int nw = 0; nw < C::NW; ++nw)
+          tmem_cp_32x128b_warpx4(tmem + t_sft + nw * 4, smem_u32(sb + s_tsf + ((kFp8 ? 0 : pp * C::NW) + nw) * 512));
+        const uint64_t sg = (uint64_t)(s * (C::STAGE >> 4));
+        if constexpr (kFp8) {
+          // a step is two K = 32 blocks (32 bytes each) of the 128-byte operand rows; block j of step pp
+          // reads byte j of the A atom (one atom per step parity) and byte 2 pp + j of the T atom
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const uint32_t kk = (uint32_t)(pp * 2 + j);
+            umma_mx8(tmem + t_acc, d_a + kk * 2, d_t + sg + kk * 2, make_idesc_mx8(128, D, (uint32_t)j, kk), tmem + t_sfa,
+                     tmem + t_sft, j > 0 ? 1u : acc);
+          }
+        } else {      // stage, then the 32-byte half of a row
+          umma_nvfp4(tmem + t_acc, d_a + pp * 2, d_t + sg + (uint64_t)(pp * 2), id_acc, tmem + t_sfa, tmem + t_sft, acc);
+        }
+      };
       auto grad_gemms = [&](int t) {
         const int pp = t & 1, s = (t >> 1) % C::NSTAGE;
         uint8_t* sb = s_stage + s * C::STAGE;
         mbar_wait(&a_full[pp], (t >> 1) & 1, &err, 8);
         tc_fence_after();
         const uint32_t acc = t > 0 ? 1u : 0u;
-        if constexpr (kFp8) {
-          // a step is two K = 32 blocks (32 bytes each) of the 128-byte operand rows; block j of step pp
-          // reads byte j of the A atom (one atom per step parity) and byte 2 pp + j of the T atom
-          const uint64_t sg = (uint64_t)(s * (C::STAGE >> 4));
-          if constexpr (kDkdv) {
-            tmem_cp_32x128b_warpx4(tmem + C::T_SFA1, smem_u32(s_res + C::O_ASF + pp * 512));
-            tmem_cp_32x128b_warpx4(tmem + C::T_SFT1, smem_u32(sb + C::S_TSF));
-          }
-          tmem_cp_32x128b_warpx4(tmem + C::T_SFA2, smem_u32(s_res + C::O_ASF + (2 + pp) * 512));
-          tmem_cp_32x128b_warpx4(tmem + C::T_SFT2, smem_u32(sb + C::S_TSF + 2 * 512));
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const uint32_t kk = (uint32_t)(pp * 2 + j);
-            const uint32_t id = make_idesc_mx8(128, 128, (uint32_t)j, kk);
-            if constexpr (kDkdv)
-              umma_mx8(tmem + C::T_ACC1, d_a1 + kk * 2, d_t1 + sg + kk * 2, id, tmem + C::T_SFA1, tmem + C::T_SFT1,
-                       j > 0 ? 1u : acc);
-            umma_mx8(tmem + C::T_ACC2, d_a2 + kk * 2, d_t2 + sg + kk * 2, id, tmem + C::T_SFA2, tmem + C::T_SFT2,
-                     j > 0 ? 1u : acc);
-          }
-          umma_commit(&a_free[pp]);
-          if (pp == 1) umma_commit(&empty[s]);
-          return;
-        }
-        const uint64_t so = (uint64_t)(s * (C::STAGE >> 4)) + (uint64_t)(pp * 2);   // stage, then the 32-byte half of a row
-        if constexpr (kDkdv) {
-          tmem_cp_32x128b_warpx4(tmem + C::T_SFA1, smem_u32(s_res + C::O_ASF + pp * 512));
-          tmem_cp_32x128b_warpx4(tmem + C::T_SFT1, smem_u32(sb + C::S_TSF + pp * 512));
-          umma_nvfp4(tmem + C::T_ACC1, d_a1 + pp * 2, d_t1 + so, id_n128, tmem + C::T_SFA1, tmem + C::T_SFT1, acc);
-        }
-        tmem_cp_32x128b_warpx4(tmem + C::T_SFA2, smem_u32(s_res + C::O_ASF + (2 + pp) * 512));
-        tmem_cp_32x128b_warpx4(tmem + C::T_SFT2, smem_u32(sb + C::S_TSF + (2 + pp) * 512));
-        umma_nvfp4(tmem + C::T_ACC2, d_a2 + pp * 2, d_t2 + so, id_n128, tmem + C::T_SFA2, tmem + C::T_SFT2, acc);
+        if constexpr (kP) one_grad(pp, s, sb, acc, C::T_ACC1, d_a1, d_t1, C::O_ASF, C::S_TSF1, C::T_SFA1, C::T_SFT1);
+        if constexpr (kDs) one_grad(pp, s, sb, acc, C::T_ACC2, d_a2, d_t2, C::O_ASF2, C::S_TSF2, C::T_SFA2, C::T_SFT2);
         umma_commit(&a_free[pp]);
         if (pp == 1) umma_commit(&empty[s]);
       };
@@ -491,19 +493,21 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
           umma_nvfp4(tmem + C::T_S + pp * 64, d_x1 + (k >> 1) * 512 + (k & 1) * 2, d_y1 + so + (k >> 1) * 512 + (k & 1) * 2,
                      id_n64, tmem + C::T_SFX1 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
         umma_commit(&s_full[pp]);
-        if (st > 0) {
-          mbar_wait(&g_free, (st - 1) & 1, &err, 9);
-          tc_fence_after();
+        if constexpr (kDs) {
+          if (st > 0) {
+            mbar_wait(&g_free, (st - 1) & 1, &err, 9);
+            tc_fence_after();
+          }
+          // dP (or dP^T)
+#pragma unroll
+          for (int c = 0; c < C::KB; ++c)
+            tmem_cp_32x128b_warpx4(tmem + C::T_SFY + 4 * c, smem_u32(sb + C::S_YSF + ((2 + pp) * C::KB + c) * 512));
+#pragma unroll
+          for (int k = 0; k < C::KB; ++k)
+            umma_nvfp4(tmem + C::T_G, d_x2 + (k >> 1) * 512 + (k & 1) * 2, d_y2 + so + (k >> 1) * 512 + (k & 1) * 2,
+                       id_n64, tmem + C::T_SFX2 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
+          umma_commit(&g_full);
         }
-        // dP (or dP^T)
-#pragma unroll
-        for (int c = 0; c < C::KB; ++c)
-          tmem_cp_32x128b_warpx4(tmem + C::T_SFY + 4 * c, smem_u32(sb + C::S_YSF + ((2 + pp) * C::KB + c) * 512));
-#pragma unroll
-        for (int k = 0; k < C::KB; ++k)
-          umma_nvfp4(tmem + C::T_G, d_x2 + (k >> 1) * 512 + (k & 1) * 2, d_y2 + so + (k >> 1) * 512 + (k & 1) * 2,
-                     id_n64, tmem + C::T_SFX2 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
-        umma_commit(&g_full);
         // The gradient GEMMs trail by two steps: S and dP of step st are queued while the team that
         // will consume them is still finishing step st - 2, so it finds them ready when it is done;
         // waiting here for step st - 1 instead would put the whole MMA round trip between two steps
@@ -536,7 +540,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
     // visible columns of this row: [lo, hi); per-row terms of the exponent and of dS
     int lo = 0, hi = 0;
     float row_e = 0.0f, row_nd = 0.0f;
-    if constexpr (kDkdv) {
+    if constexpr (kKeys) {
       if (row_ok) {
         lo = p.causal ? max(row - shift, 0) : 0;
         hi = p.s_q;
@@ -560,10 +564,10 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
       }
     }
     const uint32_t a1_s = smem_u32(s_res + C::O_A1), a2_s = smem_u32(s_res + C::O_A2);
-    const uint32_t asf_s = smem_u32(s_res + C::O_ASF);
+    const uint32_t asf1_s = smem_u32(s_res + C::O_ASF), asf2_s = smem_u32(s_res + C::O_ASF2);
     const float2 c22 = make_float2(c2, c2), cds2 = make_float2(cds, cds);
     // dQ pass: the per-row exponent offset and -delta' term; dK/dV pass: these come per column from aux
-    const float2 re2 = kDkdv ? make_float2(0.0f, 0.0f) : make_float2(row_e, row_e);
+    const float2 re2 = kKeys ? make_float2(0.0f, 0.0f) : make_float2(row_e, row_e);
     const float2 rnd2 = make_float2(row_nd, row_nd);
     for (int st = team; st < nstep; st += 2) {
       const int pp = team, sg = st >> 1, s = sg % C::NSTAGE;
@@ -574,7 +578,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
       const bool masked = !__all_sync(0xffffffffu, cs0 >= lo && cs0 + 64 <= hi);
       mbar_wait(&full_aux[s], (sg / C::NSTAGE) & 1, &err, 10);
       mbar_wait(&s_full[pp], (st >> 1) & 1, &err, 11);
-      mbar_wait(&g_full, st & 1, &err, 12);
+      if constexpr (kDs) mbar_wait(&g_full, st & 1, &err, 12);
       tc_fence_after();
       uint32_t wp[4], wd[4], scp = 0u, scd = 0u;
       float pkeep[kFp8 ? 16 : 1], dkeep[kFp8 ? 16 : 1];     // MXFP8: the even chunk of a 32-column group
@@ -585,22 +589,26 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
 #pragma unroll
         for (int e = 0; e < 16; e += 4) {
           float2 eo01 = re2, eo23 = re2, nd01 = rnd2, nd23 = rnd2;
-          if constexpr (kDkdv) {
+          if constexpr (kKeys) {
             const float4 a4 = *reinterpret_cast<const float4*>(aux + e);
-            const float4 n4 = *reinterpret_cast<const float4*>(aux + 128 + e);
             eo01 = make_float2(a4.x, a4.y); eo23 = make_float2(a4.z, a4.w);
-            nd01 = make_float2(n4.x, n4.y); nd23 = make_float2(n4.z, n4.w);
+            if constexpr (kDs) {
+              const float4 n4 = *reinterpret_cast<const float4*>(aux + 128 + e);
+              nd01 = make_float2(n4.x, n4.y); nd23 = make_float2(n4.z, n4.w);
+            }
           }
           const float2 t01 = __ffma2_rn(make_float2(__uint_as_float(cur[e]), __uint_as_float(cur[e + 1])), c22, eo01);
           const float2 t23 = __ffma2_rn(make_float2(__uint_as_float(cur[e + 2]), __uint_as_float(cur[e + 3])), c22, eo23);
-          const float2 a01 = __ffma2_rn(make_float2(__uint_as_float(gsrc[e]), __uint_as_float(gsrc[e + 1])), cds2, nd01);
-          const float2 a23 = __ffma2_rn(make_float2(__uint_as_float(gsrc[e + 2]), __uint_as_float(gsrc[e + 3])), cds2, nd23);
           pf[e] = t01.x; pf[e + 1] = t01.y; pf[e + 2] = t23.x; pf[e + 3] = t23.y;
-          ds[e] = a01.x; ds[e + 1] = a01.y; ds[e + 2] = a23.x; ds[e + 3] = a23.y;
+          if constexpr (kDs) {
+            const float2 a01 = __ffma2_rn(make_float2(__uint_as_float(gsrc[e]), __uint_as_float(gsrc[e + 1])), cds2, nd01);
+            const float2 a23 = __ffma2_rn(make_float2(__uint_as_float(gsrc[e + 2]), __uint_as_float(gsrc[e + 3])), cds2, nd23);
+            ds[e] = a01.x; ds[e + 1] = a01.y; ds[e + 2] = a23.x; ds[e + 3] = a23.y;
+          }
         }
         if (has_bias) {           // row bias (dK/dV pass) or column bias (dQ pass), base-2 units
 #pragma unroll
-          for (int e = 0; e < 16; ++e) pf[e] += kDkdv ? row_e : aux[e];
+          for (int e = 0; e < 16; ++e) pf[e] += kKeys ? row_e : aux[e];
         }
 #pragma unroll
         for (int e = 0; e < 16; ++e) pf[e] = ex2_bwd(pf[e]);
@@ -608,149 +616,128 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
 #pragma unroll
           for (int e = 0; e < 16; ++e) pf[e] = (cs0 + 16 * ch + e >= lo && cs0 + 16 * ch + e < hi) ? pf[e] : 0.0f;
         }
+        if constexpr (kDs) {
 #pragma unroll
         for (int e = 0; e < 16; e += 2) {
           const float2 d2 = __fmul2_rn(make_float2(pf[e], pf[e + 1]), make_float2(ds[e], ds[e + 1]));
           ds[e] = d2.x; ds[e + 1] = d2.y;
         }
+        }
         if constexpr (kFp8) {
           if (!(ch & 1)) {
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
-              if constexpr (kDkdv) pkeep[e] = pf[e];
-              dkeep[e] = ds[e];
+              if constexpr (kP) pkeep[e] = pf[e];
+              if constexpr (kDs) dkeep[e] = ds[e];
             }
           } else {
             if (ch == NCH * h + 1 && st >= 2) mbar_wait(&a_free[pp], ((st >> 1) - 1) & 1, &err, 13);
             const int gi = ch >> 1;                       // which 32 columns of the step
             const uint32_t byte0 = (uint32_t)(pp * 64 + gi * 32);
             uint32_t w[8];
-            if constexpr (kDkdv) {
+            if constexpr (kP) {
               const uint32_t sb8 = pack_group32_mx8(pkeep, pf, w);
               sts_v4(a1_s + sw128_offset(row_in, byte0), w[0], w[1], w[2], w[3]);
               sts_v4(a1_s + sw128_offset(row_in, byte0 + 16), w[4], w[5], w[6], w[7]);
-              sts_b8(asf_s + pp * 512 + sf_atom_offset(row_in, gi), sb8);
+              sts_b8(asf1_s + pp * 512 + sf_atom_offset(row_in, gi), sb8);
             }
-            const uint32_t sd8 = pack_group32_mx8(dkeep, ds, w);
-            sts_v4(a2_s + sw128_offset(row_in, byte0), w[0], w[1], w[2], w[3]);
-            sts_v4(a2_s + sw128_offset(row_in, byte0 + 16), w[4], w[5], w[6], w[7]);
-            sts_b8(asf_s + (2 + pp) * 512 + sf_atom_offset(row_in, gi), sd8);
+            if constexpr (kDs) {
+              const uint32_t sd8 = pack_group32_mx8(dkeep, ds, w);
+              sts_v4(a2_s + sw128_offset(row_in, byte0), w[0], w[1], w[2], w[3]);
+              sts_v4(a2_s + sw128_offset(row_in, byte0 + 16), w[4], w[5], w[6], w[7]);
+              sts_b8(asf2_s + pp * 512 + sf_atom_offset(row_in, gi), sd8);
+            }
           }
         } else {
         // random-bit counters: (tensor, row of the CTA's unit) and the quad's column within the unit
         if constexpr (kSr) {
-          const uint32_t sr_row = (uint32_t)((int64_t)rb * R + row) * 4u + (kDkdv ? 0u : 2u);
+          const uint32_t sr_row = (uint32_t)((int64_t)rb * R + row) * 4u + (kKeys ? 0u : 2u);
           const uint32_t sr_col = (uint32_t)(st * 16 + ch * 4);
-          if constexpr (kDkdv)
+          if constexpr (kP)
             scp |= b4_pack16<false>(pf, wp[2 * (ch & 1)], wp[2 * (ch & 1) + 1], p.sr_p != 0, p.seed, sr_row + 1u, sr_col)
                    << (8 * (ch & 1));
-          scd |= b4_pack16<true>(ds, wd[2 * (ch & 1)], wd[2 * (ch & 1) + 1], p.sr_ds != 0, p.seed, sr_row, sr_col)
-                 << (8 * (ch & 1));
+          if constexpr (kDs)
+            scd |= b4_pack16<true>(ds, wd[2 * (ch & 1)], wd[2 * (ch & 1) + 1], p.sr_ds != 0, p.seed, sr_row, sr_col)
+                   << (8 * (ch & 1));
         } else {
-          if constexpr (kDkdv) scp |= b4_pack16<false>(pf, wp[2 * (ch & 1)], wp[2 * (ch & 1) + 1]) << (8 * (ch & 1));
-          scd |= b4_pack16<true>(ds, wd[2 * (ch & 1)], wd[2 * (ch & 1) + 1]) << (8 * (ch & 1));
+          if constexpr (kP) scp |= b4_pack16<false>(pf, wp[2 * (ch & 1)], wp[2 * (ch & 1) + 1]) << (8 * (ch & 1));
+          if constexpr (kDs) scd |= b4_pack16<true>(ds, wd[2 * (ch & 1)], wd[2 * (ch & 1) + 1]) << (8 * (ch & 1));
         }
         if (ch & 1) {
           // the operand tiles of step st - 2 (same half of the rows' bytes) must have been consumed
           if (ch == NCH * h + 1 && st >= 2) mbar_wait(&a_free[pp], ((st >> 1) - 1) & 1, &err, 13);
           const int c2i = ch >> 1;      // which 32 columns of the step
-          if constexpr (kDkdv) {
+          if constexpr (kP) {
             sts_v4(a1_s + sw64_offset(row_in, pp * 32 + c2i * 16), wp[0], wp[1], wp[2], wp[3]);
-            sts_b16(asf_s + pp * 512 + sf_atom_offset(row_in, c2i * 2), scp);
+            sts_b16(asf1_s + pp * 512 + sf_atom_offset(row_in, c2i * 2), scp);
             scp = 0u;
           }
-          sts_v4(a2_s + sw64_offset(row_in, pp * 32 + c2i * 16), wd[0], wd[1], wd[2], wd[3]);
-          sts_b16(asf_s + (2 + pp) * 512 + sf_atom_offset(row_in, c2i * 2), scd);
-          scd = 0u;
+          if constexpr (kDs) {
+            sts_v4(a2_s + sw64_offset(row_in, pp * 32 + c2i * 16), wd[0], wd[1], wd[2], wd[3]);
+            sts_b16(asf2_s + pp * 512 + sf_atom_offset(row_in, c2i * 2), scd);
+            scd = 0u;
+          }
         }
         }
       };
-      if constexpr (NP == 1) {
-        // dP (or dP^T): all 64 columns at once, so the single slot goes back to the issuer right away;
-        // S in 16-column chunks, the next one in flight while the current one is worked on
-        uint32_t g0[32], g1[32], sa[16], sb[16];
-        tmem_ld32(tmem + lane_addr + C::T_G, g0);
-        tmem_ld32(tmem + lane_addr + C::T_G + 32, g1);
-        tmem_ld16(tmem + lane_addr + C::T_S + pp * 64, sa);
+      // this thread's 32 columns of dP (or dP^T) arrive with the first S chunk, so the single dP slot
+      // goes back to the issuer after one round trip; the S slot follows with the second chunk
+      uint32_t gq[kDs ? 32 : 1];
+      if constexpr (kDs) tmem_ld32(tmem + lane_addr + C::T_G + 32 * h, gq);
+#pragma unroll
+      for (int cc = 0; cc < NCH; ++cc) {
+        const int ch = NCH * h + cc;
+        uint32_t cur[16];
+        tmem_ld16(tmem + lane_addr + C::T_S + pp * 64 + 16 * ch, cur);
         tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&g_free);
-#pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-          if (ch < 3) {
-            if (ch & 1) tmem_ld16(tmem + lane_addr + C::T_S + pp * 64 + 16 * (ch + 1), sa);
-            else tmem_ld16(tmem + lane_addr + C::T_S + pp * 64 + 16 * (ch + 1), sb);
-          }
-          chunk(ch, (ch & 1) ? sb : sa, ch < 2 ? g0 + 16 * ch : g1 + 16 * (ch - 2));
-          if (ch < 3) {
-            tmem_ld_wait();
-            if (ch == 2) {          // the last chunk of S is in registers: the slot goes back
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&s_free[pp]);
-            }
+        if (cc == 0 || cc == NCH - 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            if (kDs && cc == 0) mbar_arrive(&g_free);
+            if (cc == NCH - 1) mbar_arrive(&s_free[pp]);
           }
         }
-      } else {
-        // this thread's 32 columns of dP (or dP^T) arrive with the first S chunk, so the single dP slot
-        // goes back to the issuer after one round trip; the S slot follows with the second chunk
-        uint32_t gq[32];
-        tmem_ld32(tmem + lane_addr + C::T_G + 32 * h, gq);
-#pragma unroll
-        for (int cc = 0; cc < NCH; ++cc) {
-          const int ch = NCH * h + cc;
-          uint32_t cur[16];
-          tmem_ld16(tmem + lane_addr + C::T_S + pp * 64 + 16 * ch, cur);
-          tmem_ld_wait();
-          if (cc == 0 || cc == NCH - 1) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-              if (cc == 0) mbar_arrive(&g_free);
-              if (cc == NCH - 1) mbar_arrive(&s_free[pp]);
-            }
-          }
-          chunk(ch, cur, gq + 16 * cc);
-        }
+        chunk(ch, cur, kDs ? gq + 16 * cc : gq);
       }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&a_full[pp]);
     }
-    // ---- epilogue: thread `part` of a row writes gradient columns [EC part, EC part + EC), EC = 64 / NP,
-    // of this CTA's 128-wide half
+    // ---- epilogue: thread `part` of a row writes gradient columns [EC part, EC part + EC)
     const float m1 = gs * 4.8828125e-4f;       // 2^-11
     const float m2 = gs * 1.953125e-3f;        // 2^-9
-    TG* o1 = nullptr;
-    constexpr int EC = 64 / NP;
-    TG* o2 = static_cast<TG*>(p.out2) + ((int64_t)rb * R + row) * D + half * 128 + part * EC;
-    if constexpr (kDkdv) o1 = static_cast<TG*>(p.out1) + ((int64_t)rb * R + row) * D + half * 128 + part * EC;
+    constexpr int EC = D / (2 * NP);
+    TG* o1 = kP ? static_cast<TG*>(p.out1) + ((int64_t)rb * R + row) * D + part * EC : nullptr;
+    TG* o2 = kDs ? static_cast<TG*>(p.out2) + ((int64_t)rb * R + row) * D + part * EC : nullptr;
     if (nstep > 0) {
       mbar_wait(&acc_done, 0, &err, 14);
       tc_fence_after();
 #pragma unroll
       for (int c = 0; c < EC / 32; ++c) {
         uint32_t r[32];
-        if constexpr (kDkdv) {
+        if constexpr (kP) {
           tmem_ld32(tmem + lane_addr + C::T_ACC1 + part * EC + c * 32, r);
           tmem_ld_wait();
           if (row_ok) store_row32<TG>(o1 + c * 32, r, m1);
         }
-        tmem_ld32(tmem + lane_addr + C::T_ACC2 + part * EC + c * 32, r);
-        tmem_ld_wait();
-        if (row_ok) store_row32<TG>(o2 + c * 32, r, m2);
+        if constexpr (kDs) {
+          tmem_ld32(tmem + lane_addr + C::T_ACC2 + part * EC + c * 32, r);
+          tmem_ld_wait();
+          if (row_ok) store_row32<TG>(o2 + c * 32, r, m2);
+        }
       }
       tc_fence_before();
     } else if (row_ok) {
-      if constexpr (kDkdv) zero_row(o1, EC);
-      zero_row(o2, EC);
+      if constexpr (kP) zero_row(o1, EC);
+      if constexpr (kDs) zero_row(o2, EC);
     }
   }
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && err != 0 && p.status != nullptr) atomicExch(p.status, err);
   if (warp == 1) tmem_dealloc(tmem, 512);
+  if (p.late_wait) griddep_wait();
 }
 
 }  // namespace nvfp4
@@ -816,47 +803,64 @@ extern "C" int nvfp4_bwd_fp4(const uint8_t* qnv, const uint8_t* qsc, const uint8
   p.h = (int)h; p.hk = (int)hk; p.g = (int)(h / hk); p.s_q = (int)s_q; p.s_kv = (int)s_kv;
   p.scaling = scaling; p.causal = (flags & NVFP4_FWD_CAUSAL) ? 1 : 0; p.status = status;
   p.seed = seed; p.sr_p = 0; p.sr_ds = 0;
-  const unsigned halves = (unsigned)(d / 128);
-  auto launch = [&](auto kdkdv, auto kdq, int smem, int threads) -> int {
-    if (int r0 = allow_smem("nvfp4_bwd_fp4", reinterpret_cast<const void*>(kdkdv), smem)) return r0;
-    if (int r0 = allow_smem("nvfp4_bwd_fp4", reinterpret_cast<const void*>(kdq), smem)) return r0;
-    // dK / dV: rows = keys (K, V packs), columns = queries (Q, dO' packs; dO'^T, Q^T transposed packs)
+  p.late_wait = 0;
+  // The passes are independent of one another: the first waits for the work before it, the later ones
+  // start filling the SMs that its last CTAs leave and wait for it only at their end.
+  bool first = true;
+  auto launch_pass = [&](const char* what, auto kern, int smem, int threads, bool keys) -> int {
+    if (int r0 = allow_smem(what, reinterpret_cast<const void*>(kern), smem)) return r0;
     B4Params a = p;
-    a.x1sc = ksc; a.x2sc = vdsc; a.y1sc = qsc; a.y2sc = dosc; a.t1sc = dotsc; a.t2sc = qtsc;
-    a.out1 = dv; a.out2 = dk; a.c_pad = (int)sq_pad;
-    a.sr_p = (flags & NVFP4_BWD_SR_P_DV) ? 1 : 0; a.sr_ds = (flags & NVFP4_BWD_SR_DS_DK) ? 1 : 0;
-    dim3 g1((unsigned)zhk, (unsigned)((s_kv + 127) / 128), halves);
-    if (int r1 = nvfp4::launch("nvfp4_bwd_fp4(dkdv)", kdkdv, g1, threads, smem, st, t_k, t_vd, t_q, t_do, t_dot, t_qt, a))
-      return r1;
+    a.late_wait = first ? 0 : 1;
+    first = false;
+    if (keys) {   // dV / dK: rows = keys (K, V packs), columns = queries (Q, dO' packs; dO'^T, Q^T transposed packs)
+      a.x1sc = ksc; a.x2sc = vdsc; a.y1sc = qsc; a.y2sc = dosc; a.t1sc = dotsc; a.t2sc = qtsc;
+      a.out1 = dv; a.out2 = dk; a.c_pad = (int)sq_pad;
+      a.sr_p = (flags & NVFP4_BWD_SR_P_DV) ? 1 : 0; a.sr_ds = (flags & NVFP4_BWD_SR_DS_DK) ? 1 : 0;
+      return launch(what, kern, dim3((unsigned)zhk, (unsigned)((s_kv + 127) / 128)), threads, smem, st, t_k, t_vd, t_q, t_do,
+                    t_dot, t_qt, a);
+    }
     // dQ: rows = queries (Q, dO' packs), columns = keys (K, V packs; K^T transposed pack)
-    B4Params b = p;
-    b.x1sc = qsc; b.x2sc = dosc; b.y1sc = ksc; b.y2sc = vdsc; b.t1sc = nullptr; b.t2sc = ktsc;
-    b.out1 = nullptr; b.out2 = dq; b.c_pad = (int)skv_pad;
-    b.sr_ds = (flags & NVFP4_BWD_SR_DS_DQ) ? 1 : 0;
-    dim3 g2((unsigned)zh, (unsigned)((s_q + 127) / 128), halves);
-    return nvfp4::launch("nvfp4_bwd_fp4(dq)", kdq, g2, threads, smem, st, t_q, t_do, t_k, t_vd, t_kt, t_kt, b);
+    a.x1sc = qsc; a.x2sc = dosc; a.y1sc = ksc; a.y2sc = vdsc; a.t1sc = nullptr; a.t2sc = ktsc;
+    a.out1 = nullptr; a.out2 = dq; a.c_pad = (int)skv_pad;
+    a.sr_ds = (flags & NVFP4_BWD_SR_DS_DQ) ? 1 : 0;
+    return launch(what, kern, dim3((unsigned)zh, (unsigned)((s_q + 127) / 128)), threads, smem, st, t_q, t_do, t_k, t_vd,
+                  t_kt, t_kt, a);
   };
   const bool any_sr = (flags & (NVFP4_BWD_SR_DS_DK | NVFP4_BWD_SR_P_DV | NVFP4_BWD_SR_DS_DQ)) != 0;
-#define NVFP4_B4_LAUNCH(DD, TT)                                                                                   \
-  (fp8      ? launch(bwd4_kernel<DD, true, TT, 2>, bwd4_kernel<DD, false, TT, 2>, B4Cfg<DD, true>::TOTAL,         \
-                     B4Cfg<DD, true>::THREADS)                                                                    \
-   : any_sr ? launch(bwd4_kernel<DD, true, TT, 1>, bwd4_kernel<DD, false, TT, 1>, B4Cfg<DD, false>::TOTAL,        \
-                     B4Cfg<DD, false>::THREADS)                                                                   \
-            : launch(bwd4_kernel<DD, true, TT, 0>, bwd4_kernel<DD, false, TT, 0>, B4Cfg<DD, false>::TOTAL,        \
-                     B4Cfg<DD, false>::THREADS))
+#define NVFP4_B4_PASS(DD, PASS, TT, MODE)                                                                     \
+  launch_pass("nvfp4_bwd_fp4(" #PASS ")", bwd4_kernel<DD, PASS, TT, MODE>, B4Cfg<DD, PASS, MODE == 2>::TOTAL,  \
+              B4Cfg<DD, PASS, MODE == 2>::THREADS, PASS != kB4Dq)
+#define NVFP4_B4_MODE(DD, TT, MODE)                                        \
+  {                                                                        \
+    if constexpr (DD == 128) {                                             \
+      if ((rc = NVFP4_B4_PASS(128, kB4DkDv, TT, MODE))) return rc;         \
+    } else {                                                               \
+      if ((rc = NVFP4_B4_PASS(256, kB4Dk, TT, MODE))) return rc;           \
+      if ((rc = NVFP4_B4_PASS(256, kB4Dv, TT, MODE))) return rc;           \
+    }                                                                      \
+    return NVFP4_B4_PASS(DD, kB4Dq, TT, MODE);                             \
+  }
+#define NVFP4_B4_LAUNCH(DD, TT)          \
+  {                                      \
+    if (fp8) NVFP4_B4_MODE(DD, TT, 2)    \
+    if (any_sr) NVFP4_B4_MODE(DD, TT, 1) \
+    NVFP4_B4_MODE(DD, TT, 0)             \
+  }
   if (d == 128) {
     switch (grad_dtype) {
-      case NVFP4_DT_BF16: return NVFP4_B4_LAUNCH(128, __nv_bfloat16);
-      case NVFP4_DT_FP16: return NVFP4_B4_LAUNCH(128, __half);
-      case NVFP4_DT_FP32: return NVFP4_B4_LAUNCH(128, float);
+      case NVFP4_DT_BF16: NVFP4_B4_LAUNCH(128, __nv_bfloat16)
+      case NVFP4_DT_FP16: NVFP4_B4_LAUNCH(128, __half);
+      case NVFP4_DT_FP32: NVFP4_B4_LAUNCH(128, float);
       default: return fail(-1, "nvfp4_bwd_fp4: unknown grad dtype %d", grad_dtype);
     }
   }
   switch (grad_dtype) {
-    case NVFP4_DT_BF16: return NVFP4_B4_LAUNCH(256, __nv_bfloat16);
-    case NVFP4_DT_FP16: return NVFP4_B4_LAUNCH(256, __half);
-    case NVFP4_DT_FP32: return NVFP4_B4_LAUNCH(256, float);
+    case NVFP4_DT_BF16: NVFP4_B4_LAUNCH(256, __nv_bfloat16);
+    case NVFP4_DT_FP16: NVFP4_B4_LAUNCH(256, __half);
+    case NVFP4_DT_FP32: NVFP4_B4_LAUNCH(256, float);
     default: return fail(-1, "nvfp4_bwd_fp4: unknown grad dtype %d", grad_dtype);
   }
 #undef NVFP4_B4_LAUNCH
+#undef NVFP4_B4_MODE
+#undef NVFP4_B4_PASS
 }
