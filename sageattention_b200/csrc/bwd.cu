@@ -15,12 +15,17 @@
 // tiles; the same tile serves as a K-major operand (contraction along D) and as an MN-major
 // operand (contraction along the rows), so no transposed copies exist anywhere.
 //
-// Pipeline of one CTA (384 threads): warp 0 TMA producer, warp 1 MMA issuer, warp 2 scale-atom /
-// row-statistics loader, warps 4-7 and 8-11 two softmax groups that alternate steps.  S has two
-// TMEM slots, dP one (a group pulls it into registers and hands the slot back at once); P^T / dS^T
-// are written back as bf16 pairs into the S slot they were computed from and enter the gradient
+// Pipeline of one CTA (640 threads): warp 0 TMA producer, warp 1 MMA issuer, warp 2 scale-atom /
+// row-statistics loader, warps 4-11 and 12-19 two softmax teams that alternate steps, two threads per
+// row.  S has two TMEM slots, dP one (a team pulls it into registers and hands the slot back at once);
+// P^T / dS^T are written back as bf16 pairs into the S slot they were computed from and enter the gradient
 // GEMMs as TMEM A operands, so the probabilities never touch shared memory and the tensor pipe
-// works on step t+1 while a group is still busy with step t.  Causal masking is bottom-right
+// works on step t+1 while a team is still busy with step t.  (One team of eight warps that took every step:
+// S8192 H32 Hk8 1629 -> 1554 us for pre-pass, dK/dV and dQ.)
+// Where the key tiles are too few or too unequal to fill the chip, the steps of a tile are dealt to the
+// CTAs of a cluster and their accumulators added over distributed shared memory: S1024 H16 Hk4 101 -> 58
+// us, S3805 372 -> 265 us.  dQ does not depend on dK / dV and starts while their last CTAs run.
+// Causal masking is bottom-right
 // aligned; packed varlen is block-diagonal, expressed as a per-row visible range.  Head dim 128,
 // or 256 as two 128-wide output halves per tile (both halves recompute S and dP).  Every barrier
 // wait is bounded.
@@ -33,7 +38,7 @@
 
 namespace nvfp4 {
 
-constexpr int kBwdThreads = 384;
+constexpr int kBwdThreads = 640;
 constexpr float kBwdLog2e = 1.4426950408889634f;
 constexpr int kBwdPrefetch = 8;   // stage loads are prefetched into L2 this many steps ahead
 
@@ -186,22 +191,24 @@ struct BwdParams {
   int s_q, s_kv;
   float scaling;
   int causal;
+  int split;            // CTAs (of one cluster) that share a tile's steps
+  int late_wait;        // independent of the kernel before it: wait for it at the end, not at the start
   int* status;
 };
 
-// P for 32 columns of one accumulator row: exp2(s * c2 + offsets).  Per-column statistics (the
-// dK/dV kernel): `nl` points at the raw lse of the 32 columns in shared memory and `nl_row` is a
+// P for 16 columns of one accumulator row: exp2(s * c2 + offsets).  Per-column statistics (the
+// dK/dV kernel): `nl` points at the raw lse of the 16 columns in shared memory and `nl_row` is a
 // per-thread offset (the key's bias * log2e, or 0).  Per-row (the dQ kernel): `nl_row` is
-// -lse*log2e of the row and `nl`, when not null, points at the raw key bias of the 32 columns.
+// -lse*log2e of the row and `nl`, when not null, points at the raw key bias of the 16 columns.
 // Columns outside [lo, hi) relative to the chunk's first column are masked when `masked`.
 template <bool kPerColumn, bool kColumnBias = false>
-__device__ __forceinline__ void prob_chunk(const uint32_t (&sr)[32], float (&pf)[32], float c2, const float* nl,
+__device__ __forceinline__ void prob_chunk(const uint32_t* sr, float (&pf)[16], float c2, const float* nl,
                                            float nl_row, bool masked, int lo, int hi) {
   const float2 c22 = make_float2(c2, c2);
   const float2 row2 = make_float2(nl_row, nl_row);
   const float2 ml2 = make_float2(kPerColumn ? -kBwdLog2e : kBwdLog2e, kPerColumn ? -kBwdLog2e : kBwdLog2e);
 #pragma unroll
-  for (int e = 0; e < 32; e += 4) {
+  for (int e = 0; e < 16; e += 4) {
     float2 n01 = row2, n23 = row2;
     if constexpr (kPerColumn || kColumnBias) {
       const float4 l4 = *reinterpret_cast<const float4*>(nl + e);
@@ -217,16 +224,16 @@ __device__ __forceinline__ void prob_chunk(const uint32_t (&sr)[32], float (&pf)
   }
   if (masked) {
 #pragma unroll
-    for (int e = 0; e < 32; ++e) pf[e] = (e >= lo && e < hi) ? pf[e] : 0.0f;
+    for (int e = 0; e < 16; ++e) pf[e] = (e >= lo && e < hi) ? pf[e] : 0.0f;
   }
 }
-// dS = P o (dP - delta) for 32 columns, packed to bf16 pairs.  Per-column: `nd` points at the raw
+// dS = P o (dP - delta) for 16 columns, packed to bf16 pairs.  Per-column: `nd` points at the raw
 // delta values; per-row: `nd_row` is -delta.
 template <bool kPerColumn>
-__device__ __forceinline__ void ds_chunk(const float (&pf)[32], const uint32_t (&dr)[32], uint32_t (&dw)[16],
+__device__ __forceinline__ void ds_chunk(const float (&pf)[16], const uint32_t* dr, uint32_t (&dw)[8],
                                          const float* nd, float nd_row) {
 #pragma unroll
-  for (int e = 0; e < 32; e += 4) {
+  for (int e = 0; e < 16; e += 4) {
     float2 a0, a1;
     const float2 d01 = make_float2(__uint_as_float(dr[e]), __uint_as_float(dr[e + 1]));
     const float2 d23 = make_float2(__uint_as_float(dr[e + 2]), __uint_as_float(dr[e + 3]));
@@ -273,7 +280,19 @@ struct DkdvSmem {
   static_assert(STAGE % 1024 == 0 && (V + KP) % 1024 == 0, "128-byte-swizzled tiles need 1 KB alignment");
 };
 
-template <int D, typename TG>
+// position in the step list of a key tile: query head of the group, 64-query step
+struct StepCursor {
+  int gq, i;
+  __device__ __forceinline__ StepCursor(int st, int n_i) : gq(n_i > 0 ? st / n_i : 0), i(n_i > 0 ? st - gq * n_i : 0) {}
+  __device__ __forceinline__ void next(int n_i) {
+    if (++i == n_i) {
+      i = 0;
+      ++gq;
+    }
+  }
+};
+
+template <int D, typename TG, bool kSplit>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant__ CUtensorMap tm_qp,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -295,7 +314,9 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int jt = blockIdx.y;           // key tile (low tiles have the most visible queries: first)
   const int unit = blockIdx.x;         // z * hk + kh
-  const int half = blockIdx.z;         // 128-wide slice of the head dim owned by this CTA
+  const int split = kSplit ? p.split : 1;   // CTAs (of one cluster) that share the tile's steps
+  const int half = blockIdx.z / split;      // 128-wide slice of the head dim owned by this CTA
+  const int rank = kSplit ? blockIdx.z % split : 0;
   const int zi = unit / p.hk, kh = unit % p.hk;
   const int n0 = jt * 128;
   const int shift = p.s_kv - p.s_q;
@@ -329,7 +350,8 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
   }
   const int i_lo = q_lo / 64, i_hi = (q_hi + 63) / 64;
   const int n_i = max(i_hi - i_lo, 0);
-  const int nstep = n_i * p.g;
+  const int st0 = n_i * p.g * rank / split;
+  const int nstep = n_i * p.g * (rank + 1) / split - st0;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -349,9 +371,8 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
       for (int c = 0; c < L::DS; ++c) tma_load_3d(s_v + c * 16384, &tm_v, &kv_full, c * 64, n0, unit);
       // L2 prefetch kBwdPrefetch steps ahead: co-resident CTAs walk the same query tiles in step,
       // so without it every stage load is a first touch that waits on HBM
-      auto prefetch = [&](int t) {
-        const int gq = t / n_i, i = i_lo + t % n_i;
-        const int zh = zi * p.h + kh * p.g + gq;
+      auto prefetch = [&](const StepCursor& c0) {
+        const int i = i_lo + c0.i, zh = zi * p.h + kh * p.g + c0.gq;
 #pragma unroll
         for (int c = 0; c < L::KSUB; ++c) tma_prefetch_3d(&tm_qp, c * 64, i * 64, zh);
 #pragma unroll
@@ -359,12 +380,16 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
         tma_prefetch_3d(&tm_q, half * 128, i * 64, zh);
         tma_prefetch_3d(&tm_q, half * 128 + 64, i * 64, zh);
       };
-      for (int t = L::NSTAGE; t < min(nstep, kBwdPrefetch); ++t) prefetch(t);
-      for (int st = 0; st < nstep; ++st) {
+      StepCursor cur(st0, n_i), ahead(st0 + L::NSTAGE, n_i);
+      for (int t = L::NSTAGE; t < min(nstep, kBwdPrefetch); ++t, ahead.next(n_i)) prefetch(ahead);
+      for (int st = 0; st < nstep; ++st, cur.next(n_i)) {
         const int s = st % L::NSTAGE;
-        const int gq = st / n_i, i = i_lo + st % n_i;
-        const int zh = zi * p.h + kh * p.g + gq;
-        if (st + kBwdPrefetch < nstep) prefetch(st + kBwdPrefetch);
+        const int i = i_lo + cur.i;
+        const int zh = zi * p.h + kh * p.g + cur.gq;
+        if (st + kBwdPrefetch < nstep) {
+          prefetch(ahead);
+          ahead.next(n_i);
+        }
         if (st >= L::NSTAGE) mbar_wait(&empty[s], ((st / L::NSTAGE) & 1) ^ 1, &err, 1);
         uint8_t* sb = s_stage + s * L::STAGE;
         mbar_expect_tx(&full_tma[s], L::QP + L::DO + L::Q);
@@ -397,10 +422,11 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&ksf_full);
-      for (int st = 0; st < nstep; ++st) {
+      StepCursor cur(st0, n_i);
+      for (int st = 0; st < nstep; ++st, cur.next(n_i)) {
         const int s = st % L::NSTAGE;
-        const int gq = st / n_i, i = i_lo + st % n_i;
-        const int zh = zi * p.h + kh * p.g + gq;
+        const int i = i_lo + cur.i;
+        const int zh = zi * p.h + kh * p.g + cur.gq;
         if (st >= L::NSTAGE) mbar_wait(&empty[s], ((st / L::NSTAGE) & 1) ^ 1, &err, 2);
         uint8_t* sb = s_stage + s * L::STAGE;
         const uint32_t qsf = smem_u32(sb + L::O_QSF);
@@ -498,7 +524,9 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
     __syncwarp();
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ softmax groups, epilogue
-    const int grp = (warp - 4) >> 2;
+    const int team = (warp - 4) >> 3;   // steps of this parity
+    const int grp = ((warp - 4) >> 2) & 1;
+    const int part = team * 2 + grp;    // 32-column slice of the gradients this thread stores
     const int wq = warp & 3;
     const int row = wq * 32 + lane;     // key within the tile
     const int key = n0 + row;
@@ -517,16 +545,18 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
       }
       qh = max(qh, ql);
     }
-    // both groups work on every step: group g owns queries [32g, 32g+32) of the 64-query tile
-    for (int st = 0; st < nstep; ++st) {
-      const int s = st % L::NSTAGE, b = st & 1, k2 = st >> 1;
-      const int q0 = (i_lo + st % n_i) * 64 + grp * 32;
-      uint8_t* sb = s_stage + s * L::STAGE;
-      const float* aux = reinterpret_cast<const float*>(sb + L::O_AUX) + grp * 32;
-      const uint32_t slot = tmem + lane_addr + T_ST + b * 64 + grp * 32;
+    // the teams alternate steps; thread g of a row owns queries [32g, 32g+32) of the 64-query tile
+    StepCursor cur(st0 + team, n_i);
+    for (int st = team; st < nstep; st += 2) {
+      const int s = st % L::NSTAGE, k2 = st >> 1;
+      const int q0 = (i_lo + cur.i) * 64 + grp * 32;
+      cur.next(n_i);
+      cur.next(n_i);
+      const float* aux = reinterpret_cast<const float*>(s_stage + s * L::STAGE + L::O_AUX) + grp * 32;
+      const uint32_t slot = tmem + lane_addr + T_ST + team * 64 + grp * 32;
       const bool masked = !__all_sync(0xffffffffu, q0 >= ql && q0 + 32 <= qh);
       mbar_wait(&full_aux[s], (st / L::NSTAGE) & 1, &err, 10);
-      mbar_wait(&s_full[b], k2 & 1, &err, 11);
+      mbar_wait(&s_full[team], k2 & 1, &err, 11);
       mbar_wait(&dp_full, st & 1, &err, 13);
       tc_fence_after();
       // dP^T first: the single dP^T slot goes back to the issuer before any arithmetic
@@ -538,42 +568,57 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
       __syncwarp();
       if (lane == 0) mbar_arrive(&dp_free);
       // P^T -> 16 columns, dS^T -> the next 16, over the S^T columns just read
-      {
-        float pf[32];
-        uint32_t w[16];
-        prob_chunk<true>(sr, pf, c2, aux, bk2, masked, ql - q0, qh - q0);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) w[e] = pack_bf16x2(pf[2 * e], pf[2 * e + 1]);
-        tmem_st16(slot, w);
-        ds_chunk<true>(pf, dr, w, aux + 64, 0.0f);
-        tmem_st16(slot + 16, w);
+      for (int c = 0; c < 2; ++c) {
+        float pf[16];
+        uint32_t w[8];
+        prob_chunk<true>(sr + 16 * c, pf, c2, aux + 16 * c, bk2, masked, ql - q0 - 16 * c, qh - q0 - 16 * c);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[e] = pack_bf16x2(pf[2 * e], pf[2 * e + 1]);
+        tmem_st8(slot + 8 * c, w);
+        ds_chunk<true>(pf, dr + 16 * c, w, aux + 64 + 16 * c, 0.0f);
+        tmem_st8(slot + 16 + 8 * c, w);
       }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&pds_full[b]);
+      if (lane == 0) mbar_arrive(&pds_full[team]);
     }
-    // ---- epilogue: group g writes gradient columns [64g, 64g+64)
-    TG* dkrow = static_cast<TG*>(p.dk) + ((int64_t)unit * p.s_kv + key) * D + half * 128 + grp * 64;
-    TG* dvrow = static_cast<TG*>(p.dv) + ((int64_t)unit * p.s_kv + key) * D + half * 128 + grp * 64;
+    // ---- epilogue: thread `part` of a row writes gradient columns [32 part, 32 part + 32)
+    TG* dkrow = static_cast<TG*>(p.dk) + ((int64_t)unit * p.s_kv + key) * D + half * 128 + part * 32;
+    TG* dvrow = static_cast<TG*>(p.dv) + ((int64_t)unit * p.s_kv + key) * D + half * 128 + part * 32;
+    const uint32_t red = smem_u32(smem);      // the operand tiles are idle once the accumulators are complete
     if (nstep > 0) {
       mbar_wait(&acc_done, 0, &err, 14);
       tc_fence_after();
+    }
+    if (nstep > 0 || kSplit) {
+      uint32_t r[32];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t r[32];
-        tmem_ld32(tmem + lane_addr + T_DV + grp * 64 + c * 32, r);
-        tmem_ld_wait();
-        if (key < p.s_kv) store_row32<TG>(dvrow + c * 32, r, 1.0f);
-        tmem_ld32(tmem + lane_addr + T_DK + grp * 64 + c * 32, r);
-        tmem_ld_wait();
-        if (key < p.s_kv) store_row32<TG>(dkrow + c * 32, r, p.scaling);
+      for (int o = 0; o < 2; ++o) {         // dV, dK
+        if (nstep > 0) {
+          tmem_ld32(tmem + lane_addr + (o ? T_DK : T_DV) + part * 32, r);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) r[e] = 0u;
+        }
+        if (kSplit) red_store32(red, row, o * 128 + part * 32, r);
+        else if (key < p.s_kv) store_row32<TG>(o ? dkrow : dvrow, r, o ? p.scaling : 1.0f);
       }
       tc_fence_before();
     } else if (key < p.s_kv) {
-      zero_row(dkrow, 64);
-      zero_row(dvrow, 64);
+      zero_row(dkrow, 32);
+      zero_row(dvrow, 32);
     }
+  }
+  if (kSplit) {
+    __syncwarp();
+    cluster_sync_all();
+    TG* base_k = static_cast<TG*>(p.dk) + ((int64_t)unit * p.s_kv + n0) * D + half * 128;
+    TG* base_v = static_cast<TG*>(p.dv) + ((int64_t)unit * p.s_kv + n0) * D + half * 128;
+    red_sum_store<TG>(smem_u32(smem), rank, split, tid, kBwdThreads, p.s_kv - n0, base_v, base_k, D, 1.0f, p.scaling);
+    cluster_sync_all();
   }
   tc_fence_before();
   __syncthreads();
@@ -651,7 +696,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&tmem_base_s, 512);
-  griddep_wait();
+  if (!p.late_wait) griddep_wait();
   int k_lo = 0, k_hi = p.s_kv;
   if (p.causal) k_hi = max(0, min(p.s_kv, m0 + 128 + shift));
   if (varlen) {
@@ -803,7 +848,9 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
     }
     __syncwarp();
   } else if (warp >= 4) {
-    const int grp = (warp - 4) >> 2;
+    const int team = (warp - 4) >> 3;   // steps of this parity
+    const int grp = ((warp - 4) >> 2) & 1;
+    const int part = team * 2 + grp;    // 32-column slice of dQ this thread stores
     const int wq = warp & 3;
     const int row_in = wq * 32 + lane;
     const int row = m0 + row_in;
@@ -822,11 +869,11 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
       }
       kh = max(kh, kl);
     }
-    // both groups work on every step: group g owns keys [32g, 32g+32) of the 64-key tile
-    for (int st = 0; st < nstep; ++st) {
-      const int b = st & 1, k2 = st >> 1;
+    // the teams alternate steps; thread g of a row owns keys [32g, 32g+32) of the 64-key tile
+    for (int st = team; st < nstep; st += 2) {
+      const int k2 = st >> 1;
       const int key0 = (j_lo + st) * 64 + grp * 32;
-      const uint32_t slot = tmem + lane_addr + T_S + b * 64;
+      const uint32_t slot = tmem + lane_addr + T_S + team * 64 + grp * 32;
       const bool masked = !__all_sync(0xffffffffu, key0 >= kl && key0 + 32 <= kh);
       const float* kbias = nullptr;
       if (p.bias != nullptr) {      // the stage's key bias (landed with the scale atoms)
@@ -834,50 +881,49 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
         mbar_wait(&full_sf[sg], (st / L::NSTAGE) & 1, &err, 10);
         kbias = reinterpret_cast<const float*>(s_stage + sg * L::STAGE + L::O_AUX) + grp * 32;
       }
-      mbar_wait(&s_full[b], k2 & 1, &err, 11);
+      mbar_wait(&s_full[team], k2 & 1, &err, 11);
       mbar_wait(&dp_full, st & 1, &err, 13);
       tc_fence_after();
       uint32_t dr[32], sr[32];
       tmem_ld32(tmem + lane_addr + T_DP + grp * 32, dr);
-      tmem_ld32(slot + grp * 32, sr);
+      tmem_ld32(slot, sr);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&dp_free);
-      {
-        float pf[32];
-        uint32_t w[16];
-        if (kbias != nullptr) prob_chunk<false, true>(sr, pf, c2, kbias, nl, masked, kl - key0, kh - key0);
-        else prob_chunk<false, false>(sr, pf, c2, nullptr, nl, masked, kl - key0, kh - key0);
-        ds_chunk<false>(pf, dr, w, nullptr, nd);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        float pf[16];
+        uint32_t w[8];
+        if (kbias != nullptr) prob_chunk<false, true>(sr + 16 * c, pf, c2, kbias + 16 * c, nl, masked, kl - key0 - 16 * c, kh - key0 - 16 * c);
+        else prob_chunk<false, false>(sr + 16 * c, pf, c2, nullptr, nl, masked, kl - key0 - 16 * c, kh - key0 - 16 * c);
+        ds_chunk<false>(pf, dr + 16 * c, w, nullptr, nd);
         // dS of keys [32g, 32g+32) replaces the first 16 of the S columns this thread just read
-        tmem_st16(slot + grp * 32, w);
+        tmem_st8(slot + 8 * c, w);
       }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ds_full[b]);
+      if (lane == 0) mbar_arrive(&ds_full[team]);
     }
-    TG* dqrow = static_cast<TG*>(p.dq) + ((int64_t)zh * p.s_q + row) * D + half * 128 + grp * 64;
+    TG* dqrow = static_cast<TG*>(p.dq) + ((int64_t)zh * p.s_q + row) * D + half * 128 + part * 32;
     if (nstep > 0) {
       mbar_wait(&acc_done, 0, &err, 14);
       tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t r[32];
-        tmem_ld32(tmem + lane_addr + T_DQ + grp * 64 + c * 32, r);
-        tmem_ld_wait();
-        if (row_ok) store_row32<TG>(dqrow + c * 32, r, p.scaling);
-      }
+      uint32_t r[32];
+      tmem_ld32(tmem + lane_addr + T_DQ + part * 32, r);
+      tmem_ld_wait();
+      if (row_ok) store_row32<TG>(dqrow, r, p.scaling);
       tc_fence_before();
     } else if (row_ok) {
-      zero_row(dqrow, 64);
+      zero_row(dqrow, 32);
     }
   }
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && err != 0 && p.status != nullptr) atomicExch(p.status, err);
   if (warp == 1) tmem_dealloc(tmem, 512);
+  if (p.late_wait) griddep_wait();
 }
 
 template <typename T>
@@ -963,19 +1009,30 @@ extern "C" int nvfp4_bwd_hp(const uint8_t* qnv, const uint8_t* qsc, const uint8_
   p.dq = dq; p.dk = dk; p.dv = dv;
   p.h = (int)h; p.hk = (int)hk; p.g = (int)(h / hk); p.s_q = (int)s_q; p.s_kv = (int)s_kv;
   p.scaling = scaling; p.causal = (flags & NVFP4_FWD_CAUSAL) ? 1 : 0; p.status = status;
+  p.split = 1; p.late_wait = 0;
   const unsigned halves = (unsigned)(d / 128);
-  auto launch = [&](auto kdkdv, auto kdq, int smem_dkdv, int smem_dq) -> int {
-    if (int r0 = allow_smem("nvfp4_bwd_hp", reinterpret_cast<const void*>(kdkdv), smem_dkdv)) return r0;
+  auto launch = [&](auto kwhole, auto ksplit, auto kdq, int smem_dkdv, int smem_dq) -> int {
     if (int r0 = allow_smem("nvfp4_bwd_hp", reinterpret_cast<const void*>(kdq), smem_dq)) return r0;
-    dim3 g1((unsigned)zhk, (unsigned)((s_kv + 127) / 128), halves);
-    if (int r1 = nvfp4::launch("nvfp4_bwd_hp(dkdv)", kdkdv, g1, kBwdThreads, smem_dkdv, st, t_kp128, t_qp64, t_v128, t_do64,
-                               t_q64, p))
+    // steps of a key tile: all queries of the group without a causal mask, fewer for later tiles with one;
+    // of packed rows the sample lengths are not known here, an even spread is assumed
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t tiles = (s_kv + 127) / 128, longest = (h / hk) * ((s_q + 63) / 64);
+    const bool tri = p.causal && !varlen;
+    p.split = varlen ? 1 : cluster_split(zhk * tiles * halves, longest, tri ? (h / hk) * 2 : longest, sms);
+    auto kdkdv = p.split > 1 ? ksplit : kwhole;
+    if (int r0 = allow_smem("nvfp4_bwd_hp", reinterpret_cast<const void*>(kdkdv), smem_dkdv)) return r0;
+    dim3 g1((unsigned)zhk, (unsigned)tiles, halves * p.split);
+    if (int r1 = launch_cluster("nvfp4_bwd_hp(dkdv)", kdkdv, g1, p.split, kBwdThreads, smem_dkdv, st, t_kp128, t_qp64, t_v128,
+                                t_do64, t_q64, p))
       return r1;
+    p.late_wait = 1;
     dim3 g2((unsigned)zh, (unsigned)((s_q + 127) / 128), halves);
     return nvfp4::launch("nvfp4_bwd_hp(dq)", kdq, g2, kBwdThreads, smem_dq, st, t_qp128, t_kp64, t_do128, t_v64, t_k64, p);
   };
 #define NVFP4_BWD_LAUNCH(DD, TT) \
-  launch(bwd_dkdv_kernel<DD, TT>, bwd_dq_kernel<DD, TT>, DkdvSmem<DD>::TOTAL, DqSmem<DD>::TOTAL)
+  launch(bwd_dkdv_kernel<DD, TT, false>, bwd_dkdv_kernel<DD, TT, true>, bwd_dq_kernel<DD, TT>, DkdvSmem<DD>::TOTAL, DqSmem<DD>::TOTAL)
   if (d == 128) {
     switch (grad_dtype) {
       case NVFP4_DT_BF16: return NVFP4_BWD_LAUNCH(128, __nv_bfloat16);

@@ -1,5 +1,6 @@
 // Small device helpers shared by the backward kernels (high-precision and all-FP4 gradient GEMMs).
 #pragma once
+#include <algorithm>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -110,6 +111,57 @@ __device__ __forceinline__ void zero_row(TG* dst, int n) {
 }
 
 
+// ---- split of a CTA's column steps over a thread-block cluster
+// Where a grid has too few CTAs, or one CTA far more steps than the average, the steps of a tile are
+// dealt to `n` CTAs of a cluster; each leaves its fp32 accumulators in its own shared memory and every
+// rank adds up 128 / n rows over the cluster, in rank order (results do not depend on timing).
+constexpr int kRedStride = 260;        // floats per row: 256 columns, padded so that 16-byte row accesses spread over the banks
+
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t saddr, uint32_t rank) {
+  uint32_t a;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+// 32 accumulator columns of one row into the reduction buffer
+__device__ __forceinline__ void red_store32(uint32_t buf, int row, int col, const uint32_t (&r)[32]) {
+  const uint32_t a = buf + (uint32_t)(row * kRedStride + col) * 4u;
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a + 16u * e), "r"(r[4 * e]), "r"(r[4 * e + 1]),
+                 "r"(r[4 * e + 2]), "r"(r[4 * e + 3]) : "memory");
+}
+// Sum rows [rank * 128 / n, (rank + 1) * 128 / n) of the cluster's buffers: columns below 128 of a row go
+// to o1 * mul1, the others to o2 * mul2 (with o1 null all 256 go to o2, with o2 null to o1); rows from `rows` on are not written.
+template <typename TG>
+__device__ __forceinline__ void red_sum_store(uint32_t buf, int rank, int n, int tid, int nthreads, int rows, TG* o1, TG* o2,
+                                              int64_t stride, float mul1, float mul2) {
+  const int per = 128 / n;
+  for (int idx = tid; idx < per * 64; idx += nthreads) {
+    const int row = rank * per + (idx >> 6), col = (idx & 63) * 4;
+    if (row >= rows) continue;
+    const uint32_t a = buf + (uint32_t)(row * kRedStride + col) * 4u;
+    float4 v = ld_cluster_f4(a, 0);
+    for (int k = 1; k < n; ++k) {
+      const float4 w = ld_cluster_f4(a, k);
+      v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+    }
+    const bool first = o2 == nullptr || (o1 != nullptr && col < 128);
+    const float m = first ? mul1 : mul2;
+    TG* o = (first ? o1 : o2) + row * stride + ((o1 != nullptr && o2 != nullptr) ? (col & 127) : col);
+    if constexpr (sizeof(TG) == 2) {
+      const TG t[4] = {from_f32<TG>(v.x * m), from_f32<TG>(v.y * m), from_f32<TG>(v.z * m), from_f32<TG>(v.w * m)};
+      *reinterpret_cast<uint2*>(o) = *reinterpret_cast<const uint2*>(t);
+    } else {
+      *reinterpret_cast<float4*>(o) = make_float4(v.x * m, v.y * m, v.z * m, v.w * m);
+    }
+  }
+}
+
 // Smallest power of two >= a for a positive normal a; 1 for zero, denormals and non-finite input.
 // Dividing a tensor by it is exact, which is what makes it usable as a global pre-scale of packs.
 __host__ __device__ __forceinline__ float pow2_ceil(float a) {
@@ -132,6 +184,21 @@ __host__ __device__ __forceinline__ float pow2_ceil(float a) {
   memcpy(&f, &r, 4);
   return f;
 #endif
+}
+
+// CTAs per tile for a pass of `tiles` tiles whose step counts run from `longest` down to `shortest`: the
+// split with the smallest estimate of max(longest CTA, all work over all SMs), a CTA costing `fixed`
+// steps on top of its share (launch, operand loads, epilogue and, split, the reduction; measured at
+// about six steps on a B200).
+inline int cluster_split(int64_t tiles, int64_t longest, int64_t shortest, int sm_count, double fixed = 6.0) {
+  int best = 1;
+  double best_cost = 1e300;
+  for (int n = 1; n <= 8; n *= 2) {
+    const double total = (double)tiles * ((double)(longest + shortest) * 0.5 + n * fixed);
+    const double cost = std::max((double)longest / n + fixed, total / sm_count);
+    if (cost < best_cost * 0.97) { best_cost = cost; best = n; }
+  }
+  return best;
 }
 
 }  // namespace nvfp4

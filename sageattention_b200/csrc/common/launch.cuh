@@ -44,10 +44,11 @@ inline int allow_smem(const char* what, const void* kern, int bytes) {
   return 0;
 }
 
-// Launch with programmatic stream serialisation.
+// Launch with programmatic stream serialisation; launch_cluster: clusters of `cluster` CTAs along z.
 template <typename... P, typename... A>
-int launch(const char* what, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
-  cudaLaunchAttribute attr[1];
+int launch_cluster(const char* what, void (*kern)(P...), dim3 grid, unsigned cluster, unsigned threads, size_t smem,
+                   cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
@@ -57,12 +58,24 @@ int launch(const char* what, void (*kern)(P...), dim3 grid, unsigned threads, si
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (cluster > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = cluster;
+    cfg.numAttrs = 2;
+  }
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, P(args)...);
   if (e != cudaSuccess) {
     cudaGetLastError();          // the failure is reported here; leave no sticky code behind
     return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
   }
   return 0;
+}
+
+template <typename... P, typename... A>
+int launch(const char* what, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
+  return launch_cluster(what, kern, grid, 1, threads, smem, st, static_cast<A&&>(args)...);
 }
 
 }  // namespace nvfp4
