@@ -179,6 +179,8 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const T* __restrict__ x, 
 struct BwdParams {
   const uint8_t* qsc;   // [ZH, Sq, 8]
   const uint8_t* ksc;   // [ZHk, Skv, 8]
+  const __nv_bfloat16* v;    // [ZHk, Skv, D]
+  const __nv_bfloat16* dout; // [ZH, Sq, D]
   const float* lse;     // [ZH, Sq] natural log
   const float* delta;   // [ZH, Sq]
   const float* bias;    // [Z, Skv] additive key bias (after the scaling) or null
@@ -195,6 +197,27 @@ struct BwdParams {
   int late_wait;        // independent of the kernel before it: wait for it at the end, not at the start
   int* status;
 };
+
+// The operand of dP that a CTA keeps for all its steps -- V rows in the dK/dV kernel, dO rows in the dQ
+// kernel -- goes to tensor memory as far as there is room: an N = 64 MMA with both operands in shared
+// memory reads 4 KB of A and 2 KB of B, 48 clocks of its 128 bytes per clock for 32 clocks of arithmetic,
+// and shared memory bandwidth (operands, TMA writes) is what the kernels run out of first.
+// One thread fills kCols columns (two elements each) of its lane; a null row is zeros.
+template <int kCols>
+__device__ __forceinline__ void fill_a_tmem(uint32_t taddr, const __nv_bfloat16* row) {
+#pragma unroll
+  for (int c = 0; c < kCols; c += 32) {
+    uint32_t r[32];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const uint4 w = row != nullptr ? __ldg(reinterpret_cast<const uint4*>(row + 2 * c) + e) : make_uint4(0u, 0u, 0u, 0u);
+      r[4 * e] = w.x; r[4 * e + 1] = w.y; r[4 * e + 2] = w.z; r[4 * e + 3] = w.w;
+    }
+    tmem_st32(taddr + c, r);
+  }
+  tmem_st_wait();
+  tc_fence_before();
+}
 
 // P for 16 columns of one accumulator row: exp2(s * c2 + offsets).  Per-column statistics (the
 // dK/dV kernel): `nl` points at the raw lse of the 16 columns in shared memory and `nl_row` is a
@@ -280,18 +303,6 @@ struct DkdvSmem {
   static_assert(STAGE % 1024 == 0 && (V + KP) % 1024 == 0, "128-byte-swizzled tiles need 1 KB alignment");
 };
 
-// position in the step list of a key tile: query head of the group, 64-query step
-struct StepCursor {
-  int gq, i;
-  __device__ __forceinline__ StepCursor(int st, int n_i) : gq(n_i > 0 ? st / n_i : 0), i(n_i > 0 ? st - gq * n_i : 0) {}
-  __device__ __forceinline__ void next(int n_i) {
-    if (++i == n_i) {
-      i = 0;
-      ++gq;
-    }
-  }
-};
-
 template <int D, typename TG, bool kSplit>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant__ CUtensorMap tm_qp,
@@ -307,7 +318,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
   uint8_t* s_ksf = s_stage + L::NSTAGE * L::STAGE;
 
   __shared__ uint64_t full_tma[L::NSTAGE], full_aux[L::NSTAGE], empty[L::NSTAGE];
-  __shared__ uint64_t kv_full, ksf_full, s_full[2], dp_full, dp_free, pds_full[2], acc_done;
+  __shared__ uint64_t kv_full, ksf_full, a_full, s_full[2], dp_full, dp_free, pds_full[2], acc_done;
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
 
@@ -330,6 +341,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
     }
     mbar_init(&kv_full, 1);
     mbar_init(&ksf_full, 1);
+    mbar_init(&a_full, 4);
     mbar_init(&dp_full, 1);
     mbar_init(&dp_free, 8);
     mbar_init(&acc_done, 1);
@@ -359,16 +371,18 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
   const uint32_t tmem = tmem_base_s;
   constexpr uint32_t T_DV = 0, T_DK = 128, T_ST = 256, T_DPT = 384, T_SFK = 448, T_SFQ = T_SFK + L::KB * 4;
   constexpr uint32_t SFQ_SLOT = L::KB * 4;
-  static_assert(T_SFQ + 2 * SFQ_SLOT <= 512, "TMEM budget");
+  constexpr int KT = D == 128 ? 4 : 0;              // K = 16 blocks of V held in tensor memory
+  constexpr uint32_t T_V = T_SFQ + 2 * SFQ_SLOT;
+  static_assert(T_V + KT * 8 <= 512 && KT % 4 == 0, "TMEM budget");
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one() && nstep > 0) {
-      mbar_expect_tx(&kv_full, L::KP + L::V);
+      mbar_expect_tx(&kv_full, L::KP + L::V - KT / 4 * 16384);
 #pragma unroll
       for (int c = 0; c < L::KSUB; ++c) tma_load_3d(s_kp + c * 8192, &tm_kp, &kv_full, c * 64, n0, unit);
 #pragma unroll
-      for (int c = 0; c < L::DS; ++c) tma_load_3d(s_v + c * 16384, &tm_v, &kv_full, c * 64, n0, unit);
+      for (int c = KT / 4; c < L::DS; ++c) tma_load_3d(s_v + c * 16384, &tm_v, &kv_full, c * 64, n0, unit);
       // L2 prefetch kBwdPrefetch steps ahead: co-resident CTAs walk the same query tiles in step,
       // so without it every stage load is a first touch that waits on HBM
       auto prefetch = [&](const StepCursor& c0) {
@@ -459,6 +473,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
       const uint32_t id_acc = make_idesc_bf16(128, 128, true);
       mbar_wait(&kv_full, 0, &err, 3);
       mbar_wait(&ksf_full, 0, &err, 4);
+      if (KT > 0) mbar_wait(&a_full, 0, &err, 15);
       tc_fence_after();
 #pragma unroll
       for (int c = 0; c < L::KB; ++c) tmem_cp_32x128b_warpx4(tmem + T_SFK + 4 * c, smem_u32(s_ksf + c * 512));
@@ -505,7 +520,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
           tc_fence_after();
         }
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k)
+        for (int k = 0; k < KT; ++k)
+          umma_bf16_ta(tmem + T_DPT, tmem + T_V + k * 8, x_do + (k >> 2) * 512 + (k & 3) * 2, id_dp, k > 0);
+#pragma unroll
+        for (int k = KT; k < D / 16; ++k)
           umma_bf16(tmem + T_DPT, b_v + (k >> 2) * 1024 + (k & 3) * 2, x_do + (k >> 2) * 512 + (k & 3) * 2, id_dp,
                     k > 0);
         umma_commit(&dp_full);
@@ -531,6 +549,12 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
     const int row = wq * 32 + lane;     // key within the tile
     const int key = n0 + row;
     const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
+    if (KT > 0 && part == 0) {
+      fill_a_tmem<(KT > 0 ? KT : 4) * 8>(tmem + lane_addr + T_V,
+                                         key < p.s_kv ? p.v + ((int64_t)unit * p.s_kv + key) * D : nullptr);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&a_full);
+    }
     const float c2 = p.scaling * kBwdLog2e;
     // additive bias of this key, in the exponent's base-2 units (-inf masks the key)
     const float bk2 = (p.bias != nullptr && key < p.s_kv) ? p.bias[(int64_t)zi * p.s_kv + key] * kBwdLog2e : 0.0f;
@@ -629,14 +653,13 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
 // ------------------------------------------------------------------------------------------
 // dQ
 // TMEM: dQ [0,128) | S slots [128,192) [192,256) | dP [256,320) | SFQ [320, 320+D/16) |
-//       two SFK slots of D/16 columns.  Head dim 256: blockIdx.z picks a 128-wide half of dQ.
+//       two SFK slots of D/16 columns | dO, D/2 columns.  Head dim 256: blockIdx.z picks a 128-wide half of dQ.
 // dS (bf16 pairs, 32 columns) is written back into the S slot it came from and feeds the dQ GEMM
 // as a TMEM A operand.
 // ------------------------------------------------------------------------------------------
 template <int D>
 struct DqSmem {
   static constexpr int DS = D / 64, KSUB = D / 128, KB = D / 64;
-  static constexpr int DO = DS * 16384;    // dO bf16 [128 q x D] as 16 KB sub-tiles
   static constexpr int QP = KSUB * 8192;   // Q pack tile, 128 queries x D/2 B
   static constexpr int QSF = KB * 512;
   // per stage: V bf16 [64 keys x D] and the 128-wide half of K bf16 (8 KB sub-tiles), K pack
@@ -644,27 +667,25 @@ struct DqSmem {
   static constexpr int V = DS * 8192, K = 16384, KP = KSUB * 4096, KSF = KB * 512, AUX = 1024;
   static constexpr int O_V = 0, O_K = V, O_KP = V + K, O_KSF = O_KP + KP, O_AUX = O_KSF + KSF;   // AUX: key bias [64]
   static constexpr int STAGE = V + K + KP + KSF + AUX;
-  static constexpr int NSTAGE = D == 128 ? 4 : 2;
-  static constexpr int TOTAL = DO + QP + NSTAGE * STAGE + QSF + 1024;
-  static_assert(STAGE % 1024 == 0 && (DO + QP) % 1024 == 0, "128-byte-swizzled tiles need 1 KB alignment");
+  static constexpr int NSTAGE = D == 128 ? 5 : 2;
+  static constexpr int TOTAL = QP + NSTAGE * STAGE + QSF + 1024;
+  static_assert(STAGE % 1024 == 0 && QP % 1024 == 0, "128-byte-swizzled tiles need 1 KB alignment");
 };
 
 template <int D, typename TG>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__ CUtensorMap tm_kp,
-              const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_v,
-              const __grid_constant__ CUtensorMap tm_k, const BwdParams p) {
+              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_k, const BwdParams p) {
   using L = DqSmem<D>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint8_t* s_do = smem;
-  uint8_t* s_qp = s_do + L::DO;
+  uint8_t* s_qp = smem;
   uint8_t* s_stage = s_qp + L::QP;
   uint8_t* s_qsf = s_stage + L::NSTAGE * L::STAGE;
 
   __shared__ uint64_t full_tma[L::NSTAGE], full_sf[L::NSTAGE], empty[L::NSTAGE];
-  __shared__ uint64_t q_full, qsf_full, s_full[2], dp_full, dp_free, ds_full[2], acc_done;
+  __shared__ uint64_t q_full, qsf_full, a_full, s_full[2], dp_full, dp_free, ds_full[2], acc_done;
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
 
@@ -686,6 +707,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
     }
     mbar_init(&q_full, 1);
     mbar_init(&qsf_full, 1);
+    mbar_init(&a_full, 4);
     mbar_init(&dp_full, 1);
     mbar_init(&dp_free, 8);
     mbar_init(&acc_done, 1);
@@ -711,15 +733,14 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
   griddep_launch();
   const uint32_t tmem = tmem_base_s;
   constexpr uint32_t T_DQ = 0, T_S = 128, T_DP = 256, T_SFQ = 320, T_SFK = T_SFQ + L::KB * 4;
-  constexpr uint32_t SFK_SLOT = L::KB * 4;
+  constexpr uint32_t SFK_SLOT = L::KB * 4, T_DO = T_SFK + 2 * SFK_SLOT;      // dO: D / 2 columns
+  static_assert(T_DO + D / 2 <= 512, "TMEM budget");
 
   if (warp == 0) {
     if (elect_one() && nstep > 0) {
-      mbar_expect_tx(&q_full, L::QP + L::DO);
+      mbar_expect_tx(&q_full, L::QP);
 #pragma unroll
       for (int c = 0; c < L::KSUB; ++c) tma_load_3d(s_qp + c * 8192, &tm_qp, &q_full, c * 64, m0, zh);
-#pragma unroll
-      for (int c = 0; c < L::DS; ++c) tma_load_3d(s_do + c * 16384, &tm_do, &q_full, c * 64, m0, zh);
       auto prefetch = [&](int t) {
         const int key0 = (j_lo + t) * 64;
 #pragma unroll
@@ -794,10 +815,11 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
       const uint32_t id_acc = make_idesc_bf16(128, 128, true);
       mbar_wait(&q_full, 0, &err, 3);
       mbar_wait(&qsf_full, 0, &err, 4);
+      mbar_wait(&a_full, 0, &err, 15);
       tc_fence_after();
 #pragma unroll
       for (int c = 0; c < L::KB; ++c) tmem_cp_32x128b_warpx4(tmem + T_SFQ + 4 * c, smem_u32(s_qsf + c * 512));
-      const uint64_t b_do = desc_sw128(s_do, 0), b_qp = desc_sw64(s_qp, 0);
+      const uint64_t b_qp = desc_sw64(s_qp, 0);
       const uint64_t b_v = desc_sw128(s_stage + L::O_V, 0), b_k_mn = desc_sw128_mn(s_stage + L::O_K, 0, 8192);
       const uint64_t b_kp = desc_sw64(s_stage + L::O_KP, 0);
       auto grad_gemm = [&](int t) {   // dQ += dS K of step t
@@ -831,8 +853,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
         }
 #pragma unroll
         for (int k = 0; k < D / 16; ++k)
-          umma_bf16(tmem + T_DP, b_do + (k >> 2) * 1024 + (k & 3) * 2, x_v + (k >> 2) * 512 + (k & 3) * 2, id_dp,
-                    k > 0);
+          umma_bf16_ta(tmem + T_DP, tmem + T_DO + k * 8, x_v + (k >> 2) * 512 + (k & 3) * 2, id_dp, k > 0);
         umma_commit(&dp_full);
         if (st > 0) {
           mbar_wait(&ds_full[b ^ 1], ((st - 1) >> 1) & 1, &err, 8);
@@ -857,6 +878,11 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
     const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
     const float c2 = p.scaling * kBwdLog2e;
     const bool row_ok = row < p.s_q;
+    if (part == 0) {
+      fill_a_tmem<D / 2>(tmem + lane_addr + T_DO, row_ok ? p.dout + ((int64_t)zh * p.s_q + row) * D : nullptr);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&a_full);
+    }
     const float nl = row_ok ? -p.lse[(int64_t)zh * p.s_q + row] * kBwdLog2e : 0.0f;
     const float nd = row_ok ? -p.delta[(int64_t)zh * p.s_q + row] : 0.0f;
     // visible keys of this row: [kl, kh)
@@ -990,7 +1016,7 @@ extern "C" int nvfp4_bwd_hp(const uint8_t* qnv, const uint8_t* qsc, const uint8_
                 "nvfp4_bwd_hp: grid too large");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t zh = z * h, zhk = z * hk;
-  CUtensorMap t_qp64, t_qp128, t_kp64, t_kp128, t_v64, t_v128, t_do64, t_do128, t_q64, t_k64;
+  CUtensorMap t_qp64, t_qp128, t_kp64, t_kp128, t_v64, t_v128, t_do64, t_q64, t_k64;
   int rc;
   const uint64_t pb = (uint64_t)d / 2, hb = (uint64_t)d * 2;   // bytes per pack row / bf16 row
   if ((rc = make_tmap_u8_3d_sw64(&t_qp64, qnv, pb, s_q, zh, pb, (uint64_t)s_q * pb, 64, "nvfp4_bwd_hp(Qp64)"))) return rc;
@@ -1000,10 +1026,10 @@ extern "C" int nvfp4_bwd_hp(const uint8_t* qnv, const uint8_t* qsc, const uint8_
   if ((rc = make_tmap_bf16_3d_sw128(&t_v64, v_bf16, d, s_kv, zhk, hb, (uint64_t)s_kv * hb, 64, "nvfp4_bwd_hp(V64)"))) return rc;
   if ((rc = make_tmap_bf16_3d_sw128(&t_v128, v_bf16, d, s_kv, zhk, hb, (uint64_t)s_kv * hb, 128, "nvfp4_bwd_hp(V128)"))) return rc;
   if ((rc = make_tmap_bf16_3d_sw128(&t_do64, do_bf16, d, s_q, zh, hb, (uint64_t)s_q * hb, 64, "nvfp4_bwd_hp(dO64)"))) return rc;
-  if ((rc = make_tmap_bf16_3d_sw128(&t_do128, do_bf16, d, s_q, zh, hb, (uint64_t)s_q * hb, 128, "nvfp4_bwd_hp(dO128)"))) return rc;
   if ((rc = make_tmap_bf16_3d_sw128(&t_q64, q_bf16, d, s_q, zh, hb, (uint64_t)s_q * hb, 64, "nvfp4_bwd_hp(Q64)"))) return rc;
   if ((rc = make_tmap_bf16_3d_sw128(&t_k64, k_bf16, d, s_kv, zhk, hb, (uint64_t)s_kv * hb, 64, "nvfp4_bwd_hp(K64)"))) return rc;
   BwdParams p;
+  p.v = static_cast<const __nv_bfloat16*>(v_bf16); p.dout = static_cast<const __nv_bfloat16*>(do_bf16);
   p.qsc = qsc; p.ksc = ksc; p.lse = lse; p.delta = delta; p.bias = key_bias;
   p.seq_start = seq_start; p.seq_end = seq_end;
   p.dq = dq; p.dk = dk; p.dv = dv;
@@ -1013,14 +1039,11 @@ extern "C" int nvfp4_bwd_hp(const uint8_t* qnv, const uint8_t* qsc, const uint8_
   const unsigned halves = (unsigned)(d / 128);
   auto launch = [&](auto kwhole, auto ksplit, auto kdq, int smem_dkdv, int smem_dq) -> int {
     if (int r0 = allow_smem("nvfp4_bwd_hp", reinterpret_cast<const void*>(kdq), smem_dq)) return r0;
-    // steps of a key tile: all queries of the group without a causal mask, fewer for later tiles with one;
-    // of packed rows the sample lengths are not known here, an even spread is assumed
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t tiles = (s_kv + 127) / 128, longest = (h / hk) * ((s_q + 63) / 64);
-    const bool tri = p.causal && !varlen;
-    p.split = varlen ? 1 : cluster_split(zhk * tiles * halves, longest, tri ? (h / hk) * 2 : longest, sms);
+    p.split = cluster_split(zhk * tiles * halves, longest, p.causal ? (h / hk) * 2 : longest, varlen, sms, 6.0);
     auto kdkdv = p.split > 1 ? ksplit : kwhole;
     if (int r0 = allow_smem("nvfp4_bwd_hp", reinterpret_cast<const void*>(kdkdv), smem_dkdv)) return r0;
     dim3 g1((unsigned)zhk, (unsigned)tiles, halves * p.split);
@@ -1029,7 +1052,7 @@ extern "C" int nvfp4_bwd_hp(const uint8_t* qnv, const uint8_t* qsc, const uint8_
       return r1;
     p.late_wait = 1;
     dim3 g2((unsigned)zh, (unsigned)((s_q + 127) / 128), halves);
-    return nvfp4::launch("nvfp4_bwd_hp(dq)", kdq, g2, kBwdThreads, smem_dq, st, t_qp128, t_kp64, t_do128, t_v64, t_k64, p);
+    return nvfp4::launch("nvfp4_bwd_hp(dq)", kdq, g2, kBwdThreads, smem_dq, st, t_qp128, t_kp64, t_v64, t_k64, p);
   };
 #define NVFP4_BWD_LAUNCH(DD, TT) \
   launch(bwd_dkdv_kernel<DD, TT, false>, bwd_dkdv_kernel<DD, TT, true>, bwd_dq_kernel<DD, TT>, DkdvSmem<DD>::TOTAL, DqSmem<DD>::TOTAL)

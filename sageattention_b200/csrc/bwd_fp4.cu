@@ -136,6 +136,7 @@ struct B4Params {
   int s_q, s_kv, c_pad;  // c_pad: padded column extent of the transposed packs
   float scaling;
   int causal;
+  int split;             // dV / dK passes: CTAs (of one cluster along z) that share a tile's stages
   int late_wait;         // independent of the kernel before it: wait for it at the end, not at the start
   int sr_p, sr_ds;       // stochastic rounding of the in-kernel P / dS packs (fp4_legacy mode)
   uint32_t seed;
@@ -291,7 +292,9 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   }
   const int i_lo = c_lo / 128;
   const int n_i = max((c_hi + 127) / 128 - i_lo, 0);
-  const int nstage = (kKeys ? p.g : 1) * n_i;
+  const int rank = kKeys ? blockIdx.z : 0;
+  const int sg0 = kKeys ? p.g * n_i * rank / p.split : 0;
+  const int nstage = kKeys ? p.g * n_i * (rank + 1) / p.split - sg0 : n_i;
   const int nstep = 2 * nstage;
 
   tc_fence_before();
@@ -301,15 +304,10 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   const uint32_t tmem = tmem_base_s;
   const float gs = gs_s;
 
-  // stage index -> (column batch entry, first column)
-  auto stage_cols = [&](int sg, int& cb, int& col0) {
-    if constexpr (kKeys) {
-      cb = cb0 + sg / n_i;
-      col0 = (i_lo + sg % n_i) * 128;
-    } else {
-      cb = cb0;
-      col0 = (i_lo + sg) * 128;
-    }
+  // a stage's column batch entry and first column, from its position in the list
+  auto stage_cols = [&](const StepCursor& c, int& cb, int& col0) {
+    cb = cb0 + c.gq;
+    col0 = (i_lo + c.i) * 128;
   };
 
   if (warp == 0) {
@@ -321,24 +319,28 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
         tma_load_3d(s_res + C::O_X1 + c * 8192, &tm_x1, &x_full, c * 64, row0, rb);
         if constexpr (kDs) tma_load_3d(s_res + C::O_X2 + c * 8192, &tm_x2, &x_full, c * 64, row0, rb);
       }
-      auto prefetch = [&](int sg) {
+      auto prefetch = [&](const StepCursor& c) {
         int cb, col0;
-        stage_cols(sg, cb, col0);
+        stage_cols(c, cb, col0);
         const int tc = kFp8 ? col0 : col0 / 2;
 #pragma unroll
-        for (int c = 0; c < C::KSUB; ++c) {
-          tma_prefetch_3d(&tm_y1, c * 64, col0, cb);
-          if constexpr (kDs) tma_prefetch_3d(&tm_y2, c * 64, col0, cb);
-          if constexpr (kP) tma_prefetch_3d(&tm_t1, tc, c * 128, cb);
-          if constexpr (kDs) tma_prefetch_3d(&tm_t2, tc, c * 128, cb);
+        for (int k = 0; k < C::KSUB; ++k) {
+          tma_prefetch_3d(&tm_y1, k * 64, col0, cb);
+          if constexpr (kDs) tma_prefetch_3d(&tm_y2, k * 64, col0, cb);
+          if constexpr (kP) tma_prefetch_3d(&tm_t1, tc, k * 128, cb);
+          if constexpr (kDs) tma_prefetch_3d(&tm_t2, tc, k * 128, cb);
         }
       };
-      for (int sg = C::NSTAGE; sg < min(nstage, C::NSTAGE + kB4Prefetch); ++sg) prefetch(sg);
-      for (int sg = 0; sg < nstage; ++sg) {
+      StepCursor cur(sg0, n_i), ahead(sg0 + C::NSTAGE, n_i);
+      for (int sg = C::NSTAGE; sg < min(nstage, C::NSTAGE + kB4Prefetch); ++sg, ahead.next(n_i)) prefetch(ahead);
+      for (int sg = 0; sg < nstage; ++sg, cur.next(n_i)) {
         const int s = sg % C::NSTAGE;
         int cb, col0;
-        stage_cols(sg, cb, col0);
-        if (sg + C::NSTAGE + kB4Prefetch < nstage) prefetch(sg + C::NSTAGE + kB4Prefetch);
+        stage_cols(cur, cb, col0);
+        if (sg + C::NSTAGE + kB4Prefetch < nstage) {
+          prefetch(ahead);
+          ahead.next(n_i);
+        }
         if (sg >= C::NSTAGE) mbar_wait(&empty[s], ((sg / C::NSTAGE) & 1) ^ 1, &err, 1);
         uint8_t* sb = s_stage + s * C::STAGE;
         const int tc = kFp8 ? col0 : col0 / 2;
@@ -375,10 +377,11 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
       if (lane == 0) mbar_arrive(&xsf_full);
       const float inv_gs = 1.0f / gs;
       const int csc = p.c_pad / (kFp8 ? 32 : 16);      // scale bytes per row of a transposed pack
-      for (int sg = 0; sg < nstage; ++sg) {
+      StepCursor cur(sg0, n_i);
+      for (int sg = 0; sg < nstage; ++sg, cur.next(n_i)) {
         const int s = sg % C::NSTAGE;
         int cb, col0;
-        stage_cols(sg, cb, col0);
+        stage_cols(cur, cb, col0);
         if (sg >= C::NSTAGE) mbar_wait(&empty[s], ((sg / C::NSTAGE) & 1) ^ 1, &err, 2);
         uint8_t* sb = s_stage + s * C::STAGE;
         const uint32_t ysf = smem_u32(sb + C::S_YSF), tsf1 = smem_u32(sb + C::S_TSF1), tsf2 = smem_u32(sb + C::S_TSF2);
@@ -569,10 +572,11 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
     // dQ pass: the per-row exponent offset and -delta' term; dK/dV pass: these come per column from aux
     const float2 re2 = kKeys ? make_float2(0.0f, 0.0f) : make_float2(row_e, row_e);
     const float2 rnd2 = make_float2(row_nd, row_nd);
-    for (int st = team; st < nstep; st += 2) {
+    StepCursor cur(sg0, n_i);
+    for (int st = team; st < nstep; st += 2, cur.next(n_i)) {
       const int pp = team, sg = st >> 1, s = sg % C::NSTAGE;
       int cb, col0;
-      stage_cols(sg, cb, col0);
+      stage_cols(cur, cb, col0);
       const float* aux0 = reinterpret_cast<const float*>(s_stage + s * C::STAGE + C::S_AUX) + 64 * pp;
       const int cs0 = col0 + 64 * pp;                // first column of the step
       const bool masked = !__all_sync(0xffffffffu, cs0 >= lo && cs0 + 64 <= hi);
@@ -652,7 +656,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
         // random-bit counters: (tensor, row of the CTA's unit) and the quad's column within the unit
         if constexpr (kSr) {
           const uint32_t sr_row = (uint32_t)((int64_t)rb * R + row) * 4u + (kKeys ? 0u : 2u);
-          const uint32_t sr_col = (uint32_t)(st * 16 + ch * 4);
+          const uint32_t sr_col = (uint32_t)((2 * sg0 + st) * 16 + ch * 4);
           if constexpr (kP)
             scp |= b4_pack16<false>(pf, wp[2 * (ch & 1)], wp[2 * (ch & 1) + 1], p.sr_p != 0, p.seed, sr_row + 1u, sr_col)
                    << (8 * (ch & 1));
@@ -710,27 +714,43 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
     constexpr int EC = D / (2 * NP);
     TG* o1 = kP ? static_cast<TG*>(p.out1) + ((int64_t)rb * R + row) * D + part * EC : nullptr;
     TG* o2 = kDs ? static_cast<TG*>(p.out2) + ((int64_t)rb * R + row) * D + part * EC : nullptr;
+    const bool split = kKeys && p.split > 1;
     if (nstep > 0) {
       mbar_wait(&acc_done, 0, &err, 14);
       tc_fence_after();
+    }
+    if (nstep > 0 || split) {
+      auto column32 = [&](uint32_t t_acc, int c, TG* o, float mul, int red_col) {
+        uint32_t r[32];
+        if (nstep > 0) {
+          tmem_ld32(tmem + lane_addr + t_acc + part * EC + c * 32, r);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) r[e] = 0u;
+        }
+        if (split) red_store32(smem_u32(smem), row_in, red_col + part * EC + c * 32, r);   // the operand tiles are idle by now
+        else if (row_ok) store_row32<TG>(o + c * 32, r, mul);
+      };
 #pragma unroll
       for (int c = 0; c < EC / 32; ++c) {
-        uint32_t r[32];
-        if constexpr (kP) {
-          tmem_ld32(tmem + lane_addr + C::T_ACC1 + part * EC + c * 32, r);
-          tmem_ld_wait();
-          if (row_ok) store_row32<TG>(o1 + c * 32, r, m1);
-        }
-        if constexpr (kDs) {
-          tmem_ld32(tmem + lane_addr + C::T_ACC2 + part * EC + c * 32, r);
-          tmem_ld_wait();
-          if (row_ok) store_row32<TG>(o2 + c * 32, r, m2);
-        }
+        if constexpr (kP) column32(C::T_ACC1, c, o1, m1, 0);
+        if constexpr (kDs) column32(C::T_ACC2, c, o2, m2, kP ? 128 : 0);
       }
       tc_fence_before();
     } else if (row_ok) {
       if constexpr (kP) zero_row(o1, EC);
       if constexpr (kDs) zero_row(o2, EC);
+    }
+  }
+  if constexpr (kKeys) {
+    if (p.split > 1) {
+      __syncwarp();
+      cluster_sync_all();
+      const int64_t first = ((int64_t)rb * R + row0) * D;
+      red_sum_store<TG>(smem_u32(smem), rank, p.split, tid, C::THREADS, R - row0, kP ? static_cast<TG*>(p.out1) + first : nullptr,
+                        kDs ? static_cast<TG*>(p.out2) + first : nullptr, D, gs * 4.8828125e-4f, gs * 1.953125e-3f);
+      cluster_sync_all();
     }
   }
   tc_fence_before();
@@ -803,10 +823,13 @@ extern "C" int nvfp4_bwd_fp4(const uint8_t* qnv, const uint8_t* qsc, const uint8
   p.h = (int)h; p.hk = (int)hk; p.g = (int)(h / hk); p.s_q = (int)s_q; p.s_kv = (int)s_kv;
   p.scaling = scaling; p.causal = (flags & NVFP4_FWD_CAUSAL) ? 1 : 0; p.status = status;
   p.seed = seed; p.sr_p = 0; p.sr_ds = 0;
-  p.late_wait = 0;
+  p.late_wait = 0; p.split = 1;
   // The passes are independent of one another: the first waits for the work before it, the later ones
   // start filling the SMs that its last CTAs leave and wait for it only at their end.
   bool first = true;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   auto launch_pass = [&](const char* what, auto kern, int smem, int threads, bool keys) -> int {
     if (int r0 = allow_smem(what, reinterpret_cast<const void*>(kern), smem)) return r0;
     B4Params a = p;
@@ -816,8 +839,10 @@ extern "C" int nvfp4_bwd_fp4(const uint8_t* qnv, const uint8_t* qsc, const uint8
       a.x1sc = ksc; a.x2sc = vdsc; a.y1sc = qsc; a.y2sc = dosc; a.t1sc = dotsc; a.t2sc = qtsc;
       a.out1 = dv; a.out2 = dk; a.c_pad = (int)sq_pad;
       a.sr_p = (flags & NVFP4_BWD_SR_P_DV) ? 1 : 0; a.sr_ds = (flags & NVFP4_BWD_SR_DS_DK) ? 1 : 0;
-      return launch(what, kern, dim3((unsigned)zhk, (unsigned)((s_kv + 127) / 128)), threads, smem, st, t_k, t_vd, t_q, t_do,
-                    t_dot, t_qt, a);
+      const int64_t g = h / hk, tiles = (s_kv + 127) / 128;
+      a.split = cluster_split(zhk * tiles, g * ((s_q + 127) / 128), p.causal ? g : g * ((s_q + 127) / 128), varlen, sms, 3.0);
+      return launch_cluster(what, kern, dim3((unsigned)zhk, (unsigned)tiles, (unsigned)a.split), a.split, threads, smem, st, t_k,
+                            t_vd, t_q, t_do, t_dot, t_qt, a);
     }
     // dQ: rows = queries (Q, dO' packs), columns = keys (K, V packs; K^T transposed pack)
     a.x1sc = qsc; a.x2sc = dosc; a.y1sc = ksc; a.y2sc = vdsc; a.t1sc = nullptr; a.t2sc = ktsc;

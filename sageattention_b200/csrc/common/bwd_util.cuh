@@ -111,6 +111,18 @@ __device__ __forceinline__ void zero_row(TG* dst, int n) {
 }
 
 
+// Position in the step list of a key tile: query head of the group, step among its n_i.
+struct StepCursor {
+  int gq, i;
+  __device__ __forceinline__ StepCursor(int st, int n_i) : gq(n_i > 0 ? st / n_i : 0), i(n_i > 0 ? st - gq * n_i : 0) {}
+  __device__ __forceinline__ void next(int n_i) {
+    if (++i == n_i) {
+      i = 0;
+      ++gq;
+    }
+  }
+};
+
 // ---- split of a CTA's column steps over a thread-block cluster
 // Where a grid has too few CTAs, or one CTA far more steps than the average, the steps of a tile are
 // dealt to `n` CTAs of a cluster; each leaves its fp32 accumulators in its own shared memory and every
@@ -188,9 +200,11 @@ __host__ __device__ __forceinline__ float pow2_ceil(float a) {
 
 // CTAs per tile for a pass of `tiles` tiles whose step counts run from `longest` down to `shortest`: the
 // split with the smallest estimate of max(longest CTA, all work over all SMs), a CTA costing `fixed`
-// steps on top of its share (launch, operand loads, epilogue and, split, the reduction; measured at
-// about six steps on a B200).
-inline int cluster_split(int64_t tiles, int64_t longest, int64_t shortest, int sm_count, double fixed = 6.0) {
+// steps on top of its share (launch, operand loads, epilogue and, split, the reduction; a few us against
+// about one per 64-query step on a B200).  Of packed rows the host does not know the sample lengths:
+// they are taken to be an eighth of the row.
+inline int cluster_split(int64_t tiles, int64_t longest, int64_t shortest, bool packed, int sm_count, double fixed) {
+  if (packed) longest = std::max<int64_t>(longest / 8, shortest);
   int best = 1;
   double best_cost = 1e300;
   for (int n = 1; n <= 8; n *= 2) {
