@@ -25,82 +25,78 @@ inline TensorMapEncodeTiledFn tensor_map_encoder() {
   return fn;
 }
 
+// One encoded map, remembered per thread by the arguments it was made from (a map is a pure function of
+// them): a decode step or a training step asks for the same four to nine maps again and again, and an
+// encode costs the driver about as much as an allocation.
+struct TmapKey {
+  const void* base;
+  uint64_t n0, n1, n2, s1, s2;
+  uint32_t type, swizzle, promotion, b0, b1;
+  bool operator==(const TmapKey& o) const {
+    return base == o.base && n0 == o.n0 && n1 == o.n1 && n2 == o.n2 && s1 == o.s1 && s2 == o.s2 && type == o.type &&
+           swizzle == o.swizzle && promotion == o.promotion && b0 == o.b0 && b1 == o.b1;
+  }
+};
+inline int encode_tmap(CUtensorMap* m, const TmapKey& k, const char* what) {
+  struct Entry { TmapKey key; CUtensorMap map; bool used; };
+  constexpr int kEntries = 64;         // 64 x 216 bytes per thread, direct mapped
+  static thread_local Entry cache[kEntries];
+  uint64_t h = reinterpret_cast<uintptr_t>(k.base) ^ (k.n1 * 0x9E3779B97F4A7C15ull) ^ (k.n0 << 20) ^ (k.s1 << 40) ^
+               ((uint64_t)k.b1 << 8) ^ k.b0 ^ ((uint64_t)k.swizzle << 16);
+  h = (h ^ (h >> 29)) * 0xBF58476D1CE4E5B9ull;
+  Entry& e = cache[(h >> 40) % kEntries];
+  if (e.used && e.key == k) {
+    *m = e.map;
+    return 0;
+  }
+  TensorMapEncodeTiledFn enc = tensor_map_encoder();
+  if (!enc) return fail(-1, "%s: cuTensorMapEncodeTiled is unavailable", what);
+  if ((reinterpret_cast<uintptr_t>(k.base) & 15) || (k.s1 & 15) || (k.s2 & 15))
+    return fail(-1, "%s: base and strides must be 16-byte aligned for TMA", what);
+  cuuint64_t dims[3] = {k.n0, k.n1, k.n2};
+  cuuint64_t strides[2] = {k.s1, k.s2};
+  cuuint32_t box[3] = {k.b0, k.b1, 1};
+  cuuint32_t es[3] = {1, 1, 1};
+  CUresult r = enc(m, (CUtensorMapDataType)k.type, 3, const_cast<void*>(k.base), dims, strides, box, es,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, (CUtensorMapSwizzle)k.swizzle, (CUtensorMapL2promotion)k.promotion,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(-1, "%s: cuTensorMapEncodeTiled failed with %d", what, (int)r);
+  e.key = k;
+  e.map = *m;
+  e.used = true;
+  return 0;
+}
+
 // Byte tensor [n2][n1][n0] (n0 innermost, contiguous) with byte strides s1, s2 (multiples of 16),
 // box [1][b1][b0] with b0 == 64 bytes and the 64-byte shared-memory swizzle; out-of-range
 // coordinates read as zero.
-inline int make_tmap_u8_3d_sw64(CUtensorMap* m, const void* base, uint64_t n0, uint64_t n1,
-                                uint64_t n2, uint64_t s1, uint64_t s2, uint32_t b1,
-                                const char* what) {
-  TensorMapEncodeTiledFn enc = tensor_map_encoder();
-  if (!enc) return fail(-1, "%s: cuTensorMapEncodeTiled is unavailable", what);
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (s1 & 15) || (s2 & 15))
-    return fail(-1, "%s: base and strides must be 16-byte aligned for TMA", what);
-  cuuint64_t dims[3] = {n0, n1, n2};
-  cuuint64_t strides[2] = {s1, s2};
-  cuuint32_t box[3] = {64, b1, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box,
-                   es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(-1, "%s: cuTensorMapEncodeTiled failed with %d", what, (int)r);
-  return 0;
+inline int make_tmap_u8_3d_sw64(CUtensorMap* m, const void* base, uint64_t n0, uint64_t n1, uint64_t n2, uint64_t s1,
+                                uint64_t s2, uint32_t b1, const char* what) {
+  return encode_tmap(m, {base, n0, n1, n2, s1, s2, CU_TENSOR_MAP_DATA_TYPE_UINT8, CU_TENSOR_MAP_SWIZZLE_64B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, 64, b1}, what);
 }
 
 // Map used only for L2 prefetch of wide row segments: the same bytes seen as 32-bit words,
 // [n2][n1][n0w] with a box of [1][b1][b0w] words (b0w <= 256, i.e. up to 1 KB per row), no swizzle.
-inline int make_tmap_u32_3d_prefetch(CUtensorMap* m, const void* base, uint64_t n0_bytes,
-                                     uint64_t n1, uint64_t n2, uint64_t s1, uint64_t s2,
-                                     uint32_t b0_words, uint32_t b1, const char* what) {
-  TensorMapEncodeTiledFn enc = tensor_map_encoder();
-  if (!enc) return fail(-1, "%s: cuTensorMapEncodeTiled is unavailable", what);
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (s1 & 15) || (s2 & 15) || (n0_bytes & 3))
-    return fail(-1, "%s: base and strides must be 16-byte aligned for TMA", what);
-  cuuint64_t dims[3] = {n0_bytes / 4, n1, n2};
-  cuuint64_t strides[2] = {s1, s2};
-  cuuint32_t box[3] = {b0_words, b1, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void*>(base), dims, strides, box,
-                   es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(-1, "%s: cuTensorMapEncodeTiled failed with %d", what, (int)r);
-  return 0;
+inline int make_tmap_u32_3d_prefetch(CUtensorMap* m, const void* base, uint64_t n0_bytes, uint64_t n1, uint64_t n2,
+                                     uint64_t s1, uint64_t s2, uint32_t b0_words, uint32_t b1, const char* what) {
+  if (n0_bytes & 3) return fail(-1, "%s: row length must be a multiple of four bytes", what);
+  return encode_tmap(m, {base, n0_bytes / 4, n1, n2, s1, s2, CU_TENSOR_MAP_DATA_TYPE_UINT32, CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, b0_words, b1}, what);
 }
 
 // Byte tensor as make_tmap_u8_3d_sw64, with rows of 128 bytes per box and the 128-byte swizzle.
-inline int make_tmap_u8_3d_sw128(CUtensorMap* m, const void* base, uint64_t n0, uint64_t n1,
-                                 uint64_t n2, uint64_t s1, uint64_t s2, uint32_t b1,
-                                 const char* what) {
-  TensorMapEncodeTiledFn enc = tensor_map_encoder();
-  if (!enc) return fail(-1, "%s: cuTensorMapEncodeTiled is unavailable", what);
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (s1 & 15) || (s2 & 15))
-    return fail(-1, "%s: base and strides must be 16-byte aligned for TMA", what);
-  cuuint64_t dims[3] = {n0, n1, n2};
-  cuuint64_t strides[2] = {s1, s2};
-  cuuint32_t box[3] = {128, b1, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box,
-                   es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(-1, "%s: cuTensorMapEncodeTiled failed with %d", what, (int)r);
-  return 0;
+inline int make_tmap_u8_3d_sw128(CUtensorMap* m, const void* base, uint64_t n0, uint64_t n1, uint64_t n2, uint64_t s1,
+                                 uint64_t s2, uint32_t b1, const char* what) {
+  return encode_tmap(m, {base, n0, n1, n2, s1, s2, CU_TENSOR_MAP_DATA_TYPE_UINT8, CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, 128, b1}, what);
 }
 
 // bf16 tensor [n2][n1][n0] with 128-byte swizzle, box [1][b1][64 elements]
-inline int make_tmap_bf16_3d_sw128(CUtensorMap* m, const void* base, uint64_t n0, uint64_t n1, uint64_t n2,
-                                   uint64_t s1_bytes, uint64_t s2_bytes, uint32_t b1, const char* what) {
-  TensorMapEncodeTiledFn enc = tensor_map_encoder();
-  if (!enc) return fail(-1, "%s: cuTensorMapEncodeTiled is unavailable", what);
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (s1_bytes & 15) || (s2_bytes & 15))
-    return fail(-1, "%s: base and strides must be 16-byte aligned for TMA", what);
-  cuuint64_t dims[3] = {n0, n1, n2};
-  cuuint64_t strides[2] = {s1_bytes, s2_bytes};
-  cuuint32_t box[3] = {64, b1, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, es,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(-1, "%s: cuTensorMapEncodeTiled failed with %d", what, (int)r);
-  return 0;
+inline int make_tmap_bf16_3d_sw128(CUtensorMap* m, const void* base, uint64_t n0, uint64_t n1, uint64_t n2, uint64_t s1_bytes,
+                                   uint64_t s2_bytes, uint32_t b1, const char* what) {
+  return encode_tmap(m, {base, n0, n1, n2, s1_bytes, s2_bytes, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, 64, b1}, what);
 }
 
 }  // namespace nvfp4

@@ -571,8 +571,17 @@ Tensor hybrid_decode(const Tensor& query, const Tensor& knv, const Tensor& ksc, 
 // Views of the first `cut` tokens of a cache, the V^T axis up to `s_pad` keys.
 std::tuple<Tensor, Tensor, Tensor, Tensor> packed_views(const Tensor& knv, const Tensor& ksc, const Tensor& vnv,
                                                         const Tensor& vsc, int64_t cut, int64_t s_pad) {
-  c10::NoGradGuard no_grad;
-  return {knv.narrow(1, 0, cut), ksc.narrow(1, 0, cut), vnv.narrow(2, 0, s_pad / 2), vsc.narrow(2, 0, s_pad / 16)};
+  // Plain strided views of buffers that never take part in autograd, made without a trip through the
+  // dispatcher (four narrow() calls cost a decode step as much as a kernel launch).
+  auto prefix = [](const Tensor& t, int64_t axis, int64_t n) {
+    require(t.dim() == 3 && n >= 0 && n <= t.size(axis), "view exceeds the cache");
+    Tensor v = at::detail::make_tensor<c10::TensorImpl>(c10::TensorImpl::VIEW, c10::Storage(t.storage()), t.key_set(), t.dtype());
+    int64_t sizes[3] = {t.size(0), t.size(1), t.size(2)};
+    sizes[axis] = n;
+    v.unsafeGetTensorImpl()->set_sizes_and_strides(at::IntArrayRef(sizes, 3), t.strides(), t.storage_offset());
+    return v;
+  };
+  return {prefix(knv, 1, cut), prefix(ksc, 1, cut), prefix(vnv, 2, s_pad / 2), prefix(vsc, 2, s_pad / 16)};
 }
 
 void append_token(const Tensor& key_new, const Tensor& value_new, const Tensor& knv, const Tensor& ksc, const Tensor& vnv,

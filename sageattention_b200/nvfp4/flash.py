@@ -458,18 +458,15 @@ class _NVFP4FlashAttn(torch.autograd.Function):
             query, key, value, scaling, causal=causal, num_key_value_groups=num_key_value_groups,
             key_pad_bias=key_pad_bias, return_lse=True, return_packs=True, out_layout=out_layout,
             q_packs=q_in, k_packs=k_in, _varlen_arrays=varlen)
-        bias = key_pad_bias if key_pad_bias is not None else torch.empty(0, device=query.device)
-        ctx.save_for_backward(query, key, value, out, lse, packs[0], packs[1], packs[2], packs[3], bias, *extra)
+        ctx.save_for_backward(query, key, value, out, lse, packs[0], packs[1], packs[2], packs[3], key_pad_bias, *extra)
         ctx.meta = (float(scaling), bool(causal), int(num_key_value_groups), varlen, out_layout,
-                    backward_grad_dots, key_pad_bias is not None,
-                    (bool(sr), backward_p_dv_sr, backward_dot_dv_sr, backward_ds_dq_sr))
+                    backward_grad_dots, (bool(sr), backward_p_dv_sr, backward_dot_dv_sr, backward_ds_dq_sr))
         return out
 
     @staticmethod
     def backward(ctx, grad_out):
         query, key, value, out, lse, qnv, qsc, knv, ksc, bias, *extra = ctx.saved_tensors
-        scaling, causal, g, varlen, out_layout, mode, has_bias, srk = ctx.meta
-        bias = bias if has_bias else None
+        scaling, causal, g, varlen, out_layout, mode, srk = ctx.meta
         if mode == "bf16":
             dq, dk, dv = _run_bwd_hp(query, key, value, out, lse, grad_out, scaling, causal, g, varlen,
                                      out_layout, q_packs=(qnv, qsc), k_packs=(knv, ksc), key_pad_bias=bias)

@@ -76,7 +76,6 @@ class NVFP4KVCache:
             self.rv = torch.zeros(z, hk, self.ring_cap, d, dtype=dtype, device=dev)
 
     # ------------------------------------------------------------------ prefill
-    @torch.no_grad()
     def prefill(self, key: torch.Tensor, value: torch.Tensor):
         """Pack a prompt's K/V ([Z, Hk, S, D]) into the cache (kv_cache.py:187-224)."""
         z, hk, s, d = key.shape
@@ -87,6 +86,7 @@ class NVFP4KVCache:
             self._prefill_converting(key, value)
         self.length, self.partial_len = s, s % self.GROUP
 
+    @torch.no_grad()
     def _prefill_converting(self, key, value):
         """Operands of another dtype than the cache's (or strided along D): packed as they are, while the
         open V group and the rings hold them rounded to the cache's dtype."""
@@ -113,7 +113,6 @@ class NVFP4KVCache:
             self.rv[:, :, slots] = value[:, :, s - w :].to(self.dtype)
 
     # ------------------------------------------------------------------ append
-    @torch.no_grad()
     def append(self, key_new: torch.Tensor, value_new: torch.Tensor):
         """Append one decode token ([Z, Hk, 1, D]); a single kernel launch (kv_cache.py:227-257)."""
         z, hk, sq, d = key_new.shape
@@ -121,12 +120,10 @@ class NVFP4KVCache:
         t = self.length
         assert t < self.max_seq_len, "append exceeds capacity"
         ring = self.recent_window > 0
-        append_token(key_new, value_new, self.knv, self.ksc, self.vnv, self.vsc, self.v_partial_bf16,
-                     self.rk if ring else None, self.rv if ring else None, t)
+        _lib.native().append_token(key_new, value_new, self.knv, self.ksc, self.vnv, self.vsc, self.v_partial_bf16,
+                                   self.rk if ring else None, self.rv if ring else None, t)
         self.length = t + 1
-        self.partial_len = (t % self.GROUP) + 1
-        if self.partial_len == self.GROUP:
-            self.partial_len = 0
+        self.partial_len = (t + 1) % self.GROUP
 
     # ------------------------------------------------------------------ views
     def get_packed(self) -> tuple:
@@ -140,7 +137,6 @@ class NVFP4KVCache:
         return (*_lib.native().packed_views(self.knv, self.ksc, self.vnv, self.vsc, cut, s_pad), cut, s_pad)
 
     # ------------------------------------------------------------------ hybrid decode
-    @torch.no_grad()
     def hybrid_decode(self, query: torch.Tensor, scaling: float, g: int) -> torch.Tensor:
         """Recent-window bf16 attention + FP4 attention over the older prefix, merged by LSE.
 
