@@ -12,6 +12,10 @@
 #include <c10/core/GradMode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <cstdlib>
@@ -808,6 +812,80 @@ std::tuple<Tensor, Tensor, Tensor> bwd_fp4(const Tensor& q, const Tensor& k, con
   return {dq, dk, dv};
 }
 
+// ---------------------------------------------------------------- autograd
+// The differentiable attention as a graph node of its own: a Python autograd.Function with the
+// operator's 26 arguments costs ~55 us per forward and backward before any kernel is launched, more than
+// the kernels of a short training step.  The node keeps the operands and calls the package's backward
+// entry (flash._attention_backward, which picks the kernels by mode).
+PyObject* g_backward = nullptr;        // set once by the package; never released
+
+void set_backward(py::object fn) { g_backward = fn.release().ptr(); }
+
+struct AttentionBackward : torch::autograd::Node {
+  torch::autograd::SavedVariable q, k, v, out, lse, qnv, qsc, knv, ksc, bias, seq_id, seq_start, seq_end;
+  double scaling = 0.0;
+  bool causal = false, zshd = false, sr = false;
+  int64_t g = 1;
+  std::string mode;
+  std::optional<bool> sr_p_dv, sr_dot_dv, sr_ds_dq;
+
+  std::string name() const override { return "NVFP4AttentionBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (auto* x : {&q, &k, &v, &out, &lse, &qnv, &qsc, &knv, &ksc, &bias, &seq_id, &seq_start, &seq_end}) x->reset_data();
+  }
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    if (!grads[0].defined()) return torch::autograd::variable_list(3);
+    Tensor qt, kt, vt, ot, lt;
+    OptTensor o[8];
+    {   // not held while waiting for the interpreter's lock
+      std::lock_guard<std::mutex> lock(mutex_);
+      qt = q.unpack(), kt = k.unpack(), vt = v.unpack(), ot = out.unpack(shared_from_this()), lt = lse.unpack();
+      const torch::autograd::SavedVariable* saved[8] = {&seq_id, &seq_start, &seq_end, &qnv, &qsc, &knv, &ksc, &bias};
+      for (int i = 0; i < 8; ++i)
+        if (Tensor t = saved[i]->unpack(); t.defined()) o[i] = t;
+    }
+    py::gil_scoped_acquire gil;
+    py::object r = py::reinterpret_borrow<py::object>(g_backward)(
+        qt, kt, vt, ot, lt, grads[0], scaling, causal, g, o[0], o[1], o[2], zshd, mode, o[3], o[4], o[5], o[6], o[7], sr,
+        sr_p_dv, sr_dot_dv, sr_ds_dq);
+    auto t = r.cast<std::tuple<Tensor, Tensor, Tensor>>();
+    return {std::get<0>(t), std::get<1>(t), std::get<2>(t)};
+  }
+};
+
+Tensor attention(const Tensor& query, const Tensor& key, const Tensor& value, double scaling, bool causal, int64_t g,
+                 const OptTensor& bias, const OptTensor& seq_id, const OptTensor& seq_start, const OptTensor& seq_end, bool zshd,
+                 const OptTensor& qnv, const OptTensor& qsc, const OptTensor& knv, const OptTensor& ksc, const std::string& mode,
+                 bool sr, std::optional<bool> sr_p_dv, std::optional<bool> sr_dot_dv, std::optional<bool> sr_ds_dq) {
+  const bool record = c10::GradMode::is_enabled() && (query.requires_grad() || key.requires_grad() || value.requires_grad());
+  c10::AutoGradMode no_grad(false);
+  auto [out, lse, packs] = flash_attention(query, key, value, scaling, causal, g, bias, false, seq_id, seq_start, zshd, true,
+                                           record, qnv, qsc, knv, ksc);
+  if (!record) return out;
+  std::shared_ptr<AttentionBackward> node(new AttentionBackward(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(query, key, value));
+  using torch::autograd::SavedVariable;
+  auto keep = [](const OptTensor& t) { return SavedVariable(t.has_value() ? *t : Tensor(), false); };
+  node->q = SavedVariable(query, false);
+  node->k = SavedVariable(key, false);
+  node->v = SavedVariable(value, false);
+  node->lse = SavedVariable(*lse, false);
+  node->qnv = SavedVariable(packs[0], false);
+  node->qsc = SavedVariable(packs[1], false);
+  node->knv = SavedVariable(packs[2], false);
+  node->ksc = SavedVariable(packs[3], false);
+  node->bias = keep(bias);
+  node->seq_id = keep(seq_id);
+  node->seq_start = keep(seq_start);
+  node->seq_end = keep(seq_end);
+  node->scaling = scaling; node->causal = causal; node->zshd = zshd; node->g = g; node->mode = mode;
+  node->sr = sr; node->sr_p_dv = sr_p_dv; node->sr_dot_dv = sr_dot_dv; node->sr_ds_dq = sr_ds_dq;
+  torch::autograd::set_history(out, node);
+  node->out = SavedVariable(out, true);
+  return out;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_native, m) {
@@ -841,4 +919,6 @@ PYBIND11_MODULE(_native, m) {
   m.def("bf16_rows", &bf16_rows, nogil());
   m.def("bwd_hp", &bwd_hp, nogil());
   m.def("bwd_fp4", &bwd_fp4, nogil());
+  m.def("set_backward", &set_backward);
+  m.def("attention", &attention, nogil());
 }

@@ -167,53 +167,80 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(
 // Half-split convention ("rotate_half"): y[i] = x[i] cos[i] - x[i + D/2] sin[i] for i < D/2,
 // y[i] = x[i] cos[i - D/2] + x[i - D/2] sin[i - D/2] otherwise; computed in fp32, rounded once to
 // the input dtype (what an unfused rotary kernel would have stored), then packed like pack_rows.
+//
+// One thread = the two 16-groups that rotate into each other, over `nb` batch entries (heads).  x is read
+// once, and cos / sin -- 128 bytes a thread, four times the bytes of a 16-bit group -- once for all the
+// entries: one thread per group and entry was bound by the L1 / L2 reads of the tables and of the
+// partner group.
 template <typename T>
-__global__ void __launch_bounds__(256) rope_pack_rows_kernel(
-    const T* __restrict__ x, int64_t R, int d, int ngroups_log2, int64_t per_batch, int64_t sxb,
+__global__ void __launch_bounds__(256, 2) rope_pack_rows_kernel(
+    const T* __restrict__ x, int B, int d, int pairs_log2, int64_t npairs, int nb, int64_t sxb,
     int64_t sxr, const float* __restrict__ cs, const float* __restrict__ sn,
     const int32_t* __restrict__ positions, int64_t pos0, uint8_t* __restrict__ nib, int64_t snb,
-    int64_t snr, uint8_t* __restrict__ sc, int64_t ssb, int64_t ssr, int vec_in) {
+    int64_t snr, uint8_t* __restrict__ sc, int64_t ssb, int64_t ssr, int align) {
+  constexpr int kW = 16 * sizeof(T) / 4;          // 32-bit words per group
   griddep_launch();
   griddep_wait();
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= per_batch) return;
-  const int64_t b = blockIdx.y;
-  const int ngroups = d >> 4, half = d >> 1;
-  const int g = (int)(gid & (ngroups - 1));
-  const int64_t r = gid >> ngroups_log2;
-  const bool upper = g * 16 >= half;
-  const int gp = upper ? g - (ngroups >> 1) : g + (ngroups >> 1);      // partner group
-  const T* row = x + b * sxb + r * sxr;
+  if (gid >= npairs) return;
+  const int half = d >> 1;
+  const int g = (int)(gid & ((1 << pairs_log2) - 1));
+  const int64_t r = gid >> pairs_log2;
   const int64_t pos = positions ? (int64_t)positions[r] : pos0 + r;
-  const float* c = cs + pos * half + (upper ? gp : g) * 16;
-  const float* s_ = sn + pos * half + (upper ? gp : g) * 16;
-  float a[16], pa[16];
-  {
-    float t0[8], t1[8];
-    load8<T>(row + g * 16, vec_in, 16, t0);
-    load8<T>(row + g * 16 + 8, vec_in, 8, t1);
+  const float4* c4 = reinterpret_cast<const float4*>(cs + pos * half + g * 16);
+  const float4* s4 = reinterpret_cast<const float4*>(sn + pos * half + g * 16);
+  float c[16], s[16];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { a[i] = t0[i]; a[8 + i] = t1[i]; }
-    load8<T>(row + gp * 16, vec_in, 16, t0);
-    load8<T>(row + gp * 16 + 8, vec_in, 8, t1);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { pa[i] = t0[i]; pa[8 + i] = t1[i]; }
+  for (int i = 0; i < 4; ++i) {
+    const float4 a = c4[i], b = s4[i];
+    c[4 * i] = a.x; c[4 * i + 1] = a.y; c[4 * i + 2] = a.z; c[4 * i + 3] = a.w;
+    s[4 * i] = b.x; s[4 * i + 1] = b.y; s[4 * i + 2] = b.z; s[4 * i + 3] = b.w;
   }
-  float v[16];
+  auto fetch = [&](const T* p, uint32_t (&raw)[kW]) {
+    if (align == 32) {
 #pragma unroll
-  for (int i = 0; i < 16; i += 4) {
-    const float4 c4 = *reinterpret_cast<const float4*>(c + i), s4 = *reinterpret_cast<const float4*>(s_ + i);
-    const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
+      for (int j = 0; j < kW / 8; ++j)
+        ldg256(reinterpret_cast<const uint32_t*>(p) + 8 * j, *reinterpret_cast<uint32_t(*)[8]>(&raw[8 * j]));
+    } else if (align == 16) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float rot = upper ? pa[i + e] : -pa[i + e];
-      v[i + e] = to_f32<T>(from_f32<T>(__fmaf_rn(rot, ss[e], a[i + e] * cc[e])));
+      for (int j = 0; j < kW / 4; ++j) {
+        const uint4 w = reinterpret_cast<const uint4*>(p)[j];
+        raw[4 * j] = w.x; raw[4 * j + 1] = w.y; raw[4 * j + 2] = w.z; raw[4 * j + 3] = w.w;
+      }
+    } else {
+      T* e = reinterpret_cast<T*>(raw);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) e[j] = p[j];
     }
+  };
+  const int b0 = blockIdx.y * nb, b1 = min(b0 + nb, B);
+  const T* row = x + b0 * sxb + r * sxr + g * 16;
+  uint32_t lo[kW], hi[kW];
+  fetch(row, lo);
+  fetch(row + half, hi);
+  for (int b = b0; b < b1; ++b) {
+    float u[16], v[16];
+    const T* el = reinterpret_cast<const T*>(lo);
+    const T* eh = reinterpret_cast<const T*>(hi);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float a = to_f32<T>(el[i]), h = to_f32<T>(eh[i]);
+      u[i] = to_f32<T>(from_f32<T>(__fmaf_rn(-h, s[i], a * c[i])));
+      v[i] = to_f32<T>(from_f32<T>(__fmaf_rn(a, s[i], h * c[i])));
+    }
+    if (b + 1 < b1) {                             // the next entry's loads fly under this one's pack
+      row += sxb;
+      fetch(row, lo);
+      fetch(row + half, hi);
+    }
+    uint32_t w0, w1;
+    uint8_t* pn = nib + b * snb + r * snr + g * 8;
+    uint8_t* ps = sc + b * ssb + r * ssr + g;
+    ps[0] = pack_group16(u, w0, w1);
+    *reinterpret_cast<uint2*>(pn) = make_uint2(w0, w1);
+    ps[half >> 4] = pack_group16(v, w0, w1);
+    *reinterpret_cast<uint2*>(pn + (half >> 1)) = make_uint2(w0, w1);
   }
-  uint32_t lo, hi;
-  const uint8_t sb = pack_group16(v, lo, hi);
-  *reinterpret_cast<uint2*>(nib + b * snb + r * snr + g * 8) = make_uint2(lo, hi);
-  sc[b * ssb + r * ssr + g] = sb;
 }
 
 // ---------------------------------------------------------------- rows contiguous (V^T)
@@ -993,18 +1020,22 @@ extern "C" int nvfp4_rope_pack(const void* x, int dtype, int64_t B, int64_t R, i
                 "nvfp4_rope_pack: cos / sin tables must be 16-byte aligned");
   if (B == 0 || R == 0) return 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int ngroups = d / 16;
+  const int pairs = d / 32;
   int lg = 0;
-  while ((1 << lg) < ngroups) ++lg;
-  const int64_t per_batch = R * ngroups;
-  const int64_t blocks = (per_batch + 255) / 256;
+  while ((1 << lg) < pairs) ++lg;
+  const int64_t npairs = R * pairs;
+  const int64_t blocks = (npairs + 255) / 256;
   NVFP4_REQUIRE(blocks < (1LL << 31), "nvfp4_rope_pack: tensor too large");
-  dim3 grid((unsigned)blocks, (unsigned)B);
+  // Entries per block: up to 8, beyond which the tables' share of the reads no longer falls, while the
+  // grid keeps 1024 blocks -- three waves of two blocks on each of 148 SMs; a short tensor is bound by latency.
+  const int nb = (int)std::max<int64_t>(1, std::min<int64_t>(8, B * blocks / 1024));
+  dim3 grid((unsigned)blocks, (unsigned)((B + nb - 1) / nb));
   const int es = dtype == NVFP4_DT_FP32 ? 4 : 2;
-  const int vec = ((uintptr_t)x % 16 == 0) && (sxb * es) % 16 == 0 && (sxr * es) % 16 == 0;
+  const int64_t bits = (int64_t)(uintptr_t)x | (sxb * es) | (sxr * es);
+  const int align = bits % 32 == 0 ? 32 : (bits % 16 == 0 ? 16 : 1);
 #define NVFP4_ROPE(T)                                                                              \
-  return launch("nvfp4_rope_pack", rope_pack_rows_kernel<T>, grid, 256, 0, st, static_cast<const T*>(x), R, d, lg, \
-                per_batch, sxb, sxr, cos_tab, sin_tab, positions, pos0, nib, snb, snr, sc, ssb, ssr, vec)
+  return launch("nvfp4_rope_pack", rope_pack_rows_kernel<T>, grid, 256, 0, st, static_cast<const T*>(x), (int)B, d, lg, \
+                npairs, nb, sxb, sxr, cos_tab, sin_tab, positions, pos0, nib, snb, snr, sc, ssb, ssr, align)
   switch (dtype) {
     case NVFP4_DT_BF16: NVFP4_ROPE(__nv_bfloat16);
     case NVFP4_DT_FP16: NVFP4_ROPE(__half);

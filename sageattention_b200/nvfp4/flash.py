@@ -468,16 +468,28 @@ class _NVFP4FlashAttn(torch.autograd.Function):
         query, key, value, out, lse, qnv, qsc, knv, ksc, bias, *extra = ctx.saved_tensors
         scaling, causal, g, varlen, out_layout, mode, srk = ctx.meta
         if mode == "bf16":
-            dq, dk, dv = _run_bwd_hp(query, key, value, out, lse, grad_out, scaling, causal, g, varlen,
+            grads = _run_bwd_hp(query, key, value, out, lse, grad_out, scaling, causal, g, varlen,
                                      out_layout, q_packs=(qnv, qsc), k_packs=(knv, ksc), key_pad_bias=bias)
         else:
-            dq, dk, dv = _run_bwd(query, key, value, out, lse, grad_out, scaling, causal, g, varlen,
+            grads = _run_bwd(query, key, value, out, lse, grad_out, scaling, causal, g, varlen,
                                   out_layout, mode=mode, q_packs=(qnv, qsc), k_packs=(knv, ksc),
                                   key_pad_bias=bias, sr=srk[0], sr_p_dv=srk[1], sr_dot_dv=srk[2],
                                   sr_ds_dq=srk[3], qt_packs=tuple(extra[0:2]) if extra else None,
                                   kt_packs=tuple(extra[2:4]) if extra else None,
                                   vd_packs=tuple(extra[4:6]) if extra else None)
-        return (dq, dk, dv) + (None,) * 23
+        return (*grads,) + (None,) * 23
+
+
+def _attention_backward(query, key, value, out, lse, grad_out, scaling, causal, g, seq_id, seq_start, seq_end, zshd, mode,
+                        qnv, qsc, knv, ksc, bias, sr, sr_p_dv, sr_dot_dv, sr_ds_dq):
+    """Backward entry of the native graph node of ``nvfp4_flash_attn_func``: ``(dq, dk, dv)``."""
+    varlen = (seq_id, seq_start, seq_end) if seq_id is not None else None
+    layout = "zshd" if zshd else "zhsd"
+    if mode == "bf16":
+        return _run_bwd_hp(query, key, value, out, lse, grad_out, scaling, causal, g, varlen, layout, q_packs=(qnv, qsc),
+                           k_packs=(knv, ksc), key_pad_bias=bias)
+    return _run_bwd(query, key, value, out, lse, grad_out, scaling, causal, g, varlen, layout, mode=mode, q_packs=(qnv, qsc),
+                    k_packs=(knv, ksc), key_pad_bias=bias, sr=sr, sr_p_dv=sr_p_dv, sr_dot_dv=sr_dot_dv, sr_ds_dq=sr_ds_dq)
 
 
 def nvfp4_flash_attn_func(query, key, value, scaling, causal=False, num_key_value_groups=1,
@@ -509,6 +521,8 @@ def nvfp4_flash_attn_func(query, key, value, scaling, causal=False, num_key_valu
         # AUTO on the effective sequence: s_kv, or the mean sample length of a packed row
         eff = s_kv if cu_seqlens is None else s_q / max(1, cu_seqlens.numel() - 1)
         backward_grad_dots = _resolve_backward_grad_dots(None, eff, save_backward_packs, num_key_value_groups)
+    else:
+        backward_grad_dots = _resolve_backward_grad_dots(backward_grad_dots, s_kv, save_backward_packs, num_key_value_groups)
     seq_id = seq_start = seq_end = None
     if cu_seqlens is not None:
         assert causal, "varlen (cu_seqlens) implements block-diagonal causal attention; pass causal=True"
@@ -521,6 +535,13 @@ def nvfp4_flash_attn_func(query, key, value, scaling, causal=False, num_key_valu
             "(the saved pack set must come from the same fused HP read)")
     qnv_in, qsc_in = q_packs if q_packs is not None else (None, None)
     knv_in, ksc_in = k_packs if k_packs is not None else (None, None)
+    if not save_backward_packs:
+        optional = lambda x: None if x is None else bool(x)
+        return _lib.native().attention(
+            query, key, value, scaling, causal, num_key_value_groups, key_pad_bias, seq_id, seq_start, seq_end,
+            out_layout == "zshd", qnv_in, qsc_in, knv_in, ksc_in, backward_grad_dots, bool(stochastic_rounding),
+            optional(backward_p_dv_stochastic_rounding), optional(backward_dot_dv_stochastic_rounding),
+            optional(backward_ds_dq_stochastic_rounding))
     return _NVFP4FlashAttn.apply(
         query, key, value, scaling, causal, num_key_value_groups, key_pad_bias, stochastic_rounding,
         save_backward_packs, backward_p_dv_stochastic_rounding, backward_dot_dv_stochastic_rounding,
