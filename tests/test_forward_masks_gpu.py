@@ -1,0 +1,60 @@
+"""Forward masks at the edges of key tiles: biases that are zero in whole tiles and not in others, and samples of
+packed rows that end at, before and behind tile and chunk boundaries, causal or not, with and without a bias."""
+
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import cos, seeded_bf16
+from oracle import nvfp4_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+MAXABS = 2e-2
+
+
+def _check(q, k, v, qf, kf, vf, h, hk, causal, bias=None, cu=None):
+    import sageattention_b200.nvfp4 as nv
+    from sageattention_b200 import _lib
+    z, _, sq, d = q.shape
+    skv = k.shape[2]
+    packs = nv.nvfp4_flash_attention(q, k, v, d ** -0.5, num_key_value_groups=h // hk, return_packs=True)[1]
+    out = nv.nvfp4_flash_attention_packed(
+        *packs, z, h, hk, sq, skv, d, d ** -0.5, torch.float32, causal=causal,
+        key_pad_bias=None if bias is None else torch.from_numpy(bias).cuda(),
+        cu_seqlens=None if cu is None else torch.tensor(cu, dtype=torch.int32, device="cuda"))
+    assert _lib.read_status("cuda") == 0
+    ref, _ = O.attention_mode_b(qf, kf, vf, d ** -0.5, causal, h // hk, cu_seqlens=cu, key_pad_bias=bias)
+    o = out.cpu().numpy()
+    assert np.isfinite(o).all()
+    assert cos(o, ref) >= 0.9999 and np.abs(o - ref).max() <= MAXABS, (cos(o, ref), np.abs(o - ref).max())
+
+
+@pytest.mark.parametrize("d", [128, 256])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("keys", [(), (127,), (128,), (255, 256), range(256, 700), range(640, 700), (0, 699)])
+def test_bias_in_some_tiles(d, causal, keys):
+    z, h, hk, sq, skv = 2, 2, 1, 150, 700
+    q, qf = seeded_bf16((z, h, sq, d), 51)
+    k, kf = seeded_bf16((z, hk, skv, d), 52)
+    v, vf = seeded_bf16((z, hk, skv, d), 53)
+    bias = np.zeros((z, skv), np.float32)
+    bias[1, list(keys)] = -np.inf                  # the other entry of the batch has no bias at all
+    if len(keys) == 2:
+        bias[1, keys[0]] = 2.5
+    _check(q, k, v, qf, kf, vf, h, hk, causal, bias=bias)
+
+
+@pytest.mark.parametrize("d", [128, 256])
+@pytest.mark.parametrize("causal,biased", [(True, False), (True, True), (False, False), (False, True)])
+@pytest.mark.parametrize("lens", [(128, 128, 128), (1, 127, 129, 31, 32, 33), (400, 3, 300), (63, 65, 1, 1, 254, 17)])
+def test_packed_samples(d, causal, biased, lens):
+    h, hk, s = 2, 1, sum(lens)
+    q, qf = seeded_bf16((1, h, s, d), 61)
+    k, kf = seeded_bf16((1, hk, s, d), 62)
+    v, vf = seeded_bf16((1, hk, s, d), 63)
+    bias = None
+    if biased:
+        bias = np.zeros((1, s), np.float32)
+        bias[0, 1::7] = -3.0
+    _check(q, k, v, qf, kf, vf, h, hk, causal, bias=bias, cu=np.cumsum((0,) + lens))
