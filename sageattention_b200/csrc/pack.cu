@@ -1026,9 +1026,15 @@ extern "C" int nvfp4_rope_pack(const void* x, int dtype, int64_t B, int64_t R, i
   const int64_t npairs = R * pairs;
   const int64_t blocks = (npairs + 255) / 256;
   NVFP4_REQUIRE(blocks < (1LL << 31), "nvfp4_rope_pack: tensor too large");
-  // Entries per block: up to 8, beyond which the tables' share of the reads no longer falls, while the
-  // grid keeps 1024 blocks -- three waves of two blocks on each of 148 SMs; a short tensor is bound by latency.
-  const int nb = (int)std::max<int64_t>(1, std::min<int64_t>(8, B * blocks / 1024));
+  // Entries per block: two blocks fit an SM; where up to four entries a block bring the grid into one wave, as
+  // many (a second wave costs more than a block's second entry: [32, 2048, 128] 9.9 us with one, 7.5 with
+  // four), else as many, up to eight, as leave four waves to even out.
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  auto entries = [&](int64_t grid) { return (B * blocks + grid - 1) / grid; };
+  int nb = (int)entries(2 * sms);
+  if (nb > 4) nb = (int)std::min<int64_t>(8, entries(8 * sms));
   dim3 grid((unsigned)blocks, (unsigned)((B + nb - 1) / nb));
   const int es = dtype == NVFP4_DT_FP32 ? 4 : 2;
   const int64_t bits = (int64_t)(uintptr_t)x | (sxb * es) | (sxr * es);

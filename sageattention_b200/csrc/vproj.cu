@@ -8,9 +8,14 @@
 // tokens on its columns: the 16-token groups of the pack are thread-local in the epilogue and a
 // thread writes 64 contiguous nibble bytes + 8 scale bytes of its row.
 //
-// One CTA = 128 features x 128 tokens of one batch entry; K loop over the hidden dim in 64-element
+// One tile = 128 features x 128 tokens of one batch entry; K loop over the hidden dim in 64-element
 // stages (TMA, 128-byte swizzle, 4-stage ring), tcgen05.mma kind::f16 M128 N128 K16, accumulator in
-// 128 TMEM columns.  Warps: 0 TMA producer, 1 MMA issuer, 2-5 epilogue.
+// 128 TMEM columns.  Warps: 0 TMA producer, 1 MMA issuer, 2-17 epilogue (32 tokens of 32 features each).
+//
+// What bounds it: a stage's 32 KB take ~470 clocks to arrive (an SM's share of L2; the MMAs need 260; a ring of six stages
+// is no faster), so a tile of hidden 4096 costs 16 us however few there are.  Where tiles are fewer than
+// SMs, a cluster of 2, 4 or 8 CTAs shares one: each takes a range of the hidden dim, leaves its fp32 partial
+// in its shared memory, and finishes its share of the tokens from all partials in rank order.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
 #include "common/launch.cuh"
@@ -20,9 +25,12 @@
 
 namespace nvfp4 {
 
-constexpr int kVpThreads = 192;
+constexpr int kVpThreads = 576;
 constexpr int kVpStages = 4;
 constexpr int kVpTile = 128 * 64 * 2;      // bytes of one operand tile of a stage
+// A partial in shared memory, in place of the ring: [token / 4][feature][token % 4], so that a warp, a feature per lane,
+// writes and (through the cluster) reads 512 consecutive bytes at a time.
+static_assert(128 * 128 * 4 <= kVpStages * 2 * kVpTile, "a partial takes the place of the ring");
 
 struct VprojParams {
   const void* bias;      // [features] in the operand dtype, or null
@@ -30,10 +38,45 @@ struct VprojParams {
   uint8_t* vsc;          // [Z*Hk, D, s_pad/16]
   void* v_out;           // [Z, S, features] (element strides svb, svs; unit feature stride) or null
   int64_t svb, svs;
-  int features, d, hk, s, s_pad, hidden;
+  int features, d, hk, s, s_pad, hidden, split;
   int f16;
   int* status;
 };
+
+// 16 tokens from `tok` of feature f: bias, rounding to the operand dtype (what an unfused projection would have
+// stored), the value and its pack; tokens behind S are +0.0, groups behind the padded extent do not exist.
+template <typename T>
+__device__ __forceinline__ void vproj_store(const VprojParams& p, int zi, int f, int tok, float (&v)[16]) {
+  if (f >= p.features || tok >= p.s_pad) return;
+  const float b = p.bias != nullptr ? to_f32<T>(static_cast<const T*>(p.bias)[f]) : 0.0f;
+  T* vo = p.v_out ? static_cast<T*>(p.v_out) + (int64_t)zi * p.svb + f : nullptr;
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    const T hv = from_f32<T>(v[e] + b);
+    v[e] = (tok + e < p.s) ? to_f32<T>(hv) : 0.0f;
+    if (vo != nullptr && tok + e < p.s) vo[(int64_t)(tok + e) * p.svs] = hv;
+  }
+  uint32_t lo, hi;
+  const uint8_t sb = pack_group16(v, lo, hi);
+  const int64_t row = ((int64_t)zi * p.hk + f / p.d) * p.d + f % p.d;
+  *reinterpret_cast<uint2*>(p.vnv + row * (p.s_pad / 2) + tok / 2) = make_uint2(lo, hi);
+  p.vsc[row * (p.s_pad / 16) + tok / 16] = sb;
+}
+
+// CTAs per tile: the split with the fewest waves x (stages of a CTA + 12 for its start and epilogue, + 6 for the
+// exchange of a split one), in units of a stage's ~0.25 us.  Clusters of eight do not fill the chip (sixteen of
+// them took two waves), hence three quarters of it.  [S, hidden] x 1024 features: 509 x 4096 22.6 -> 11.4 us,
+// 2430 x 4096 44.9 -> 36.5; sixteen epilogue warps instead of four are 2.5 us of each wave, 2048 x 4096 23.8 -> 21.1.
+inline int vproj_split(int64_t tiles, int stages, int sms) {
+  int best = 1;
+  int64_t best_cost = INT64_MAX / 2;
+  for (int n = 1; n <= 8 && n <= stages; n *= 2) {
+    const int64_t room = n == 8 ? sms * 3 / 4 : sms;
+    const int64_t cost = (tiles * n + room - 1) / room * ((stages + n - 1) / n + 12 + (n > 1 ? 6 : 0));
+    if (cost < best_cost - best_cost / 16) { best_cost = cost; best = n; }
+  }
+  return best;
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kVpThreads, 1)
@@ -46,8 +89,10 @@ vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int f0 = blockIdx.x * 128, t0 = blockIdx.y * 128, zi = blockIdx.z;
-  const int nstage = (p.hidden + 63) / 64;
+  const int f0 = blockIdx.x * 128, t0 = blockIdx.y * 128;
+  const int zi = blockIdx.z / p.split, rank = blockIdx.z - zi * p.split;     // rank of the CTA in its cluster
+  const int all = (p.hidden + 63) / 64;
+  const int st0 = (int)((int64_t)all * rank / p.split), nstage = (int)((int64_t)all * (rank + 1) / p.split) - st0;
   if (tid == 0) {
     err = 0;
     for (int i = 0; i < kVpStages; ++i) {
@@ -72,8 +117,8 @@ vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         if (st >= kVpStages) mbar_wait(&empty[s], ((st / kVpStages) & 1) ^ 1, &err, 1);
         uint8_t* sb = smem + s * 2 * kVpTile;
         mbar_expect_tx(&full[s], 2 * kVpTile);
-        tma_load_3d(sb, &tm_w, &full[s], st * 64, f0, 0);
-        tma_load_3d(sb + kVpTile, &tm_x, &full[s], st * 64, t0, zi);
+        tma_load_3d(sb, &tm_w, &full[s], (st0 + st) * 64, f0, 0);
+        tma_load_3d(sb + kVpTile, &tm_x, &full[s], (st0 + st) * 64, t0, zi);
       }
     }
     __syncwarp();
@@ -94,45 +139,49 @@ vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     }
     __syncwarp();
   } else {
-    // epilogue: thread = feature row f0 + 32 (warp % 4) + lane, columns = 128 tokens
-    const int wq = warp & 3;
-    const int f = f0 + wq * 32 + lane;
-    const bool f_ok = f < p.features;
-    const float b = (f_ok && p.bias != nullptr) ? to_f32<T>(static_cast<const T*>(p.bias)[f]) : 0.0f;
+    // epilogue: thread = feature row 32 (warp % 4) + lane, 32 of the tokens
+    const int ep = tid - 64, row = (warp & 3) * 32 + lane, c = ep >> 7;
     mbar_wait(&acc_done, 0, &err, 3);
     tc_fence_after();
-    const int64_t unit = (int64_t)zi * p.hk + (f_ok ? f / p.d : 0);
-    const int dr = f_ok ? f % p.d : 0;
-    uint8_t* nrow = p.vnv + (unit * p.d + dr) * (int64_t)(p.s_pad / 2) + t0 / 2;
-    uint8_t* srow = p.vsc + (unit * p.d + dr) * (int64_t)(p.s_pad / 16) + t0 / 16;
-    T* vo = p.v_out ? static_cast<T*>(p.v_out) + (int64_t)zi * p.svb + f : nullptr;
-#pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
-      uint32_t r[32];
-      tmem_ld32(tmem + ((uint32_t)(wq * 32) << 16) + c * 32, r);
-      tmem_ld_wait();
+    uint32_t r[32];
+    tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c * 32, r);
+    tmem_ld_wait();
+    tc_fence_before();
+    if (p.split == 1) {
 #pragma unroll
       for (int gi = 0; gi < 2; ++gi) {
-        const int tok = t0 + c * 32 + gi * 16;
-        if (tok >= p.s_pad) continue;       // groups behind the padded extent do not exist
         float v[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          // what an unfused projection would have stored: rounded once to the operand dtype;
-          // tokens behind S are +0.0
-          const T hv = from_f32<T>(__uint_as_float(r[gi * 16 + e]) + b);
-          v[e] = (tok + e < p.s) ? to_f32<T>(hv) : 0.0f;
-          if (vo != nullptr && f_ok && tok + e < p.s) vo[(int64_t)(tok + e) * p.svs] = hv;
-        }
-        uint32_t lo, hi;
-        const uint8_t sb = pack_group16(v, lo, hi);
-        if (f_ok) {
-          *reinterpret_cast<uint2*>(nrow + (c * 32 + gi * 16) / 2) = make_uint2(lo, hi);
-          srow[(c * 32 + gi * 16) / 16] = sb;
+        for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r[gi * 16 + e]);
+        vproj_store<T>(p, zi, f0 + row, t0 + c * 32 + gi * 16, v);
+      }
+    } else {
+      float4* part = reinterpret_cast<float4*>(smem) + c * 8 * 128 + row;
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        part[e * 128] = make_float4(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1]), __uint_as_float(r[4 * e + 2]),
+                              __uint_as_float(r[4 * e + 3]));
+    }
+  }
+  if (p.split > 1) {
+    cluster_sync_all();
+    const int ep = tid - 64, groups = 8 / p.split;         // 16-token groups of this CTA
+    if (ep >= 0 && (ep >> 7) < groups) {
+      const int row = ep & 127, gt = (rank * groups + (ep >> 7)) * 16;
+      const uint32_t a = smem_u32(smem) + (uint32_t)(gt / 4 * 128 + row) * 16u;
+      float v[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) v[e] = 0.0f;
+      for (int k = 0; k < p.split; ++k) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float4 x = ld_cluster_f4(a + 2048 * e, k);
+          v[4 * e] += x.x; v[4 * e + 1] += x.y; v[4 * e + 2] += x.z; v[4 * e + 3] += x.w;
         }
       }
+      vproj_store<T>(p, zi, f0 + row, t0 + gt, v);
     }
-    tc_fence_before();
+    cluster_sync_all();                                    // the partials stay until every CTA has read them
   }
   __syncthreads();
   if (tid == 0 && err != 0 && p.status != nullptr) atomicExch(p.status, err);
@@ -170,11 +219,16 @@ extern "C" int nvfp4_vproj_pack(const void* x, const void* w, const void* bias, 
   p.f16 = dtype == NVFP4_DT_FP16 ? 1 : 0; p.status = status;
   const int smem = kVpStages * 2 * kVpTile + 1024;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  dim3 grid((unsigned)((features + 127) / 128), (unsigned)((s_pad + 127) / 128), (unsigned)z);
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t tf = (features + 127) / 128, tt = (s_pad + 127) / 128;
+  p.split = z * 8 < 65536 ? vproj_split(tf * tt * z, (int)((hidden + 63) / 64), sms) : 1;
+  dim3 grid((unsigned)tf, (unsigned)tt, (unsigned)(z * p.split));
 #define NVFP4_VP(T)                                                                                       \
   {                                                                                                       \
     if ((rc = allow_smem("nvfp4_vproj_pack", reinterpret_cast<const void*>(vproj_pack_kernel<T>), smem))) return rc; \
-    return launch("nvfp4_vproj_pack", vproj_pack_kernel<T>, grid, kVpThreads, smem, st, t_w, t_x, p);     \
+    return launch_cluster("nvfp4_vproj_pack", vproj_pack_kernel<T>, grid, p.split, kVpThreads, smem, st, t_w, t_x, p); \
   }
   if (dtype == NVFP4_DT_BF16) NVFP4_VP(__nv_bfloat16)
   NVFP4_VP(__half)

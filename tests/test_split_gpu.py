@@ -85,3 +85,17 @@ def test_combine_of_many_pieces(d, s, split_kv):
     assert _status() == 0
     assert float((lse - whole_lse).abs().max()) <= 1e-3
     assert cos(out.cpu().numpy(), whole.cpu().numpy()) >= 0.99     # P is rounded against another running maximum
+
+
+@pytest.mark.parametrize("s,hidden,hk,d", [(1000, 1000, 8, 128), (450, 1544, 8, 128), (130, 584, 3, 64), (17, 4096, 2, 256)])
+def test_split_projection_matches_product(s, hidden, hk, d):
+    """V projection whose tiles are shared by 2, 4 and 8 CTAs, hidden sizes that do not divide evenly."""
+    import sageattention_b200.nvfp4 as nv
+    x, _ = seeded_bf16((1, s, hidden), 71)
+    w, _ = seeded_bf16((hk * d, hidden), 72, scale=hidden ** -0.5)
+    vnv, vsc, v = nv.vproj_quant_nvfp4(x, w, None, hk, d)
+    assert _status() == 0
+    ref = (x.float().double() @ w.double().T).view(1, s, hk, d).permute(0, 2, 1, 3)
+    assert float((v.double() - ref).abs().max()) <= 2.0 ** -8 * max(1.0, float(ref.abs().max())) * 1.01
+    n2, s2 = nv._quant_nvfp4(v.reshape(hk, s, d), transpose=True, k_pad=-(-s // 128) * 128)
+    assert torch.equal(vnv, n2) and torch.equal(vsc.view(torch.uint8), s2.view(torch.uint8))
