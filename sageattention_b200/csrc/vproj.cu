@@ -9,8 +9,8 @@
 // thread writes 64 contiguous nibble bytes + 8 scale bytes of its row.
 //
 // One tile = 128 features x 128 tokens of one batch entry; K loop over the hidden dim in 64-element
-// stages (TMA, 128-byte swizzle, 4-stage ring), tcgen05.mma kind::f16 M128 N128 K16, accumulator in
-// 128 TMEM columns.  Warps: 0 TMA producer, 1 MMA issuer, 2-17 epilogue (32 tokens of 32 features each).
+// stages (TMA, 128-byte swizzle, ring of 4 or 3), tcgen05.mma kind::f16 M128 N128 K16, accumulator in
+// 128 TMEM columns.  Warps: 0 TMA producer, 1 MMA issuer, the others epilogue (32 tokens of 32 features at a time).
 //
 // What bounds it: a stage's 32 KB take ~470 clocks to arrive (an SM's share of L2; the MMAs need 260; a ring of six stages
 // is no faster), so a tile of hidden 4096 costs 16 us however few there are.  Where tiles are fewer than
@@ -25,12 +25,16 @@
 
 namespace nvfp4 {
 
-constexpr int kVpThreads = 576;
-constexpr int kVpStages = 4;
+template <int kPerSm>                      // CTAs per SM the kernel is built for
+struct VpCfg {
+  static constexpr int STAGES = kPerSm == 1 ? 4 : 3;
+  static constexpr int EPI = kPerSm == 1 ? 512 : 256;       // epilogue threads
+  static constexpr int THREADS = 64 + EPI;
+};
 constexpr int kVpTile = 128 * 64 * 2;      // bytes of one operand tile of a stage
 // A partial in shared memory, in place of the ring: [token / 4][feature][token % 4], so that a warp, a feature per lane,
 // writes and (through the cluster) reads 512 consecutive bytes at a time.
-static_assert(128 * 128 * 4 <= kVpStages * 2 * kVpTile, "a partial takes the place of the ring");
+static_assert(128 * 128 * 4 <= VpCfg<2>::STAGES * 2 * kVpTile, "a partial takes the place of the ring");
 
 struct VprojParams {
   const void* bias;      // [features] in the operand dtype, or null
@@ -63,25 +67,30 @@ __device__ __forceinline__ void vproj_store(const VprojParams& p, int zi, int f,
   p.vsc[row * (p.s_pad / 16) + tok / 16] = sb;
 }
 
-// CTAs per tile: the split with the fewest waves x (stages of a CTA + 12 for its start and epilogue, + 6 for the
-// exchange of a split one), in units of a stage's ~0.25 us.  Clusters of eight do not fill the chip (sixteen of
-// them took two waves), hence three quarters of it.  [S, hidden] x 1024 features: 509 x 4096 22.6 -> 11.4 us,
-// 2430 x 4096 44.9 -> 36.5; sixteen epilogue warps instead of four are 2.5 us of each wave, 2048 x 4096 23.8 -> 21.1.
-inline int vproj_split(int64_t tiles, int stages, int sms) {
-  int best = 1;
+// CTAs per tile and per SM, in units of a stage's ~0.25 us.  One CTA per SM: waves x (stages of a CTA + 12 for its
+// start and epilogue, + 6 for the exchange of a split one); clusters of eight do not fill the chip (sixteen of
+// them took two waves), hence three quarters of it.  Two per SM, one's start and epilogue under the other's
+// loads: the stages of the busiest SM, + 2 a CTA (8 split), + 16.  [S, hidden] x features: 509 x 4096 x 1024 22.6 -> 11.4 us
+// (split), 8192 x 4096 x 1024 109 -> 77 and 7486 x 1024 x 2048 80 -> 56 (two per SM, which at 2048 x 4096 x
+// 1024, one wave, takes 30 us against 21); sixteen epilogue warps instead of four are 2.5 us of a wave.
+struct VpPlan { int split, per_sm; };
+inline VpPlan vproj_plan(int64_t tiles, int stages, int sms) {
+  VpPlan best = {1, 1};
   int64_t best_cost = INT64_MAX / 2;
-  for (int n = 1; n <= 8 && n <= stages; n *= 2) {
-    const int64_t room = n == 8 ? sms * 3 / 4 : sms;
-    const int64_t cost = (tiles * n + room - 1) / room * ((stages + n - 1) / n + 12 + (n > 1 ? 6 : 0));
-    if (cost < best_cost - best_cost / 16) { best_cost = cost; best = n; }
-  }
+  for (int per_sm = 1; per_sm <= 2; ++per_sm)
+    for (int n = 1; n <= (per_sm == 1 ? 8 : 2) && n <= stages; n *= 2) {
+      const int64_t room = n == 8 ? sms * 3 / 4 : sms, waves = (tiles * n + room - 1) / room, mine = (stages + n - 1) / n;
+      const int64_t cost = per_sm == 1 ? waves * (mine + 12 + (n > 1 ? 6 : 0)) : waves * (mine + (n > 1 ? 8 : 2)) + 16;
+      if (cost < best_cost - best_cost / 16) { best_cost = cost; best = {n, per_sm}; }
+    }
   return best;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kVpThreads, 1)
+template <typename T, int kPerSm>
+__global__ void __launch_bounds__(VpCfg<kPerSm>::THREADS, kPerSm)
 vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                   const VprojParams p) {
+  constexpr int kVpStages = VpCfg<kPerSm>::STAGES, kStep = VpCfg<kPerSm>::EPI / 128;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -140,34 +149,37 @@ vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     __syncwarp();
   } else {
     // epilogue: thread = feature row 32 (warp % 4) + lane, 32 of the tokens
-    const int ep = tid - 64, row = (warp & 3) * 32 + lane, c = ep >> 7;
+    const int row = (warp & 3) * 32 + lane;
     mbar_wait(&acc_done, 0, &err, 3);
     tc_fence_after();
-    uint32_t r[32];
-    tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c * 32, r);
-    tmem_ld_wait();
-    tc_fence_before();
-    if (p.split == 1) {
+#pragma unroll 1
+    for (int c = (tid - 64) >> 7; c < 4; c += kStep) {
+      uint32_t r[32];
+      tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c * 32, r);
+      tmem_ld_wait();
+      if (p.split == 1) {
 #pragma unroll
-      for (int gi = 0; gi < 2; ++gi) {
-        float v[16];
+        for (int gi = 0; gi < 2; ++gi) {
+          float v[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r[gi * 16 + e]);
-        vproj_store<T>(p, zi, f0 + row, t0 + c * 32 + gi * 16, v);
+          for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r[gi * 16 + e]);
+          vproj_store<T>(p, zi, f0 + row, t0 + c * 32 + gi * 16, v);
+        }
+      } else {
+        float4* part = reinterpret_cast<float4*>(smem) + c * 8 * 128 + row;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          part[e * 128] = make_float4(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1]), __uint_as_float(r[4 * e + 2]),
+                                      __uint_as_float(r[4 * e + 3]));
       }
-    } else {
-      float4* part = reinterpret_cast<float4*>(smem) + c * 8 * 128 + row;
-#pragma unroll
-      for (int e = 0; e < 8; ++e)
-        part[e * 128] = make_float4(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1]), __uint_as_float(r[4 * e + 2]),
-                              __uint_as_float(r[4 * e + 3]));
     }
+    tc_fence_before();
   }
   if (p.split > 1) {
     cluster_sync_all();
     const int ep = tid - 64, groups = 8 / p.split;         // 16-token groups of this CTA
-    if (ep >= 0 && (ep >> 7) < groups) {
-      const int row = ep & 127, gt = (rank * groups + (ep >> 7)) * 16;
+    for (int gi = ep < 0 ? groups : ep >> 7; gi < groups; gi += kStep) {
+      const int row = ep & 127, gt = (rank * groups + gi) * 16;
       const uint32_t a = smem_u32(smem) + (uint32_t)(gt / 4 * 128 + row) * 16u;
       float v[16];
 #pragma unroll
@@ -217,20 +229,23 @@ extern "C" int nvfp4_vproj_pack(const void* x, const void* w, const void* bias, 
   p.bias = bias; p.vnv = vnv; p.vsc = vsc; p.v_out = v_out; p.svb = svb; p.svs = svs;
   p.features = (int)features; p.d = d; p.hk = (int)hk; p.s = (int)s; p.s_pad = (int)s_pad; p.hidden = (int)hidden;
   p.f16 = dtype == NVFP4_DT_FP16 ? 1 : 0; p.status = status;
-  const int smem = kVpStages * 2 * kVpTile + 1024;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int64_t tf = (features + 127) / 128, tt = (s_pad + 127) / 128;
-  p.split = z * 8 < 65536 ? vproj_split(tf * tt * z, (int)((hidden + 63) / 64), sms) : 1;
+  const VpPlan plan = z * 8 < 65536 ? vproj_plan(tf * tt * z, (int)((hidden + 63) / 64), sms) : VpPlan{1, 2};
+  p.split = plan.split;
   dim3 grid((unsigned)tf, (unsigned)tt, (unsigned)(z * p.split));
-#define NVFP4_VP(T)                                                                                       \
-  {                                                                                                       \
-    if ((rc = allow_smem("nvfp4_vproj_pack", reinterpret_cast<const void*>(vproj_pack_kernel<T>), smem))) return rc; \
-    return launch_cluster("nvfp4_vproj_pack", vproj_pack_kernel<T>, grid, p.split, kVpThreads, smem, st, t_w, t_x, p); \
-  }
-  if (dtype == NVFP4_DT_BF16) NVFP4_VP(__nv_bfloat16)
-  NVFP4_VP(__half)
+  auto run = [&](auto kern, int threads, int stages) -> int {
+    const int smem = stages * 2 * kVpTile + 1024;
+    if (int r0 = allow_smem("nvfp4_vproj_pack", reinterpret_cast<const void*>(kern), smem)) return r0;
+    return launch_cluster("nvfp4_vproj_pack", kern, grid, p.split, threads, smem, st, t_w, t_x, p);
+  };
+#define NVFP4_VP(T)                                                                                            \
+  return plan.per_sm == 1 ? run(vproj_pack_kernel<T, 1>, VpCfg<1>::THREADS, VpCfg<1>::STAGES)                  \
+                          : run(vproj_pack_kernel<T, 2>, VpCfg<2>::THREADS, VpCfg<2>::STAGES)
+  if (dtype == NVFP4_DT_BF16) { NVFP4_VP(__nv_bfloat16); }
+  NVFP4_VP(__half);
 #undef NVFP4_VP
 }

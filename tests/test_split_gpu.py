@@ -87,9 +87,10 @@ def test_combine_of_many_pieces(d, s, split_kv):
     assert cos(out.cpu().numpy(), whole.cpu().numpy()) >= 0.99     # P is rounded against another running maximum
 
 
-@pytest.mark.parametrize("s,hidden,hk,d", [(1000, 1000, 8, 128), (450, 1544, 8, 128), (130, 584, 3, 64), (17, 4096, 2, 256)])
+@pytest.mark.parametrize("s,hidden,hk,d", [(1000, 1000, 8, 128), (450, 1544, 8, 128), (130, 584, 3, 64), (17, 4096, 2, 256),
+                                           (2430, 1000, 8, 128), (2500, 200, 16, 128)])
 def test_split_projection_matches_product(s, hidden, hk, d):
-    """V projection whose tiles are shared by 2, 4 and 8 CTAs, hidden sizes that do not divide evenly."""
+    """V projection whose tiles are shared by 2, 4 and 8 CTAs, hidden sizes that do not divide evenly; two CTAs per SM."""
     import sageattention_b200.nvfp4 as nv
     x, _ = seeded_bf16((1, s, hidden), 71)
     w, _ = seeded_bf16((hk * d, hidden), 72, scale=hidden ** -0.5)
