@@ -253,7 +253,10 @@ int nvfp4_decode_static(const void* q, int q_dtype, int64_t s_qz, int64_t s_qh, 
  * such partials per unit (they follow the kernel's own slots: extra_base = own slots, total_slots =
  * own slots + Z*Hk*n_extra; workspace_bytes must cover them).  out / lse are the attention over
  * prefix and window together, written once in the query dtype.
+ * NVFP4_DECODE_AFTER_WINDOW, or-ed to n_extra, says that nvfp4_window_partials was the stream's last
+ * launch before this call: the split-K kernel then starts beside it instead of behind it.
  */
+#define NVFP4_DECODE_AFTER_WINDOW 0x100
 int nvfp4_window_partials(const void* q, int dtype, int64_t s_qz, int64_t s_qh, const void* rk,
                           const void* rv, int64_t z, int64_t hk, int g, int d, int64_t ring_cap,
                           int64_t first_pos, int64_t count, float scaling, int pieces,

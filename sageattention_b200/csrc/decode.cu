@@ -91,6 +91,7 @@ struct DecodeParams {
   float* ws_l;    // [nitems][16]
   int64_t extra_base;   // first of the partial slots appended by another kernel (n_extra per unit)
   int n_extra;
+  int late_wait;        // independent of the kernel before it: wait for it at the end, not at the start
   int* status;
 };
 
@@ -193,7 +194,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     mbar_fence_init();
   }
   __syncthreads();
-  griddep_wait();
+  if (!p.late_wait) griddep_wait();
   // The TMA producer (warp 0) and the scale loader (warp 2) need nothing but the barriers and the
   // stage buffers: they start streaming now, while the other warps allocate TMEM and clear the
   // operand buffers behind a barrier of their own.
@@ -716,6 +717,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
+  if (p.late_wait) griddep_wait();       // the combine, which waits for this kernel, needs the window's partials too
   if (tid == 0 && err != 0 && p.status != nullptr) atomicExch(p.status, err);
   if (warp == 1) tmem_dealloc(tmem, C::T_COLS);
 }
@@ -942,6 +944,11 @@ extern "C" int nvfp4_decode_hybrid(const void* q, int q_dtype, int64_t s_qz, int
                                    size_t workspace_bytes, int nsplit, int64_t split_kv, int n_extra,
                                    int* status, nvfp4_stream_t stream) {
   using namespace nvfp4;
+  // The window kernel lets its successor start once all its CTAs have seen the work before it complete, so the
+  // split-K kernel, which reads nothing of the window's, streams the cache beside it (H16 Hk4 S17558 window
+  // 128 23.9 -> 19.5 us with the append; 256 window CTAs at two per SM leave it no room: Z8 S8190 window 512 unchanged).
+  const bool after_window = (n_extra & ~0xFF) == NVFP4_DECODE_AFTER_WINDOW;
+  if (after_window) n_extra &= 0xFF;
   NVFP4_REQUIRE(n_extra >= 0 && n_extra <= 64, "nvfp4_decode: extra partials per unit must be in [0, 64]");
   NVFP4_REQUIRE(d == 128 || d == 256, "nvfp4_decode: D must be 128 or 256");
   NVFP4_REQUIRE(g >= 1 && g <= 16, "nvfp4_decode: GQA group %d must be <= 16", g);
@@ -1010,6 +1017,7 @@ extern "C" int nvfp4_decode_hybrid(const void* q, int q_dtype, int64_t s_qz, int
   p.ws_l = p.ws_m + slots * 16;
   p.extra_base = own_slots;
   p.n_extra = n_extra;
+  p.late_wait = after_window ? 1 : 0;
   p.status = status;
 
 #define NVFP4_DECODE(DD, T) return decode_launch<DD, T>(tm_k, tm_v, tm_vpf, tm_vpf4, p, zhk, out, lse, sm_count, st)

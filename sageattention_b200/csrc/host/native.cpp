@@ -525,7 +525,7 @@ std::tuple<Tensor, OptTensor> decode_core(const Call& c, const Tensor& query, co
                              u8(*a.ksc), a.ksc->stride(0), u8(*a.vnv), a.vnv->stride(0), a.vnv->stride(1), u8(*a.vsc),
                              a.vsc->stride(0), a.vsc->stride(1), a.z, hk, (int)a.g, (int)a.d, a.s_kv, (float)a.scaling,
                              out.data_ptr(), opt_ptr<float>(lse), ws.data_ptr(), (size_t)(slots * slot_bytes), nsplit, split_kv,
-                             (int)extra, c.status, c.stream),
+                             (int)extra | (win ? NVFP4_DECODE_AFTER_WINDOW : 0), c.status, c.stream),
          "nvfp4_decode");
   return {out, lse};
 }
