@@ -7,7 +7,8 @@
 namespace nvfp4 {
 
 // One block per (z, kv-head) unit, one thread per head-dim element.
-//  * threads [0, D/16) pack the new K row (one 16-group each);
+//  * a warp of its own, threads [D, D + D/16), packs the new K row (one 16-group each): in front of the V
+//    work of warp 0 its trip to memory came on top of the other one;
 //  * every thread stores its element of the new V token into the partial-group buffer and
 //    re-packs "its" V^T row of the current 16-key group (8 bytes + 1 scale);
 //  * ring slots are written when the rings exist.
@@ -25,15 +26,18 @@ __global__ void kv_append_kernel(const T* __restrict__ k_new, const T* __restric
   const int t = threadIdx.x;
   const T* kr = k_new + u * s_new;
   const T* vr = v_new + u * s_new;
-  if (t < d / 16) {
+  if (t >= d) {
+    const int gi = t - d;
+    if (gi >= d / 16) return;
     float v[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = to_f32<T>(kr[t * 16 + i]);
+    for (int i = 0; i < 16; ++i) v[i] = to_f32<T>(kr[gi * 16 + i]);
     uint32_t lo, hi;
     const uint8_t sb = pack_group16(v, lo, hi);
-    uint8_t* pn = knv + u * knv_unit + pos * (d / 2) + t * 8;
+    uint8_t* pn = knv + u * knv_unit + pos * (d / 2) + gi * 8;
     *reinterpret_cast<uint2*>(pn) = make_uint2(lo, hi);
-    ksc[u * ksc_unit + pos * (d / 16) + t] = sb;
+    ksc[u * ksc_unit + pos * (d / 16) + gi] = sb;
+    return;
   }
   const int slot = (int)(pos % 16);
   const int64_t gidx = pos / 16;
@@ -485,7 +489,7 @@ int append_launch(const void* k_new, const void* v_new, int64_t s_new, int64_t z
                   int64_t vsc_row, void* partial, void* ring_k, void* ring_v, int64_t ring_cap,
                   cudaStream_t st) {
   return launch(
-      "nvfp4_kv_append", kv_append_kernel<T>, dim3((unsigned)zhk), d, 0, st, static_cast<const T*>(k_new), static_cast<const T*>(v_new), s_new, d, pos, knv, knv_unit, ksc,
+      "nvfp4_kv_append", kv_append_kernel<T>, dim3((unsigned)zhk), d + 32, 0, st, static_cast<const T*>(k_new), static_cast<const T*>(v_new), s_new, d, pos, knv, knv_unit, ksc,
       ksc_unit, vnv, vnv_unit, vnv_row, vsc, vsc_unit, vsc_row, static_cast<T*>(partial),
       static_cast<T*>(ring_k), static_cast<T*>(ring_v), ring_cap);
 }
