@@ -328,6 +328,14 @@ int nvfp4_bwd_prep(const void* x, int dtype, int64_t sxb1, int64_t sxb2, int64_t
                    int d, void* xc, float* delta, float* amax, nvfp4_stream_t stream);
 
 /*
+ * Contiguous bf16 copies out[k] [B1*B2, S, D] of n <= 4 strided bf16 / fp16 operands x[k] [B1, B2, S, D]
+ * (one dtype, unit stride along D, rows 32-byte aligned) in one launch; strides [n][3] in elements,
+ * extents [n][3] = B1, B2, S (host arrays).  What nvfp4_bwd_prep copies one operand at a time.
+ */
+int nvfp4_bf16_copies(int n, const void* const* x, void* const* out, int dtype, const int64_t* strides,
+                      const int64_t* extents, int d, nvfp4_stream_t stream);
+
+/*
  * Backward with high-precision gradient GEMMs: dQ, dK, dV of the forward above.  Replaces
  * `_run_bwd_hp` and its kernels `_flash_bwd_dkdv_hp_kernel` / `_flash_bwd_dq_hp_kernel`
  * (flash.py:2008-2399, 3459-3805): S is recomputed from the NVFP4 packs of Q and K, P uses the

@@ -66,6 +66,7 @@ SIGNATURES = {
     "nvfp4_rope_pack": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int, c_int64, c_int64, c_void_p, c_void_p,
                                 c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64,
                                 c_void_p]),
+    "nvfp4_bf16_copies": (c_int, [c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p]),
     "nvfp4_bwd_prep": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, c_void_p,
                                c_int64, c_int64, c_int64, c_int64, c_int, c_void_p, c_void_p, c_void_p,
                                c_void_p]),

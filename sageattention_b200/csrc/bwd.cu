@@ -257,6 +257,50 @@ __global__ void __launch_bounds__(256, 4) prep_wide_kernel(const T* __restrict__
   }
 }
 
+// bf16 copies of up to four 16-bit operands (Q, K, V of an fp16 training step) in one launch, blockIdx.y the
+// operand: bound by memory and, for short sequences, by the launches that three kernels would be (fp16 training step
+// S1024 H16 Hk4 97 -> 91 us, S3000 H32 Hk8 418 -> 412).
+struct CopyArgs {
+  const void* x[4];
+  __nv_bfloat16* out[4];
+  int64_t sb1[4], sb2[4], ss[4], rows[4];
+  int nb2[4], s[4], flat[4];
+};
+template <typename T, int D>
+__global__ void __launch_bounds__(256, 4) bf16_copies_kernel(const CopyArgs a) {
+  griddep_launch();
+  griddep_wait();
+  constexpr int kLanes = D / 16, kPer = 32 / kLanes, kRows = 4;
+  const int k = blockIdx.y, lane = threadIdx.x & 31, sub = lane / kLanes, col = (lane % kLanes) * 16;
+  const T* x = static_cast<const T*>(a.x[k]);
+  const int64_t rows = a.rows[k], step = (int64_t)gridDim.x * 8 * kPer * kRows;
+  for (int64_t base = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * (kPer * kRows); base < rows; base += step) {
+    uint32_t rx[kRows][8];
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      const int64_t r = min(base + kPer * j + sub, rows - 1);
+      int64_t o = r * a.ss[k];
+      if (!a.flat[k]) {
+        const uint32_t b = (uint32_t)r / (uint32_t)a.s[k], b1 = b / (uint32_t)a.nb2[k];
+        o = (int64_t)b1 * a.sb1[k] + (int64_t)(b - b1 * (uint32_t)a.nb2[k]) * a.sb2[k] + (r - (int64_t)b * a.s[k]) * a.ss[k];
+      }
+      prep_ldg32(x + o + col, rx[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      const int64_t r = base + kPer * j + sub;
+      if (r >= rows) continue;
+      const T* e = reinterpret_cast<const T*>(rx[j]);
+      uint32_t w[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) w[i] = pack_bf16x2(to_f32<T>(e[2 * i]), to_f32<T>(e[2 * i + 1]));
+      uint4* o = reinterpret_cast<uint4*>(a.out[k] + r * D + col);
+      o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+      o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+  }
+}
+
 struct BwdParams {
   const uint8_t* qsc;   // [ZH, Sq, 8]
   const uint8_t* ksc;   // [ZHk, Skv, 8]
@@ -1075,6 +1119,34 @@ int prep_launch(const void* x, int64_t sxb1, int64_t sxb2, int64_t sxs, int64_t 
 }
 
 }  // namespace nvfp4
+
+extern "C" int nvfp4_bf16_copies(int n, const void* const* x, void* const* out, int dtype, const int64_t* strides,
+                                 const int64_t* extents, int d, nvfp4_stream_t stream) {
+  using namespace nvfp4;
+  NVFP4_REQUIRE(n >= 1 && n <= 4 && x && out && strides && extents, "nvfp4_bf16_copies: one to four operands");
+  NVFP4_REQUIRE(dtype == NVFP4_DT_BF16 || dtype == NVFP4_DT_FP16, "nvfp4_bf16_copies: operands must be bf16 or fp16");
+  NVFP4_REQUIRE(d == 128 || d == 256, "nvfp4_bf16_copies: D must be 128 or 256");
+  CopyArgs a = {};
+  int64_t most = 0;
+  for (int k = 0; k < n; ++k) {
+    const int64_t *st = strides + 3 * k, b1 = extents[3 * k], b2 = extents[3 * k + 1], s = extents[3 * k + 2];
+    NVFP4_REQUIRE(x[k] && out[k] && b1 >= 1 && b2 >= 1 && s >= 1 && b1 * b2 * s < (1LL << 31), "nvfp4_bf16_copies: bad extents");
+    NVFP4_REQUIRE((((uintptr_t)x[k] | (uint64_t)(st[0] * 2) | (uint64_t)(st[1] * 2) | (uint64_t)(st[2] * 2)) & 31) == 0 &&
+                      ((uintptr_t)out[k] & 15) == 0,
+                  "nvfp4_bf16_copies: rows must be 32-byte aligned");
+    a.x[k] = x[k]; a.out[k] = static_cast<__nv_bfloat16*>(out[k]);
+    a.sb1[k] = st[0]; a.sb2[k] = st[1]; a.ss[k] = st[2];
+    a.nb2[k] = (int)b2; a.s[k] = (int)s; a.rows[k] = b1 * b2 * s;
+    a.flat[k] = (b2 == 1 || st[1] == s * st[2]) && (b1 == 1 || st[0] == b2 * s * st[2]);
+    most = std::max(most, a.rows[k]);
+  }
+  const int64_t per_block = 8 * (512 / d) * 4;
+  const dim3 grid((unsigned)std::min<int64_t>((most + per_block - 1) / per_block, 148 * 8), (unsigned)n);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  auto run = [&](auto kern) { return launch("nvfp4_bf16_copies", kern, grid, 256, 0, st, a); };
+  if (dtype == NVFP4_DT_BF16) return d == 128 ? run(bf16_copies_kernel<__nv_bfloat16, 128>) : run(bf16_copies_kernel<__nv_bfloat16, 256>);
+  return d == 128 ? run(bf16_copies_kernel<__half, 128>) : run(bf16_copies_kernel<__half, 256>);
+}
 
 extern "C" int nvfp4_bwd_prep(const void* x, int dtype, int64_t sxb1, int64_t sxb2, int64_t sxs,
                               int64_t nb1, int64_t nb2, const void* y, int64_t syb1, int64_t syb2,

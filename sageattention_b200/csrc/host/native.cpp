@@ -18,6 +18,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <array>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -681,6 +682,36 @@ Tensor bf16_rows_call(const Call& c, const Tensor& x) {
   if (x.scalar_type() == at::kBFloat16 && x.is_contiguous()) return x;
   return *bwd_prep_call(c, x, std::nullopt, true, false).copy;
 }
+// The same for Q, K and V: those that need a copy in one launch where their rows allow it.
+std::array<Tensor, 3> bf16_rows3(const Call& c, const Tensor& q, const Tensor& k, const Tensor& v) {
+  const Tensor* in[3] = {&q, &k, &v};
+  std::array<Tensor, 3> r;
+  const void* x[3];
+  void* out[3];
+  int64_t strides[9], extents[9];
+  int n = 0;
+  bool one = true;
+  for (int i = 0; i < 3; ++i) {
+    const Tensor& t = *in[i];
+    if (t.scalar_type() == at::kBFloat16 && t.is_contiguous()) { r[i] = t; continue; }
+    one = one && t.stride(3) == 1 && t.element_size() == 2 && t.scalar_type() == q.scalar_type() &&
+          ((reinterpret_cast<uintptr_t>(t.data_ptr()) | (uint64_t)(t.stride(0) * 2) | (uint64_t)(t.stride(1) * 2) |
+            (uint64_t)(t.stride(2) * 2)) & 31) == 0 && t.numel() > 0 && t.size(0) * t.size(1) * t.size(2) < (1LL << 31);
+    x[n] = t.data_ptr();
+    for (int e = 0; e < 3; ++e) { strides[3 * n + e] = t.stride(e); extents[3 * n + e] = t.size(e); }
+    ++n;
+  }
+  if (n < 2 || !one) return {bf16_rows_call(c, q), bf16_rows_call(c, k), bf16_rows_call(c, v)};
+  n = 0;
+  for (int i = 0; i < 3; ++i)
+    if (!r[i].defined()) {
+      r[i] = c.empty(in[i]->sizes(), at::kBFloat16);
+      out[n++] = r[i].data_ptr();
+    }
+  c.done(nvfp4_bf16_copies(n, x, out, dtype_code(q.scalar_type()), strides, extents, (int)q.size(3), c.stream),
+         "nvfp4_bf16_copies");
+  return r;
+}
 Tensor bf16_rows(const Tensor& x) {
   require_cuda(x, "x");
   Call c(x);
@@ -714,7 +745,7 @@ std::tuple<Tensor, Tensor, Tensor> bwd_hp(const Tensor& q, const Tensor& k, cons
   const bool need_copy = !(gdt == at::kBFloat16 && dout.is_contiguous());
   Prep pp = bwd_prep_call(c, dout, out, need_copy, false);
   const Tensor doc = need_copy ? *pp.copy : dout;
-  const Tensor qc = bf16_rows_call(c, q), kc = bf16_rows_call(c, k), vc = bf16_rows_call(c, v);
+  const auto [qc, kc, vc] = bf16_rows3(c, q, k, v);
   Pack qp = given_or_quant(c, qnv_in, qsc_in, rows_of(q), q.scalar_type(), kQPacks);
   Pack kp = given_or_quant(c, knv_in, ksc_in, rows_of(k), k.scalar_type(), kKPacks);
   Tensor dq = c.empty({z, h, s_q, d}, gdt), dk = c.empty({z, hk, s_kv, d}, gdt), dv = c.empty({z, hk, s_kv, d}, gdt);
