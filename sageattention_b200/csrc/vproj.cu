@@ -8,14 +8,15 @@
 // tokens on its columns: the 16-token groups of the pack are thread-local in the epilogue and a
 // thread writes 64 contiguous nibble bytes + 8 scale bytes of its row.
 //
-// One tile = 128 features x 128 tokens of one batch entry; K loop over the hidden dim in 64-element
-// stages (TMA, 128-byte swizzle, ring of 4 or 3), tcgen05.mma kind::f16 M128 N128 K16, accumulator in
-// 128 TMEM columns.  Warps: 0 TMA producer, 1 MMA issuer, the others epilogue (32 tokens of 32 features at a time).
+// One CTA = 128 features x NT tokens (128, 64 or 32) of one batch entry; K loop over the hidden dim in 64-element
+// stages (TMA, 128-byte swizzle, ring of 3 to 8), tcgen05.mma kind::f16 M128 N=NT K16, accumulator in
+// NT TMEM columns.  Warps: 0 TMA producer, 1 MMA issuer, the others epilogue (32 tokens of 32 features at a time).
 //
-// What bounds it: a stage's 32 KB take ~470 clocks to arrive (an SM's share of L2; the MMAs need 260; a ring of six stages
-// is no faster), so a tile of hidden 4096 costs 16 us however few there are.  Where tiles are fewer than
-// SMs, a cluster of 2, 4 or 8 CTAs shares one: each takes a range of the hidden dim, leaves its fp32 partial
-// in its shared memory, and finishes its share of the tokens from all partials in rank order.
+// What bounds it: a stage's 32 KB (NT = 128) take ~470 clocks to arrive (an SM's share of L2; the MMAs need 260; a
+// ring of six stages is no faster), so a tile of hidden 4096 costs 16 us however few there are.  The hidden dim
+// is not split: V is rounded, packed to FP4 and attended, and a sum in another order moves single outputs by
+// as much as their size.  Where tiles are fewer than SMs they are cut along the tokens instead, with
+// 24 or 20 KB a stage.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
 #include "common/launch.cuh"
@@ -25,16 +26,15 @@
 
 namespace nvfp4 {
 
-template <int kPerSm>                      // CTAs per SM the kernel is built for
+constexpr int kVpTile = 128 * 64 * 2;      // bytes of the W tile of a stage
+
+template <int kNT, int kPerSm>             // tokens of a tile, CTAs per SM the kernel is built for
 struct VpCfg {
-  static constexpr int STAGES = kPerSm == 1 ? 4 : 3;
-  static constexpr int EPI = kPerSm == 1 ? 512 : 256;       // epilogue threads
+  static constexpr int STAGES = kPerSm == 2 ? 3 : (kNT == 128 ? 4 : 8);     // a narrow tile is bound by latency
+  static constexpr int STAGE_BYTES = kVpTile + kNT * 128;
+  static constexpr int EPI = kPerSm == 1 ? kNT * 4 : 256;   // epilogue threads
   static constexpr int THREADS = 64 + EPI;
 };
-constexpr int kVpTile = 128 * 64 * 2;      // bytes of one operand tile of a stage
-// A partial in shared memory, in place of the ring: [token / 4][feature][token % 4], so that a warp, a feature per lane,
-// writes and (through the cluster) reads 512 consecutive bytes at a time.
-static_assert(128 * 128 * 4 <= VpCfg<2>::STAGES * 2 * kVpTile, "a partial takes the place of the ring");
 
 struct VprojParams {
   const void* bias;      // [features] in the operand dtype, or null
@@ -42,7 +42,7 @@ struct VprojParams {
   uint8_t* vsc;          // [Z*Hk, D, s_pad/16]
   void* v_out;           // [Z, S, features] (element strides svb, svs; unit feature stride) or null
   int64_t svb, svs;
-  int features, d, hk, s, s_pad, hidden, split;
+  int features, d, hk, s, s_pad, hidden;
   int f16;
   int* status;
 };
@@ -67,30 +67,22 @@ __device__ __forceinline__ void vproj_store(const VprojParams& p, int zi, int f,
   p.vsc[row * (p.s_pad / 16) + tok / 16] = sb;
 }
 
-// CTAs per tile and per SM, in units of a stage's ~0.25 us.  One CTA per SM: waves x (stages of a CTA + 12 for its
-// start and epilogue, + 6 for the exchange of a split one); clusters of eight do not fill the chip (sixteen of
-// them took two waves), hence three quarters of it.  Two per SM, one's start and epilogue under the other's
-// loads: the stages of the busiest SM, + 2 a CTA (8 split), + 16.  [S, hidden] x features: 509 x 4096 x 1024 22.6 -> 11.4 us
-// (split), 8192 x 4096 x 1024 109 -> 77 and 7486 x 1024 x 2048 80 -> 56 (two per SM, which at 2048 x 4096 x
-// 1024, one wave, takes 30 us against 21); sixteen epilogue warps instead of four are 2.5 us of a wave.
-struct VpPlan { int split, per_sm; };
-inline VpPlan vproj_plan(int64_t tiles, int stages, int sms) {
-  VpPlan best = {1, 1};
-  int64_t best_cost = INT64_MAX / 2;
-  for (int per_sm = 1; per_sm <= 2; ++per_sm)
-    for (int n = 1; n <= (per_sm == 1 ? 8 : 2) && n <= stages; n *= 2) {
-      const int64_t room = n == 8 ? sms * 3 / 4 : sms, waves = (tiles * n + room - 1) / room, mine = (stages + n - 1) / n;
-      const int64_t cost = per_sm == 1 ? waves * (mine + 12 + (n > 1 ? 6 : 0)) : waves * (mine + (n > 1 ? 8 : 2)) + 16;
-      if (cost < best_cost - best_cost / 16) { best_cost = cost; best = {n, per_sm}; }
-    }
-  return best;
+// Tokens of a tile and CTAs per SM: the narrowest tile of which one wave covers the problem; beyond a wave of
+// the widest, two CTAs per SM, one's start and epilogue under the other's loads.  [S, hidden] x features: 509 x 4096 x 1024
+// 22.6 us (128 tokens) -> 17.4 (32), 128 x 2048 x 512 14.9 -> 10.3, 2430 x 4096 x 1024 44.9 -> 33, 8192 x 4096 x 1024 109 -> 76, 7486 x 1024 x 2048 80 -> 58.
+struct VpPlan { int nt, per_sm; };
+inline VpPlan vproj_plan(int64_t row_tiles, int64_t s_pad, int sms) {
+  for (int nt = 32; nt <= 128; nt *= 2)
+    if (row_tiles * ((s_pad + nt - 1) / nt) <= sms) return {nt, 1};
+  return {128, 2};
 }
 
-template <typename T, int kPerSm>
-__global__ void __launch_bounds__(VpCfg<kPerSm>::THREADS, kPerSm)
+template <typename T, int kNT, int kPerSm>
+__global__ void __launch_bounds__(VpCfg<kNT, kPerSm>::THREADS, kPerSm)
 vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                   const VprojParams p) {
-  constexpr int kVpStages = VpCfg<kPerSm>::STAGES, kStep = VpCfg<kPerSm>::EPI / 128;
+  using C = VpCfg<kNT, kPerSm>;
+  constexpr int kVpStages = C::STAGES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -98,10 +90,8 @@ vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int f0 = blockIdx.x * 128, t0 = blockIdx.y * 128;
-  const int zi = blockIdx.z / p.split, rank = blockIdx.z - zi * p.split;     // rank of the CTA in its cluster
-  const int all = (p.hidden + 63) / 64;
-  const int st0 = (int)((int64_t)all * rank / p.split), nstage = (int)((int64_t)all * (rank + 1) / p.split) - st0;
+  const int f0 = blockIdx.x * 128, t0 = blockIdx.y * kNT, zi = blockIdx.z;
+  const int nstage = (p.hidden + 63) / 64;
   if (tid == 0) {
     err = 0;
     for (int i = 0; i < kVpStages; ++i) {
@@ -124,21 +114,21 @@ vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       for (int st = 0; st < nstage; ++st) {
         const int s = st % kVpStages;
         if (st >= kVpStages) mbar_wait(&empty[s], ((st / kVpStages) & 1) ^ 1, &err, 1);
-        uint8_t* sb = smem + s * 2 * kVpTile;
-        mbar_expect_tx(&full[s], 2 * kVpTile);
-        tma_load_3d(sb, &tm_w, &full[s], (st0 + st) * 64, f0, 0);
-        tma_load_3d(sb + kVpTile, &tm_x, &full[s], (st0 + st) * 64, t0, zi);
+        uint8_t* sb = smem + s * C::STAGE_BYTES;
+        mbar_expect_tx(&full[s], C::STAGE_BYTES);
+        tma_load_3d(sb, &tm_w, &full[s], st * 64, f0, 0);
+        tma_load_3d(sb + kVpTile, &tm_x, &full[s], st * 64, t0, zi);
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     if (elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(128, 128, false, p.f16 != 0);
+      const uint32_t idesc = make_idesc_bf16(128, kNT, false, p.f16 != 0);
       for (int st = 0; st < nstage; ++st) {
         const int s = st % kVpStages;
         mbar_wait(&full[s], (st / kVpStages) & 1, &err, 2);
         tc_fence_after();
-        const uint8_t* sb = smem + s * 2 * kVpTile;
+        const uint8_t* sb = smem + s * C::STAGE_BYTES;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           umma_bf16(tmem, desc_sw128(sb, k), desc_sw128(sb + kVpTile, k), idesc, (st > 0 || k > 0) ? 1u : 0u);
@@ -153,47 +143,19 @@ vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     mbar_wait(&acc_done, 0, &err, 3);
     tc_fence_after();
 #pragma unroll 1
-    for (int c = (tid - 64) >> 7; c < 4; c += kStep) {
+    for (int c = (tid - 64) >> 7; c < kNT / 32; c += C::EPI / 128) {
       uint32_t r[32];
       tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c * 32, r);
       tmem_ld_wait();
-      if (p.split == 1) {
 #pragma unroll
-        for (int gi = 0; gi < 2; ++gi) {
-          float v[16];
+      for (int gi = 0; gi < 2; ++gi) {
+        float v[16];
 #pragma unroll
-          for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r[gi * 16 + e]);
-          vproj_store<T>(p, zi, f0 + row, t0 + c * 32 + gi * 16, v);
-        }
-      } else {
-        float4* part = reinterpret_cast<float4*>(smem) + c * 8 * 128 + row;
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-          part[e * 128] = make_float4(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1]), __uint_as_float(r[4 * e + 2]),
-                                      __uint_as_float(r[4 * e + 3]));
+        for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r[gi * 16 + e]);
+        vproj_store<T>(p, zi, f0 + row, t0 + c * 32 + gi * 16, v);
       }
     }
     tc_fence_before();
-  }
-  if (p.split > 1) {
-    cluster_sync_all();
-    const int ep = tid - 64, groups = 8 / p.split;         // 16-token groups of this CTA
-    for (int gi = ep < 0 ? groups : ep >> 7; gi < groups; gi += kStep) {
-      const int row = ep & 127, gt = (rank * groups + gi) * 16;
-      const uint32_t a = smem_u32(smem) + (uint32_t)(gt / 4 * 128 + row) * 16u;
-      float v[16];
-#pragma unroll
-      for (int e = 0; e < 16; ++e) v[e] = 0.0f;
-      for (int k = 0; k < p.split; ++k) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float4 x = ld_cluster_f4(a + 2048 * e, k);
-          v[4 * e] += x.x; v[4 * e + 1] += x.y; v[4 * e + 2] += x.z; v[4 * e + 3] += x.w;
-        }
-      }
-      vproj_store<T>(p, zi, f0 + row, t0 + gt, v);
-    }
-    cluster_sync_all();                                    // the partials stay until every CTA has read them
   }
   __syncthreads();
   if (tid == 0 && err != 0 && p.status != nullptr) atomicExch(p.status, err);
@@ -217,35 +179,38 @@ extern "C" int nvfp4_vproj_pack(const void* x, const void* w, const void* bias, 
   const int64_t features = hk * d;
   NVFP4_REQUIRE(features < (1LL << 30) && s_pad < (1LL << 30) && z < 65536 && (s_pad + 127) / 128 < 65536,
                 "nvfp4_vproj_pack: problem too large");
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t tf = (features + 127) / 128;
+  const VpPlan plan = vproj_plan(tf * z, s_pad, sms);
   CUtensorMap t_w, t_x;
   int rc;
   if ((rc = make_tmap_bf16_3d_sw128(&t_w, w, (uint64_t)hidden, (uint64_t)features, 1, (uint64_t)hidden * 2,
                                     (uint64_t)features * hidden * 2, 128, "nvfp4_vproj_pack(W)")))
     return rc;
   if ((rc = make_tmap_bf16_3d_sw128(&t_x, x, (uint64_t)hidden, (uint64_t)s, (uint64_t)z, (uint64_t)sxs * 2,
-                                    (uint64_t)(z > 1 ? sxb : s * sxs) * 2, 128, "nvfp4_vproj_pack(X)")))
+                                    (uint64_t)(z > 1 ? sxb : s * sxs) * 2, (uint32_t)plan.nt, "nvfp4_vproj_pack(X)")))
     return rc;
   VprojParams p;
   p.bias = bias; p.vnv = vnv; p.vsc = vsc; p.v_out = v_out; p.svb = svb; p.svs = svs;
   p.features = (int)features; p.d = d; p.hk = (int)hk; p.s = (int)s; p.s_pad = (int)s_pad; p.hidden = (int)hidden;
   p.f16 = dtype == NVFP4_DT_FP16 ? 1 : 0; p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t tf = (features + 127) / 128, tt = (s_pad + 127) / 128;
-  const VpPlan plan = z * 8 < 65536 ? vproj_plan(tf * tt * z, (int)((hidden + 63) / 64), sms) : VpPlan{1, 2};
-  p.split = plan.split;
-  dim3 grid((unsigned)tf, (unsigned)tt, (unsigned)(z * p.split));
-  auto run = [&](auto kern, int threads, int stages) -> int {
-    const int smem = stages * 2 * kVpTile + 1024;
-    if (int r0 = allow_smem("nvfp4_vproj_pack", reinterpret_cast<const void*>(kern), smem)) return r0;
-    return launch_cluster("nvfp4_vproj_pack", kern, grid, p.split, threads, smem, st, t_w, t_x, p);
+  const dim3 grid((unsigned)tf, (unsigned)((s_pad + plan.nt - 1) / plan.nt), (unsigned)z);
+  auto run = [&](auto kern, int threads, int ring) -> int {
+    if (int r0 = allow_smem("nvfp4_vproj_pack", reinterpret_cast<const void*>(kern), ring + 1024)) return r0;
+    return launch("nvfp4_vproj_pack", kern, grid, threads, ring + 1024, st, t_w, t_x, p);
   };
-#define NVFP4_VP(T)                                                                                            \
-  return plan.per_sm == 1 ? run(vproj_pack_kernel<T, 1>, VpCfg<1>::THREADS, VpCfg<1>::STAGES)                  \
-                          : run(vproj_pack_kernel<T, 2>, VpCfg<2>::THREADS, VpCfg<2>::STAGES)
-  if (dtype == NVFP4_DT_BF16) { NVFP4_VP(__nv_bfloat16); }
-  NVFP4_VP(__half);
+#define NVFP4_VP(T, NT, PER) \
+  run(vproj_pack_kernel<T, NT, PER>, VpCfg<NT, PER>::THREADS, VpCfg<NT, PER>::STAGES * VpCfg<NT, PER>::STAGE_BYTES)
+#define NVFP4_VP_T(T)                                      \
+  return plan.per_sm == 2 ? NVFP4_VP(T, 128, 2)            \
+         : plan.nt == 128 ? NVFP4_VP(T, 128, 1)            \
+         : plan.nt == 64  ? NVFP4_VP(T, 64, 1)             \
+                          : NVFP4_VP(T, 32, 1)
+  if (dtype == NVFP4_DT_BF16) { NVFP4_VP_T(__nv_bfloat16); }
+  NVFP4_VP_T(__half);
+#undef NVFP4_VP_T
 #undef NVFP4_VP
 }

@@ -1,5 +1,5 @@
 """Work split over CTAs: the dK / dV passes of the backward with the query steps of a key tile shared by a
-cluster, and the decode combine with many pieces per unit."""
+cluster, the decode combine with many pieces per unit, and the tile widths of the V projection."""
 
 import numpy as np
 import pytest
@@ -89,8 +89,8 @@ def test_combine_of_many_pieces(d, s, split_kv):
 
 @pytest.mark.parametrize("s,hidden,hk,d", [(1000, 1000, 8, 128), (450, 1544, 8, 128), (130, 584, 3, 64), (17, 4096, 2, 256),
                                            (2430, 1000, 8, 128), (2500, 200, 16, 128)])
-def test_split_projection_matches_product(s, hidden, hk, d):
-    """V projection whose tiles are shared by 2, 4 and 8 CTAs, hidden sizes that do not divide evenly; two CTAs per SM."""
+def test_projection_tiles_match_product(s, hidden, hk, d):
+    """V projection in tiles of 32, 64 and 128 tokens, one and two CTAs per SM, hidden sizes that leave a remainder."""
     import sageattention_b200.nvfp4 as nv
     x, _ = seeded_bf16((1, s, hidden), 71)
     w, _ = seeded_bf16((hk * d, hidden), 72, scale=hidden ** -0.5)
