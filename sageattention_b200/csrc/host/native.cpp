@@ -153,6 +153,14 @@ Rows rows_of(const Tensor& t) {
   return {c, c.data_ptr(), b, sz[2], sz[3], sz[2] * sz[3], sz[3], 1};
 }
 
+// A [Z, H, S, D] operand of known extents: as it is, or (any other shape of as many elements) reshaped to
+// [Z*H, S, D] rows.  Throws where the elements do not make up the extents: the kernels take their sizes from
+// one operand and would read past the end of another.
+Tensor as_rows(const Tensor& t, int64_t b, int64_t s, int64_t d) {
+  if (t.dim() == 4 && t.size(0) * t.size(1) == b && t.size(2) == s && t.size(3) == d) return t;
+  return t.reshape({b, s, d});
+}
+
 // ---------------------------------------------------------------- packers
 void pack_rows_call(const Call& c, const Rows& x, int dt, int64_t r, int64_t k_read, int64_t kp, int64_t sxr, int64_t sxk,
                     uint8_t* nib, int64_t snb, int64_t snr, uint8_t* sc, int64_t ssb, int64_t ssr) {
@@ -311,7 +319,7 @@ struct FwdPacks {
   Tensor qn, qs, kn, ks, vn, vs;
 };
 bool qkv_fusable(const Rows& q, const Rows& k, const Rows& v, bool same_dtype, int64_t s_pad) {
-  return same_dtype && q.sk == 1 && k.sk == 1 && v.sk == 1 && v.b == k.b && v.r == k.r && v.k == k.k &&
+  return same_dtype && q.sk == 1 && k.sk == 1 && v.sk == 1 && v.b == k.b && v.r == k.r && v.k == k.k && k.k == q.k &&
          (q.k == 64 || q.k == 128 || q.k == 256) && s_pad % 16 == 0 && q.b * q.r * k.b * k.r > 0;
 }
 FwdPacks quant_qkv_rows(const Call& c, const Tensor& qt, const Tensor& kt, const Tensor& vt, const Rows& q, const Rows& k,
@@ -432,7 +440,7 @@ std::tuple<Tensor, OptTensor, std::vector<Tensor>> flash_attention(
   c.same(key);
   c.same(value);
   const int64_t s_pad = next_mult(s_kv, kKeyTile);
-  const Rows q = rows_of(query), k = rows_of(key), v = rows_of(value);
+  const Rows q = rows_of(query), k = rows_of(as_rows(key, z * hk, s_kv, d)), v = rows_of(as_rows(value, z * hk, s_kv, d));
   FwdPacks p;
   if (!qnv.has_value() && !knv.has_value()) {
     p = quant_qkv_rows(c, query, key, value, q, k, v, s_pad);       // one launch
@@ -727,6 +735,17 @@ Pack given_or_quant(const Call& c, const OptTensor& nv, const OptTensor& sc, con
   c.same(p.sc);
   return p;
 }
+// The kernels take Z, H, Sq, D from q and Hk, Skv from k; every other operand has to have as many rows.
+void check_bwd_operands(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse,
+                        const Tensor& dout) {
+  auto rows = [](const Tensor& t, int64_t b, int64_t s, int64_t d) {
+    return (t.dim() == 4 ? t.size(0) * t.size(1) == b : t.dim() == 3 && t.size(0) == b) && t.size(-2) == s && t.size(-1) == d;
+  };
+  const int64_t b = q.size(0) * q.size(1), bk = q.size(0) * k.size(1), s = q.size(2), d = q.size(3);
+  if (!rows(q, b, s, d) || !rows(k, bk, k.size(2), d) || !rows(v, bk, k.size(2), d) || !rows(out, b, s, d) ||
+      !rows(dout, b, s, d) || lse.numel() != b * s)
+    throw std::runtime_error("backward operands: shape mismatch between q, k, v, out, lse and the gradient of out");
+}
 constexpr const char* kQPacks = "q_packs layout mismatch: expected along-D packs of the query rows";
 constexpr const char* kKPacks = "k_packs layout mismatch: expected along-D packs of the key rows";
 
@@ -741,6 +760,7 @@ std::tuple<Tensor, Tensor, Tensor> bwd_hp(const Tensor& q, const Tensor& k, cons
   const int64_t z = q.size(0), h = q.size(1), s_q = q.size(2), d = q.size(3), hk = k.size(1), s_kv = k.size(2);
   require(d == 128 || d == 256, "D must be 128 or 256");
   const Tensor out = zshd ? out_in.transpose(1, 2) : out_in, dout = zshd ? dout_in.transpose(1, 2) : dout_in;
+  check_bwd_operands(q, k, v, out, lse_in, dout);
   const auto gdt = dout.scalar_type();
   const bool need_copy = !(gdt == at::kBFloat16 && dout.is_contiguous());
   Prep pp = bwd_prep_call(c, dout, out, need_copy, false);
@@ -775,6 +795,7 @@ std::tuple<Tensor, Tensor, Tensor> bwd_fp4(const Tensor& q, const Tensor& k, con
   const int64_t z = q.size(0), h = q.size(1), s_q = q.size(2), d = q.size(3), hk = k.size(1), s_kv = k.size(2);
   require(d == 128 || d == 256, "D must be 128 or 256");
   const Tensor out = zshd ? out_in.transpose(1, 2) : out_in, dout = zshd ? dout_in.transpose(1, 2) : dout_in;
+  check_bwd_operands(q, k, v, out, lse_in, dout);
   const auto gdt = dout.scalar_type();
   Prep pp = bwd_prep_call(c, dout, out, false, true);          // strided reads: no copy for the pre-pass
   const float* amax = pp.amax->data_ptr<float>();
