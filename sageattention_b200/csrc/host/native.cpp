@@ -605,11 +605,13 @@ void append_token(const Tensor& key_new, const Tensor& value_new, const Tensor& 
   c.same(value_new);
   const int64_t zhk = knv.size(0), d = knv.size(2) * 2;
   const auto t = v_partial.scalar_type();
-  // one row per (batch, kv head) unit: [Z, Hk, 1, D] or [Z*Hk, D]
+  require(key_new.numel() == zhk * d && value_new.numel() == zhk * d, "one token per (batch, kv head) unit");
+  // one row per (batch, kv head) unit: [Z, Hk, 1, D] or [Z*Hk, D] is read in place; any other shape of as many
+  // elements ([Z, 1, Hk, D], say) is brought to rows first
   auto rows = [&](const Tensor& x, int64_t& stride) -> Tensor {
-    if (x.scalar_type() == t && x.stride(-1) == 1) {
+    if (x.scalar_type() == t && x.stride(-1) == 1 && x.size(-1) == d) {
       if (x.dim() == 2) { stride = x.stride(0); return x; }
-      if (x.dim() == 4 && (x.size(0) == 1 || x.size(1) == 1 || x.stride(0) == x.size(1) * x.stride(1))) {
+      if (x.dim() == 4 && x.size(2) == 1 && (x.size(0) == 1 || x.size(1) == 1 || x.stride(0) == x.size(1) * x.stride(1))) {
         stride = x.size(1) == 1 ? x.stride(0) : x.stride(1);
         return x;
       }
@@ -617,7 +619,6 @@ void append_token(const Tensor& key_new, const Tensor& value_new, const Tensor& 
     stride = d;
     return x.reshape({zhk, d}).to(t).contiguous();
   };
-  require(key_new.numel() == zhk * d && value_new.numel() == zhk * d, "one token per (batch, kv head) unit");
   int64_t sk = 0, sv = 0;
   Tensor kn = rows(key_new, sk), vn = rows(value_new, sv);
   if (sk != sv) {

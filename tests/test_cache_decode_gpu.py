@@ -322,3 +322,27 @@ def test_decode_demo_small_model():
     assert rep["fp4"]["logit_cos"] > 0.97 and rep["hybrid"]["logit_cos"] > 0.97
     assert rep["fp4"]["bf16_bytes"] / rep["fp4"]["bytes"] > 2.5
     assert _status() == 0
+
+
+@pytest.mark.parametrize("z,hk", [(1, 4), (3, 4), (3, 1)])
+def test_append_takes_tokens_of_any_layout(z, hk):
+    """A token as [Z, Hk, 1, D], as rows, token-major ([Z, 1, Hk, D], a projection's own output) and strided:
+    the same cache."""
+    from sageattention_b200.nvfp4 import kv_cache
+    d, s = 128, 21
+    k, _ = seeded_bf16((z, hk, s, d), 61)
+    v, _ = seeded_bf16((z, hk, s, d), 62)
+    layouts = [lambda t: t, lambda t: t.contiguous().view(z * hk, d), lambda t: t.reshape(z, 1, hk, d).contiguous(),
+               lambda t: t.reshape(z, hk, d // 2, 2).contiguous(), lambda t: t.reshape(1, z * hk * d).contiguous(),
+               lambda t: t.transpose(0, 3).contiguous().transpose(0, 3)]
+    caches = []
+    for i, f in enumerate(layouts):
+        c = _n().NVFP4KVCache(z, hk, d, 64, "cuda", torch.bfloat16, recent_window=16)
+        for t in range(s):
+            kv_cache.append_token(f(k[:, :, t:t + 1]), layouts[(i + t) % 6](v[:, :, t:t + 1]), c.knv, c.ksc, c.vnv, c.vsc,
+                                  c.v_partial_bf16, c.rk, c.rv, t)
+        caches.append(c)
+    for c in caches[1:]:
+        for name in ("knv", "ksc", "vnv", "vsc", "v_partial_bf16", "rk", "rv"):
+            a, b = getattr(caches[0], name), getattr(c, name)
+            assert torch.equal(a.view(torch.uint8), b.view(torch.uint8)), name
