@@ -637,14 +637,15 @@ void append_token(const Tensor& key_new, const Tensor& value_new, const Tensor& 
 bool kv_prefill(const Tensor& key, const Tensor& value, const Tensor& knv, const Tensor& ksc, const Tensor& vnv,
                 const Tensor& vsc, const Tensor& v_partial, const OptTensor& rk, const OptTensor& rv) {
   require_cuda(key, "key");
+  require(key.dim() == 4, "key must be [Z, Hk, S, D]");
   Call c(knv);
   c.same(key);
   c.same(value);
   const auto t = v_partial.scalar_type();
   if (key.scalar_type() != t || value.scalar_type() != t) return false;
-  const Rows k = rows_of(key), v = rows_of(value);
+  const Rows k = rows_of(key), v = rows_of(as_rows(value, key.size(0) * key.size(1), key.size(2), key.size(3)));
   if (k.sk != 1 || v.sk != 1) return false;
-  require(k.b == knv.size(0) && v.b == k.b && v.r == k.r && v.k == k.k, "key and value must be [Z, Hk, S, D] of the cache");
+  require(k.b == knv.size(0) && k.k == knv.size(2) * 2, "key must be [Z, Hk, S, D] of the cache");
   require(k.r <= knv.size(1), "prefill exceeds capacity");
   c.done(nvfp4_kv_prefill(k.p, v.p, dtype_code(t), k.b, k.r, (int)k.k, k.sb, k.sr, v.sb, v.sr, u8(knv), knv.stride(0), u8(ksc),
                           ksc.stride(0), u8(vnv), vnv.stride(0), vnv.stride(1), u8(vsc), vsc.stride(0), vsc.stride(1),

@@ -27,3 +27,19 @@ def test_prefill_equals_general_path(s, d, window, dtype):
         for n in names:
             x, y = getattr(a, n), getattr(b, n)
             assert torch.equal(x.contiguous().view(torch.uint8), y.contiguous().view(torch.uint8)), n
+
+
+def test_prefill_takes_values_of_another_shape():
+    """A value of as many elements is taken as [Z*Hk, S, D] rows, any other is refused."""
+    import sageattention_b200.nvfp4 as nv
+    z, hk, s, d = 2, 3, 70, 128
+    k, v = (torch.randn(z, hk, s, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    caches = []
+    for other in (v, v.view(z * hk, s, d), v.view(1, z * hk, s, d), v.view(-1, d), v.view(z, hk, s, 2, d // 2)):
+        caches.append(nv.NVFP4KVCache(z, hk, d, 128, "cuda"))
+        caches[-1].prefill(k, other)
+    for c in caches[1:]:
+        assert torch.equal(caches[0].vnv, c.vnv) and torch.equal(caches[0].v_partial_bf16, c.v_partial_bf16)
+    for other in (v[:, :, 1:], v[:1], v[..., :64]):
+        with pytest.raises((RuntimeError, AssertionError)):
+            caches[0].prefill(k, other)
