@@ -557,6 +557,7 @@ Tensor hybrid_decode(const Tensor& query, const Tensor& knv, const Tensor& ksc, 
   c.same(rk);
   c.same(rv);
   const int64_t z = query.size(0), h = query.size(1), d = query.size(3), hk = rk.size(1), cap = rk.size(2);
+  require(rk.dim() == 4 && rk.size(0) == z && rk.size(3) == d && h == hk * g, "query does not fit the window's rings");
   const int64_t cut = std::max<int64_t>(0, length - recent_window) / 16 * 16, count = length - cut;
   Tensor q = query.stride(3) == 1 ? query : query.contiguous();
   if (q.scalar_type() != rk.scalar_type()) q = q.to(rk.scalar_type());

@@ -43,3 +43,14 @@ def test_prefill_takes_values_of_another_shape():
     for other in (v[:, :, 1:], v[:1], v[..., :64]):
         with pytest.raises((RuntimeError, AssertionError)):
             caches[0].prefill(k, other)
+
+
+@pytest.mark.parametrize("s", [20, 400])         # inside the window, and behind it
+def test_hybrid_decode_refuses_other_head_counts(s):
+    import sageattention_b200.nvfp4 as nv
+    c = nv.NVFP4KVCache(2, 2, 128, 512, "cuda", recent_window=128)
+    c.prefill(*(torch.randn(2, 2, s, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2)))
+    assert c.hybrid_decode(torch.randn(2, 4, 1, 128, device="cuda"), 0.1, 2).shape == (2, 4, 1, 128)
+    for shape, g in (((2, 4, 1, 128), 4), ((1, 4, 1, 128), 2), ((2, 4, 1, 64), 2)):
+        with pytest.raises((RuntimeError, AssertionError)):
+            c.hybrid_decode(torch.randn(*shape, device="cuda"), 0.1, g)
