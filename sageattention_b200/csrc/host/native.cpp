@@ -43,6 +43,9 @@ struct AssertionFailure : std::runtime_error {
 struct UnsupportedType : std::runtime_error {
   using std::runtime_error::runtime_error;
 };
+struct NotImplemented : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
 
 inline void require(bool ok, const char* msg) {
   if (__builtin_expect(!ok, 0)) throw AssertionFailure(msg);
@@ -923,6 +926,10 @@ Tensor attention(const Tensor& query, const Tensor& key, const Tensor& value, do
                  const OptTensor& bias, const OptTensor& seq_id, const OptTensor& seq_start, const OptTensor& seq_end, bool zshd,
                  const OptTensor& qnv, const OptTensor& qsc, const OptTensor& knv, const OptTensor& ksc, const std::string& mode,
                  bool sr, std::optional<bool> sr_p_dv, std::optional<bool> sr_dot_dv, std::optional<bool> sr_ds_dq) {
+  // A node made here has no rule for tangents, and the kernels would drop them without a word.
+  auto dual = [](const Tensor& t) { return t._fw_grad(0).defined(); };
+  if (dual(query) || dual(key) || dual(value) || (bias.has_value() && dual(*bias)))
+    throw NotImplemented("nvfp4_flash_attn_func does not implement forward-mode AD (no jvp)");
   const bool record = c10::GradMode::is_enabled() && (query.requires_grad() || key.requires_grad() || value.requires_grad());
   c10::AutoGradMode no_grad(false);
   auto [out, lse, packs] = flash_attention(query, key, value, scaling, causal, g, bias, false, seq_id, seq_start, zshd, true,
@@ -962,6 +969,8 @@ PYBIND11_MODULE(_native, m) {
       PyErr_SetString(PyExc_AssertionError, x.what());
     } catch (const UnsupportedType& x) {
       PyErr_SetString(PyExc_TypeError, x.what());
+    } catch (const NotImplemented& x) {
+      PyErr_SetString(PyExc_NotImplementedError, x.what());
     }
   });
   using nogil = py::call_guard<py::gil_scoped_release>;
