@@ -930,7 +930,9 @@ Tensor attention(const Tensor& query, const Tensor& key, const Tensor& value, do
   auto dual = [](const Tensor& t) { return t._fw_grad(0).defined(); };
   if (dual(query) || dual(key) || dual(value) || (bias.has_value() && dual(*bias)))
     throw NotImplemented("nvfp4_flash_attn_func does not implement forward-mode AD (no jvp)");
-  const bool record = c10::GradMode::is_enabled() && (query.requires_grad() || key.requires_grad() || value.requires_grad());
+  // A bias that requires a gradient gets none, but it makes the output part of the graph.
+  const bool record = c10::GradMode::is_enabled() && (query.requires_grad() || key.requires_grad() || value.requires_grad() ||
+                                                      (bias.has_value() && bias->requires_grad()));
   c10::AutoGradMode no_grad(false);
   auto [out, lse, packs] = flash_attention(query, key, value, scaling, causal, g, bias, false, seq_id, seq_start, zshd, true,
                                            record, qnv, qsc, knv, ksc);

@@ -42,3 +42,16 @@ def test_function_transforms_are_refused():
         torch.func.vmap(_attend)(q[None], k[None], v[None])
     with pytest.raises((RuntimeError, NotImplementedError)):
         torch.func.jvp(lambda q: _attend(q, k, v), (q,), (q,))
+
+
+@pytest.mark.parametrize("operands", [False, True])
+def test_bias_that_requires_a_gradient(operands):
+    """The bias gets no gradient; the output is part of the graph all the same, and backward runs."""
+    q, k, v, do = _inputs()
+    for t in (q, k, v):
+        t.requires_grad_(operands)
+    bias = torch.zeros(Z, S, device="cuda", requires_grad=True)
+    out = _attend(q, k, v, key_pad_bias=bias)
+    assert out.requires_grad
+    out.backward(do)
+    assert bias.grad is None and all((t.grad is not None) == operands for t in (q, k, v))
