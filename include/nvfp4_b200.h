@@ -240,7 +240,7 @@ int nvfp4_decode_static(const void* q, int q_dtype, int64_t s_qz, int64_t s_qh, 
                         int* status, nvfp4_stream_t stream);
 
 /*
- * Hybrid decode in two calls, replacing the torch code of `NVFP4KVCache.hybrid_decode`
+ * Hybrid decode, replacing the torch code of `NVFP4KVCache.hybrid_decode`
  * (kv_cache.py:293-351: FP4 prefix decode, bf16 window attention, log-sum-exp merge).
  *
  * nvfp4_window_partials: exact attention of one query token per head over `count` high-precision
@@ -253,10 +253,11 @@ int nvfp4_decode_static(const void* q, int q_dtype, int64_t s_qz, int64_t s_qh, 
  * such partials per unit (they follow the kernel's own slots: extra_base = own slots, total_slots =
  * own slots + Z*Hk*n_extra; workspace_bytes must cover them).  out / lse are the attention over
  * prefix and window together, written once in the query dtype.
- * NVFP4_DECODE_AFTER_WINDOW, or-ed to n_extra, says that nvfp4_window_partials was the stream's last
- * launch before this call: the split-K kernel then starts beside it instead of behind it.
+ *
+ * nvfp4_decode_window: both in one call, nvfp4_window_partials with extra_base = own slots and then
+ * the decode over prefix and window, with the split-K kernel beside the window's instead of behind
+ * it (which only the call that launches both can promise).
  */
-#define NVFP4_DECODE_AFTER_WINDOW 0x100
 int nvfp4_window_partials(const void* q, int dtype, int64_t s_qz, int64_t s_qh, const void* rk,
                           const void* rv, int64_t z, int64_t hk, int g, int d, int64_t ring_cap,
                           int64_t first_pos, int64_t count, float scaling, int pieces,
@@ -269,6 +270,14 @@ int nvfp4_decode_hybrid(const void* q, int q_dtype, int64_t s_qz, int64_t s_qh, 
                         float scaling, void* out, float* lse, void* workspace,
                         size_t workspace_bytes, int nsplit, int64_t split_kv, int n_extra,
                         int* status, nvfp4_stream_t stream);
+int nvfp4_decode_window(const void* q, int q_dtype, int64_t s_qz, int64_t s_qh, const uint8_t* knv,
+                        int64_t knv_unit, const uint8_t* ksc, int64_t ksc_unit, const uint8_t* vnv,
+                        int64_t vnv_unit, int64_t vnv_row, const uint8_t* vsc, int64_t vsc_unit,
+                        int64_t vsc_row, int64_t z, int64_t hk, int g, int d, int64_t s_kv,
+                        float scaling, void* out, float* lse, void* workspace,
+                        size_t workspace_bytes, int nsplit, int64_t split_kv, const void* rk,
+                        const void* rv, int64_t ring_cap, int64_t first_pos, int64_t count,
+                        int pieces, int* status, nvfp4_stream_t stream);
 
 /*
  * Exact merge of two attention results over disjoint key sets from their log-sum-exps:

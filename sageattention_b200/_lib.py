@@ -50,6 +50,11 @@ SIGNATURES = {
                                     c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int64, c_int64,
                                     c_int, c_int, c_int64, c_float, c_void_p, c_void_p, c_void_p, c_size_t,
                                     c_int, c_int64, c_int, c_void_p, c_void_p]),
+    "nvfp4_decode_window": (c_int, [c_void_p, c_int, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64,
+                                    c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int64, c_int64,
+                                    c_int, c_int, c_int64, c_float, c_void_p, c_void_p, c_void_p, c_size_t,
+                                    c_int, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int,
+                                    c_void_p, c_void_p]),
     "nvfp4_window_partials": (c_int, [c_void_p, c_int, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_int64,
                                       c_int, c_int, c_int64, c_int64, c_int64, c_float, c_int, c_void_p,
                                       c_int64, c_int64, c_void_p]),

@@ -935,20 +935,21 @@ extern "C" int nvfp4_decode(const void* q, int q_dtype, int64_t s_qz, int64_t s_
                              nsplit, split_kv, 0, status, stream);
 }
 
-extern "C" int nvfp4_decode_hybrid(const void* q, int q_dtype, int64_t s_qz, int64_t s_qh,
-                                   const uint8_t* knv, int64_t knv_unit, const uint8_t* ksc,
-                                   int64_t ksc_unit, const uint8_t* vnv, int64_t vnv_unit,
-                                   int64_t vnv_row, const uint8_t* vsc, int64_t vsc_unit,
-                                   int64_t vsc_row, int64_t z, int64_t hk, int g, int d, int64_t s_kv,
-                                   float scaling, void* out, float* lse, void* workspace,
-                                   size_t workspace_bytes, int nsplit, int64_t split_kv, int n_extra,
-                                   int* status, nvfp4_stream_t stream) {
-  using namespace nvfp4;
-  // The window kernel lets its successor start once all its CTAs have seen the work before it complete, so the
-  // split-K kernel, which reads nothing of the window's, streams the cache beside it (H16 Hk4 S17558 window
-  // 128 23.9 -> 19.5 us with the append; 256 window CTAs at two per SM leave it no room: Z8 S8190 window 512 unchanged).
-  const bool after_window = (n_extra & ~0xFF) == NVFP4_DECODE_AFTER_WINDOW;
-  if (after_window) n_extra &= 0xFF;
+namespace nvfp4 {
+
+struct DecodeWindow {
+  const void *rk, *rv;
+  int64_t ring_cap, first_pos, count;
+};
+
+// Checks, tensor maps and launches of all decode entries: `n_extra` further partials per unit, which the caller
+// has written or, with `window`, which the window kernel launched here writes.
+static int decode_call(const void* q, int q_dtype, int64_t s_qz, int64_t s_qh, const uint8_t* knv, int64_t knv_unit,
+                       const uint8_t* ksc, int64_t ksc_unit, const uint8_t* vnv, int64_t vnv_unit, int64_t vnv_row,
+                       const uint8_t* vsc, int64_t vsc_unit, int64_t vsc_row, int64_t z, int64_t hk, int g, int d,
+                       int64_t s_kv, float scaling, void* out, float* lse, void* workspace, size_t workspace_bytes,
+                       int nsplit, int64_t split_kv, int n_extra, const DecodeWindow* window, int* status,
+                       nvfp4_stream_t stream) {
   NVFP4_REQUIRE(n_extra >= 0 && n_extra <= 64, "nvfp4_decode: extra partials per unit must be in [0, 64]");
   NVFP4_REQUIRE(d == 128 || d == 256, "nvfp4_decode: D must be 128 or 256");
   NVFP4_REQUIRE(g >= 1 && g <= 16, "nvfp4_decode: GQA group %d must be <= 16", g);
@@ -1017,8 +1018,17 @@ extern "C" int nvfp4_decode_hybrid(const void* q, int q_dtype, int64_t s_qz, int
   p.ws_l = p.ws_m + slots * 16;
   p.extra_base = own_slots;
   p.n_extra = n_extra;
-  p.late_wait = after_window ? 1 : 0;
+  p.late_wait = window != nullptr ? 1 : 0;
   p.status = status;
+  if (window != nullptr) {
+    // The window kernel lets its successor start once all its CTAs have seen the work before it complete, so the
+    // split-K kernel, which reads nothing of the window's, streams the cache beside it (H16 Hk4 S17558 window
+    // 128 23.9 -> 19.5 us with the append; 256 window CTAs at two per SM leave it no room: Z8 S8190 window 512
+    // unchanged).  That holds for a split-K kernel directly behind the window's, which is why both are launched here.
+    const int rw = nvfp4_window_partials(q, q_dtype, s_qz, s_qh, window->rk, window->rv, z, hk, g, d, window->ring_cap,
+                                         window->first_pos, window->count, scaling, n_extra, ws, slots, own_slots, stream);
+    if (rw) return rw;
+  }
 
 #define NVFP4_DECODE(DD, T) return decode_launch<DD, T>(tm_k, tm_v, tm_vpf, tm_vpf4, p, zhk, out, lse, sm_count, st)
   if (d == 128) {
@@ -1036,6 +1046,38 @@ extern "C" int nvfp4_decode_hybrid(const void* q, int q_dtype, int64_t s_qz, int
   }
 #undef NVFP4_DECODE
   return fail(-1, "nvfp4_decode: unknown dtype %d", q_dtype);
+}
+
+}  // namespace nvfp4
+
+extern "C" int nvfp4_decode_hybrid(const void* q, int q_dtype, int64_t s_qz, int64_t s_qh,
+                                   const uint8_t* knv, int64_t knv_unit, const uint8_t* ksc,
+                                   int64_t ksc_unit, const uint8_t* vnv, int64_t vnv_unit,
+                                   int64_t vnv_row, const uint8_t* vsc, int64_t vsc_unit,
+                                   int64_t vsc_row, int64_t z, int64_t hk, int g, int d, int64_t s_kv,
+                                   float scaling, void* out, float* lse, void* workspace,
+                                   size_t workspace_bytes, int nsplit, int64_t split_kv, int n_extra,
+                                   int* status, nvfp4_stream_t stream) {
+  return nvfp4::decode_call(q, q_dtype, s_qz, s_qh, knv, knv_unit, ksc, ksc_unit, vnv, vnv_unit, vnv_row, vsc, vsc_unit,
+                            vsc_row, z, hk, g, d, s_kv, scaling, out, lse, workspace, workspace_bytes, nsplit, split_kv,
+                            n_extra, nullptr, status, stream);
+}
+
+extern "C" int nvfp4_decode_window(const void* q, int q_dtype, int64_t s_qz, int64_t s_qh,
+                                   const uint8_t* knv, int64_t knv_unit, const uint8_t* ksc,
+                                   int64_t ksc_unit, const uint8_t* vnv, int64_t vnv_unit,
+                                   int64_t vnv_row, const uint8_t* vsc, int64_t vsc_unit,
+                                   int64_t vsc_row, int64_t z, int64_t hk, int g, int d, int64_t s_kv,
+                                   float scaling, void* out, float* lse, void* workspace,
+                                   size_t workspace_bytes, int nsplit, int64_t split_kv, const void* rk,
+                                   const void* rv, int64_t ring_cap, int64_t first_pos, int64_t count, int pieces,
+                                   int* status, nvfp4_stream_t stream) {
+  using namespace nvfp4;
+  NVFP4_REQUIRE(pieces >= 1, "nvfp4_decode_window: pieces must be in [1, 64]");
+  const DecodeWindow window = {rk, rv, ring_cap, first_pos, count};
+  return decode_call(q, q_dtype, s_qz, s_qh, knv, knv_unit, ksc, ksc_unit, vnv, vnv_unit, vnv_row, vsc, vsc_unit,
+                            vsc_row, z, hk, g, d, s_kv, scaling, out, lse, workspace, workspace_bytes, nsplit, split_kv,
+                            pieces, &window, status, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

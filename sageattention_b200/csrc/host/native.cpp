@@ -522,23 +522,23 @@ std::tuple<Tensor, OptTensor> decode_core(const Call& c, const Tensor& query, co
     nsplit = (int)((a.s_kv + split_kv - 1) / split_kv);
     wbytes = (size_t)(zhk * nsplit * slot_bytes);
   }
-  const int64_t own = (int64_t)wbytes / slot_bytes;
-  const int64_t extra = win ? win->pieces : 0, slots = own + zhk * extra;
-  Tensor ws = c.empty({slots * slot_bytes}, at::kByte);
-  if (win)
-    c.done(nvfp4_window_partials(q.data_ptr(), dtype_code(q.scalar_type()), q.stride(0), q.stride(1), win->rk->data_ptr(),
-                                 win->rv->data_ptr(), a.z, hk, (int)a.g, (int)a.d, win->ring_cap, win->first, win->count,
-                                 (float)a.scaling, win->pieces, ws.data_ptr(), slots, own, c.stream),
-           "nvfp4_window_partials");
+  wbytes += (size_t)(win ? zhk * win->pieces * slot_bytes : 0);       // the window's partials behind the decode's own
+  Tensor ws = c.empty({(int64_t)wbytes}, at::kByte);
   Tensor out = c.empty({a.z, a.h, 1, a.d}, q.scalar_type());
   OptTensor lse;
   if (want_lse) lse = c.empty({a.z, a.h}, at::kFloat);
-  c.done(nvfp4_decode_hybrid(q.data_ptr(), dtype_code(q.scalar_type()), q.stride(0), q.stride(1), u8(*a.knv), a.knv->stride(0),
-                             u8(*a.ksc), a.ksc->stride(0), u8(*a.vnv), a.vnv->stride(0), a.vnv->stride(1), u8(*a.vsc),
-                             a.vsc->stride(0), a.vsc->stride(1), a.z, hk, (int)a.g, (int)a.d, a.s_kv, (float)a.scaling,
-                             out.data_ptr(), opt_ptr<float>(lse), ws.data_ptr(), (size_t)(slots * slot_bytes), nsplit, split_kv,
-                             (int)extra | (win ? NVFP4_DECODE_AFTER_WINDOW : 0), c.status, c.stream),
-         "nvfp4_decode");
+  auto run = [&](auto entry, const char* what, auto... window) {
+    c.done(entry(q.data_ptr(), dtype_code(q.scalar_type()), q.stride(0), q.stride(1), u8(*a.knv), a.knv->stride(0), u8(*a.ksc),
+                 a.ksc->stride(0), u8(*a.vnv), a.vnv->stride(0), a.vnv->stride(1), u8(*a.vsc), a.vsc->stride(0),
+                 a.vsc->stride(1), a.z, hk, (int)a.g, (int)a.d, a.s_kv, (float)a.scaling, out.data_ptr(), opt_ptr<float>(lse),
+                 ws.data_ptr(), wbytes, nsplit, split_kv, window..., c.status, c.stream),
+           what);
+  };
+  if (win)
+    run(nvfp4_decode_window, "nvfp4_decode_window", win->rk->data_ptr(), win->rv->data_ptr(), win->ring_cap, win->first,
+        win->count, win->pieces);
+  else
+    run(nvfp4_decode, "nvfp4_decode");
   return {out, lse};
 }
 

@@ -80,3 +80,19 @@ def test_host_policy_tables():
     assert sid.tolist() == [0, 0, 0, 2, 2, 2, 2, 2, 2, 2] and st.tolist()[3] == 3 and en.tolist()[0] == 3
     with pytest.raises(AssertionError, match=r"cu_seqlens\[-1\]"):
         flash._varlen_seq_arrays(torch.tensor([0, 4], dtype=torch.int32), 10, "cpu")
+
+
+def test_hybrid_decode_takes_no_ordering_promise():
+    """Bits above the count of extra partials are an invalid count, not a promise of the caller about what was
+    launched before; the call that launches window and decode itself checks its own count."""
+    from sageattention_b200 import _lib
+    if not os.path.exists(_lib.LIB_PATH):
+        pytest.skip("library not built")
+    L = _lib.lib()
+    args = (0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 1, 1, 128, 128, 1.0, 0, 0, 0, 0, 1, 128)
+    for n_extra in (0x100, 0x101, 65, -1):
+        assert L.nvfp4_decode_hybrid(*args, n_extra, None, None) < 0
+        assert b"extra partials" in L.nvfp4_last_error()
+    for pieces in (0, 65, 0x101):
+        assert L.nvfp4_decode_window(*args, None, None, 16, 0, 16, pieces, None, None) < 0
+        assert b"partials" in L.nvfp4_last_error() or b"pieces" in L.nvfp4_last_error()

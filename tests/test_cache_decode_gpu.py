@@ -346,3 +346,32 @@ def test_append_takes_tokens_of_any_layout(z, hk):
         for name in ("knv", "ksc", "vnv", "vsc", "v_partial_bf16", "rk", "rv"):
             a, b = getattr(caches[0], name), getattr(c, name)
             assert torch.equal(a.view(torch.uint8), b.view(torch.uint8)), name
+
+
+@pytest.mark.parametrize("d,z,hk,s,window", [(128, 1, 4, 5000, 128), (128, 3, 2, 700, 512), (256, 2, 2, 1500, 200)])
+def test_hybrid_decode_equals_its_two_calls(d, z, hk, s, window):
+    """The decode beside the window kernel (one C call) against the decode behind it (two)."""
+    from sageattention_b200 import _lib
+    from sageattention_b200.nvfp4 import flash
+    n, g = _n(), 2
+    c = n.NVFP4KVCache(z, hk, d, s + 128, "cuda", torch.bfloat16, recent_window=window)
+    q, _ = seeded_bf16((z, g * hk, 1, d), 71)
+    c.prefill(seeded_bf16((z, hk, s, d), 72)[0], seeded_bf16((z, hk, s, d), 73)[0])
+    one = c.hybrid_decode(q, d ** -0.5, g)
+    cut = (s - window) // 16 * 16
+    count, slot = s - cut, (16 * d + 32) * 4
+    pieces = -(-count // 144)
+    nsplit, split_kv, own_bytes = flash._decode_plan(cut, z * hk, d, "cuda")
+    own = own_bytes // slot
+    slots = own + z * hk * pieces
+    ws, out = torch.empty(slots * slot, dtype=torch.uint8, device="cuda"), torch.empty_like(q)
+    st, dt = _lib.stream_ptr("cuda"), _lib.dtype_code(q.dtype)
+    dev = torch.device("cuda")
+    _lib.call("nvfp4_window_partials", dev, q.data_ptr(), dt, q.stride(0), q.stride(1), c.rk.data_ptr(), c.rv.data_ptr(), z,
+              hk, g, d, c.ring_cap, cut, count, d ** -0.5, pieces, ws.data_ptr(), slots, own, st)
+    _lib.call("nvfp4_decode_hybrid", dev, q.data_ptr(), dt, q.stride(0), q.stride(1), c.knv.data_ptr(), c.knv.stride(0),
+              c.ksc.data_ptr(), c.ksc.stride(0), c.vnv.data_ptr(), c.vnv.stride(0), c.vnv.stride(1), c.vsc.data_ptr(),
+              c.vsc.stride(0), c.vsc.stride(1), z, hk, g, d, cut, d ** -0.5, out.data_ptr(), None, ws.data_ptr(), ws.numel(),
+              nsplit, split_kv, pieces, None, st)
+    assert _status() == 0
+    assert torch.equal(one, out)
