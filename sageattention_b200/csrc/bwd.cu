@@ -319,7 +319,7 @@ struct BwdParams {
   float scaling;
   int causal;
   int split;            // CTAs (of one cluster) that share a tile's steps
-  int late_wait;        // independent of the kernel before it: wait for it at the end, not at the start
+  int late_wait;        // dQ kernel: wait for the kernel before it at the end, not at the start (launch.cuh)
   int* status;
 };
 
@@ -477,7 +477,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&tmem_base_s, 512);
-  griddep_wait();
+  griddep_wait();                 // before griddep_launch(): the dQ kernel behind it waits late (launch.cuh)
   // 64-query steps that can see a key of this tile
   int q_lo = 0, q_hi = p.s_q;
   if (p.causal) q_lo = max(0, n0 - shift);
@@ -843,7 +843,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&tmem_base_s, 512);
-  if (!p.late_wait) griddep_wait();
+  griddep_start(p.late_wait != 0);
   int k_lo = 0, k_hi = p.s_kv;
   if (p.causal) k_hi = max(0, min(p.s_kv, m0 + 128 + shift));
   if (varlen) {

@@ -137,7 +137,7 @@ struct B4Params {
   float scaling;
   int causal;
   int split;             // dV / dK passes: CTAs (of one cluster along z) that share a tile's stages
-  int late_wait;         // independent of the kernel before it: wait for it at the end, not at the start
+  int late_wait;         // a later pass: wait for the kernel before it at the end, not at the start (launch.cuh)
   int sr_p, sr_ds;       // stochastic rounding of the in-kernel P / dS packs (fp4_legacy mode)
   uint32_t seed;
   int* status;
@@ -259,7 +259,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&tmem_base_s, 512);
-  if (!p.late_wait) griddep_wait();
+  griddep_start(p.late_wait != 0);     // before griddep_launch(): the passes behind the first wait late (launch.cuh)
   if (tid == 0) gs_s = pow2_ceil(p.amax != nullptr ? *p.amax : 1.0f);
 
   // ---- rows of this CTA, and the range of 128-column stages it has to visit

@@ -8,6 +8,22 @@
 //     complete and visible, and since no kernel finishes without it, completion is transitive;
 //   * a kernel that allocates tensor memory calls griddep_launch() only after its allocation, so a
 //     dependent that starts on the same SM cannot take columns its predecessor still waits for.
+// One exception, the late wait: a kernel that needs nothing of the kernel P launched directly before it may
+// take the operands that were there before P at once and call griddep_wait() at its END, where it keeps
+// completion transitive.  It then starts as soon as P has signalled, and rests on three conditions:
+//   * P executes griddep_wait() BEFORE griddep_launch(): its signal says that everything before P is
+//     complete.  (P may be a late waiter itself, directly behind such a kernel: it starts after that signal.)
+//     Swapping the two lines in P would be a race that no test is sure to show;
+//   * one host call launches both.  A launch that another thread puts between them does no harm, it cannot start
+//     before P's signal either; but only a caller that launches P knows that nothing it needs comes after P;
+//   * it reads nothing that P writes and writes nothing that P reads or writes.
+// No wait of its own stands between those operands and its first loads, so griddep_start() puts a fence there: what
+// an SM's L1 kept from before their writers completed is not read.  TMA reads L2; a warp that only issues such
+// loads need not stand behind the fence's ~0.3 us.
+// Late waiters, and what each stands behind:
+//   bwd_dq_kernel   behind bwd_dkdv_kernel (nvfp4_bwd_hp)
+//   bwd4_kernel     passes after the first, behind bwd4_kernel (nvfp4_bwd_fp4)
+//   decode_kernel   behind window_mma_kernel or window_attention_kernel (nvfp4_decode_window)
 #pragma once
 #include <cuda_runtime.h>
 #include <atomic>
@@ -18,6 +34,11 @@ namespace nvfp4 {
 
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Start of a kernel that can be a late waiter (its end calls griddep_wait() if `late`); `l1`: the thread loads through L1.
+__device__ __forceinline__ void griddep_start(bool late, bool l1 = true) {
+  if (!late) griddep_wait();
+  else if (l1) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+}
 
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per kernel and device: a fixed open-addressing
 // table of kernel addresses (the library has fewer kernels than slots), lock-free, so that a launch

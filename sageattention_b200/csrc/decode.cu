@@ -91,7 +91,7 @@ struct DecodeParams {
   float* ws_l;    // [nitems][16]
   int64_t extra_base;   // first of the partial slots appended by another kernel (n_extra per unit)
   int n_extra;
-  int late_wait;        // independent of the kernel before it: wait for it at the end, not at the start
+  int late_wait;        // behind the window kernel: wait for it at the end, not at the start (launch.cuh)
   int* status;
 };
 
@@ -194,7 +194,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     mbar_fence_init();
   }
   __syncthreads();
-  if (!p.late_wait) griddep_wait();
+  griddep_start(p.late_wait != 0, warp != 0);
   // The TMA producer (warp 0) and the scale loader (warp 2) need nothing but the barriers and the
   // stage buffers: they start streaming now, while the other warps allocate TMEM and clear the
   // operand buffers behind a barrier of their own.

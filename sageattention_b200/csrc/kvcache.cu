@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(512) window_attention_kernel(
     float* __restrict__ ws_acc, float* __restrict__ ws_m, float* __restrict__ ws_l, int64_t extra_base) {
   extern __shared__ __align__(16) float sm[];
   griddep_wait();
-  griddep_launch();                       // in this order: see nvfp4_decode_window
+  griddep_launch();                       // in this order: the decode kernel behind it waits late (launch.cuh)
   const bool partial = ws_acc != nullptr;
   const int k0 = partial ? (int)blockIdx.y * chunk : 0;
   const int count = partial ? min(chunk, count_all - k0) : count_all;
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kWinThreads, D == 128 ? 2 : 1) window_mma_kern
   constexpr int kChunks = D / 8;          // 16-byte chunks of a row
   extern __shared__ __align__(128) uint8_t wsm[];
   griddep_wait();
-  griddep_launch();                       // in this order: see nvfp4_decode_window
+  griddep_launch();                       // in this order: the decode kernel behind it waits late (launch.cuh)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int k0 = (int)blockIdx.y * chunk;
   const int count = min(chunk, count_all - k0);
