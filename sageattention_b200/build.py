@@ -4,7 +4,8 @@
 (in parallel, skipping objects newer than all sources and headers) and links one shared library next
 to this file.  No torch headers are involved: the library is a plain C ABI
 (``include/nvfp4_b200.h``).  The operators' host path (``csrc/host/native.cpp``, a Python extension on
-torch's C++ API) is compiled with the host compiler beside them and linked against that library.
+torch's C++ API) is compiled with the host compiler beside them and linked against that library, again
+when torch is another one than it was compiled against.
 """
 
 from __future__ import annotations
@@ -60,6 +61,22 @@ def _run(cmd, what: str) -> str:
     return r.stderr
 
 
+def _native_tag(cmd) -> str:
+    """What the host path's object depends on besides its sources: torch (its headers, its ABI) and the command."""
+    import torch
+    return "\n".join([torch.__version__, str(torch.version.git_version), *cmd])
+
+
+def _native_stale(obj: str, cmd) -> bool:
+    """Older than its sources, or compiled against another torch: the stamp beside the object says which."""
+    if not os.path.exists(obj) or not os.path.exists(obj + ".tag"):
+        return True
+    with open(obj + ".tag") as f:
+        if f.read() != _native_tag(cmd):
+            return True
+    return os.path.getmtime(obj) < max(os.path.getmtime(NATIVE_SRC), os.path.getmtime(_headers()[0]))
+
+
 def _headers():
     out = [os.path.join(os.path.dirname(HERE), "include", "nvfp4_b200.h")]
     for root, _, files in os.walk(CSRC):
@@ -80,8 +97,8 @@ def build(verbose: bool = False, force: bool = False) -> str:
         cmd = [nvcc, *(["-Xptxas=-v"] if verbose else []), *NVCC_FLAGS, "-c", s, "-o", o]
         jobs.append((cmd, s, o, stale))
     native_obj, native_compile, native_link = _native_commands(nvcc)
-    jobs.append((native_compile, NATIVE_SRC, native_obj, force or not os.path.exists(native_obj) or
-                 os.path.getmtime(native_obj) < max(os.path.getmtime(NATIVE_SRC), os.path.getmtime(_headers()[0]))))
+    native_stale = force or _native_stale(native_obj, native_compile)
+    jobs.append((native_compile, NATIVE_SRC, native_obj, native_stale))
 
     def compile_one(job):
         cmd, s, _, stale = job
@@ -92,6 +109,9 @@ def build(verbose: bool = False, force: bool = False) -> str:
 
     with ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
         logs = list(ex.map(compile_one, jobs))
+    if native_stale:
+        with open(native_obj + ".tag", "w") as f:
+            f.write(_native_tag(native_compile))
     if verbose:
         for log in logs:
             if log:
