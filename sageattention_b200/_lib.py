@@ -120,7 +120,7 @@ def native():
             raise RuntimeError("sageattention_b200/_native.so is missing or unusable: build it with "
                                f"`python -m sageattention_b200.build` ({exc})") from exc
         from .nvfp4 import flash
-        ext.set_backward(flash._attention_backward, vars(flash))
+        ext.set_backward(flash._attention_backward)
         _native = ext
     return _native
 

@@ -874,15 +874,11 @@ std::tuple<Tensor, Tensor, Tensor> bwd_fp4(const Tensor& q, const Tensor& k, con
 // The differentiable attention as a graph node of its own: a Python autograd.Function with the
 // operator's 26 arguments costs ~55 us per forward and backward before any kernel is launched, more than
 // the kernels of a short training step.  The node keeps the operands.  Backward with bf16 gradient products
-// calls bwd_hp below without entering the interpreter, as long as the package's _run_bwd_hp is its own (a
-// program may have wrapped it); everything else goes through flash._attention_backward, which picks the kernels by mode.
-PyObject *g_backward = nullptr, *g_namespace = nullptr, *g_bwd_hp = nullptr;        // set once; never released
+// calls bwd_hp above without entering the interpreter; the block-scaled modes go through flash._attention_backward
+// (stochastic-rounding defaults and seed).  The node's name states the mode.
+PyObject* g_backward = nullptr;        // set once; never released
 
-void set_backward(py::object fn, py::dict ns) {
-  g_backward = fn.release().ptr();
-  g_bwd_hp = py::object(ns["_run_bwd_hp"]).release().ptr();
-  g_namespace = ns.release().ptr();
-}
+void set_backward(py::object fn) { g_backward = fn.release().ptr(); }
 
 struct AttentionBackward : torch::autograd::Node {
   torch::autograd::SavedVariable q, k, v, out, lse, qnv, qsc, knv, ksc, bias, seq_id, seq_start, seq_end;
@@ -892,7 +888,7 @@ struct AttentionBackward : torch::autograd::Node {
   std::string mode;
   std::optional<bool> sr_p_dv, sr_dot_dv, sr_ds_dq;
 
-  std::string name() const override { return "NVFP4AttentionBackward"; }
+  std::string name() const override { return "NVFP4AttentionBackward[" + mode + "]"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
     for (auto* x : {&q, &k, &v, &out, &lse, &qnv, &qsc, &knv, &ksc, &bias, &seq_id, &seq_start, &seq_end}) x->reset_data();
@@ -908,12 +904,11 @@ struct AttentionBackward : torch::autograd::Node {
       for (int i = 0; i < 8; ++i)
         if (Tensor t = saved[i]->unpack(); t.defined()) o[i] = t;
     }
-    py::gil_scoped_acquire gil;
-    if (mode == "bf16" && PyDict_GetItemString(g_namespace, "_run_bwd_hp") == g_bwd_hp) {
-      py::gil_scoped_release open;
+    if (mode == "bf16") {
       auto [dq, dk, dv] = bwd_hp(qt, kt, vt, ot, lt, grads[0], scaling, causal, o[1], o[2], zshd, o[3], o[4], o[5], o[6], o[7]);
       return {dq, dk, dv};
     }
+    py::gil_scoped_acquire gil;
     py::object r = py::reinterpret_borrow<py::object>(g_backward)(
         qt, kt, vt, ot, lt, grads[0], scaling, causal, g, o[0], o[1], o[2], zshd, mode, o[3], o[4], o[5], o[6], o[7], sr,
         sr_p_dv, sr_dot_dv, sr_ds_dq);

@@ -482,12 +482,10 @@ class _NVFP4FlashAttn(torch.autograd.Function):
 
 def _attention_backward(query, key, value, out, lse, grad_out, scaling, causal, g, seq_id, seq_start, seq_end, zshd, mode,
                         qnv, qsc, knv, ksc, bias, sr, sr_p_dv, sr_dot_dv, sr_ds_dq):
-    """Backward entry of the native graph node of ``nvfp4_flash_attn_func``: ``(dq, dk, dv)``."""
+    """Block-scaled modes of the native graph node of ``nvfp4_flash_attn_func``: ``(dq, dk, dv)``.  (The node runs
+    the "bf16" mode without coming here.)"""
     varlen = (seq_id, seq_start, seq_end) if seq_id is not None else None
     layout = "zshd" if zshd else "zhsd"
-    if mode == "bf16":
-        return _run_bwd_hp(query, key, value, out, lse, grad_out, scaling, causal, g, varlen, layout, q_packs=(qnv, qsc),
-                           k_packs=(knv, ksc), key_pad_bias=bias)
     return _run_bwd(query, key, value, out, lse, grad_out, scaling, causal, g, varlen, layout, mode=mode, q_packs=(qnv, qsc),
                     k_packs=(knv, ksc), key_pad_bias=bias, sr=sr, sr_p_dv=sr_p_dv, sr_dot_dv=sr_dot_dv, sr_ds_dq=sr_ds_dq)
 

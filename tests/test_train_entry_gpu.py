@@ -63,54 +63,42 @@ def test_entry_rejects_bad_arguments():
     assert _status() == 0
 
 
-def test_auto_gate_and_deprecated_alias_dispatch(monkeypatch):
+def test_auto_gate_and_deprecated_alias_dispatch():
     """``backward_grad_dots=None`` resolves on s_kv (or the mean sample length of a packed row);
-    the legacy boolean maps True -> "bf16", False -> "fp4_legacy"."""
+    the legacy boolean maps True -> "bf16", False -> "fp4_legacy".  The graph node's name states the mode;
+    the gradients are those of that mode's kernels, to the bit."""
     from sageattention_b200.nvfp4 import flash
-    calls = []
-    real_hp, real_fp4 = flash._run_bwd_hp, flash._run_bwd
-
-    nested = [0]                       # the FP4-mode entry runs on the high-precision kernels here
-
-    def spy_hp(*a, **kw):
-        if not nested[0]:
-            calls.append("bf16")
-        return real_hp(*a, **kw)
-
-    def spy_fp4(*a, **kw):
-        calls.append(kw.get("mode", "fp4_legacy"))
-        nested[0] += 1
-        try:
-            return real_fp4(*a, **kw)
-        finally:
-            nested[0] -= 1
-
-    monkeypatch.setattr(flash, "_run_bwd_hp", spy_hp)
-    monkeypatch.setattr(flash, "_run_bwd", spy_fp4)
     d = 128
 
-    def run(s, cu=None, **kw):
+    def run(mode, s, cu=None, **kw):
         (q, _), (k, _), (v, _) = _qkv(1, 2, 2, s, d, s)
+        args = dict(causal=True, num_key_value_groups=1, cu_seqlens=cu)
+        out, lse, packs = flash.nvfp4_flash_attention(q, k, v, d ** -0.5, return_lse=True, return_packs=True, **args)
+        do = torch.ones_like(out)
+        arrays = None if cu is None else flash._varlen_seq_arrays(cu, s, q.device)
+        back = flash._run_bwd_hp if mode == "bf16" else flash._run_bwd
+        ref = back(q, k, v, out, lse, do, d ** -0.5, True, 1, arrays, q_packs=packs[0:2], k_packs=packs[2:4],
+                   **({} if mode == "bf16" else {"mode": mode}))
         q, k, v = (t.requires_grad_(True) for t in (q, k, v))
-        out = flash.nvfp4_flash_attn_func(q, k, v, d ** -0.5, causal=True, num_key_value_groups=1,
-                                          cu_seqlens=cu, stochastic_rounding=False, **kw)
-        out.backward(torch.ones_like(out))
-        for t in (q.grad, k.grad, v.grad):
-            assert t is not None and torch.isfinite(t).all()
+        got = flash.nvfp4_flash_attn_func(q, k, v, d ** -0.5, stochastic_rounding=False, **args, **kw)
+        name = got.grad_fn.name()
+        got.backward(do)
+        for t, r in zip((q.grad, k.grad, v.grad), ref):
+            assert torch.isfinite(t).all() and torch.equal(t, r), mode
+        return name
 
-    run(256)
-    assert calls[-1] == "bf16"
-    run(4096)
-    assert calls[-1] == "fp4_rownorm"
+    def native(mode):
+        return f"NVFP4AttentionBackward[{mode}]"
+
+    assert run("bf16", 256) == native("bf16")
+    assert run("fp4_rownorm", 4096) == native("fp4_rownorm")
     cu = torch.tensor([512 * i for i in range(10)], dtype=torch.int32)
-    run(4608, cu=cu)                                      # S > 4096, mean sample length 512
-    assert calls[-1] == "bf16"
-    run(128, backward_bf16_grad_dots=True)
-    assert calls[-1] == "bf16"
-    run(128, backward_bf16_grad_dots=False)
-    assert calls[-1] == "fp4_legacy"
-    run(128, save_backward_packs=True)                    # only packs saved: "bf16" downgrades
-    assert calls[-1] == "fp4_rownorm"
+    assert run("bf16", 4608, cu=cu) == native("bf16")                    # S > 4096, mean sample length 512
+    assert run("bf16", 128, backward_bf16_grad_dots=True) == native("bf16")
+    assert run("fp4_legacy", 128, backward_bf16_grad_dots=False) == native("fp4_legacy")
+    assert run("fp8_rownorm", 128, backward_grad_dots="fp8_rownorm") == native("fp8_rownorm")
+    # only packs saved: "bf16" downgrades (and the packs are kept by the Python function)
+    assert "NVFP4FlashAttn" in run("fp4_rownorm", 128, save_backward_packs=True)
     assert _status() == 0
 
 
