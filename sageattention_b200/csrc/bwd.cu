@@ -1219,7 +1219,10 @@ extern "C" int nvfp4_bwd_hp(const uint8_t* qnv, const uint8_t* qsc, const uint8_
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t tiles = (s_kv + 127) / 128, longest = (h / hk) * ((s_q + 63) / 64);
-    p.split = cluster_split(zhk * tiles * halves, longest, p.causal ? (h / hk) * 2 : longest, varlen, sms, 6.0);
+    if (int r0 = allow_smem("nvfp4_bwd_hp", reinterpret_cast<const void*>(ksplit), smem_dkdv)) return r0;
+    int slots[4];
+    cluster_slots(reinterpret_cast<const void*>(ksplit), kBwdThreads, smem_dkdv, sms, slots);
+    p.split = cluster_split(zhk * tiles * halves, longest, p.causal ? (h / hk) * 2 : longest, varlen, slots);
     auto kdkdv = p.split > 1 ? ksplit : kwhole;
     if (int r0 = allow_smem("nvfp4_bwd_hp", reinterpret_cast<const void*>(kdkdv), smem_dkdv)) return r0;
     dim3 g1((unsigned)zhk, (unsigned)tiles, halves * p.split);

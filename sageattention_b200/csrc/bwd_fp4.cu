@@ -840,7 +840,9 @@ extern "C" int nvfp4_bwd_fp4(const uint8_t* qnv, const uint8_t* qsc, const uint8
       a.out1 = dv; a.out2 = dk; a.c_pad = (int)sq_pad;
       a.sr_p = (flags & NVFP4_BWD_SR_P_DV) ? 1 : 0; a.sr_ds = (flags & NVFP4_BWD_SR_DS_DK) ? 1 : 0;
       const int64_t g = h / hk, tiles = (s_kv + 127) / 128;
-      a.split = cluster_split(zhk * tiles, g * ((s_q + 127) / 128), p.causal ? g : g * ((s_q + 127) / 128), varlen, sms, 3.0);
+      int slots[4];
+      cluster_slots(reinterpret_cast<const void*>(kern), threads, smem, sms, slots);
+      a.split = cluster_split(zhk * tiles, g * ((s_q + 127) / 128), p.causal ? g : g * ((s_q + 127) / 128), varlen, slots);
       return launch_cluster(what, kern, dim3((unsigned)zhk, (unsigned)tiles, (unsigned)a.split), a.split, threads, smem, st, t_k,
                             t_vd, t_q, t_do, t_dot, t_qt, a);
     }

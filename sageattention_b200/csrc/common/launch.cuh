@@ -65,6 +65,34 @@ inline int allow_smem(const char* what, const void* kern, int bytes) {
   return 0;
 }
 
+// Clusters of 1, 2, 4 and 8 CTAs of a kernel that are resident at once, asked once per device: for kernels that leave
+// room for one CTA per SM only (the answer depends on that alone).  allow_smem() has been called for `kern`.
+inline void cluster_slots(const void* kern, unsigned threads, int smem, int sms, int (&slots)[4]) {
+  static std::atomic<int> known[64][4];
+  int dev = 0;
+  const bool keep = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
+  for (int i = 0; i < 4; ++i) {
+    slots[i] = keep ? known[dev][i].load(std::memory_order_relaxed) : 0;
+    if (slots[i] > 0) continue;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1u << i;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, 1u << i);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&slots[i], kern, &cfg) != cudaSuccess || slots[i] < 1) {
+      cudaGetLastError();
+      slots[i] = sms >> i;
+    } else if (keep) {
+      known[dev][i].store(slots[i], std::memory_order_relaxed);
+    }
+  }
+}
+
 // Launch with programmatic stream serialisation; launch_cluster: clusters of `cluster` CTAs along z.
 template <typename... P, typename... A>
 int launch_cluster(const char* what, void (*kern)(P...), dim3 grid, unsigned cluster, unsigned threads, size_t smem,

@@ -27,9 +27,9 @@ def _grads(q, k, v, do, g, causal, mode, cu=None):
     return q.grad, k.grad, v.grad
 
 
-# One batch entry alone leaves most SMs idle, so its key tiles are split; among `copies` of itself there are
-# enough tiles that they are not (or less).  Split 8 of few steps: CTAs of a cluster with none; ragged ends;
-# a head dim of two halves; keys that only the last rows see.
+# One batch entry alone leaves most SMs idle, so its key tiles are split where they have enough steps; among
+# `copies` of itself there are enough tiles that they are not (or less).  CTAs of a cluster without a step; ragged
+# ends; a head dim of two halves; keys that only the last rows see.
 @pytest.mark.parametrize("mode", ["bf16", "fp4_rownorm", "fp8_rownorm"])
 @pytest.mark.parametrize("d,h,hk,sq,skv,causal,copies", [
     (128, 1, 1, 129, 129, False, 160),
@@ -38,6 +38,8 @@ def _grads(q, k, v, do, g, causal, mode, cu=None):
     (128, 4, 2, 700, 1300, False, 32),
     (256, 4, 1, 333, 333, True, 64),
     (256, 2, 2, 1, 140, True, 64),
+    (128, 1, 1, 1900, 1900, True, 40),      # split by eight: the last tiles have fewer steps than CTAs
+    (256, 1, 1, 880, 880, True, 40),
 ])
 def test_split_key_tiles_match_whole_ones(d, h, hk, sq, skv, causal, copies, mode):
     q, _ = seeded_bf16((1, h, sq, d), 21)
