@@ -862,9 +862,12 @@ int decode_launch(const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtens
   c.ntiles = p.ntiles; c.nctas = grid; c.maxseg = p.maxseg; c.total_tiles = p.total_tiles;
   c.extra_base = p.extra_base; c.n_extra = p.n_extra; c.hk = p.hk; c.g = p.g;
   c.out = out; c.lse = lse;
-  // a warp for every piece or two of a unit, at most eight
+  // Threads by the pieces of a unit: a warp for each up to four, eight warps where there is much to fetch.  A step in us
+  // with 64 / 128 / 256 threads: one piece 12.45 / 12.6 / 12.8 (Z1 S600), 14.5 / 14.8 / 14.9 (Z16 S1024); 2 to 8 pieces
+  // at 128 up to 0.8 less than at 64 (0.1 more at worst) and up to 0.5 less than at 256 (0.3 more at worst); 16 pieces
+  // 13.3 / 12.6 / 12.9, at D 256 15.3 / 14.0 / 13.75; 36 pieces 16.6 / 15.3 / 14.9; 64 pieces 17.0 / 14.9 / 14.2.
   const int64_t pieces = (p.balanced ? ((int64_t)p.ntiles * grid + p.total_tiles - 1) / p.total_tiles + 1 : p.nsplit) + p.n_extra;
-  const unsigned threads = pieces > 8 ? 256 : (pieces > 4 ? 128 : 64);
+  const unsigned threads = pieces * (D / 128) > 16 ? 256 : (pieces > 1 ? 128 : 64);
   return nvfp4::launch("nvfp4_decode(combine)", decode_combine_kernel<D, TQ>, dim3((unsigned)(zhk * p.g)), threads, 0, st, c);
 }
 
