@@ -423,7 +423,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll
         for (int k = 0; k < N / 32; ++k) {
           const int off = i * 128 + c + 32 * k, lim = lim0 - off;         // last visible of these 32 columns
-          if constexpr (kBias && !kVarlen) {       // (a compare and a select: 106.5 us where the bits take 108)
+          // With a bias a compare and a select per score are faster at D = 128 than the bits: Z2 H32 Sq1029 Skv2309 111.3
+          // us (113.3), causal Z1 H32 S4096 173.7 (176.1), Z2 H8 S3000 99.5 (101.1); equal at D = 256.
+          if constexpr (kBias && !kVarlen) {
 #pragma unroll
             for (int e = 0; e < 32; ++e) sv[32 * k + e] = (e <= lim) ? sv[32 * k + e] : -INFINITY;
           } else {
