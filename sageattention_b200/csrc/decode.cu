@@ -194,7 +194,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     mbar_fence_init();
   }
   __syncthreads();
-  griddep_start(p.late_wait != 0, warp != 0);
+  griddep_start(p.late_wait != 0);
   // The TMA producer (warp 0) and the scale loader (warp 2) need nothing but the barriers and the
   // stage buffers: they start streaming now, while the other warps allocate TMEM and clear the
   // operand buffers behind a barrier of their own.
