@@ -861,13 +861,14 @@ def run_profile_case(args):
         x, w = rn(1, 8192, 4096), rn(1024, 4096) * (4096 ** -0.5)
         w = w.to(torch.bfloat16)
         fn = lambda: nv.vproj_quant_nvfp4(x, w, None, 8, 128)
-    elif case in ("bwd", "bwd_fp4", "bwd_fp8"):   # Z1 H32 Hk8 S4096 D128 causal fwd+bwd: 0.48 TFLOP per step
-        q, k, v, do = rn(1, 32, 4096, 128), rn(1, 8, 4096, 128), rn(1, 8, 4096, 128), rn(1, 32, 4096, 128)
+    elif case in ("bwd", "bwd_fp4", "bwd_fp8", "bwd_fp4_d256"):   # Z1 H32 Hk8 S4096 D128 (H16 Hk4 D256) causal fwd+bwd: 0.48 TFLOP per step
+        d, h = (256, 16) if case == "bwd_fp4_d256" else (128, 32)
+        q, k, v, do = rn(1, h, 4096, d), rn(1, h // 4, 4096, d), rn(1, h // 4, 4096, d), rn(1, h, 4096, d)
         q.requires_grad_(True), k.requires_grad_(True), v.requires_grad_(True)
-        mode = {"bwd": "bf16", "bwd_fp4": "fp4_rownorm", "bwd_fp8": "fp8_rownorm"}[case]
+        mode = {"bwd": "bf16", "bwd_fp4": "fp4_rownorm", "bwd_fp8": "fp8_rownorm", "bwd_fp4_d256": "fp4_rownorm"}[case]
 
         def fn():
-            o = nv.nvfp4_flash_attn_func(q, k, v, 128 ** -0.5, causal=True, num_key_value_groups=4,
+            o = nv.nvfp4_flash_attn_func(q, k, v, d ** -0.5, causal=True, num_key_value_groups=4,
                                          backward_grad_dots=mode)
             o.backward(do)
             q.grad = k.grad = v.grad = None
@@ -898,7 +899,8 @@ def run_profile_case(args):
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--profile-case", default=None,
-                    choices=["fwd", "fwd_d256", "decode", "pack", "bwd", "bwd_fp4", "bwd_fp8", "hybrid", "vproj", "umma_peak"],
+                    choices=["fwd", "fwd_d256", "decode", "pack", "bwd", "bwd_fp4", "bwd_fp8", "bwd_fp4_d256", "hybrid", "vproj",
+                             "umma_peak"],
                     help="run one small kernel case --steps times (for ncu) and exit")
     ap.add_argument("--gpus", type=int, default=1)
     ap.add_argument("--steps", type=int, default=20)
