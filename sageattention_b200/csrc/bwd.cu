@@ -23,8 +23,8 @@
 // works on step t+1 while a team is still busy with step t.  (One team of eight warps that took every step:
 // S8192 H32 Hk8 1629 -> 1554 us for pre-pass, dK/dV and dQ.)
 // Where the key tiles are too few or too unequal to fill the chip, the steps of a tile are dealt to the
-// CTAs of a cluster and their accumulators added over distributed shared memory: S1024 H16 Hk4 101 -> 58
-// us, S3805 372 -> 265 us.  dQ does not depend on dK / dV and starts while their last CTAs run.
+// CTAs of a cluster and their accumulators added over distributed shared memory: S1024 H16 Hk4 101 -> 36 us
+// (cluster_split chooses the number).  dQ does not depend on dK / dV and starts while their last CTAs run.
 // Causal masking is bottom-right
 // aligned; packed varlen is block-diagonal, expressed as a per-row visible range.  Head dim 128,
 // or 256 as two 128-wide output halves per tile (both halves recompute S and dP).  Every barrier
