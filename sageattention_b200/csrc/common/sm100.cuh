@@ -118,6 +118,46 @@ __device__ __forceinline__ bool mbar_spin_wait(uint64_t* bar, uint32_t parity, v
   return true;
 }
 
+// Wait of a hand-over that goes on when the CTA has recorded an error, so that all warps keep to the same sequence
+// of work items (and of the barriers in them) until the last one: 16 times the budget of a data wait, which by then
+// has run out and let everything else drain.
+__device__ __forceinline__ void mbar_wait_item(uint64_t* bar, uint32_t parity, volatile int* err, int site) {
+#pragma unroll 1
+  for (uint32_t i = 0; !mbar_try_wait(bar, parity); ++i)
+    if (i >= (NVFP4_WAIT_SPINS << 4)) {
+      *err = KSTAT_WAIT_TIMEOUT | site;
+      return;
+    }
+}
+
+// ------------------------------------------------------------------ cluster launch control
+// A running CTA takes over the work of one that has not been launched yet: one thread asks (16 bytes arrive at
+// `resp`, counted by `bar`), then any thread reads the answer.  After an answer without a CTA nothing may be asked again.
+__device__ __forceinline__ void clc_request(void* resp, uint64_t* bar) {
+  mbar_expect_tx(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(resp)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// block index of the CTA taken over, or false where none was left
+__device__ __forceinline__ bool clc_answer(const void* resp, int& x, int& y, int& z) {
+  uint32_t got, bx = 0, by = 0, bz = 0;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
+      "ld.shared.b128 r, [%4];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, _}, r;\n\t}\n"
+      : "=r"(got), "+r"(bx), "+r"(by), "+r"(bz)
+      : "r"(smem_u32(resp))
+      : "memory");
+  x = (int)bx;
+  y = (int)by;
+  z = (int)bz;
+  return got != 0;
+}
+
 // barrier among a subset of warps (id 1..15, nthreads multiple of 32)
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
@@ -152,6 +192,23 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, uin
       "%4, %5}], [%2];" ::"r"(smem_u32(dst)),
       "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
+}
+
+__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* m) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
+}
+
+// Shared-memory box -> global memory, asynchronous in the issuing thread's bulk group.
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, const void* src, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(m)),
+               "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {      // all but the last N stores have read their shared memory
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
 
 // L2 prefetch of a tensor-map box (no shared memory, no barrier).

@@ -32,9 +32,10 @@ struct TmapKey {
   const void* base;
   uint64_t n0, n1, n2, s1, s2;
   uint32_t type, swizzle, promotion, b0, b1;
+  uint64_t n3 = 0, s3 = 0;             // n3 = 0: three dimensions
   bool operator==(const TmapKey& o) const {
     return base == o.base && n0 == o.n0 && n1 == o.n1 && n2 == o.n2 && s1 == o.s1 && s2 == o.s2 && type == o.type &&
-           swizzle == o.swizzle && promotion == o.promotion && b0 == o.b0 && b1 == o.b1;
+           swizzle == o.swizzle && promotion == o.promotion && b0 == o.b0 && b1 == o.b1 && n3 == o.n3 && s3 == o.s3;
   }
 };
 inline int encode_tmap(CUtensorMap* m, const TmapKey& k, const char* what) {
@@ -51,13 +52,13 @@ inline int encode_tmap(CUtensorMap* m, const TmapKey& k, const char* what) {
   }
   TensorMapEncodeTiledFn enc = tensor_map_encoder();
   if (!enc) return fail(-1, "%s: cuTensorMapEncodeTiled is unavailable", what);
-  if ((reinterpret_cast<uintptr_t>(k.base) & 15) || (k.s1 & 15) || (k.s2 & 15))
+  if ((reinterpret_cast<uintptr_t>(k.base) & 15) || (k.s1 & 15) || (k.s2 & 15) || (k.s3 & 15))
     return fail(-1, "%s: base and strides must be 16-byte aligned for TMA", what);
-  cuuint64_t dims[3] = {k.n0, k.n1, k.n2};
-  cuuint64_t strides[2] = {k.s1, k.s2};
-  cuuint32_t box[3] = {k.b0, k.b1, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(m, (CUtensorMapDataType)k.type, 3, const_cast<void*>(k.base), dims, strides, box, es,
+  cuuint64_t dims[4] = {k.n0, k.n1, k.n2, k.n3};
+  cuuint64_t strides[3] = {k.s1, k.s2, k.s3};
+  cuuint32_t box[4] = {k.b0, k.b1, 1, 1};
+  cuuint32_t es[4] = {1, 1, 1, 1};
+  CUresult r = enc(m, (CUtensorMapDataType)k.type, k.n3 ? 4 : 3, const_cast<void*>(k.base), dims, strides, box, es,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, (CUtensorMapSwizzle)k.swizzle, (CUtensorMapL2promotion)k.promotion,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(-1, "%s: cuTensorMapEncodeTiled failed with %d", what, (int)r);
@@ -90,6 +91,13 @@ inline int make_tmap_u8_3d_sw128(CUtensorMap* m, const void* base, uint64_t n0, 
                                  uint64_t s2, uint32_t b1, const char* what) {
   return encode_tmap(m, {base, n0, n1, n2, s1, s2, CU_TENSOR_MAP_DATA_TYPE_UINT8, CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, 128, b1}, what);
+}
+
+// The same over [n3][n2][n1][n0]
+inline int make_tmap_u8_4d_sw128(CUtensorMap* m, const void* base, uint64_t n0, uint64_t n1, uint64_t n2, uint64_t n3,
+                                 uint64_t s1, uint64_t s2, uint64_t s3, uint32_t b1, const char* what) {
+  return encode_tmap(m, {base, n0, n1, n2, s1, s2, CU_TENSOR_MAP_DATA_TYPE_UINT8, CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, 128, b1, n3, s3}, what);
 }
 
 // bf16 tensor [n2][n1][n0] with 128-byte swizzle, box [1][b1][64 elements]
