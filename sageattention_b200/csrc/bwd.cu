@@ -10,12 +10,13 @@
 //   bwd_dkdv_kernel  one CTA per 128-key tile of a (batch, kv-head) unit; walks 64-query steps of
 //                    every query head of the GQA group, so dK / dV are reduced over the group in
 //                    TMEM and written once.
-//   bwd_dq_kernel    one CTA per 128-query tile of a head; walks 64-key steps.
+//   bwd_dq_kernel    walks the 64-key steps of 128-query tiles of a head; at D = 128 a CTA takes over tiles of the grid
+//                    that have not been launched.
 // Every bf16 operand is read from the row-major [rows, 128] tensors by TMA into 128-byte-swizzled
 // tiles; the same tile serves as a K-major operand (contraction along D) and as an MN-major
 // operand (contraction along the rows), so no transposed copies exist anywhere.
 //
-// Pipeline of one CTA (640 threads): warp 0 TMA producer, warp 1 MMA issuer, warp 2 scale-atom /
+// Pipeline of a dK/dV CTA (640 threads; dQ's is described at its kernel): warp 0 TMA producer, warp 1 MMA issuer, warp 2 scale-atom /
 // row-statistics loader, warps 4-11 and 12-19 two softmax teams that alternate steps, two threads per
 // row.  S has two TMEM slots, dP one (a team pulls it into registers and hands the slot back at once);
 // P^T / dS^T are written back as bf16 pairs into the S slot they were computed from and enter the gradient
@@ -777,97 +778,160 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
 
 // ------------------------------------------------------------------------------------------
 // dQ
-// TMEM: dQ [0,128) | S slots [128,192) [192,256) | dP [256,320) | SFQ [320, 320+D/16) |
-//       two SFK slots of D/16 columns | dO, D/2 columns.  Head dim 256: blockIdx.z picks a 128-wide half of dQ.
-// dS (bf16 pairs, 32 columns) is written back into the S slot it came from and feeds the dQ GEMM
-// as a TMEM A operand.
+// TMEM: dQ [0,128) | S 64 | three dP slots of 64 (D = 256: two) | SFQ, D/16 columns an item | two SFK slots of D/16
+//       columns | dO, D/2 columns.  Head dim 256: blockIdx.z picks a 128-wide half of dQ.
+// dS (bf16 pairs, 32 columns) is written back into the dP slot it came from and feeds the dQ GEMM
+// as a TMEM A operand.  What bounded a step was the thread that issued its products: a wait that finds its phase complete
+// costs it 110 to 130 clocks, fourteen MMAs and their commits 400 more, 1160 of a step's 1280 clocks where the
+// products take 650.  So two threads issue, one S and dP and one the dQ GEMMs; the operands of a stage complete on one
+// barrier; and the one slot that both teams share is that of S, which a team reads first and hands back before anything else.
+// Whole backward (pre-pass, dK/dV, dQ), against one CTA per tile and one issuer: S3072 H32 Hk8 283 -> 239 us, S8192
+// 1525 -> 1398, eight samples in 16384 tokens 1038 -> 900, H16 Hk4 D256 S2048 246 -> 220.
+// An item is a query tile of a head.  At D = 128 a CTA that is through with one takes over another that has not been
+// launched (clusterlaunchcontrol): a CTA's start and end were 13000 clocks, of 640 a step.  Steps count through all
+// items; rings, parities and the turns of the teams run on, and the team that has no part in an item's last step is at
+// the next item while the other brings out dQ.  At D = 256 the second item's operands do not fit: a CTA has one.
+// dO lands in shared memory by TMA and goes from there to tensor memory (rows read by their threads from global
+// memory took 2300 clocks of an item's start); dQ leaves through a tile in shared memory as 64-byte row segments.
 // ------------------------------------------------------------------------------------------
 template <int D>
 struct DqSmem {
+  static constexpr bool kMany = D == 128;  // a CTA walks several items
+  static constexpr int NI = kMany ? 2 : 1; // items whose Q operands are held
+  static constexpr int NG = D == 128 ? 3 : 2;   // dP slots
   static constexpr int DS = D / 64, KSUB = D / 128, KB = D / 64;
   static constexpr int QP = KSUB * 8192;   // Q pack tile, 128 queries x D/2 B
   static constexpr int QSF = KB * 512;
+  static constexpr int LAND = DS * 16384;  // dO bf16 [128 queries x D] on its way to tensor memory
+  static constexpr int OUT = 8 * 2048;     // per warp of a team 32 rows x 64 bytes of dQ
   // per stage: V bf16 [64 keys x D] and the 128-wide half of K bf16 (8 KB sub-tiles), K pack
   // [64 keys x D/2 B], K scale atoms
   static constexpr int V = DS * 8192, K = 16384, KP = KSUB * 4096, KSF = KB * 512, AUX = 1024;
   static constexpr int O_V = 0, O_K = V, O_KP = V + K, O_KSF = O_KP + KP, O_AUX = O_KSF + KSF;   // AUX: key bias [64]
   static constexpr int STAGE = V + K + KP + KSF + AUX;
-  static constexpr int NSTAGE = D == 128 ? 5 : 2;
-  static constexpr int TOTAL = QP + NSTAGE * STAGE + QSF + 1024;
+  static constexpr int NSTAGE = D == 128 ? 4 : 2;
+  static constexpr int TOTAL = NI * (QP + QSF) + LAND + OUT + NSTAGE * STAGE + 1024;
   static_assert(STAGE % 1024 == 0 && QP % 1024 == 0, "128-byte-swizzled tiles need 1 KB alignment");
+  static_assert(NI * QSF % 512 == 0, "the output tiles are swizzled");
+};
+
+struct __align__(16) DqItem {   // one query tile of one head; steps count from the CTA's first one on
+  int r0, r1;                   // its 64-key steps [r0, r1); r1 = -1: no more items
+  int j0;                       // key step of running step 0 (may be negative)
+  int m0, zh, unit, zi, half;
 };
 
 template <int D, typename TG>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__ CUtensorMap tm_kp,
-              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_k, const BwdParams p) {
+              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_k,
+              const __grid_constant__ CUtensorMap tm_do, const BwdParams p) {
   using L = DqSmem<D>;
+  constexpr int NI = L::NI;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint8_t* s_qp = smem;
-  uint8_t* s_stage = s_qp + L::QP;
-  uint8_t* s_qsf = s_stage + L::NSTAGE * L::STAGE;
+  uint8_t* s_qp = smem;                          // NI items
+  uint8_t* s_land = s_qp + NI * L::QP;
+  uint8_t* s_stage = s_land + L::LAND;
+  uint8_t* s_qsf = s_stage + L::NSTAGE * L::STAGE;   // NI items
+  uint8_t* s_out = s_qsf + NI * L::QSF;
 
-  __shared__ uint64_t full_tma[L::NSTAGE], full_sf[L::NSTAGE], empty[L::NSTAGE];
-  __shared__ uint64_t q_full, qsf_full, a_full, s_full[2], dp_full, dp_free, ds_full[2], acc_done;
+  __shared__ uint64_t full[L::NSTAGE], empty[L::NSTAGE];      // empty: also, the dQ GEMM of the stage's step is complete
+  __shared__ uint64_t q_full[2], qsf_full[2], a_full[2], do_full, do_free;
+  __shared__ uint64_t s_full[2], s_free, ds_full[2], acc_done, dq_free;
+  __shared__ uint64_t item_full[2], item_free[2], clc_full;
+  __shared__ __align__(16) uint4 clc_resp;
+  __shared__ DqItem s_item[2];
+  __shared__ float4 s_rows[NI][128];             // -lse * log2e, -delta, visible keys [first, end) of a row
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int mblk = gridDim.y - 1 - blockIdx.y;   // late query tiles see the most keys: first
-  const int zh = blockIdx.x;
-  const int half = blockIdx.z;         // 128-wide slice of the head dim owned by this CTA
-  const int zi = zh / p.h, hi = zh % p.h;
-  const int unit = zi * p.hk + hi / p.g;
-  const int m0 = mblk * 128;
   const int shift = p.s_kv - p.s_q;
   const bool varlen = p.seq_start != nullptr;
-  if (tid == 0) {
-    err = 0;
-    for (int i = 0; i < L::NSTAGE; ++i) {
-      mbar_init(&full_tma[i], 1);
-      mbar_init(&full_sf[i], 1);
-      mbar_init(&empty[i], 1);
+  if (warp == 0) {
+    if (lane < L::NSTAGE) {
+      mbar_init(&full[lane], 2);             // TMA producer (and its bytes), scale loader
+      mbar_init(&empty[lane], 1);
     }
-    mbar_init(&q_full, 1);
-    mbar_init(&qsf_full, 1);
-    mbar_init(&a_full, 4);
-    mbar_init(&dp_full, 1);
-    mbar_init(&dp_free, 8);
-    mbar_init(&acc_done, 1);
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&s_full[b], 1);
-      mbar_init(&ds_full[b], 8);
+    if (lane < 2) {
+      mbar_init(&q_full[lane], 1);
+      mbar_init(&qsf_full[lane], 1);
+      mbar_init(&a_full[lane], 8);
+      mbar_init(&s_full[lane], 1);
+      mbar_init(&ds_full[lane], 8);
+      mbar_init(&item_full[lane], 1);
+      mbar_init(&item_free[lane], 19);
+    }
+    if (lane == 0) {
+      err = 0;
+      mbar_init(&do_full, 1);
+      mbar_init(&do_free, 8);
+      mbar_init(&s_free, 8);
+      mbar_init(&acc_done, 1);
+      mbar_init(&dq_free, 8);
+      mbar_init(&clc_full, 1);
     }
     mbar_fence_init();
+    if (lane == 0) tma_prefetch_map(&tm_qp);
+    if (lane == 1) tma_prefetch_map(&tm_kp);
+    if (lane == 2) tma_prefetch_map(&tm_v);
+    if (lane == 3) tma_prefetch_map(&tm_k);
+    if (lane == 4) tma_prefetch_map(&tm_do);
   }
   if (warp == 1) tmem_alloc(&tmem_base_s, 512);
+  // (warp 0) the query tile of the CTA with block index (bx, by, bz), as item `sl` whose steps count from r0
+  auto decode = [&](int bx, int by, int bz, int r0, int sl) {
+    const int m0 = ((int)gridDim.y - 1 - by) * 128;      // late query tiles see the most keys: first
+    const int zi = bx / p.h, hi = bx - zi * p.h;
+    int k_lo = 0, k_hi = p.s_kv;
+    if (p.causal) k_hi = max(0, min(p.s_kv, m0 + 128 + shift));
+    if (varlen) {
+      k_lo = p.seq_start[min(m0, p.s_q - 1)];
+      k_hi = min(k_hi, (int)p.seq_end[min(m0 + 127, p.s_q - 1)]);
+    }
+    const int j_lo = k_lo / 64;
+    if (lane == 0) s_item[sl] = DqItem{r0, r0 + max((k_hi + 63) / 64 - j_lo, 0), j_lo - r0, m0, bx, zi * p.hk + hi / p.g, zi, bz};
+    __syncwarp();
+  };
   griddep_start(p.late_wait != 0);
-  int k_lo = 0, k_hi = p.s_kv;
-  if (p.causal) k_hi = max(0, min(p.s_kv, m0 + 128 + shift));
-  if (varlen) {
-    k_lo = p.seq_start[min(m0, p.s_q - 1)];
-    k_hi = min(k_hi, (int)p.seq_end[min(m0 + 127, p.s_q - 1)]);
-  }
-  const int j_lo = k_lo / 64;
-  const int nstep = max((k_hi + 63) / 64 - j_lo, 0);
+  if (warp == 0) decode(blockIdx.x, blockIdx.y, blockIdx.z, 0, 0);
+  if (tid == 0) mbar_arrive(&item_full[0]);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   griddep_launch();
   const uint32_t tmem = tmem_base_s;
-  constexpr uint32_t T_DQ = 0, T_S = 128, T_DP = 256, T_SFQ = 320, T_SFK = T_SFQ + L::KB * 4;
-  constexpr uint32_t SFK_SLOT = L::KB * 4, T_DO = T_SFK + 2 * SFK_SLOT;      // dO: D / 2 columns
+  constexpr uint32_t SF = L::KB * 4;
+  constexpr uint32_t T_DQ = 0, T_S = 128, T_DP = 192, T_SFQ = T_DP + L::NG * 64, T_SFK = T_SFQ + NI * SF;
+  constexpr uint32_t T_DO = T_SFK + 2 * SF;
   static_assert(T_DO + D / 2 <= 512, "TMEM budget");
 
   if (warp == 0) {
-    if (elect_one() && nstep > 0) {
-      mbar_expect_tx(&q_full, L::QP);
+    // ------------------------------------------------------------------ items, TMA producer
+    const bool leader = elect_one();
+    uint32_t landed = 0;             // dO tiles loaded
+    for (int it = 0;; ++it) {
+      const int sl = it & 1, sb_i = sl % NI;
+      const int r0 = s_item[sl].r0, r1 = s_item[sl].r1, m0 = s_item[sl].m0, zh = s_item[sl].zh, unit = s_item[sl].unit;
+      const int half = s_item[sl].half, j0 = s_item[sl].j0;
+      if (leader) {
+        mbar_expect_tx(&q_full[sl], L::QP);
 #pragma unroll
-      for (int c = 0; c < L::KSUB; ++c) tma_load_3d(s_qp + c * 8192, &tm_qp, &q_full, c * 64, m0, zh);
-      auto prefetch = [&](int t) {
-        const int key0 = (j_lo + t) * 64;
+        for (int c = 0; c < L::KSUB; ++c) tma_load_3d(s_qp + sb_i * L::QP + c * 8192, &tm_qp, &q_full[sl], c * 64, m0, zh);
+      }
+      if (r1 > r0) {
+        if (landed > 0) mbar_wait(&do_free, (landed - 1) & 1, &err, 18);
+        ++landed;
+        if (leader) {
+          mbar_expect_tx(&do_full, L::LAND);
+#pragma unroll
+          for (int c = 0; c < L::DS; ++c) tma_load_3d(s_land + c * 16384, &tm_do, &do_full, c * 64, m0, zh);
+        }
+      }
+      auto prefetch = [&](int r) {
+        const int key0 = (j0 + r) * 64;
 #pragma unroll
         for (int c = 0; c < L::KSUB; ++c) tma_prefetch_3d(&tm_kp, c * 64, key0, unit);
 #pragma unroll
@@ -875,199 +939,331 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
         tma_prefetch_3d(&tm_k, half * 128, key0, unit);
         tma_prefetch_3d(&tm_k, half * 128 + 64, key0, unit);
       };
-      for (int t = L::NSTAGE; t < min(nstep, kBwdPrefetch); ++t) prefetch(t);
-      for (int st = 0; st < nstep; ++st) {
-        const int s = st % L::NSTAGE, key0 = (j_lo + st) * 64;
-        if (st + kBwdPrefetch < nstep) prefetch(st + kBwdPrefetch);
-        if (st >= L::NSTAGE) mbar_wait(&empty[s], ((st / L::NSTAGE) & 1) ^ 1, &err, 1);
-        uint8_t* sb = s_stage + s * L::STAGE;
-        mbar_expect_tx(&full_tma[s], L::KP + L::V + L::K);
+#pragma unroll 1
+      for (int r = r0; r < r1; ++r) {
+        const int s = r % L::NSTAGE, key0 = (j0 + r) * 64;
+        if (leader && r + kBwdPrefetch < r1) prefetch(r + kBwdPrefetch);
+        if (r >= L::NSTAGE) mbar_wait(&empty[s], ((r / L::NSTAGE) & 1) ^ 1, &err, 1);
+        if (leader) {
+          uint8_t* sb = s_stage + s * L::STAGE;
+          mbar_expect_tx(&full[s], L::KP + L::V + L::K);
 #pragma unroll
-        for (int c = 0; c < L::KSUB; ++c)
-          tma_load_3d(sb + L::O_KP + c * 4096, &tm_kp, &full_tma[s], c * 64, key0, unit);
+          for (int c = 0; c < L::KSUB; ++c)
+            tma_load_3d(sb + L::O_KP + c * 4096, &tm_kp, &full[s], c * 64, key0, unit);
 #pragma unroll
-        for (int c = 0; c < L::DS; ++c) tma_load_3d(sb + L::O_V + c * 8192, &tm_v, &full_tma[s], c * 64, key0, unit);
-        tma_load_3d(sb + L::O_K, &tm_k, &full_tma[s], half * 128, key0, unit);
-        tma_load_3d(sb + L::O_K + 8192, &tm_k, &full_tma[s], half * 128 + 64, key0, unit);
+          for (int c = 0; c < L::DS; ++c) tma_load_3d(sb + L::O_V + c * 8192, &tm_v, &full[s], c * 64, key0, unit);
+          tma_load_3d(sb + L::O_K, &tm_k, &full[s], half * 128, key0, unit);
+          tma_load_3d(sb + L::O_K + 8192, &tm_k, &full[s], half * 128 + 64, key0, unit);
+        }
       }
+      bool more = false;
+      int bx = 0, by = 0, bz = 0;
+      if (L::kMany) {
+        if (leader) clc_request(&clc_resp, &clc_full);      // late: the next item goes to who is through first
+        __syncwarp();
+        mbar_wait_item(&clc_full, it & 1, &err, 21);
+        more = clc_answer(&clc_resp, bx, by, bz);
+        fence_proxy_async_smem();       // read before the next answer may overwrite it
+        __syncwarp();
+      }
+      const int next = sl ^ 1;
+      if (it >= 1) mbar_wait_item(&item_free[next], (((it + 1) >> 1) & 1) ^ 1, &err, 20);
+      if (more) decode(bx, by, bz, r1, next);
+      else if (lane == 0) s_item[next].r1 = -1;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&item_full[next]);
+      if (!more) break;
     }
     __syncwarp();
   } else if (warp == 2) {
-    if (nstep > 0) {
+    // ------------------------------------------------------------------ scale atoms (+ key bias), row statistics, visible ranges
+    for (int it = 0;; ++it) {
+      const int sl = it & 1;
+      mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+      const int r0 = s_item[sl].r0, r1 = s_item[sl].r1;
+      if (r1 < 0) break;
+      const int m0 = s_item[sl].m0, zh = s_item[sl].zh, unit = s_item[sl].unit, zi = s_item[sl].zi, j0 = s_item[sl].j0;
       const uint8_t* qsrc = p.qsc + (int64_t)zh * p.s_q * (D / 16);
+      const uint32_t qsf = smem_u32(s_qsf + (sl % NI) * L::QSF);
 #pragma unroll
       for (int r4 = 0; r4 < 4; ++r4) {
         const int r = lane + 32 * r4;
         const bool ok = m0 + r < p.s_q;
         const uint8_t* g = qsrc + (int64_t)(ok ? m0 + r : 0) * (D / 16);
 #pragma unroll
-        for (int c = 0; c < L::KB; ++c)
-          cp_async_4(smem_u32(s_qsf) + c * 512 + sf_atom_offset(r, 0), g + 4 * c, ok ? 4u : 0u);
+        for (int c = 0; c < L::KB; ++c) cp_async_4(qsf + c * 512 + sf_atom_offset(r, 0), g + 4 * c, ok ? 4u : 0u);
       }
       cp_async_commit();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int row = m0 + lane + 32 * j;
+        float4 v = make_float4(0.0f, 0.0f, __int_as_float(0), __int_as_float(0));
+        if (row < p.s_q) {
+          int kl = 0, kh = p.causal ? min(p.s_kv, row + shift + 1) : p.s_kv;
+          if (varlen) {
+            kl = p.seq_start[row];
+            kh = min(kh, (int)p.seq_end[row]);
+          }
+          v = make_float4(-p.lse[(int64_t)zh * p.s_q + row] * kBwdLog2e, -p.delta[(int64_t)zh * p.s_q + row],
+                          __int_as_float(kl), __int_as_float(max(kh, kl)));
+        }
+        s_rows[sl % NI][lane + 32 * j] = v;
+      }
       cp_async_wait<0>();
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&qsf_full);
+      if (lane == 0) mbar_arrive(&qsf_full[sl]);
       const uint8_t* ksrc = p.ksc + (int64_t)unit * p.s_kv * (D / 16);
-      for (int st = 0; st < nstep; ++st) {
-        const int s = st % L::NSTAGE, key0 = (j_lo + st) * 64;
-        if (st >= L::NSTAGE) mbar_wait(&empty[s], ((st / L::NSTAGE) & 1) ^ 1, &err, 2);
+#pragma unroll 1
+      for (int r = r0; r < r1; ++r) {
+        const int s = r % L::NSTAGE, key0 = (j0 + r) * 64;
+        if (r >= L::NSTAGE) mbar_wait(&empty[s], ((r / L::NSTAGE) & 1) ^ 1, &err, 2);
         const uint32_t ksf = smem_u32(s_stage + s * L::STAGE + L::O_KSF);
 #pragma unroll
         for (int r2 = 0; r2 < 2; ++r2) {
-          const int r = lane + 32 * r2;
-          const int key = key0 + r;
+          const int rr = lane + 32 * r2;
+          const int key = key0 + rr;
           const bool ok = key < p.s_kv;
           const uint8_t* g = ksrc + (int64_t)(ok ? key : 0) * (D / 16);
 #pragma unroll
-          for (int c = 0; c < L::KB; ++c) cp_async_4(ksf + c * 512 + sf_atom_offset(r, 0), g + 4 * c, ok ? 4u : 0u);
+          for (int c = 0; c < L::KB; ++c) cp_async_4(ksf + c * 512 + sf_atom_offset(rr, 0), g + 4 * c, ok ? 4u : 0u);
           if (p.bias != nullptr)
-            cp_async_4(smem_u32(s_stage + s * L::STAGE + L::O_AUX) + r * 4,
+            cp_async_4(smem_u32(s_stage + s * L::STAGE + L::O_AUX) + rr * 4,
                        p.bias + (int64_t)zi * p.s_kv + (ok ? key : 0), ok ? 4u : 0u);
         }
         cp_async_commit();
         cp_async_wait<0>();
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&full_sf[s]);
+        if (lane == 0) mbar_arrive(&full[s]);
       }
+      if (lane == 0) mbar_arrive(&item_free[sl]);
     }
   } else if (warp == 1) {
-    if (elect_one() && nstep > 0) {
+    // ------------------------------------------------------------------ S and dP issuer
+    if (elect_one()) {
       const uint32_t id_s = make_idesc_nvfp4(128, 64);
       const uint32_t id_dp = make_idesc_bf16(128, 64, false);
-      const uint32_t id_acc = make_idesc_bf16(128, 128, true);
-      mbar_wait(&q_full, 0, &err, 3);
-      mbar_wait(&qsf_full, 0, &err, 4);
-      mbar_wait(&a_full, 0, &err, 15);
-      tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < L::KB; ++c) tmem_cp_32x128b_warpx4(tmem + T_SFQ + 4 * c, smem_u32(s_qsf + c * 512));
-      const uint64_t b_qp = desc_sw64(s_qp, 0);
-      const uint64_t b_v = desc_sw128(s_stage + L::O_V, 0), b_k_mn = desc_sw128_mn(s_stage + L::O_K, 0, 8192);
-      const uint64_t b_kp = desc_sw64(s_stage + L::O_KP, 0);
-      auto grad_gemm = [&](int t) {   // dQ += dS K of step t
-        const uint32_t a_ds = tmem + T_S + (t & 1) * 64;
-        const uint64_t x_k = b_k_mn + (uint64_t)((t % L::NSTAGE) * (L::STAGE >> 4));
-        const uint32_t acc0 = t > 0 ? 1u : 0u;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          umma_bf16_ta(tmem + T_DQ, a_ds + (k >> 1) * 32 + (k & 1) * 8, x_k + 128 * k, id_acc, k > 0 ? 1u : acc0);
-      };
-      for (int st = 0; st < nstep; ++st) {
-        const int s = st % L::NSTAGE, b = st & 1;
-        const uint32_t ph = (st / L::NSTAGE) & 1;
-        uint8_t* sb = s_stage + s * L::STAGE;
-        mbar_wait(&full_tma[s], ph, &err, 5);
-        mbar_wait(&full_sf[s], ph, &err, 6);
+      const uint64_t b_v = desc_sw128(s_stage + L::O_V, 0), b_kp = desc_sw64(s_stage + L::O_KP, 0);
+      int r = 0;
+      for (int it = 0;; ++it) {
+        const int sl = it & 1, si = sl % NI;
+        mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+        const int r1 = s_item[sl].r1;
+        if (r1 < 0) break;
+        mbar_wait(&q_full[sl], (it >> 1) & 1, &err, 3);
+        mbar_wait(&qsf_full[sl], (it >> 1) & 1, &err, 4);
+        if (r1 > r) mbar_wait(&a_full[sl], (it >> 1) & 1, &err, 15);
         tc_fence_after();
+        const uint64_t b_qp = desc_sw64(s_qp + si * L::QP, 0);
+        const uint32_t sfq = tmem + T_SFQ + si * SF;
 #pragma unroll
-        for (int c = 0; c < L::KB; ++c)
-          tmem_cp_32x128b_warpx4(tmem + T_SFK + b * SFK_SLOT + 4 * c, smem_u32(sb + L::O_KSF + c * 512));
-        const uint64_t so = (uint64_t)(s * (L::STAGE >> 4));
-        const uint64_t x_kp = b_kp + so, x_v = b_v + so;
-#pragma unroll
-        for (int k = 0; k < L::KB; ++k)
-          umma_nvfp4(tmem + T_S + b * 64, b_qp + (k >> 1) * 512 + (k & 1) * 2, x_kp + (k >> 1) * 256 + (k & 1) * 2,
-                     id_s, tmem + T_SFQ + k * 4, tmem + T_SFK + b * SFK_SLOT + k * 4, k > 0);
-        umma_commit(&s_full[b]);
-        if (st > 0) {
-          mbar_wait(&dp_free, (st - 1) & 1, &err, 7);
+        for (int c = 0; c < L::KB; ++c) tmem_cp_32x128b_warpx4(sfq + 4 * c, smem_u32(s_qsf + si * L::QSF + c * 512));
+#pragma unroll 1
+        for (; r < r1; ++r) {
+          const int s = r % L::NSTAGE, b = r & 1;
+          // the operands of the step; what its dP slot held, dS of step r - NG, has been consumed
+          if (r >= L::NG)
+            mbar_wait_all(&full[s], (r / L::NSTAGE) & 1, &empty[(r - L::NG) % L::NSTAGE], ((r - L::NG) / L::NSTAGE) & 1, &err, 5);
+          else
+            mbar_wait(&full[s], (r / L::NSTAGE) & 1, &err, 5);
           tc_fence_after();
-        }
+          const uint64_t so = (uint64_t)(s * (L::STAGE >> 4));
+          const uint64_t x_kp = b_kp + so, x_v = b_v + so;
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k)
-          umma_bf16_ta(tmem + T_DP, tmem + T_DO + k * 8, x_v + (k >> 2) * 512 + (k & 3) * 2, id_dp, k > 0);
-        umma_commit(&dp_full);
-        if (st > 0) {
-          mbar_wait(&ds_full[b ^ 1], ((st - 1) >> 1) & 1, &err, 8);
-          tc_fence_after();
-          grad_gemm(st - 1);
-          umma_commit(&empty[(st - 1) % L::NSTAGE]);
+          for (int k = 0; k < D / 16; ++k)
+            umma_bf16_ta(tmem + T_DP + (r % L::NG) * 64, tmem + T_DO + k * 8, x_v + (k >> 2) * 512 + (k & 3) * 2, id_dp, k > 0);
+          const uint32_t ksf = smem_u32(s_stage + L::O_KSF) + s * L::STAGE;
+#pragma unroll
+          for (int c = 0; c < L::KB; ++c) tmem_cp_32x128b_warpx4(tmem + T_SFK + b * SF + 4 * c, ksf + c * 512);
+          if (r > 0) {
+            mbar_wait(&s_free, (r - 1) & 1, &err, 7);
+            tc_fence_after();
+          }
+#pragma unroll
+          for (int k = 0; k < L::KB; ++k)
+            umma_nvfp4(tmem + T_S, b_qp + (k >> 1) * 512 + (k & 1) * 2, x_kp + (k >> 1) * 256 + (k & 1) * 2,
+                       id_s, sfq + k * 4, tmem + T_SFK + b * SF + k * 4, k > 0);
+          umma_commit(&s_full[b]);
         }
+        mbar_arrive(&item_free[sl]);
       }
-      mbar_wait(&ds_full[(nstep - 1) & 1], ((nstep - 1) >> 1) & 1, &err, 9);
-      tc_fence_after();
-      grad_gemm(nstep - 1);
-      umma_commit(&acc_done);
     }
     __syncwarp();
-  } else if (warp >= 4) {
+  } else if (warp == 3) {
+    // ------------------------------------------------------------------ dQ issuer
+    if (elect_one()) {
+      const uint32_t id_acc = make_idesc_bf16(128, 128, true);
+      const uint64_t b_k_mn = desc_sw128_mn(s_stage + L::O_K, 0, 8192);
+      int r = 0;
+      uint32_t n = 0;                     // items with steps so far
+      for (int it = 0;; ++it) {
+        const int sl = it & 1;
+        mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+        const int r1 = s_item[sl].r1;
+        if (r1 < 0) break;
+        const int first = r;
+#pragma unroll 1
+        for (; r < r1; ++r) {
+          // K of the stage landed before S and dP of the step were issued, but this thread has to observe it itself;
+          // it does so while dS is still being written
+          mbar_wait(&full[r % L::NSTAGE], (r / L::NSTAGE) & 1, &err, 6);
+          if (r == first && n > 0) mbar_wait(&dq_free, (n - 1) & 1, &err, 16);
+          mbar_wait(&ds_full[r & 1], (r >> 1) & 1, &err, 8);
+          tc_fence_after();
+          const uint32_t a_ds = tmem + T_DP + (r % L::NG) * 64;
+          const uint64_t x_k = b_k_mn + (uint64_t)((r % L::NSTAGE) * (L::STAGE >> 4));
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            umma_bf16_ta(tmem + T_DQ, a_ds + (k >> 1) * 32 + (k & 1) * 8, x_k + 128 * k, id_acc, (k > 0 || r > first) ? 1u : 0u);
+          umma_commit(&empty[r % L::NSTAGE]);
+        }
+        if (r1 > first) {
+          umma_commit(&acc_done);
+          ++n;
+        }
+        mbar_arrive(&item_free[sl]);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ softmax teams, end of an item
     const int team = (warp - 4) >> 3;   // steps of this parity
     const int grp = ((warp - 4) >> 2) & 1;
-    const int part = team * 2 + grp;    // 32-column slice of dQ this thread stores
     const int wq = warp & 3;
     const int row_in = wq * 32 + lane;
-    const int row = m0 + row_in;
     const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
     const float c2 = p.scaling * kBwdLog2e;
-    const bool row_ok = row < p.s_q;
-    if (part == 0) {
-      fill_a_tmem<D / 2>(tmem + lane_addr + T_DO, row_ok ? p.dout + ((int64_t)zh * p.s_q + row) * D : nullptr);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&a_full);
-    }
-    const float nl = row_ok ? -p.lse[(int64_t)zh * p.s_q + row] * kBwdLog2e : 0.0f;
-    const float nd = row_ok ? -p.delta[(int64_t)zh * p.s_q + row] : 0.0f;
-    // visible keys of this row: [kl, kh)
-    int kl = 0, kh = 0;
-    if (row_ok) {
-      kh = p.causal ? min(p.s_kv, row + shift + 1) : p.s_kv;
-      if (varlen) {
-        kl = p.seq_start[row];
-        kh = min(kh, (int)p.seq_end[row]);
-      }
-      kh = max(kh, kl);
-    }
-    // the teams alternate steps; thread g of a row owns keys [32g, 32g+32) of the 64-key tile
-    for (int st = team; st < nstep; st += 2) {
-      const int k2 = st >> 1;
-      const int key0 = (j_lo + st) * 64 + grp * 32;
-      const uint32_t slot = tmem + lane_addr + T_S + team * 64 + grp * 32;
-      const bool masked = !__all_sync(0xffffffffu, key0 >= kl && key0 + 32 <= kh);
-      const float* kbias = nullptr;
-      if (p.bias != nullptr) {      // the stage's key bias (landed with the scale atoms)
-        const int sg = st % L::NSTAGE;
-        mbar_wait(&full_sf[sg], (st / L::NSTAGE) & 1, &err, 10);
-        kbias = reinterpret_cast<const float*>(s_stage + sg * L::STAGE + L::O_AUX) + grp * 32;
-      }
-      mbar_wait(&s_full[team], k2 & 1, &err, 11);
-      mbar_wait(&dp_full, st & 1, &err, 13);
-      tc_fence_after();
-      uint32_t dr[32], sr[32];
-      tmem_ld32(tmem + lane_addr + T_DP + grp * 32, dr);
-      tmem_ld32(slot, sr);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&dp_free);
+    uint32_t n = 0;                     // items with steps so far
+    for (int it = 0;; ++it) {
+      const int sl = it & 1, si = sl % NI;
+      mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+      const int r0 = s_item[sl].r0, r1 = s_item[sl].r1;
+      if (r1 < 0) break;
+      if (team == (r0 & 1)) {           // the team of the first step: dO of the item to tensor memory, 2 threads a row
+        if (r1 > r0) {
+          mbar_wait(&do_full, n & 1, &err, 19);
+          if (r0 > 0) {                 // the last dP of the item before has read its dO
+            mbar_wait(&s_full[(r0 - 1) & 1], ((r0 - 1) >> 1) & 1, &err, 13);
+            tc_fence_after();
+          }
+#pragma unroll 1
+          for (int c = 0; c < L::DS / 2; ++c) {
+            const int sub = grp * (L::DS / 2) + c;
+            uint32_t w[32];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        float pf[16];
-        uint32_t w[8];
-        if (kbias != nullptr) prob_chunk<false, true>(sr + 16 * c, pf, c2, kbias + 16 * c, nl, masked, kl - key0 - 16 * c, kh - key0 - 16 * c);
-        else prob_chunk<false, false>(sr + 16 * c, pf, c2, nullptr, nl, masked, kl - key0 - 16 * c, kh - key0 - 16 * c);
-        ds_chunk<false>(pf, dr + 16 * c, w, nullptr, nd);
-        // dS of keys [32g, 32g+32) replaces the first 16 of the S columns this thread just read
-        tmem_st8(slot + 8 * c, w);
+            for (int e = 0; e < 8; ++e) {
+              const uint4 v = *reinterpret_cast<const uint4*>(s_land + sub * 16384 + sw128_offset(row_in, e * 16));
+              w[4 * e] = v.x; w[4 * e + 1] = v.y; w[4 * e + 2] = v.z; w[4 * e + 3] = v.w;
+            }
+            tmem_st32(tmem + lane_addr + T_DO + sub * 32, w);
+          }
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&do_free);
+        }
+        if (lane == 0) mbar_arrive(&a_full[sl]);
       }
-      tmem_st_wait();
-      tc_fence_before();
+      mbar_wait(&qsf_full[sl], (it >> 1) & 1, &err, 12);
+      const float4 st = s_rows[si][row_in];
+      const float nl = st.x, nd = st.y;
+      const int kl = __float_as_int(st.z), kh = __float_as_int(st.w);      // visible keys of this row: [kl, kh)
+      const int j0 = s_item[sl].j0;
+      // the teams alternate steps; thread g of a row owns keys [32g, 32g+32) of the 64-key tile
+#pragma unroll 1
+      for (int r = r0 + ((r0 ^ team) & 1); r < r1; r += 2) {
+        const int key0 = (j0 + r) * 64 + grp * 32;
+        const uint32_t slot = tmem + lane_addr + T_DP + (r % L::NG) * 64 + grp * 32;
+        const bool masked = !__all_sync(0xffffffffu, key0 >= kl && key0 + 32 <= kh);
+        const float* kbias = nullptr;
+        if (p.bias != nullptr) {      // the stage's key bias (landed with the scale atoms)
+          const int sg = r % L::NSTAGE;
+          mbar_wait(&full[sg], (r / L::NSTAGE) & 1, &err, 10);
+          kbias = reinterpret_cast<const float*>(s_stage + sg * L::STAGE + L::O_AUX) + grp * 32;
+        }
+        mbar_wait(&s_full[team], (r >> 1) & 1, &err, 11);
+        tc_fence_after();
+        uint32_t dr[32], sr[32];
+        tmem_ld32(tmem + lane_addr + T_S + grp * 32, sr);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_free);
+        tmem_ld32(slot, dr);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          float pf[16];
+          uint32_t w[8];
+          if (kbias != nullptr) prob_chunk<false, true>(sr + 16 * c, pf, c2, kbias + 16 * c, nl, masked, kl - key0 - 16 * c, kh - key0 - 16 * c);
+          else prob_chunk<false, false>(sr + 16 * c, pf, c2, nullptr, nl, masked, kl - key0 - 16 * c, kh - key0 - 16 * c);
+          if (c == 0) tmem_ld_wait();
+          ds_chunk<false>(pf, dr + 16 * c, w, nullptr, nd);
+          // dS of keys [32g, 32g+32) replaces the first 16 of the dP columns this thread just read
+          tmem_st8(slot + 8 * c, w);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ds_full[team]);
+      }
+      // ---- end of the item: the team of its last step brings out dQ, 64 columns a thread
+      if (team == (r1 > r0 ? (r1 - 1) & 1 : 0)) {
+        constexpr int PC = 64 / sizeof(TG);          // columns of a 64-byte row segment
+        const int m0 = s_item[sl].m0 + wq * 32;
+        TG* out = static_cast<TG*>(p.dq) + ((int64_t)s_item[sl].zh * p.s_q + m0) * D + s_item[sl].half * 128 + grp * 64;
+        if (r1 > r0) {
+          mbar_wait(&acc_done, n & 1, &err, 14);
+          tc_fence_after();
+        }
+        uint8_t* stg = s_out + (grp * 4 + wq) * 2048;
+#pragma unroll 1
+        for (int c = 0; c < 64; c += PC) {
+          uint4 seg[4];
+          if (r1 > r0) {
+            uint32_t w[16];
+            if constexpr (sizeof(TG) == 2) {
+              uint32_t o[32];
+              tmem_ld32(tmem + lane_addr + T_DQ + grp * 64 + c, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) {
+                const float2 v = __fmul2_rn(make_float2(__uint_as_float(o[2 * e]), __uint_as_float(o[2 * e + 1])),
+                                            make_float2(p.scaling, p.scaling));
+                w[e] = pack_16x2<TG>(v.x, v.y);
+              }
+            } else {
+              tmem_ld16(tmem + lane_addr + T_DQ + grp * 64 + c, w);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(__uint_as_float(w[e]) * p.scaling);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              *reinterpret_cast<uint4*>(stg + sw64_offset(lane, e * 16)) = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int e = 0; e < 4; ++e) seg[e] = *reinterpret_cast<const uint4*>(stg + sw64_offset(8 * e + (lane >> 2), (lane & 3) * 16));
+            __syncwarp();
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) seg[e] = make_uint4(0u, 0u, 0u, 0u);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int row = 8 * e + (lane >> 2);
+            if (m0 + row < p.s_q) *reinterpret_cast<uint4*>(out + (int64_t)row * D + c + (lane & 3) * (16 / sizeof(TG))) = seg[e];
+          }
+        }
+        if (r1 > r0) {                // dQ and the staging tile are free for the next item
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&dq_free);
+        }
+      }
+      if (r1 > r0) ++n;
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ds_full[team]);
-    }
-    TG* dqrow = static_cast<TG*>(p.dq) + ((int64_t)zh * p.s_q + row) * D + half * 128 + part * 32;
-    if (nstep > 0) {
-      mbar_wait(&acc_done, 0, &err, 14);
-      tc_fence_after();
-      uint32_t r[32];
-      tmem_ld32(tmem + lane_addr + T_DQ + part * 32, r);
-      tmem_ld_wait();
-      if (row_ok) store_row32<TG>(dqrow, r, p.scaling);
-      tc_fence_before();
-    } else if (row_ok) {
-      zero_row(dqrow, 32);
+      if (lane == 0) mbar_arrive(&item_free[sl]);
     }
   }
   tc_fence_before();
@@ -1192,7 +1388,7 @@ extern "C" int nvfp4_bwd_hp(const uint8_t* qnv, const uint8_t* qsc, const uint8_
                 "nvfp4_bwd_hp: grid too large");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t zh = z * h, zhk = z * hk;
-  CUtensorMap t_qp64, t_qp128, t_kp64, t_kp128, t_v64, t_v128, t_do64, t_q64, t_k64;
+  CUtensorMap t_qp64, t_qp128, t_kp64, t_kp128, t_v64, t_v128, t_do64, t_do128, t_q64, t_k64;
   int rc;
   const uint64_t pb = (uint64_t)d / 2, hb = (uint64_t)d * 2;   // bytes per pack row / bf16 row
   if ((rc = make_tmap_u8_3d_sw64(&t_qp64, qnv, pb, s_q, zh, pb, (uint64_t)s_q * pb, 64, "nvfp4_bwd_hp(Qp64)"))) return rc;
@@ -1202,6 +1398,7 @@ extern "C" int nvfp4_bwd_hp(const uint8_t* qnv, const uint8_t* qsc, const uint8_
   if ((rc = make_tmap_bf16_3d_sw128(&t_v64, v_bf16, d, s_kv, zhk, hb, (uint64_t)s_kv * hb, 64, "nvfp4_bwd_hp(V64)"))) return rc;
   if ((rc = make_tmap_bf16_3d_sw128(&t_v128, v_bf16, d, s_kv, zhk, hb, (uint64_t)s_kv * hb, 128, "nvfp4_bwd_hp(V128)"))) return rc;
   if ((rc = make_tmap_bf16_3d_sw128(&t_do64, do_bf16, d, s_q, zh, hb, (uint64_t)s_q * hb, 64, "nvfp4_bwd_hp(dO64)"))) return rc;
+  if ((rc = make_tmap_bf16_3d_sw128(&t_do128, do_bf16, d, s_q, zh, hb, (uint64_t)s_q * hb, 128, "nvfp4_bwd_hp(dO128)"))) return rc;
   if ((rc = make_tmap_bf16_3d_sw128(&t_q64, q_bf16, d, s_q, zh, hb, (uint64_t)s_q * hb, 64, "nvfp4_bwd_hp(Q64)"))) return rc;
   if ((rc = make_tmap_bf16_3d_sw128(&t_k64, k_bf16, d, s_kv, zhk, hb, (uint64_t)s_kv * hb, 64, "nvfp4_bwd_hp(K64)"))) return rc;
   BwdParams p;
@@ -1231,7 +1428,7 @@ extern "C" int nvfp4_bwd_hp(const uint8_t* qnv, const uint8_t* qsc, const uint8_
       return r1;
     p.late_wait = 1;
     dim3 g2((unsigned)zh, (unsigned)((s_q + 127) / 128), halves);
-    return nvfp4::launch("nvfp4_bwd_hp(dq)", kdq, g2, kBwdThreads, smem_dq, st, t_qp128, t_kp64, t_v64, t_k64, p);
+    return nvfp4::launch("nvfp4_bwd_hp(dq)", kdq, g2, kBwdThreads, smem_dq, st, t_qp128, t_kp64, t_v64, t_k64, t_do128, p);
   };
 #define NVFP4_BWD_LAUNCH(DD, TT) \
   launch(bwd_dkdv_kernel<DD, TT, false>, bwd_dkdv_kernel<DD, TT, true>, bwd_dq_kernel<DD, TT>, DkdvSmem<DD>::TOTAL, DqSmem<DD>::TOTAL)

@@ -23,6 +23,17 @@ template <> __device__ __forceinline__ float from_f32<float>(float v) { return v
 template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
 
+// two values rounded to a 16-bit type, `lo` in the low half
+template <typename T> __device__ __forceinline__ uint32_t pack_16x2(float lo, float hi);
+template <> __device__ __forceinline__ uint32_t pack_16x2<__nv_bfloat16>(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+template <> __device__ __forceinline__ uint32_t pack_16x2<__half>(float lo, float hi) {
+  const __half2 v = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
 // e4m3 byte of clamp(amax / 6, 2^-9, 448), round-to-nearest-even.
 __device__ __forceinline__ uint8_t scale_byte_from_amax(float amax) {
   float s = fminf(fmaxf(__fdiv_rn(amax, kF4Max), kScaleFloor), kScaleMax);
