@@ -403,13 +403,14 @@ __device__ __forceinline__ void ds_chunk(const float (&pf)[16], const uint32_t* 
 }
 // ------------------------------------------------------------------------------------------
 // dK / dV
-// TMEM: dV [0,128) | dK [128,256) | S^T slots [256,320) [320,384) | dP^T [384,448) |
+// TMEM: dV [0,128) | dK [128,256) | S^T [256,320) | two dP^T slots [320,384) [384,448) |
 //       SFK [448, 448+D/16) | two SFQ slots of D/16 columns
 // Head dim 256: the accumulators of a full tile would need all 512 columns, so blockIdx.z picks a
 // 128-wide half of dV / dK; S^T and dP^T still contract over the whole head dim.
-// A softmax group reads its S^T slot into registers and writes P^T and dS^T (bf16 pairs, 16
-// columns per 32 queries each) back into the same slot: the gradient GEMMs take them as TMEM A
-// operands.
+// A team reads S^T first and hands its slot back, forms P^T while dP^T is still on its way, and writes P^T and dS^T (bf16
+// pairs, 16 columns per 32 queries each) over the dP^T columns it has read: the gradient GEMMs take them as TMEM A
+// operands.  Two threads issue, one S^T and dP^T and one the gradient GEMMs: a single one paid its waits, twenty MMAs and
+// their commits one after the other, about as long as the ~1000 clocks that the products of a step take.
 // ------------------------------------------------------------------------------------------
 template <int D>
 struct DkdvSmem {
@@ -443,8 +444,8 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
   uint8_t* s_stage = s_kp + L::KP;
   uint8_t* s_ksf = s_stage + L::NSTAGE * L::STAGE;
 
-  __shared__ uint64_t full_tma[L::NSTAGE], full_aux[L::NSTAGE], empty[L::NSTAGE];
-  __shared__ uint64_t kv_full, ksf_full, a_full, s_full[2], dp_full, dp_free, pds_full[2], acc_done;
+  __shared__ uint64_t full[L::NSTAGE], empty[L::NSTAGE];      // empty: also, the gradient GEMMs of the step are complete
+  __shared__ uint64_t kv_full, ksf_full, a_full, s_full[2], s_free, dp_full[2], pds_full[2], acc_done;
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
 
@@ -461,18 +462,17 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
   if (tid == 0) {
     err = 0;
     for (int i = 0; i < L::NSTAGE; ++i) {
-      mbar_init(&full_tma[i], 1);
-      mbar_init(&full_aux[i], 1);
+      mbar_init(&full[i], 2);              // TMA producer (and its bytes), scale loader
       mbar_init(&empty[i], 1);
     }
     mbar_init(&kv_full, 1);
     mbar_init(&ksf_full, 1);
     mbar_init(&a_full, 4);
-    mbar_init(&dp_full, 1);
-    mbar_init(&dp_free, 8);
+    mbar_init(&s_free, 8);
     mbar_init(&acc_done, 1);
     for (int b = 0; b < 2; ++b) {
       mbar_init(&s_full[b], 1);
+      mbar_init(&dp_full[b], 1);
       mbar_init(&pds_full[b], 8);
     }
     mbar_fence_init();
@@ -495,7 +495,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
   tc_fence_after();
   griddep_launch();
   const uint32_t tmem = tmem_base_s;
-  constexpr uint32_t T_DV = 0, T_DK = 128, T_ST = 256, T_DPT = 384, T_SFK = 448, T_SFQ = T_SFK + L::KB * 4;
+  constexpr uint32_t T_DV = 0, T_DK = 128, T_ST = 256, T_DPT = 320, T_SFK = 448, T_SFQ = T_SFK + L::KB * 4;
   constexpr uint32_t SFQ_SLOT = L::KB * 4;
   constexpr int KT = D == 128 ? 4 : 0;              // K = 16 blocks of V held in tensor memory
   constexpr uint32_t T_V = T_SFQ + 2 * SFQ_SLOT;
@@ -532,15 +532,15 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
         }
         if (st >= L::NSTAGE) mbar_wait(&empty[s], ((st / L::NSTAGE) & 1) ^ 1, &err, 1);
         uint8_t* sb = s_stage + s * L::STAGE;
-        mbar_expect_tx(&full_tma[s], L::QP + L::DO + L::Q);
+        mbar_expect_tx(&full[s], L::QP + L::DO + L::Q);
 #pragma unroll
         for (int c = 0; c < L::KSUB; ++c)
-          tma_load_3d(sb + L::O_QP + c * 4096, &tm_qp, &full_tma[s], c * 64, i * 64, zh);
+          tma_load_3d(sb + L::O_QP + c * 4096, &tm_qp, &full[s], c * 64, i * 64, zh);
 #pragma unroll
         for (int c = 0; c < L::DS; ++c)
-          tma_load_3d(sb + L::O_DO + c * 8192, &tm_do, &full_tma[s], c * 64, i * 64, zh);
-        tma_load_3d(sb + L::O_Q, &tm_q, &full_tma[s], half * 128, i * 64, zh);
-        tma_load_3d(sb + L::O_Q + 8192, &tm_q, &full_tma[s], half * 128 + 64, i * 64, zh);
+          tma_load_3d(sb + L::O_DO + c * 8192, &tm_do, &full[s], c * 64, i * 64, zh);
+        tma_load_3d(sb + L::O_Q, &tm_q, &full[s], half * 128, i * 64, zh);
+        tma_load_3d(sb + L::O_Q + 8192, &tm_q, &full[s], half * 128 + 64, i * 64, zh);
       }
     }
     __syncwarp();
@@ -588,15 +588,14 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
         cp_async_wait<0>();
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&full_aux[s]);
+        if (lane == 0) mbar_arrive(&full[s]);
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------------ S^T and dP^T issuer
     if (elect_one() && nstep > 0) {
       const uint32_t id_s = make_idesc_nvfp4(128, 64);
       const uint32_t id_dp = make_idesc_bf16(128, 64, false);
-      const uint32_t id_acc = make_idesc_bf16(128, 128, true);
       mbar_wait(&kv_full, 0, &err, 3);
       mbar_wait(&ksf_full, 0, &err, 4);
       if (KT > 0) mbar_wait(&a_full, 0, &err, 15);
@@ -605,64 +604,67 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
       for (int c = 0; c < L::KB; ++c) tmem_cp_32x128b_warpx4(tmem + T_SFK + 4 * c, smem_u32(s_ksf + c * 512));
       // descriptors: constant fields once, then only the 16-byte-unit address field moves
       const uint64_t b_v = desc_sw128(s_v, 0), b_kp = desc_sw64(s_kp, 0);
-      const uint64_t b_do = desc_sw128(s_stage + L::O_DO, 0);
-      const uint64_t b_do_mn = desc_sw128_mn(s_stage + L::O_DO + half * 16384, 0, 8192);   // this half's two sub-tiles
-      const uint64_t b_q_mn = desc_sw128_mn(s_stage + L::O_Q, 0, 8192), b_qp = desc_sw64(s_stage + L::O_QP, 0);
-      // dV += P^T dO and dK += dS^T Q of step t (operands: slot t&1, stage t%NSTAGE)
-      auto grad_gemms = [&](int t) {
-        const uint64_t so = (uint64_t)((t % L::NSTAGE) * (L::STAGE >> 4));
-        // slot columns: [P^T q0-31 | dS^T q0-31 | P^T q32-63 | dS^T q32-63], 16 each
-        const uint32_t a_pt = tmem + T_ST + (t & 1) * 64, a_dst = a_pt + 16;
-        const uint64_t x_do = b_do_mn + so, x_q = b_q_mn + so;
-        const uint32_t acc0 = t > 0 ? 1u : 0u;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          umma_bf16_ta(tmem + T_DV, a_pt + (k >> 1) * 32 + (k & 1) * 8, x_do + 128 * k, id_acc, k > 0 ? 1u : acc0);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          umma_bf16_ta(tmem + T_DK, a_dst + (k >> 1) * 32 + (k & 1) * 8, x_q + 128 * k, id_acc, k > 0 ? 1u : acc0);
-      };
+      const uint64_t b_do = desc_sw128(s_stage + L::O_DO, 0), b_qp = desc_sw64(s_stage + L::O_QP, 0);
+#pragma unroll 1
       for (int st = 0; st < nstep; ++st) {
         const int s = st % L::NSTAGE, b = st & 1;
-        const uint32_t ph = (st / L::NSTAGE) & 1;
-        uint8_t* sb = s_stage + s * L::STAGE;
-        mbar_wait(&full_tma[s], ph, &err, 5);
-        mbar_wait(&full_aux[s], ph, &err, 6);
+        mbar_wait(&full[s], (st / L::NSTAGE) & 1, &err, 5);
         tc_fence_after();
-        // S^T slot b: its P^T / dS^T were consumed by the gradient GEMMs of step st-2, issued
-        // earlier on this in-order pipe
+        const uint32_t qsf = smem_u32(s_stage + L::O_QSF) + s * L::STAGE;
 #pragma unroll
-        for (int c = 0; c < L::KB; ++c)
-          tmem_cp_32x128b_warpx4(tmem + T_SFQ + b * SFQ_SLOT + 4 * c, smem_u32(sb + L::O_QSF + c * 512));
+        for (int c = 0; c < L::KB; ++c) tmem_cp_32x128b_warpx4(tmem + T_SFQ + b * SFQ_SLOT + 4 * c, qsf + c * 512);
         const uint64_t so = (uint64_t)(s * (L::STAGE >> 4));
         const uint64_t x_qp = b_qp + so, x_do = b_do + so;
+        if (st > 0) {
+          mbar_wait(&s_free, (st - 1) & 1, &err, 7);
+          tc_fence_after();
+        }
 #pragma unroll
         for (int k = 0; k < L::KB; ++k)
-          umma_nvfp4(tmem + T_ST + b * 64, b_kp + (k >> 1) * 512 + (k & 1) * 2, x_qp + (k >> 1) * 256 + (k & 1) * 2,
+          umma_nvfp4(tmem + T_ST, b_kp + (k >> 1) * 512 + (k & 1) * 2, x_qp + (k >> 1) * 256 + (k & 1) * 2,
                      id_s, tmem + T_SFK + k * 4, tmem + T_SFQ + b * SFQ_SLOT + k * 4, k > 0);
         umma_commit(&s_full[b]);
-        if (st > 0) {
-          mbar_wait(&dp_free, (st - 1) & 1, &err, 7);
+        if (st >= 2) {      // P^T and dS^T of step st - 2, in this dP^T slot, have been consumed
+          mbar_wait(&empty[(st - 2) % L::NSTAGE], ((st - 2) / L::NSTAGE) & 1, &err, 16);
           tc_fence_after();
         }
+        const uint32_t dpt = tmem + T_DPT + b * 64;
 #pragma unroll
         for (int k = 0; k < KT; ++k)
-          umma_bf16_ta(tmem + T_DPT, tmem + T_V + k * 8, x_do + (k >> 2) * 512 + (k & 3) * 2, id_dp, k > 0);
+          umma_bf16_ta(dpt, tmem + T_V + k * 8, x_do + (k >> 2) * 512 + (k & 3) * 2, id_dp, k > 0);
 #pragma unroll
         for (int k = KT; k < D / 16; ++k)
-          umma_bf16(tmem + T_DPT, b_v + (k >> 2) * 1024 + (k & 3) * 2, x_do + (k >> 2) * 512 + (k & 3) * 2, id_dp,
-                    k > 0);
-        umma_commit(&dp_full);
-        if (st > 0) {
-          mbar_wait(&pds_full[b ^ 1], ((st - 1) >> 1) & 1, &err, 8);
-          tc_fence_after();
-          grad_gemms(st - 1);
-          umma_commit(&empty[(st - 1) % L::NSTAGE]);
-        }
+          umma_bf16(dpt, b_v + (k >> 2) * 1024 + (k & 3) * 2, x_do + (k >> 2) * 512 + (k & 3) * 2, id_dp, k > 0);
+        umma_commit(&dp_full[b]);
       }
-      mbar_wait(&pds_full[(nstep - 1) & 1], ((nstep - 1) >> 1) & 1, &err, 9);
-      tc_fence_after();
-      grad_gemms(nstep - 1);
+    }
+    __syncwarp();
+  } else if (warp == 3) {
+    // ------------------------------------------------------------------ issuer of the gradient GEMMs
+    if (elect_one() && nstep > 0) {
+      const uint32_t id_acc = make_idesc_bf16(128, 128, true);
+      const uint64_t b_do_mn = desc_sw128_mn(s_stage + L::O_DO + half * 16384, 0, 8192);   // this half's two sub-tiles
+      const uint64_t b_q_mn = desc_sw128_mn(s_stage + L::O_Q, 0, 8192);
+#pragma unroll 1
+      for (int st = 0; st < nstep; ++st) {
+        const int s = st % L::NSTAGE, b = st & 1;
+        // dO and Q of the stage landed before S^T and dP^T of the step were issued, but this thread has to observe them
+        // itself; it does so while P^T and dS^T are still being written
+        mbar_wait(&full[s], (st / L::NSTAGE) & 1, &err, 6);
+        mbar_wait(&pds_full[b], (st >> 1) & 1, &err, 8);
+        tc_fence_after();
+        // dV += P^T dO and dK += dS^T Q; slot columns: [P^T q0-31 | dS^T q0-31 | P^T q32-63 | dS^T q32-63], 16 each
+        const uint64_t so = (uint64_t)(s * (L::STAGE >> 4));
+        const uint32_t a_pt = tmem + T_DPT + b * 64, a_dst = a_pt + 16;
+        const uint64_t x_do = b_do_mn + so, x_q = b_q_mn + so;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          umma_bf16_ta(tmem + T_DV, a_pt + (k >> 1) * 32 + (k & 1) * 8, x_do + 128 * k, id_acc, (k > 0 || st > 0) ? 1u : 0u);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          umma_bf16_ta(tmem + T_DK, a_dst + (k >> 1) * 32 + (k & 1) * 8, x_q + 128 * k, id_acc, (k > 0 || st > 0) ? 1u : 0u);
+        umma_commit(&empty[s]);
+      }
       umma_commit(&acc_done);
     }
     __syncwarp();
@@ -703,30 +705,33 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
       cur.next(n_i);
       cur.next(n_i);
       const float* aux = reinterpret_cast<const float*>(s_stage + s * L::STAGE + L::O_AUX) + grp * 32;
-      const uint32_t slot = tmem + lane_addr + T_ST + team * 64 + grp * 32;
+      const uint32_t slot = tmem + lane_addr + T_DPT + team * 64 + grp * 32;
       const bool masked = !__all_sync(0xffffffffu, q0 >= ql && q0 + 32 <= qh);
-      mbar_wait(&full_aux[s], (st / L::NSTAGE) & 1, &err, 10);
-      mbar_wait(&s_full[team], k2 & 1, &err, 11);
-      mbar_wait(&dp_full, st & 1, &err, 13);
+      // the row statistics have landed with the operands of the stage
+      mbar_wait_all(&full[s], (st / L::NSTAGE) & 1, &s_full[team], k2 & 1, &err, 10);
       tc_fence_after();
-      // dP^T first: the single dP^T slot goes back to the issuer before any arithmetic
-      uint32_t dr[32], sr[32];
-      tmem_ld32(tmem + lane_addr + T_DPT + grp * 32, dr);
-      tmem_ld32(slot, sr);
+      uint32_t sr[32], dr[32];
+      tmem_ld32(tmem + lane_addr + T_ST + grp * 32, sr);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&dp_free);
-      // P^T -> 16 columns, dS^T -> the next 16, over the S^T columns just read
+      if (lane == 0) mbar_arrive(&s_free);
+      float pf[2][16];
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        prob_chunk<true>(sr + 16 * c, pf[c], c2, aux + 16 * c, bk2, masked, ql - q0 - 16 * c, qh - q0 - 16 * c);
+      mbar_wait(&dp_full[team], k2 & 1, &err, 13);
+      tc_fence_after();
+      tmem_ld32(slot, dr);
+      tmem_ld_wait();
+      // P^T -> 16 columns, dS^T -> the next 16, over the dP^T columns just read
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        float pf[16];
         uint32_t w[8];
-        prob_chunk<true>(sr + 16 * c, pf, c2, aux + 16 * c, bk2, masked, ql - q0 - 16 * c, qh - q0 - 16 * c);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) w[e] = pack_bf16x2(pf[2 * e], pf[2 * e + 1]);
+        for (int e = 0; e < 8; ++e) w[e] = pack_bf16x2(pf[c][2 * e], pf[c][2 * e + 1]);
         tmem_st8(slot + 8 * c, w);
-        ds_chunk<true>(pf, dr + 16 * c, w, aux + 64 + 16 * c, 0.0f);
+        ds_chunk<true>(pf[c], dr + 16 * c, w, aux + 64 + 16 * c, 0.0f);
         tmem_st8(slot + 16 + 8 * c, w);
       }
       tmem_st_wait();
