@@ -759,7 +759,8 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
           for (int e = 0; e < 32; ++e) r[e] = 0u;
         }
         if (kSplit) red_store32(red, row, o * 128 + part * 32, r);
-        else if (key < p.s_kv) store_row32<TG>(o ? dkrow : dvrow, r, o ? p.scaling : 1.0f);
+        else store_rows32<TG>(smem + (warp - 4) * 4096, (o ? dkrow : dvrow) - (int64_t)lane * D, D, p.s_kv - key + lane, r,
+                              o ? p.scaling : 1.0f, lane);
       }
       tc_fence_before();
     } else if (key < p.s_kv) {

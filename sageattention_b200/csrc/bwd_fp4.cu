@@ -14,7 +14,7 @@
 //               group in turn (dV / dK are reduced over the group in TMEM and written once); one pass
 //               for both at D = 128, one each at D = 256;
 //   dQ pass     rows = queries of a head, columns = keys.
-// Per step the issuer thread queues S (or S^T) and dP as two N=64 block-scaled MMAs each; a
+// Per step one issuer thread queues S (or S^T) and dP as N=64 block-scaled MMAs, another the gradient GEMMs; a
 // softmax thread owns one row and 16-column chunks of the step's 64 columns, so the per-16 packs of
 // P and dS along the columns are thread-local: nibbles and scale bytes go to shared memory in the
 // operand layout and feed one MMA (M128, N = head dim, K64) per gradient and step.  FP4 MMAs replace
@@ -141,6 +141,7 @@ struct B4Params {
   int sr_p, sr_ds;       // stochastic rounding of the in-kernel P / dS packs (fp4_legacy mode)
   uint32_t seed;
   int* status;
+  int vec;                // scale tensors are aligned for one load a row
 };
 
 __device__ __forceinline__ float b4_max3(float a, float b, float c) {
@@ -228,8 +229,8 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   uint8_t* s_res = smem;
   uint8_t* s_stage = smem + C::RES;
 
-  __shared__ uint64_t full_tma[C::NSTAGE], full_aux[C::NSTAGE], empty[C::NSTAGE];
-  __shared__ uint64_t x_full, xsf_full, s_full[2], s_free[2], g_full, g_free, a_full[2], a_free[2], acc_done;
+  __shared__ uint64_t full[C::NSTAGE], empty[C::NSTAGE];
+  __shared__ uint64_t x_full, xsf_full, s_full[2], s_free[2], g_free, a_full[2], a_free[2], acc_done;
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
   __shared__ float gs_s;      // the power-of-two pre-scale of dO
@@ -241,13 +242,11 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   if (tid == 0) {
     err = 0;
     for (int i = 0; i < C::NSTAGE; ++i) {
-      mbar_init(&full_tma[i], 1);
-      mbar_init(&full_aux[i], 1);
+      mbar_init(&full[i], 2);              // TMA producer (and its bytes), scale loader
       mbar_init(&empty[i], 1);
     }
     mbar_init(&x_full, 1);
     mbar_init(&xsf_full, 1);
-    mbar_init(&g_full, 1);
     mbar_init(&g_free, 4 * C::NP);
     mbar_init(&acc_done, 1);
     for (int b = 0; b < 2; ++b) {
@@ -344,13 +343,13 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
         if (sg >= C::NSTAGE) mbar_wait(&empty[s], ((sg / C::NSTAGE) & 1) ^ 1, &err, 1);
         uint8_t* sb = s_stage + s * C::STAGE;
         const int tc = kFp8 ? col0 : col0 / 2;
-        mbar_expect_tx(&full_tma[s], (kDs ? 2 : 1) * C::X + ((kP ? 1 : 0) + (kDs ? 1 : 0)) * C::TB);
+        mbar_expect_tx(&full[s], (kDs ? 2 : 1) * C::X + ((kP ? 1 : 0) + (kDs ? 1 : 0)) * C::TB);
 #pragma unroll
         for (int c = 0; c < C::KSUB; ++c) {
-          tma_load_3d(sb + C::S_Y1 + c * 8192, &tm_y1, &full_tma[s], c * 64, col0, cb);
-          if constexpr (kDs) tma_load_3d(sb + C::S_Y2 + c * 8192, &tm_y2, &full_tma[s], c * 64, col0, cb);
-          if constexpr (kP) tma_load_3d(sb + C::S_T1 + c * C::AT, &tm_t1, &full_tma[s], tc, c * 128, cb);
-          if constexpr (kDs) tma_load_3d(sb + C::S_T2 + c * C::AT, &tm_t2, &full_tma[s], tc, c * 128, cb);
+          tma_load_3d(sb + C::S_Y1 + c * 8192, &tm_y1, &full[s], c * 64, col0, cb);
+          if constexpr (kDs) tma_load_3d(sb + C::S_Y2 + c * 8192, &tm_y2, &full[s], c * 64, col0, cb);
+          if constexpr (kP) tma_load_3d(sb + C::S_T1 + c * C::AT, &tm_t1, &full[s], tc, c * 128, cb);
+          if constexpr (kDs) tma_load_3d(sb + C::S_T2 + c * C::AT, &tm_t2, &full[s], tc, c * 128, cb);
         }
       }
     }
@@ -375,61 +374,121 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&xsf_full);
+      // The bytes of the next stage are fetched into registers while this one is in use: a stage that is handed back costs
+      // the warp its shared-memory stores, not a trip to L2.  It gets a load or store through in 60 to 80 clocks beside the
+      // softmax warps, so the packs' rows are taken with one load each where they are aligned (as allocated tensors are) and
+      // stored 8 and 16 bytes at a time: with a load and a store a word a stage came 1700 clocks late (D = 256 dK), with
+      // copies started when a stage is handed back 1850.  (The column rows loaded by the TMA warp instead: D = 256 1265 ->
+      // 1286 us, D = 128 1550 -> 1540.)
       const float inv_gs = 1.0f / gs;
+      constexpr int PQ = kFp8 ? 1 : 2;                 // words of a transposed row's scale bytes in a stage
       const int csc = p.c_pad / (kFp8 ? 32 : 16);      // scale bytes per row of a transposed pack
-      StepCursor cur(sg0, n_i);
-      for (int sg = 0; sg < nstage; ++sg, cur.next(n_i)) {
-        const int s = sg % C::NSTAGE;
+      uint32_t y1[4][C::KB], y2[4][kDs ? C::KB : 1], t1[C::NW][PQ][4], t2[C::NW][PQ][4];
+      float a0[4], a1[4];
+      const bool vec = p.vec != 0;
+      auto words = [&](const uint8_t* g, auto&... w) {        // 1, 2 or 4 consecutive words
+        uint32_t* o[] = {&w...};
+        constexpr int N = sizeof...(w);
+        if (N == 4 && vec) {
+          const uint4 v = __ldg(reinterpret_cast<const uint4*>(g));
+          *o[0] = v.x; *o[1 % N] = v.y; *o[2 % N] = v.z; *o[3 % N] = v.w;
+        } else if (N == 2 && vec) {
+          const uint2 v = __ldg(reinterpret_cast<const uint2*>(g));
+          *o[0] = v.x; *o[1 % N] = v.y;
+        } else {
+#pragma unroll
+          for (int k = 0; k < N; ++k) *o[k] = __ldg(reinterpret_cast<const uint32_t*>(g) + k);
+        }
+      };
+      auto row_words = [&](const uint8_t* g, uint32_t (&w)[C::KB]) {
+        if constexpr (C::KB == 4) words(g, w[0], w[1], w[2], w[3]);
+        else words(g, w[0], w[1]);
+      };
+      auto col_words = [&](const uint8_t* g, uint32_t (&w)[PQ][4], int r4) {
+        if constexpr (PQ == 2) words(g, w[0][r4], w[1][r4]);
+        else words(g, w[0][r4]);
+      };
+      auto fetch = [&](const StepCursor& c) {
         int cb, col0;
-        stage_cols(cur, cb, col0);
-        if (sg >= C::NSTAGE) mbar_wait(&empty[s], ((sg / C::NSTAGE) & 1) ^ 1, &err, 2);
-        uint8_t* sb = s_stage + s * C::STAGE;
-        const uint32_t ysf = smem_u32(sb + C::S_YSF), tsf1 = smem_u32(sb + C::S_TSF1), tsf2 = smem_u32(sb + C::S_TSF2);
-        float* aux = reinterpret_cast<float*>(sb + C::S_AUX);
+        stage_cols(c, cb, col0);
+        const int64_t y0 = ((int64_t)cb * Ccols + col0 + lane) * (D / 16);
+        const int64_t t0 = ((int64_t)cb * D + lane) * csc + col0 / (kFp8 ? 32 : 16);
 #pragma unroll
         for (int r4 = 0; r4 < 4; ++r4) {
-          const int r = lane + 32 * r4;            // column within the stage / row of a transposed tile
-          const int col = col0 + r;
+          const int col = col0 + lane + 32 * r4;   // column of the stage
           const bool ok = col < Ccols;
-          const int pp = r >> 6, rr = r & 63;
-          const int64_t gi = ((int64_t)cb * Ccols + (ok ? col : 0)) * (D / 16);
 #pragma unroll
-          for (int c = 0; c < C::KB; ++c) {
-            cp_async_4(ysf + (pp * C::KB + c) * 512 + sf_atom_offset(rr, 0), p.y1sc + gi + 4 * c, ok ? 4u : 0u);
-            if constexpr (kDs) cp_async_4(ysf + ((2 + pp) * C::KB + c) * 512 + sf_atom_offset(rr, 0), p.y2sc + gi + 4 * c, ok ? 4u : 0u);
+          for (int k = 0; k < C::KB; ++k) {
+            y1[r4][k] = 0u;
+            if constexpr (kDs) y2[r4][k] = 0u;
+          }
+          if (ok) {
+            row_words(p.y1sc + y0 + r4 * 2 * D, y1[r4]);
+            if constexpr (kDs) row_words(p.y2sc + y0 + r4 * 2 * D, y2[r4]);
           }
           // transposed packs: row = feature, 8 (MXFP8: 4) scale bytes = this stage's columns
 #pragma unroll
           for (int nw = 0; nw < C::NW; ++nw) {
-            const int64_t ti = ((int64_t)cb * D + nw * 128 + r) * csc + col0 / (kFp8 ? 32 : 16);
-#pragma unroll
-            for (int pq = 0; pq < (kFp8 ? 1 : 2); ++pq) {
-              if constexpr (kP) cp_async_4(tsf1 + (pq * C::NW + nw) * 512 + sf_atom_offset(r, 0), p.t1sc + ti + 4 * pq, 4u);
-              if constexpr (kDs) cp_async_4(tsf2 + (pq * C::NW + nw) * 512 + sf_atom_offset(r, 0), p.t2sc + ti + 4 * pq, 4u);
-            }
+            const int64_t ti = t0 + (int64_t)(nw * 128 + 32 * r4) * csc;
+            if constexpr (kP) col_words(p.t1sc + ti, t1[nw], r4);
+            if constexpr (kDs) col_words(p.t2sc + ti, t2[nw], r4);
           }
           if constexpr (kKeys) {
             // per query: -lse * log2e + 11 (exponent offset of P * 2^11) and -delta' * scaling / 4
             const int64_t qi = (int64_t)cb * p.s_q + (ok ? col : 0);
-            aux[r] = ok ? fmaf(-p.lse[qi], kB4Log2e, kB4PShift) : 0.0f;
-            if constexpr (kDs) aux[128 + r] = ok ? -p.delta[qi] * inv_gs * (p.scaling * 0.25f) : 0.0f;
+            a0[r4] = ok ? p.lse[qi] : 0.0f;
+            if constexpr (kDs) a1[r4] = ok ? p.delta[qi] : 0.0f;
           } else {
             // per key: the additive bias in base-2 units
-            aux[r] = (p.bias != nullptr && ok) ? p.bias[(int64_t)zi * p.s_kv + col] * kB4Log2e : 0.0f;
+            a0[r4] = (p.bias != nullptr && ok) ? p.bias[(int64_t)zi * p.s_kv + col] : 0.0f;
           }
         }
-        cp_async_commit();
-        cp_async_wait<0>();
+      };
+      StepCursor cur(sg0, n_i);
+      if (nstage > 0) fetch(cur);
+#pragma unroll 1
+      for (int sg = 0; sg < nstage; ++sg) {
+        const int s = sg % C::NSTAGE;
+        if (sg >= C::NSTAGE) mbar_wait(&empty[s], ((sg / C::NSTAGE) & 1) ^ 1, &err, 2);
+        uint8_t* sb = s_stage + s * C::STAGE;
+        float* aux = reinterpret_cast<float*>(sb + C::S_AUX);
+        const uint32_t at = smem_u32(sb) + lane * 16;      // rows lane, lane + 32, .. of an atom are neighbours
+#pragma unroll
+        for (int k = 0; k < C::KB; ++k)
+#pragma unroll
+          for (int pp = 0; pp < 2; ++pp) {
+            sts_v2(at + C::S_YSF + (pp * C::KB + k) * 512, y1[2 * pp][k], y1[2 * pp + 1][k]);
+            if constexpr (kDs) sts_v2(at + C::S_YSF + ((2 + pp) * C::KB + k) * 512, y2[2 * pp][k], y2[2 * pp + 1][k]);
+          }
+#pragma unroll
+        for (int nw = 0; nw < C::NW; ++nw)
+#pragma unroll
+          for (int pq = 0; pq < PQ; ++pq) {
+            if constexpr (kP) sts_v4(at + C::S_TSF1 + (pq * C::NW + nw) * 512, t1[nw][pq][0], t1[nw][pq][1], t1[nw][pq][2], t1[nw][pq][3]);
+            if constexpr (kDs) sts_v4(at + C::S_TSF2 + (pq * C::NW + nw) * 512, t2[nw][pq][0], t2[nw][pq][1], t2[nw][pq][2], t2[nw][pq][3]);
+          }
+#pragma unroll
+        for (int r4 = 0; r4 < 4; ++r4) {
+          const int r = lane + 32 * r4;
+          if constexpr (kKeys) {
+            const bool ok = (i_lo + cur.i) * 128 + r < Ccols;
+            aux[r] = ok ? fmaf(-a0[r4], kB4Log2e, kB4PShift) : 0.0f;
+            if constexpr (kDs) aux[128 + r] = -a1[r4] * inv_gs * (p.scaling * 0.25f);
+          } else {
+            aux[r] = a0[r4] * kB4Log2e;
+          }
+        }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&full_aux[s]);
+        if (lane == 0) mbar_arrive(&full[s]);
+        cur.next(n_i);
+        if (sg + 1 < nstage) fetch(cur);
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------------ S and dP issuer
     if (elect_one() && nstep > 0) {
       const uint32_t id_n64 = make_idesc_nvfp4(128, 64);
-      const uint32_t id_acc = make_idesc_nvfp4(128, D);
       mbar_wait(&x_full, 0, &err, 3);
       mbar_wait(&xsf_full, 0, &err, 4);
       tc_fence_after();
@@ -439,9 +498,48 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
         if constexpr (kDs) tmem_cp_32x128b_warpx4(tmem + C::T_SFX2 + 4 * c, smem_u32(s_res + C::O_XSF + (C::KB + c) * 512));
       }
       const uint64_t d_x1 = desc_sw64(s_res + C::O_X1, 0), d_x2 = desc_sw64(s_res + C::O_X2, 0);
+      const uint64_t d_y1 = desc_sw64(s_stage + C::S_Y1, 0), d_y2 = desc_sw64(s_stage + C::S_Y2, 0);
+#pragma unroll 1
+      for (int st = 0; st < nstep; ++st) {
+        const int pp = st & 1, sg = st >> 1, s = sg % C::NSTAGE;
+        uint8_t* sb = s_stage + s * C::STAGE;
+        if (pp == 0) mbar_wait(&full[s], (sg / C::NSTAGE) & 1, &err, 5);
+        // S slot: read by the team of step st - 2; the one dP slot: by that of step st - 1
+        if (kDs && st >= 2) mbar_wait_all(&s_free[pp], ((st >> 1) - 1) & 1, &g_free, (st - 1) & 1, &err, 7);
+        else if (kDs && st > 0) mbar_wait(&g_free, (st - 1) & 1, &err, 9);
+        else if (st >= 2) mbar_wait(&s_free[pp], ((st >> 1) - 1) & 1, &err, 7);
+        tc_fence_after();
+        const uint64_t so = (uint64_t)(s * (C::STAGE >> 4)) + (uint64_t)(pp * 256);   // 64 rows x 64 bytes further
+        // S (or S^T): rows x this step's 64 columns
+#pragma unroll
+        for (int c = 0; c < C::KB; ++c)
+          tmem_cp_32x128b_warpx4(tmem + C::T_SFY + 4 * c, smem_u32(sb + C::S_YSF + (pp * C::KB + c) * 512));
+#pragma unroll
+        for (int k = 0; k < C::KB; ++k)
+          umma_nvfp4(tmem + C::T_S + pp * 64, d_x1 + (k >> 1) * 512 + (k & 1) * 2, d_y1 + so + (k >> 1) * 512 + (k & 1) * 2,
+                     id_n64, tmem + C::T_SFX1 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
+        if constexpr (kDs) {
+          // dP (or dP^T)
+#pragma unroll
+          for (int c = 0; c < C::KB; ++c)
+            tmem_cp_32x128b_warpx4(tmem + C::T_SFY + 4 * c, smem_u32(sb + C::S_YSF + ((2 + pp) * C::KB + c) * 512));
+#pragma unroll
+          for (int k = 0; k < C::KB; ++k)
+            umma_nvfp4(tmem + C::T_G, d_x2 + (k >> 1) * 512 + (k & 1) * 2, d_y2 + so + (k >> 1) * 512 + (k & 1) * 2,
+                       id_n64, tmem + C::T_SFX2 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
+        }
+        umma_commit(&s_full[pp]);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 3) {
+    // ------------------------------------------------------------------ issuer of the gradient GEMMs
+    // A thread of its own: one thread for all products paid its waits and commits one after the other, about 1100
+    // clocks a step, and S and dP of the next step stood behind the wait for this one's operands.
+    if (elect_one() && nstep > 0) {
+      const uint32_t id_acc = make_idesc_nvfp4(128, D);
       const uint64_t d_a1 = kFp8 ? desc_sw128(s_res + C::O_A1, 0) : desc_sw64(s_res + C::O_A1, 0);
       const uint64_t d_a2 = kFp8 ? desc_sw128(s_res + C::O_A2, 0) : desc_sw64(s_res + C::O_A2, 0);
-      const uint64_t d_y1 = desc_sw64(s_stage + C::S_Y1, 0), d_y2 = desc_sw64(s_stage + C::S_Y2, 0);
       const uint64_t d_t1 = kFp8 ? desc_sw128(s_stage + C::S_T1, 0) : desc_sw64(s_stage + C::S_T1, 0);
       const uint64_t d_t2 = kFp8 ? desc_sw128(s_stage + C::S_T2, 0) : desc_sw64(s_stage + C::S_T2, 0);
       // acc += A T^T of step pp of stage s (columns [64 pp, 64 pp + 64)), one gradient
@@ -468,6 +566,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
       auto grad_gemms = [&](int t) {
         const int pp = t & 1, s = (t >> 1) % C::NSTAGE;
         uint8_t* sb = s_stage + s * C::STAGE;
+        if (pp == 0) mbar_wait(&full[s], ((t >> 1) / C::NSTAGE) & 1, &err, 6);   // the transposed tiles, seen by this thread
         mbar_wait(&a_full[pp], (t >> 1) & 1, &err, 8);
         tc_fence_after();
         const uint32_t acc = t > 0 ? 1u : 0u;
@@ -476,49 +575,8 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
         umma_commit(&a_free[pp]);
         if (pp == 1) umma_commit(&empty[s]);
       };
-      for (int st = 0; st < nstep; ++st) {
-        const int pp = st & 1, sg = st >> 1, s = sg % C::NSTAGE;
-        uint8_t* sb = s_stage + s * C::STAGE;
-        if (pp == 0) {
-          const uint32_t ph = (sg / C::NSTAGE) & 1;
-          mbar_wait(&full_tma[s], ph, &err, 5);
-          mbar_wait(&full_aux[s], ph, &err, 6);
-        }
-        if (st >= 2) mbar_wait(&s_free[pp], ((st >> 1) - 1) & 1, &err, 7);
-        tc_fence_after();
-        const uint64_t so = (uint64_t)(s * (C::STAGE >> 4)) + (uint64_t)(pp * 256);   // 64 rows x 64 bytes further
-        // S (or S^T): rows x this step's 64 columns
-#pragma unroll
-        for (int c = 0; c < C::KB; ++c)
-          tmem_cp_32x128b_warpx4(tmem + C::T_SFY + 4 * c, smem_u32(sb + C::S_YSF + (pp * C::KB + c) * 512));
-#pragma unroll
-        for (int k = 0; k < C::KB; ++k)
-          umma_nvfp4(tmem + C::T_S + pp * 64, d_x1 + (k >> 1) * 512 + (k & 1) * 2, d_y1 + so + (k >> 1) * 512 + (k & 1) * 2,
-                     id_n64, tmem + C::T_SFX1 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
-        umma_commit(&s_full[pp]);
-        if constexpr (kDs) {
-          if (st > 0) {
-            mbar_wait(&g_free, (st - 1) & 1, &err, 9);
-            tc_fence_after();
-          }
-          // dP (or dP^T)
-#pragma unroll
-          for (int c = 0; c < C::KB; ++c)
-            tmem_cp_32x128b_warpx4(tmem + C::T_SFY + 4 * c, smem_u32(sb + C::S_YSF + ((2 + pp) * C::KB + c) * 512));
-#pragma unroll
-          for (int k = 0; k < C::KB; ++k)
-            umma_nvfp4(tmem + C::T_G, d_x2 + (k >> 1) * 512 + (k & 1) * 2, d_y2 + so + (k >> 1) * 512 + (k & 1) * 2,
-                       id_n64, tmem + C::T_SFX2 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
-          umma_commit(&g_full);
-        }
-        // The gradient GEMMs trail by two steps: S and dP of step st are queued while the team that
-        // will consume them is still finishing step st - 2, so it finds them ready when it is done;
-        // waiting here for step st - 1 instead would put the whole MMA round trip between two steps
-        // of a team.
-        if (st > 1) grad_gemms(st - 2);
-      }
-      grad_gemms(nstep - 2);
-      grad_gemms(nstep - 1);
+#pragma unroll 1
+      for (int t = 0; t < nstep; ++t) grad_gemms(t);
       umma_commit(&acc_done);
     }
     __syncwarp();
@@ -580,9 +638,8 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
       const float* aux0 = reinterpret_cast<const float*>(s_stage + s * C::STAGE + C::S_AUX) + 64 * pp;
       const int cs0 = col0 + 64 * pp;                // first column of the step
       const bool masked = !__all_sync(0xffffffffu, cs0 >= lo && cs0 + 64 <= hi);
-      mbar_wait(&full_aux[s], (sg / C::NSTAGE) & 1, &err, 10);
-      mbar_wait(&s_full[pp], (st >> 1) & 1, &err, 11);
-      if constexpr (kDs) mbar_wait(&g_full, st & 1, &err, 12);
+      // the column statistics have landed with the operands of the stage
+      mbar_wait_all(&full[s], (sg / C::NSTAGE) & 1, &s_full[pp], (st >> 1) & 1, &err, 11);
       tc_fence_after();
       uint32_t wp[4], wd[4], scp = 0u, scd = 0u;
       float pkeep[kFp8 ? 16 : 1], dkeep[kFp8 ? 16 : 1];     // MXFP8: the even chunk of a 32-column group
@@ -730,7 +787,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
           for (int e = 0; e < 32; ++e) r[e] = 0u;
         }
         if (split) red_store32(smem_u32(smem), row_in, red_col + part * EC + c * 32, r);   // the operand tiles are idle by now
-        else if (row_ok) store_row32<TG>(o + c * 32, r, mul);
+        else store_rows32<TG>(smem + (warp - 4) * 4096, o + c * 32 - (int64_t)lane * D, D, R - row + lane, r, mul, lane);
       };
 #pragma unroll
       for (int c = 0; c < EC / 32; ++c) {
@@ -824,6 +881,7 @@ extern "C" int nvfp4_bwd_fp4(const uint8_t* qnv, const uint8_t* qsc, const uint8
   p.scaling = scaling; p.causal = (flags & NVFP4_FWD_CAUSAL) ? 1 : 0; p.status = status;
   p.seed = seed; p.sr_p = 0; p.sr_ds = 0;
   p.late_wait = 0; p.split = 1;
+  p.vec = (((uintptr_t)qsc | (uintptr_t)ksc | (uintptr_t)vdsc | (uintptr_t)dosc | (uintptr_t)dotsc | (uintptr_t)qtsc | (uintptr_t)ktsc) & 15) == 0;
   // The passes are independent of one another: the first waits for the work before it, the later ones
   // start filling the SMs that its last CTAs leave and wait for it only at their end.
   bool first = true;

@@ -82,28 +82,33 @@ __device__ __forceinline__ void load8(const T* src, float (&v)[8]) {
   for (int e = 0; e < 8; ++e) v[e] = to_f32<T>(src[e]);
 }
 
-// 32 fp32 accumulator columns -> 32 contiguous gradient elements
+// 32 rows (one a lane) x 32 accumulator columns of a warp -> gradient rows `stride` elements apart, of which the first
+// `rows` exist.  Through 32 x 64 (fp32: 128) bytes of shared memory, so that a store instruction covers whole 64- or
+// 128-byte row segments: 16 bytes of 32 different rows each time kept the store path of a D = 256 CTA busy for 7700 clocks.
 template <typename TG>
-__device__ __forceinline__ void store_row32(TG* dst, const uint32_t (&r)[32], float mul) {
+__device__ __forceinline__ void store_rows32(uint8_t* stg, TG* out, int64_t stride, int rows, const uint32_t (&r)[32], float mul,
+                                             int lane) {
+  constexpr int W = 8 * sizeof(TG);         // words of a row
+  constexpr int CH = W / 4;                 // 16-byte chunks of a row: lanes of a row when it is stored
+  auto at = [&](uint32_t row, uint32_t byte) { return stg + (CH == 4 ? sw64_offset(row, byte) : sw128_offset(row, byte)); };
+  uint32_t w[W];
   if constexpr (sizeof(TG) == 2) {
-    uint32_t w[16];
 #pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      const TG a0 = from_f32<TG>(__uint_as_float(r[2 * e]) * mul);
-      const TG a1 = from_f32<TG>(__uint_as_float(r[2 * e + 1]) * mul);
-      w[e] = (uint32_t)(*reinterpret_cast<const uint16_t*>(&a0)) |
-             ((uint32_t)(*reinterpret_cast<const uint16_t*>(&a1)) << 16);
-    }
-    uint4* d4 = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) d4[e] = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+    for (int e = 0; e < 16; ++e) w[e] = pack_16x2<TG>(__uint_as_float(r[2 * e]) * mul, __uint_as_float(r[2 * e + 1]) * mul);
   } else {
-    float4* d4 = reinterpret_cast<float4*>(dst);
 #pragma unroll
-    for (int e = 0; e < 8; ++e)
-      d4[e] = make_float4(__uint_as_float(r[4 * e]) * mul, __uint_as_float(r[4 * e + 1]) * mul,
-                          __uint_as_float(r[4 * e + 2]) * mul, __uint_as_float(r[4 * e + 3]) * mul);
+    for (int e = 0; e < 32; ++e) w[e] = __float_as_uint(__uint_as_float(r[e]) * mul);
   }
+#pragma unroll
+  for (int e = 0; e < CH; ++e) *reinterpret_cast<uint4*>(at(lane, e * 16)) = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int e = 0; e < CH; ++e) {
+    const int row = (32 / CH) * e + lane / CH, ch = lane % CH;
+    const uint4 v = *reinterpret_cast<const uint4*>(at(row, ch * 16));
+    if (row < rows) *reinterpret_cast<uint4*>(out + row * stride + ch * (16 / (int)sizeof(TG))) = v;
+  }
+  __syncwarp();
 }
 template <typename TG>
 __device__ __forceinline__ void zero_row(TG* dst, int n) {
