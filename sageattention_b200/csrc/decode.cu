@@ -122,7 +122,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   float* s_merge = reinterpret_cast<float*>(s_p);          // [16][D], only at the end of an item
   float* ssc = reinterpret_cast<float*>(s_p + (C::PBUF_BYTES > C::MERGE_BYTES ? C::PBUF_BYTES : C::MERGE_BYTES));
 
-  __shared__ uint64_t full_kv[C::NSTAGE], full_sf[C::NSTAGE], empty[C::NSTAGE];
+  __shared__ uint64_t full[C::NSTAGE], empty[C::NSTAGE];
   __shared__ uint64_t s_full[2], s_free[2], p_full[2], o_full[2], q_full[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
@@ -180,13 +180,12 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   if (tid == 0) {
     err = 0;
     for (int i = 0; i < C::NSTAGE; ++i) {
-      mbar_init(&full_kv[i], 1);
-      mbar_init(&full_sf[i], 1);
+      mbar_init(&full[i], 2);          // TMA producer (and its bytes), scale loader
       mbar_init(&empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
-      mbar_init(&s_free[i], 256);
+      mbar_init(&s_free[i], 8);
       mbar_init(&p_full[i], 8);
       mbar_init(&o_full[i], 1);
       mbar_init(&q_full[i], 1);
@@ -282,13 +281,13 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           const int s = it % C::NSTAGE;
           if (it >= (uint32_t)C::NSTAGE) mbar_spin_wait(&empty[s], ((it / C::NSTAGE) & 1) ^ 1, &err, 1);
           uint8_t* st = s_stage + s * C::STAGE_BYTES;
-          mbar_expect_tx(&full_kv[s], C::K_BYTES + C::V_BYTES);
+          mbar_expect_tx(&full[s], C::K_BYTES + C::V_BYTES);
 #pragma unroll
           for (int ks = 0; ks < C::KSUB; ++ks)
-            tma_load_3d(st + ks * 8192, &tm_k, &full_kv[s], ks * 64, t * 128, unit);
+            tma_load_3d(st + ks * 8192, &tm_k, &full[s], ks * 64, t * 128, unit);
 #pragma unroll
           for (int mt = 0; mt < C::MT; ++mt)
-            tma_load_3d(st + C::K_BYTES + mt * 8192, &tm_v, &full_kv[s], t * 64, mt * 128, unit);
+            tma_load_3d(st + C::K_BYTES + mt * 8192, &tm_v, &full[s], t * 64, mt * 128, unit);
         }
       }
     }
@@ -304,7 +303,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     auto publish = [&](uint32_t n) {
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&full_sf[n % C::NSTAGE]);
+      if (lane == 0) mbar_arrive(&full[n % C::NSTAGE]);
     };
     for (int wi = 0; wi < my_items; ++wi) {
       int unit, t0, t1;
@@ -386,8 +385,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           for (int j = 0; j < nt; ++j, ++it) {
             const int s = it % C::NSTAGE;
             const uint32_t ph = (it / C::NSTAGE) & 1;
-            mbar_spin_wait(&full_kv[s], ph, &err, 3);
-            mbar_spin_wait(&full_sf[s], ph, &err, 4);
+            mbar_spin_wait(&full[s], ph, &err, 3);
             tc_fence_after();
             uint8_t* st = s_stage + s * C::STAGE_BYTES;
             const uint32_t sfk = tmem + C::T_SFK + (b * C::STMAX + j) * C::KB * 4;
@@ -560,7 +558,8 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           }
         }
         tc_fence_before();
-        mbar_arrive(&s_free[b]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_free[b]);
         named_bar_sync(1, 256);
         // ---- pack role: thread = (tile ij, head ih, 16-key group ig) of the round; its sixteen
         // scores are thread-local from here on
