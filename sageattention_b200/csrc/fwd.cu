@@ -147,7 +147,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   uint8_t* s_qsf = s_psf + 2 * C::PSF_BYTES;                // two items
   uint8_t* s_out = s_qsf + 2 * C::QSF_BYTES;                // per warp of a group 32 rows x 128 bytes
 
-  __shared__ uint64_t full_kv[C::NSTAGE], full_sf[C::NSTAGE], empty[C::NSTAGE];
+  __shared__ uint64_t full[C::NSTAGE], empty[C::NSTAGE];
   __shared__ uint64_t s_full[2], s_free[2], p_full[2], pv_done[2], q_full[2], qsf_full[2], part_done[2], o_free;
   __shared__ uint64_t item_full[2], item_free[2], clc_full;
   __shared__ uint64_t mx_ready[kFwdMaxSlots][4];     // row maxima of a tile, one barrier per 32-row quadrant
@@ -168,8 +168,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   if (warp == 0) {
     mbar_init(&mx_ready[lane >> 2][lane & 3], 2);
     if (lane < C::NSTAGE) {
-      mbar_init(&full_kv[lane], 1);
-      mbar_init(&full_sf[lane], 1);
+      mbar_init(&full[lane], 2);        // TMA producer (and its bytes), scale loader
       mbar_init(&empty[lane], 1);
     }
     if (lane < 2) {
@@ -283,12 +282,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (r >= C::NSTAGE) mbar_wait(&empty[s], ((r / C::NSTAGE) & 1) ^ 1, &err, 1);
         if (leader) {
           uint8_t* st = s_stage + s * C::STAGE_BYTES;
-          mbar_expect_tx(&full_kv[s], C::K_BYTES + C::V_BYTES);
+          mbar_expect_tx(&full[s], C::K_BYTES + C::V_BYTES);
 #pragma unroll
-          for (int ks = 0; ks < C::KSUB; ++ks) tma_load_3d(st + ks * 8192, &tm_k, &full_kv[s], ks * 64, t * 128, unit);
+          for (int ks = 0; ks < C::KSUB; ++ks) tma_load_3d(st + ks * 8192, &tm_k, &full[s], ks * 64, t * 128, unit);
 #pragma unroll
           for (int nt = 0; nt < C::NT; ++nt)
-            tma_load_3d(st + C::K_BYTES + nt * 8192, &tm_v, &full_kv[s], t * 64, nt * 128, unit);
+            tma_load_3d(st + C::K_BYTES + nt * 8192, &tm_v, &full[s], t * 64, nt * 128, unit);
         }
       }
       // The next item is asked for when this one's loads are out, three or four tiles before its end: asked for at its
@@ -391,7 +390,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (r + 1 < r1) fetch(key0 + (r + 1 - r0) * 128);
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&full_sf[s]);
+        if (lane == 0) mbar_arrive(&full[s]);
       }
       if (lane == 0) mbar_arrive(&item_free[sl]);
     }
@@ -417,8 +416,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         for (; r < r1; ++r) {
           const int s = r % C::NSTAGE, b = r % C::NSBUF;
           const uint32_t ph = (r / C::NSTAGE) & 1;
-          mbar_wait(&full_kv[s], ph, &err, 5);
-          mbar_wait(&full_sf[s], ph, &err, 9);
+          mbar_wait(&full[s], ph, &err, 5);
           if (r >= C::NSBUF) {      // the S buffer's last tile has been read into registers
             const int u = r - C::NSBUF;
             mbar_spin_wait(&s_free[u & 1], (u >> 1) & 1, &err, 7);
@@ -463,8 +461,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           const int s = r % C::NSTAGE, b = r & 1;
           // the V tile and V scales of stage s landed before this tile's QK^T was issued, but this
           // thread has to observe them itself; it does so while P is still being written
-          mbar_wait(&full_kv[s], (r / C::NSTAGE) & 1, &err, 15);
-          mbar_wait(&full_sf[s], (r / C::NSTAGE) & 1, &err, 16);
+          mbar_wait(&full[s], (r / C::NSTAGE) & 1, &err, 15);
           tc_fence_after();
           uint8_t* st = s_stage + s * C::STAGE_BYTES;
           const uint32_t sfp = tmem + C::T_SFP + b * 8;
