@@ -375,44 +375,71 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
       __syncwarp();
       if (lane == 0) mbar_arrive(&xsf_full);
       // The bytes of the next stage are fetched into registers while this one is in use: a stage that is handed back costs
-      // the warp its shared-memory stores, not a trip to L2.  It gets a load or store through in 60 to 80 clocks beside the
-      // softmax warps, so the packs' rows are taken with one load each where they are aligned (as allocated tensors are) and
-      // stored 8 and 16 bytes at a time: with a load and a store a word a stage came 1700 clocks late (D = 256 dK), with
-      // copies started when a stage is handed back 1850.  (The column rows loaded by the TMA warp instead: D = 256 1265 ->
-      // 1286 us, D = 128 1550 -> 1540.)
+      // the warp its shared-memory stores, not a trip to L2.  Beside the softmax warps of its scheduler an instruction takes
+      // this warp 6 to 8 clocks, so the packs' rows are taken with one load each where they are aligned (as allocated tensors
+      // are) and stored 8 and 16 bytes at a time.  S8192 backward, D = 256 / D = 128: copies started when a stage is handed
+      // back 1500 / 1947 us (a stage up to 1850 clocks late), a load and a store a word 1305 / 1640, wide ones 1265 / 1547,
+      // with one address an operand 1231 / 1536 (column rows by the TMA warp instead: 1286 / 1540).
       const float inv_gs = 1.0f / gs;
       constexpr int PQ = kFp8 ? 1 : 2;                 // words of a transposed row's scale bytes in a stage
       const int csc = p.c_pad / (kFp8 ? 32 : 16);      // scale bytes per row of a transposed pack
       uint32_t y1[4][C::KB], y2[4][kDs ? C::KB : 1], t1[C::NW][PQ][4], t2[C::NW][PQ][4];
       float a0[4], a1[4];
       const bool vec = p.vec != 0;
-      auto words = [&](const uint8_t* g, auto&... w) {        // 1, 2 or 4 consecutive words
-        uint32_t* o[] = {&w...};
-        constexpr int N = sizeof...(w);
-        if (N == 4 && vec) {
+      auto row_vec = [](const uint8_t* g, uint32_t (&w)[C::KB]) {
+        if constexpr (C::KB == 4) {
           const uint4 v = __ldg(reinterpret_cast<const uint4*>(g));
-          *o[0] = v.x; *o[1 % N] = v.y; *o[2 % N] = v.z; *o[3 % N] = v.w;
-        } else if (N == 2 && vec) {
-          const uint2 v = __ldg(reinterpret_cast<const uint2*>(g));
-          *o[0] = v.x; *o[1 % N] = v.y;
+          w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
         } else {
-#pragma unroll
-          for (int k = 0; k < N; ++k) *o[k] = __ldg(reinterpret_cast<const uint32_t*>(g) + k);
+          const uint2 v = __ldg(reinterpret_cast<const uint2*>(g));
+          w[0] = v.x; w[1] = v.y;
         }
       };
-      auto row_words = [&](const uint8_t* g, uint32_t (&w)[C::KB]) {
-        if constexpr (C::KB == 4) words(g, w[0], w[1], w[2], w[3]);
-        else words(g, w[0], w[1]);
+      auto col_vec = [](const uint8_t* g, uint32_t (&w)[PQ][4], int r4) {
+        if constexpr (PQ == 2) {
+          const uint2 v = __ldg(reinterpret_cast<const uint2*>(g));
+          w[0][r4] = v.x; w[1][r4] = v.y;
+        } else {
+          w[0][r4] = __ldg(reinterpret_cast<const uint32_t*>(g));
+        }
       };
-      auto col_words = [&](const uint8_t* g, uint32_t (&w)[PQ][4], int r4) {
-        if constexpr (PQ == 2) words(g, w[0][r4], w[1][r4]);
-        else words(g, w[0][r4]);
-      };
+      auto word = [](const uint8_t* g) { return __ldg(reinterpret_cast<const uint32_t*>(g)); };
       auto fetch = [&](const StepCursor& c) {
         int cb, col0;
         stage_cols(c, cb, col0);
         const int64_t y0 = ((int64_t)cb * Ccols + col0 + lane) * (D / 16);
         const int64_t t0 = ((int64_t)cb * D + lane) * csc + col0 / (kFp8 ? 32 : 16);
+        if (vec && col0 + 128 <= Ccols) {
+          // a whole stage of aligned packs: one address an operand
+          const uint8_t *py1 = p.y1sc + y0, *py2 = kDs ? p.y2sc + y0 : nullptr;
+          const uint8_t *pt1 = kP ? p.t1sc + t0 : nullptr, *pt2 = kDs ? p.t2sc + t0 : nullptr;
+          const uint32_t step = 32u * (uint32_t)csc;
+#pragma unroll
+          for (int r4 = 0; r4 < 4; ++r4) {
+            row_vec(py1 + r4 * 2 * D, y1[r4]);
+            if constexpr (kDs) row_vec(py2 + r4 * 2 * D, y2[r4]);
+          }
+#pragma unroll
+          for (int nw = 0; nw < C::NW; ++nw)
+#pragma unroll
+            for (int r4 = 0; r4 < 4; ++r4) {
+              const uint32_t off = (uint32_t)(nw * 4 + r4) * step;
+              if constexpr (kP) col_vec(pt1 + off, t1[nw], r4);
+              if constexpr (kDs) col_vec(pt2 + off, t2[nw], r4);
+            }
+          if constexpr (kKeys) {
+            const float *pl = p.lse + (int64_t)cb * p.s_q + col0 + lane, *pd = p.delta + (int64_t)cb * p.s_q + col0 + lane;
+#pragma unroll
+            for (int r4 = 0; r4 < 4; ++r4) {
+              a0[r4] = pl[32 * r4];
+              if constexpr (kDs) a1[r4] = pd[32 * r4];
+            }
+          } else {
+#pragma unroll
+            for (int r4 = 0; r4 < 4; ++r4) a0[r4] = p.bias != nullptr ? p.bias[(int64_t)zi * p.s_kv + col0 + lane + 32 * r4] : 0.0f;
+          }
+          return;
+        }
 #pragma unroll
         for (int r4 = 0; r4 < 4; ++r4) {
           const int col = col0 + lane + 32 * r4;   // column of the stage
@@ -423,15 +450,21 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
             if constexpr (kDs) y2[r4][k] = 0u;
           }
           if (ok) {
-            row_words(p.y1sc + y0 + r4 * 2 * D, y1[r4]);
-            if constexpr (kDs) row_words(p.y2sc + y0 + r4 * 2 * D, y2[r4]);
+#pragma unroll
+            for (int k = 0; k < C::KB; ++k) {
+              y1[r4][k] = word(p.y1sc + y0 + r4 * 2 * D + 4 * k);
+              if constexpr (kDs) y2[r4][k] = word(p.y2sc + y0 + r4 * 2 * D + 4 * k);
+            }
           }
           // transposed packs: row = feature, 8 (MXFP8: 4) scale bytes = this stage's columns
 #pragma unroll
           for (int nw = 0; nw < C::NW; ++nw) {
             const int64_t ti = t0 + (int64_t)(nw * 128 + 32 * r4) * csc;
-            if constexpr (kP) col_words(p.t1sc + ti, t1[nw], r4);
-            if constexpr (kDs) col_words(p.t2sc + ti, t2[nw], r4);
+#pragma unroll
+            for (int pq = 0; pq < PQ; ++pq) {
+              if constexpr (kP) t1[nw][pq][r4] = word(p.t1sc + ti + 4 * pq);
+              if constexpr (kDs) t2[nw][pq][r4] = word(p.t2sc + ti + 4 * pq);
+            }
           }
           if constexpr (kKeys) {
             // per query: -lse * log2e + 11 (exponent offset of P * 2^11) and -delta' * scaling / 4
