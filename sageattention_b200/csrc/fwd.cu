@@ -33,12 +33,12 @@
 // maxima are the first to be exponentiated, without another read; reciprocal scales come from a table in
 // shared memory, not from the pipe that ex2 needs; P leaves in 16-byte stores.
 // Measured on a B200, kernel alone, causal bf16, against one CTA per query tile: Z4 H32 Hk8 S8192 D128 2033 -> 1695 us
-// (1.30 PFLOP/s), Z1 S4096 150 -> 119, S2048 51.6 -> 37.7, eight samples in 16384 tokens 403 -> 270; H16 Hk4 D256
-// S8192 334 -> 300, S2048 33.2 -> 28.6.
+// (1.30 PFLOP/s), Z1 S4096 150 -> 119, S2048 51.6 -> 37.7, eight samples in 16384 tokens 403 -> 269; H16 Hk4 D256
+// S8192 334 -> 297, S2048 33.2 -> 28.3.
 // Masks: only tiles at an edge of what a row may see -- diagonal, ragged end, ends of a packed sample -- and
 // tiles whose bias has a value other than zero (added already divided by the scaling) are edited, in tensor memory
 // before the maxima are taken, by bits of a 32-column word formed from the row's range; the loop over the others holds
-// no mask code.  Z2 H32 Sq1029 Skv2309 padded 111 -> 86 us.
+// no mask code; keys at the end that the bias hides have no tiles.  Z2 H32 Sq1029 Skv2309 padded 111 -> 78 us.
 // Registers decide here (96 per thread at twenty warps): variants that spilled even a few hundred
 // bytes took up to three times as long; O is rescaled 32 columns at a time (64: prefill Z4 S8192 1883 -> 2049 us).
 #include "common/abi.cuh"
@@ -247,15 +247,36 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       t_lo = __shfl_sync(0xffffffffu, beg[0], 0) / 128;
       i_first = (__shfl_sync(0xffffffffu, beg[3], 31) + 127) / 128 - t_lo;
     }
+    if (kBias) {
+      // Keys at the end that the bias hides from every row, as it does in a padded batch, have no tiles: 256 at a time from
+      // behind until one is visible.  Z2 H32 Sq1029 Skv2309, 11 and 22 % padded: 86.2 -> 78.0 us.
+      const float* b = p.bias + (int64_t)zi * p.s_kv;
+      int seen = 0;                       // visible key with the highest number, plus one
+      for (; hi_key > t_lo * 128; hi_key -= 256) {
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int key = hi_key - 1 - lane - 32 * j;
+          v[j] = key >= 0 ? __ldg(b + key) : -INFINITY;
+        }
+#pragma unroll
+        for (int j = 7; j >= 0; --j)
+          if (v[j] != -INFINITY) seen = hi_key - lane - 32 * j;
+        seen = __reduce_max_sync(0xffffffffu, seen);
+        if (seen > 0) break;
+      }
+      hi_key = seen;
+    }
     const int r1 = r0 + max((hi_key + 127) / 128 - t_lo, 0);
     if (lane == 0)
       s_item[sl] = FwdItem{r0, r1, r0 + i_first, r0 - t_lo + max(last_full, 0) / 128, zi, hi, m0,
                            t_lo - r0};
     __syncwarp();
   };
-  if (!kVarlen && warp == 0) decode(blockIdx.x, blockIdx.y, blockIdx.z, 0, 0);
+  constexpr bool kReads = kVarlen || kBias;         // an item's extent depends on memory: sample ids, bias
+  if (!kReads && warp == 0) decode(blockIdx.x, blockIdx.y, blockIdx.z, 0, 0);
   griddep_wait();
-  if (kVarlen && warp == 0) decode(blockIdx.x, blockIdx.y, blockIdx.z, 0, 0);      // reads the sample ids
+  if (kReads && warp == 0) decode(blockIdx.x, blockIdx.y, blockIdx.z, 0, 0);
   if (tid == 0) mbar_arrive(&item_full[0]);
   tc_fence_before();
   __syncthreads();

@@ -42,3 +42,31 @@ def test_dq_of_every_item_as_alone(dtype, z, h, hk, sq, skv, causal, cu, biased)
         for hi in sorted({0, 1, g, h // 2 + 1, h - 1}):
             one = [t[zi:zi + 1, j:j + 1].contiguous() for t, j in ((q, hi), (k, hi // g), (v, hi // g), (do, hi))]
             assert torch.equal(dq[zi, hi], _dq(*one, causal, cus, None if bias is None else bias[zi:zi + 1])[0, 0]), (zi, hi)
+
+
+@pytest.mark.parametrize("d", [128, 256])
+@pytest.mark.parametrize("mode", ["fp4_rownorm", "fp8_rownorm"])
+@pytest.mark.parametrize("shift", [4, 8])
+def test_scales_at_any_four_byte_address(d, mode, shift):
+    """Whole stages of 16-byte aligned scales are loaded a row at a time, others word by word: the same gradients."""
+    import sageattention_b200.nvfp4 as nv
+    z, h, hk, s = 1, 4, 2, 400
+    q, k, v, do = (seeded_bf16((z, n, s, d), 191 + i)[0] for i, n in enumerate((h, hk, hk, h)))
+
+    def grads(offset):
+        packs = []
+        for x in (q, k):
+            nib, sc = nv._quant_nvfp4(x.reshape(-1, s, d))
+            raw = sc.view(torch.uint8)
+            buf = torch.zeros(raw.numel() + 64, dtype=torch.uint8, device="cuda")
+            moved = buf[offset:offset + raw.numel()].view(raw.shape)
+            moved.copy_(raw)
+            packs.append((nib, moved.view(sc.dtype)))
+        t = [x.clone().requires_grad_(True) for x in (q, k, v)]
+        out = nv.nvfp4_flash_attn_func(*t, d ** -0.5, causal=True, num_key_value_groups=h // hk, backward_grad_dots=mode,
+                                       q_packs=packs[0], k_packs=packs[1])
+        assert packs[0][1].data_ptr() % 16 == offset
+        return torch.autograd.grad(out, t, do)
+
+    for a, b in zip(grads(0), grads(shift)):
+        assert torch.equal(a, b)

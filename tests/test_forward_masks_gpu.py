@@ -58,3 +58,27 @@ def test_packed_samples(d, causal, biased, lens):
         bias = np.zeros((1, s), np.float32)
         bias[0, 1::7] = -3.0
     _check(q, k, v, qf, kf, vf, h, hk, causal, bias=bias, cu=np.cumsum((0,) + lens))
+
+
+@pytest.mark.parametrize("d", [128, 256])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("visible", [0, 1, 127, 128, 129, 383, 384, 385, 443, 700])
+def test_hidden_keys_at_the_end(d, causal, visible):
+    """Tiles that the bias hides from every row are not walked, wherever the last visible key lies; one entry of the batch
+    has its own number of keys, in another only the last one is visible."""
+    z, h, hk, sq, skv = 3, 2, 1, 150, 700
+    q, qf = seeded_bf16((z, h, sq, d), 55)
+    k, kf = seeded_bf16((z, hk, skv, d), 56)
+    v, vf = seeded_bf16((z, hk, skv, d), 57)
+    bias = np.zeros((z, skv), np.float32)
+    bias[1, visible:] = -np.inf
+    bias[2, :skv - 1] = -np.inf
+    import sageattention_b200.nvfp4 as nv
+    from sageattention_b200 import _lib
+    out, lse = nv.nvfp4_flash_attention(q.float(), k.float(), v.float(), d ** -0.5, causal=causal, num_key_value_groups=h // hk,
+                                        key_pad_bias=torch.from_numpy(bias).cuda(), return_lse=True)
+    assert _lib.read_status("cuda") == 0
+    ref, ref_lse = O.attention_mode_b(qf, kf, vf, d ** -0.5, causal, h // hk, key_pad_bias=bias)
+    o = out.cpu().numpy()
+    assert np.isfinite(o).all() and np.abs(o - ref).max() <= MAXABS
+    assert np.abs(lse.cpu().numpy().reshape(ref_lse.shape) - ref_lse).max() <= 2e-3
