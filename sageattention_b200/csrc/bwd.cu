@@ -969,13 +969,12 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
       if (L::kMany) {
         if (leader) clc_request(&clc_resp, &clc_full);      // late: the next item goes to who is through first
         __syncwarp();
-        mbar_wait_item(&clc_full, it & 1, &err, 21);
-        more = clc_answer(&clc_resp, bx, by, bz);
+        more = mbar_wait_item_warp(&clc_full, it & 1, &err, 21) && clc_answer(&clc_resp, bx, by, bz);
         fence_proxy_async_smem();       // read before the next answer may overwrite it
         __syncwarp();
       }
       const int next = sl ^ 1;
-      if (it >= 1) mbar_wait_item(&item_free[next], (((it + 1) >> 1) & 1) ^ 1, &err, 20);
+      if (it >= 1) more = mbar_wait_item_warp(&item_free[next], (((it + 1) >> 1) & 1) ^ 1, &err, 20) && more;
       if (more) decode(bx, by, bz, r1, next);
       else if (lane == 0) s_item[next].r1 = -1;
       __syncwarp();
@@ -987,7 +986,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
     // ------------------------------------------------------------------ scale atoms (+ key bias), row statistics, visible ranges
     for (int it = 0;; ++it) {
       const int sl = it & 1;
-      mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+      if (!mbar_wait_item_warp(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
       const int r0 = s_item[sl].r0, r1 = s_item[sl].r1;
       if (r1 < 0) break;
       const int m0 = s_item[sl].m0, zh = s_item[sl].zh, unit = s_item[sl].unit, zi = s_item[sl].zi, j0 = s_item[sl].j0;
@@ -1056,7 +1055,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
       int r = 0;
       for (int it = 0;; ++it) {
         const int sl = it & 1, si = sl % NI;
-        mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+        if (!mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
         const int r1 = s_item[sl].r1;
         if (r1 < 0) break;
         mbar_wait(&q_full[sl], (it >> 1) & 1, &err, 3);
@@ -1107,7 +1106,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
       uint32_t n = 0;                     // items with steps so far
       for (int it = 0;; ++it) {
         const int sl = it & 1;
-        mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+        if (!mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
         const int r1 = s_item[sl].r1;
         if (r1 < 0) break;
         const int first = r;
@@ -1145,7 +1144,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
     uint32_t n = 0;                     // items with steps so far
     for (int it = 0;; ++it) {
       const int sl = it & 1, si = sl % NI;
-      mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+      if (!mbar_wait_item_warp(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
       const int r0 = s_item[sl].r0, r1 = s_item[sl].r1;
       if (r1 < 0) break;
       if (team == (r0 & 1)) {           // the team of the first step: dO of the item to tensor memory, 2 threads a row

@@ -1,10 +1,11 @@
 // Thin inline-PTX layer for sm_100a: mbarrier, TMA (cp.async.bulk.tensor), tcgen05
 // (TMEM allocation, block-scaled MMA, tcgen05.cp/ld/st, commit) and descriptor builders.
 //
-// Every wait in this file is BOUNDED: a wait that exceeds its iteration budget records a
-// status word and returns false instead of spinning forever, and once a CTA has recorded an
-// error all of its later waits return immediately, so a protocol bug ends the kernel in
-// milliseconds with a readable status instead of hanging the device.
+// Every wait in this file is BOUNDED: a wait that exceeds its budget records a status word and returns false instead of
+// spinning forever.  A wait for data has 2^20 probes that suspend for up to 2 us each (about two seconds), or 2^24
+// plain polls; once a CTA has recorded an error all of its later waits for data return at their first probe.  The
+// hand-over of work items goes on after an error and has four times that budget (mbar_wait_item).  So a protocol bug
+// ends a kernel within seconds, with a readable status, instead of hanging the device.
 #pragma once
 #include <cuda_runtime.h>
 #include <cuda.h>
@@ -136,16 +137,25 @@ __device__ __forceinline__ bool mbar_spin_wait(uint64_t* bar, uint32_t parity, v
   return true;
 }
 
-// Wait of a hand-over that goes on when the CTA has recorded an error, so that all warps keep to the same sequence
-// of work items (and of the barriers in them) until the last one: 16 times the budget of a data wait, which by then
-// has run out and let everything else drain.
-__device__ __forceinline__ void mbar_wait_item(uint64_t* bar, uint32_t parity, volatile int* err, int site) {
+// Wait of a hand-over of work items, by a whole warp or by one thread.  It goes on when the CTA has recorded an error, so
+// that all warps keep to the same sequence of items (and of the barriers in them) until the last one: by the time that
+// the budget, four times that of a data wait, runs out, an expired data wait has let everything else drain.  False when
+// it has run out: what was to be handed over is not there, and the caller leaves its loop over the items.
+__device__ __forceinline__ bool mbar_wait_item_n(uint64_t* bar, uint32_t parity, volatile int* err, int site, uint32_t spins) {
 #pragma unroll 1
   for (uint32_t i = 0; !mbar_try_wait(bar, parity); ++i)
-    if (i >= (NVFP4_WAIT_SPINS << 4)) {
-      *err = KSTAT_WAIT_TIMEOUT | site;
-      return;
+    if (i >= spins) {
+      if (*err == 0) *err = KSTAT_WAIT_TIMEOUT | site;      // the first expired wait is the one to look at
+      return false;
     }
+  return true;
+}
+__device__ __forceinline__ bool mbar_wait_item(uint64_t* bar, uint32_t parity, volatile int* err, int site) {
+  return mbar_wait_item_n(bar, parity, err, site, NVFP4_WAIT_SPINS << 2);
+}
+// the same by a whole warp, with one answer for all of its lanes
+__device__ __forceinline__ bool mbar_wait_item_warp(uint64_t* bar, uint32_t parity, volatile int* err, int site) {
+  return __all_sync(0xffffffffu, mbar_wait_item(bar, parity, err, site));
 }
 
 // ------------------------------------------------------------------ cluster launch control

@@ -315,13 +315,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       // start, the items of a grid of a wave or two would be dealt before it is known who is through first.
       if (leader) clc_request(&clc_resp, &clc_full);
       __syncwarp();
-      mbar_wait_item(&clc_full, it & 1, &err, 21);
       int bx, by, bz;
-      const bool more = clc_answer(&clc_resp, bx, by, bz);
+      bool more = mbar_wait_item_warp(&clc_full, it & 1, &err, 21) && clc_answer(&clc_resp, bx, by, bz);
       fence_proxy_async_smem();         // read before the next answer may overwrite it
       __syncwarp();
       const int next = sl ^ 1;
-      if (it >= 1) mbar_wait_item(&item_free[next], (((it + 1) >> 1) & 1) ^ 1, &err, 20);
+      if (it >= 1) more = mbar_wait_item_warp(&item_free[next], (((it + 1) >> 1) & 1) ^ 1, &err, 20) && more;
       if (more) decode(bx, by, bz, r1, next);
       else if (lane == 0) s_item[next].r1 = -1;
       __syncwarp();
@@ -337,7 +336,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     const float inv_scaling = kBias ? 1.0f / p.scaling : 0.0f;      // the bias is added to the unscaled scores
     for (int it = 0;; ++it) {
       const int sl = it & 1;
-      mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+      if (!mbar_wait_item_warp(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
       const int r0 = s_item[sl].r0, r1 = s_item[sl].r1;
       if (r1 < 0) break;
       const int zi = s_item[sl].zi, hi = s_item[sl].hi, m0 = s_item[sl].m0;
@@ -422,7 +421,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       int r = 0;
       for (int it = 0;; ++it) {
         const int sl = it & 1;
-        mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+        if (!mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
         const int r1 = s_item[sl].r1;
         if (r1 < 0) break;
         mbar_wait(&q_full[sl], (it >> 1) & 1, &err, 3);
@@ -469,7 +468,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       uint32_t o_phase = 0u;
       for (int it = 0;; ++it) {
         const int sl = it & 1;
-        mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+        if (!mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
         const int r1 = s_item[sl].r1;
         if (r1 < 0) break;
         if (r1 > r && r > 0) {          // O of the last item that had tiles has been read
@@ -573,7 +572,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 
     for (int it = 0;; ++it) {
       const int sl = it & 1;
-      mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22);
+      if (!mbar_wait_item_warp(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
       const int r0 = s_item[sl].r0, r1 = s_item[sl].r1;
       if (r1 < 0) break;
       // Tiles below r_first and from r_mask on need a test per score: the edge of a sample, the causal

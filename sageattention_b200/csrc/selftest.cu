@@ -2,11 +2,11 @@
 //
 // The production kernels never spin forever: a wait on an mbarrier gives up after a probe budget,
 // records KSTAT_WAIT_TIMEOUT | site in a CTA-shared word, every other role of the CTA then leaves
-// its loops, and thread 0 publishes the word through the `status` pointer.  This file runs exactly
-// that sequence on a barrier nobody ever completes -- no TMA copy, MMA or other asynchronous work
-// is in flight, nothing traps, and the kernel returns by itself within microseconds -- so a host
-// test can check that an expired wait really shows up in the status word and that the context stays
-// usable afterwards.
+// its loops (a hand-over of work items last, when its own larger budget has run out), and thread 0
+// publishes the word through the `status` pointer.  This file runs exactly that sequence on a barrier
+// nobody ever completes -- no TMA copy, MMA or other asynchronous work is in flight, nothing traps, and
+// the kernel returns by itself within milliseconds -- so a host test can check that an expired wait
+// really shows up in the status word and that the context stays usable afterwards.
 #include "common/abi.cuh"
 #include "common/sm100.cuh"
 
@@ -14,10 +14,11 @@ namespace nvfp4 {
 
 __global__ void __launch_bounds__(128) selftest_wait_kernel(int site, uint32_t spins, int* status) {
   __shared__ uint64_t never;     // initialised for one arrival that no thread performs
-  __shared__ int err;
+  __shared__ int err, item;      // item: what the hand-over came to
   const int tid = threadIdx.x;
   if (tid == 0) {
     err = 0;
+    item = 0;
     mbar_init(&never, 1);
     mbar_fence_init();
   }
@@ -29,8 +30,14 @@ __global__ void __launch_bounds__(128) selftest_wait_kernel(int site, uint32_t s
     // a second role waiting on the same barrier with a far larger budget: it must leave early
     // because the first one raised the CTA's error word
     mbar_wait_n(&never, 0, &err, site + 1, spins << 12);
+  } else if (tid >= 96) {
+    // a hand-over: goes on after the error, gives up when its own budget has run out and says so, and leaves the
+    // first site in the error word
+    const bool got = mbar_wait_item_n(&never, 0, &err, site + 2, spins << 2);
+    if (tid == 96) item = !got && err == (KSTAT_WAIT_TIMEOUT | site) ? 1 : 2;
   }
   __syncthreads();
+  if (tid == 0 && item != 1) err = KSTAT_WAIT_TIMEOUT | 0xFF;
   if (tid == 0 && err != 0 && status != nullptr) atomicExch(status, err);
 }
 
