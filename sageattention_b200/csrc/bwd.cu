@@ -780,7 +780,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && err != 0 && p.status != nullptr) atomicExch(p.status, err);
+  report_error(&err, p.status);
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
@@ -1275,7 +1275,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && err != 0 && p.status != nullptr) atomicExch(p.status, err);
+  report_error(&err, p.status);
   if (warp == 1) tmem_dealloc(tmem, 512);
   if (p.late_wait) griddep_wait();
 }

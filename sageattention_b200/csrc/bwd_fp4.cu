@@ -845,7 +845,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && err != 0 && p.status != nullptr) atomicExch(p.status, err);
+  report_error(&err, p.status);
   if (warp == 1) tmem_dealloc(tmem, 512);
   if (p.late_wait) griddep_wait();
 }

@@ -158,6 +158,17 @@ __device__ __forceinline__ bool mbar_wait_item_warp(uint64_t* bar, uint32_t pari
   return __all_sync(0xffffffffu, mbar_wait_item(bar, parity, err, site));
 }
 
+// End of a kernel, by all of its threads behind the last barrier and before tensor memory is given back.  Where a wait has
+// expired nothing has waited for the copies and products still under way: they get a millisecond (they take
+// microseconds) before the CTA's memory is another's, and the site of the wait goes to the status word.
+__device__ __forceinline__ void report_error(volatile int* err, int* status) {
+  const int e = *err;
+  if (e == 0) return;
+#pragma unroll 1
+  for (int i = 0; i < 1024; ++i) __nanosleep(1000);
+  if (threadIdx.x == 0 && status != nullptr) atomicExch(status, e);
+}
+
 // ------------------------------------------------------------------ cluster launch control
 // A running CTA takes over the work of one that has not been launched yet: one thread asks (16 bytes arrive at
 // `resp`, counted by `bar`), then any thread reads the answer.  After an answer without a CTA nothing may be asked again.

@@ -717,7 +717,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   if (p.late_wait) griddep_wait();       // the combine, which waits for this kernel, needs the window's partials too
-  if (tid == 0 && err != 0 && p.status != nullptr) atomicExch(p.status, err);
+  report_error(&err, p.status);
   if (warp == 1) tmem_dealloc(tmem, C::T_COLS);
 }
 

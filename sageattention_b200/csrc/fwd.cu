@@ -797,7 +797,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && err != 0 && p.status != nullptr) atomicExch(p.status, err);
+  report_error(&err, p.status);
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 

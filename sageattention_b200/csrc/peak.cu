@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(128, 1) peak_mma_kernel(int iters, int* status
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && err != 0 && status != nullptr) atomicExch(status, err);
+  report_error(&err, status);
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 

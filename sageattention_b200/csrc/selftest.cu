@@ -38,7 +38,8 @@ __global__ void __launch_bounds__(128) selftest_wait_kernel(int site, uint32_t s
   }
   __syncthreads();
   if (tid == 0 && item != 1) err = KSTAT_WAIT_TIMEOUT | 0xFF;
-  if (tid == 0 && err != 0 && status != nullptr) atomicExch(status, err);
+  __syncthreads();
+  report_error(&err, status);
 }
 
 }  // namespace nvfp4

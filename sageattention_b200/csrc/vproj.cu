@@ -158,7 +158,7 @@ vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     tc_fence_before();
   }
   __syncthreads();
-  if (tid == 0 && err != 0 && p.status != nullptr) atomicExch(p.status, err);
+  report_error(&err, p.status);
   if (warp == 1) tmem_dealloc(tmem, 128);
 }
 
