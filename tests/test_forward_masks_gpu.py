@@ -82,3 +82,22 @@ def test_hidden_keys_at_the_end(d, causal, visible):
     o = out.cpu().numpy()
     assert np.isfinite(o).all() and np.abs(o - ref).max() <= MAXABS
     assert np.abs(lse.cpu().numpy().reshape(ref_lse.shape) - ref_lse).max() <= 2e-3
+
+
+@pytest.mark.parametrize("d", [128, 256])
+@pytest.mark.parametrize("tiles", [(1, 64), (64, 1), (33, 1, 1, 30), (2, 31, 32)])
+def test_end_of_a_long_sample(d, tiles):
+    """Non-causal packed rows whose samples go on for many tiles behind a query tile: samples of whole key tiles, so that each
+    one is the same to the bit as alone."""
+    import sageattention_b200.nvfp4 as nv
+    h, hk, s = 2, 1, 128 * sum(tiles)
+    q, _ = seeded_bf16((1, h, s, d), 64)
+    k, _ = seeded_bf16((1, hk, s, d), 65)
+    v, _ = seeded_bf16((1, hk, s, d), 66)
+    cu = np.cumsum((0,) + tiles) * 128
+    packs = nv.nvfp4_flash_attention(q, k, v, d ** -0.5, num_key_value_groups=h // hk, return_packs=True)[1]
+    out = nv.nvfp4_flash_attention_packed(*packs, 1, h, hk, s, s, d, d ** -0.5, torch.bfloat16,
+                                          cu_seqlens=torch.tensor(cu, dtype=torch.int32, device="cuda"))
+    for a, b in zip(cu[:-1], cu[1:]):
+        alone = nv.nvfp4_flash_attention(q[:, :, a:b], k[:, :, a:b], v[:, :, a:b], d ** -0.5, num_key_value_groups=h // hk)
+        assert torch.equal(out[:, :, a:b], alone)
