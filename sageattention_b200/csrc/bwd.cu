@@ -986,7 +986,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
     // ------------------------------------------------------------------ scale atoms (+ key bias), row statistics, visible ranges
     for (int it = 0;; ++it) {
       const int sl = it & 1;
-      if (!mbar_wait_item_warp(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
+      if (!mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
       const int r0 = s_item[sl].r0, r1 = s_item[sl].r1;
       if (r1 < 0) break;
       const int m0 = s_item[sl].m0, zh = s_item[sl].zh, unit = s_item[sl].unit, zi = s_item[sl].zi, j0 = s_item[sl].j0;
@@ -1144,7 +1144,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
     uint32_t n = 0;                     // items with steps so far
     for (int it = 0;; ++it) {
       const int sl = it & 1, si = sl % NI;
-      if (!mbar_wait_item_warp(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
+      if (!mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
       const int r0 = s_item[sl].r0, r1 = s_item[sl].r1;
       if (r1 < 0) break;
       if (team == (r0 & 1)) {           // the team of the first step: dO of the item to tensor memory, 2 threads a row

@@ -345,7 +345,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     const float inv_scaling = kBias ? 1.0f / p.scaling : 0.0f;      // the bias is added to the unscaled scores
     for (int it = 0;; ++it) {
       const int sl = it & 1;
-      if (!mbar_wait_item_warp(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
+      if (!mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
       const int r0 = s_item[sl].r0, r1 = s_item[sl].r1;
       if (r1 < 0) break;
       const int zi = s_item[sl].zi, hi = s_item[sl].hi, m0 = s_item[sl].m0;
@@ -581,7 +581,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 
     for (int it = 0;; ++it) {
       const int sl = it & 1;
-      if (!mbar_wait_item_warp(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
+      if (!mbar_wait_item(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
       const int r0 = s_item[sl].r0, r1 = s_item[sl].r1;
       if (r1 < 0) break;
       // Tiles below r_first and from r_mask on need a test per score: the edge of a sample, the causal
