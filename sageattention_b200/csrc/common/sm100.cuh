@@ -3,8 +3,8 @@
 //
 // Every wait in this file is BOUNDED: a wait that exceeds its budget records a status word and returns false instead of
 // spinning forever.  A wait for data has 2^20 probes that suspend for up to 2 us each (about two seconds), or 2^24
-// plain polls; once a CTA has recorded an error all of its later waits for data return at their first probe.  The
-// hand-over of work items goes on after an error and has four times that budget (mbar_wait_item).  So a protocol bug
+// plain polls; once a CTA has recorded an error all of its later waits for data return after a failed
+// probe (256 plain polls).  The hand-over of work items goes on after an error and has four times that budget (mbar_wait_item).  So a protocol bug
 // ends a kernel within seconds, with a readable status, instead of hanging the device.
 #pragma once
 #include <cuda_runtime.h>

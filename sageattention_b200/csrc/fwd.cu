@@ -20,7 +20,7 @@
 // has no part in an item's last tile is at the next item's first while the other merges the row sums and brings out O
 // through a staging tile and TMA (32 rows x 128 bytes a warp; stores of 16 bytes a row took 3500 clocks).  An item
 // costs ~3000 clocks besides its tiles where a CTA cost ~11000 (of 1750 a tile).  The next item is asked for only
-// when the loads of this one are out: asked for at its start, S2048 H16 D256 takes 36.5 instead of 28.6 us.
+// when the loads of this one are out: asked for at its start, S2048 H16 D256 takes 36.5 instead of 28.5 us.
 //
 // What bounds it: the floor is one ex2 per score (16 lanes per clock and SM, 1024 clocks per tile at
 // D = 128); a softmax warp's tile is a chain -- wait, read, maxima, exchange, exponentials and pack,
@@ -33,12 +33,14 @@
 // maxima are the first to be exponentiated, without another read; reciprocal scales come from a table in
 // shared memory, not from the pipe that ex2 needs; P leaves in 16-byte stores.
 // Measured on a B200, kernel alone, causal bf16, against one CTA per query tile: Z4 H32 Hk8 S8192 D128 2033 -> 1695 us
-// (1.30 PFLOP/s), Z1 S4096 150 -> 119, S2048 51.6 -> 37.7, eight samples in 16384 tokens 403 -> 269; H16 Hk4 D256
-// S8192 334 -> 297, S2048 33.2 -> 28.3.
+// (1.30 PFLOP/s), Z1 S4096 150 -> 119, S2048 51.6 -> 37.7, eight samples in 16384 tokens 403 -> 271; H16 Hk4 D256
+// S8192 334 -> 297, S2048 33.2 -> 28.5.
 // Masks: only tiles at an edge of what a row may see -- diagonal, ragged end, ends of a packed sample -- and
 // tiles whose bias has a value other than zero (added already divided by the scaling) are edited, in tensor memory
 // before the maxima are taken, by bits of a 32-column word formed from the row's range; the loop over the others holds
 // no mask code; keys at the end that the bias hides have no tiles.  Z2 H32 Sq1029 Skv2309 padded 111 -> 78 us.
+// A bias that is non-zero in every tile edits them all: Z1 H32 S4096 not causal 235 -> 310 us at D = 128, 322 -> 374 at 256
+// (added on the two reads of S instead, one CTA per query tile: 356 and 422).
 // Registers decide here (96 per thread at twenty warps): variants that spilled even a few hundred
 // bytes took up to three times as long; O is rescaled 32 columns at a time (64: prefill Z4 S8192 1883 -> 2049 us).
 #include "common/abi.cuh"
@@ -258,7 +260,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     }
     if (kBias) {
       // Keys at the end that the bias hides from every row, as it does in a padded batch, have no tiles: 256 at a time from
-      // behind until one is visible.  Z2 H32 Sq1029 Skv2309, 11 and 22 % padded: 86.2 -> 78.0 us.
+      // behind until one is visible.  Z2 H32 Sq1029 Skv2309, 11 and 22 % padded: 86.2 -> 78.0 us,
+      // eight prompts of up to 300 H8 Hk2 15.3 -> 11.9.  It is a trip to L2 before the loads, which calls of two or three tiles
+      // without padding do not get back: Z1 H8 Hk2 S300 9.2 -> 9.7.  Left out below 256 or 384 keys, it cost padded batches of
+      // short prompts more (Z32 H16 S512 causal 47.7 -> 53.2).
       const float* b = p.bias + (int64_t)zi * p.s_kv;
       int seen = 0;                       // visible key with the highest number, plus one
       for (; hi_key > t_lo * 128; hi_key -= 256) {

@@ -368,9 +368,9 @@ def _run_bwd(q, k, v, out, lse, dout, scaling, causal, g, varlen_arrays=None, ou
     """Block-scaled backward for the ``fp4_rownorm`` / ``fp4_legacy`` / ``fp8_rownorm`` modes (stands
     in for flash.py:3811-4265): every GEMM of the backward is a block-scaled tensor-core product.
 
-    Pre-pass (four small launches): delta = rowsum(dO o O) and max|dO|; dO / 2^e packed along D and
-    along the tokens from one read; Q^T and K^T packed along the tokens; V packed along D.  Then the
-    dK/dV kernel (GQA reduced in tensor memory) and the dQ kernel.  In ``fp8_rownorm`` the operands
+    Pre-pass (five launches and a zeroed word): delta = rowsum(dO o O) and max|dO|; dO / 2^e packed along D
+    and along the tokens from one read; Q^T and K^T packed along the tokens; V packed along D.  Then the
+    dK/dV kernel (GQA reduced in tensor memory; at D = 256 a dV and a dK kernel) and the dQ kernel.  In ``fp8_rownorm`` the operands
     of the three gradient GEMMs (dO^T, Q^T, K^T from the pre-pass; P^T, dS^T, dS packed in the
     kernels) are MXFP8 -- e4m3 with an e8m0 scale per 32 -- while S and dP stay NVFP4 products.
 
