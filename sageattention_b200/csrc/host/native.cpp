@@ -53,6 +53,11 @@ inline void require(bool ok, const char* msg) {
   if (__builtin_expect(!ok, 0)) throw AssertionFailure(msg);
 }
 
+// An operand of another number of dimensions is a ValueError, as it is where a shape is unpacked.
+inline void require_dims(const Tensor& t, int64_t n, const char* msg) {
+  if (__builtin_expect(t.dim() != n, 0)) throw std::invalid_argument(msg);
+}
+
 inline int64_t next_mult(int64_t n, int64_t m) { return (n + m - 1) / m * m; }
 
 int dtype_code(at::ScalarType t) {
@@ -178,7 +183,7 @@ void pack_into(const Tensor& x, const Tensor& nib, const Tensor& sc, bool transp
   Call c(x);
   c.same(nib);
   c.same(sc);
-  require(x.dim() == 3, "x must be three-dimensional");
+  require_dims(x, 3, "x must be three-dimensional");
   const Rows xr = rows_of(x);
   const int64_t r = transpose ? xr.k : xr.r, k_read = transpose ? xr.r : xr.k;
   const int64_t sxr = transpose ? xr.sk : xr.sr, sxk = transpose ? xr.sr : xr.sk;
@@ -210,7 +215,7 @@ Pack quant_rows(const Call& c, const Rows& x, at::ScalarType t, bool transpose, 
 
 std::tuple<Tensor, Tensor> quant(const Tensor& x, bool transpose, std::optional<int64_t> k_pad) {
   require_cuda(x, "x");
-  require(x.dim() == 3, "x must be three-dimensional");
+  require_dims(x, 3, "x must be three-dimensional");
   Call c(x);
   Pack p = quant_rows(c, rows_of(x), x.scalar_type(), transpose, k_pad);
   return {p.nib, p.sc};
@@ -220,7 +225,7 @@ std::tuple<Tensor, Tensor> rope_quant(const Tensor& x, const Tensor& cos, const 
                                       int64_t pos0) {
   require_cuda(x, "x");
   Call c(x);
-  require(x.dim() == 3, "x must be [B, R, D]");
+  require_dims(x, 3, "x must be [B, R, D]");
   const int64_t b = x.size(0), r = x.size(1), d = x.size(2);
   require(x.stride(2) == 1, "rows must be contiguous along D");
   require(cos.size(-1) == d / 2 && sin.sizes() == cos.sizes() && cos.scalar_type() == at::kFloat,
@@ -244,7 +249,7 @@ std::tuple<Tensor, Tensor> rope_quant(const Tensor& x, const Tensor& cos, const 
 std::tuple<Tensor, Tensor> quant_mxfp8_t(const Tensor& x_in, int64_t s_pad, const OptTensor& amax) {
   require_cuda(x_in, "x");
   Call c(x_in);
-  require(x_in.dim() == 3, "x must be [B, S, D]");
+  require_dims(x_in, 3, "x must be [B, S, D]");
   const int64_t b = x_in.size(0), s = x_in.size(1), d = x_in.size(2);
   require(s_pad % 32 == 0 && s_pad >= s, "s_pad must be a multiple of 32 covering S");
   const Tensor x = x_in.stride(2) == 1 ? x_in : x_in.contiguous();
@@ -260,7 +265,7 @@ std::tuple<Tensor, Tensor, OptTensor> vproj_quant(const Tensor& x_in, const Tens
                                                   int64_t hk, int64_t d, std::optional<int64_t> s_pad, bool return_value) {
   require_cuda(x_in, "x");
   Call c(x_in);
-  require(x_in.dim() == 3, "x must be [Z, S, hidden]");
+  require_dims(x_in, 3, "x must be [Z, S, hidden]");
   const int64_t z = x_in.size(0), s = x_in.size(1), hidden = x_in.size(2), feats = hk * d;
   require(weight_in.dim() == 2 && weight_in.size(0) == feats && weight_in.size(1) == hidden, "weight must be [Hk*D, hidden]");
   const auto t = x_in.scalar_type();
@@ -312,7 +317,7 @@ Rows unit_rows(const Tensor& t) {      // rows with unit stride along D
 std::tuple<Tensor, Tensor, Tensor, Tensor> quant_dual(const Tensor& x, std::optional<int64_t> s_pad, const OptTensor& amax,
                                                       bool sr_d, bool sr_s, int64_t seed) {
   require_cuda(x, "x");
-  require(x.dim() == 3, "x must be [B, S, D]");
+  require_dims(x, 3, "x must be [B, S, D]");
   Call c(x);
   Dual o = quant_dual_rows(c, unit_rows(x), x.scalar_type(), s_pad.value_or(next_mult(x.size(1), 16)), opt_ptr<float>(amax),
                            (sr_d ? 1 : 0) | (sr_s ? 2 : 0), (uint32_t)(seed & 0xFFFFFFFF));
@@ -430,7 +435,7 @@ std::tuple<Tensor, OptTensor, std::vector<Tensor>> flash_attention(
     bool varlen, const OptTensor& seq_id, const OptTensor& seq_start, bool zshd, bool want_lse, bool want_packs,
     const OptTensor& qnv, const OptTensor& qsc, const OptTensor& knv, const OptTensor& ksc) {
   require_cuda(query, "query");
-  require(query.dim() == 4 && key.dim() == 4, "query and key must be [Z, H, S, D]");
+  for (const Tensor* t : {&query, &key}) require_dims(*t, 4, "query and key must be [Z, H, S, D]");
   const int64_t z = query.size(0), h = query.size(1), s_q = query.size(2), d = query.size(3);
   const int64_t hk = key.size(1), s_kv = key.size(2);
   require(h == hk * g, "num_key_value_groups must equal H // Hk");
@@ -548,7 +553,8 @@ std::tuple<Tensor, OptTensor> decode(const Tensor& query, const Tensor& knv, con
                                      const Tensor& vsc, int64_t s_kv, double scaling, int64_t g, bool want_lse,
                                      std::optional<int64_t> split_kv) {
   require_cuda(query, "query");
-  require(query.dim() == 4 && query.size(2) == 1, "nvfp4_flash_decode is for seqlen_q == 1 (decode)");
+  require_dims(query, 4, "query must be [Z, H, 1, D]");
+  require(query.size(2) == 1, "nvfp4_flash_decode is for seqlen_q == 1 (decode)");
   Call c(query);
   const DecodeArgs a{query.size(0), query.size(1), 0, query.size(3), &knv, &ksc, &vnv, &vsc, s_kv, scaling, g};
   return decode_core(c, query, a, want_lse, split_kv, nullptr);
@@ -557,7 +563,8 @@ std::tuple<Tensor, OptTensor> decode(const Tensor& query, const Tensor& knv, con
 Tensor hybrid_decode(const Tensor& query, const Tensor& knv, const Tensor& ksc, const Tensor& vnv, const Tensor& vsc,
                      const Tensor& rk, const Tensor& rv, int64_t length, int64_t recent_window, double scaling, int64_t g) {
   require_cuda(query, "query");
-  require(query.dim() == 4 && query.size(2) == 1, "nvfp4_flash_decode is for seqlen_q == 1 (decode)");
+  require_dims(query, 4, "query must be [Z, H, 1, D]");
+  require(query.size(2) == 1, "nvfp4_flash_decode is for seqlen_q == 1 (decode)");
   Call c(query);
   c.same(rk);
   c.same(rv);

@@ -52,3 +52,23 @@ def test_backward_refuses_operands_of_other_extents(which):
     for run in (flash._run_bwd_hp, flash._run_bwd):
         with pytest.raises((RuntimeError, AssertionError)):
             run(t["q"], t["k"], t["v"], t["out"], t["lse"], t["dout"], 0.1, True, 2)
+
+
+@pytest.mark.parametrize("call", ["quant", "dual", "mx8", "rope", "vproj", "attention", "train", "decode"])
+@pytest.mark.parametrize("more", [False, True])
+def test_operand_of_another_number_of_dimensions_is_a_value_error(call, more):
+    import sageattention_b200.nvfp4 as nv
+    from sageattention_b200.nvfp4 import flash
+    x3 = torch.zeros(2, 16, 128, device="cuda", dtype=torch.bfloat16)
+    x4 = torch.zeros(1, 2, 1, 128, device="cuda", dtype=torch.bfloat16)
+    x = x3[None] if more else x3[0]                      # where three are wanted
+    y = x4[None] if more else x4[0]                      # where four are wanted
+    angle = torch.zeros(16, 64, device="cuda")
+    packed = nv.nvfp4_quant_kv_decode(x4, x4)
+    calls = dict(quant=lambda: nv._quant_nvfp4(x), dual=lambda: flash._quant_nvfp4_dual(x), mx8=lambda: flash._quant_mxfp8_t(x, 32),
+                 rope=lambda: nv.rope_quant_nvfp4(x, angle, angle), vproj=lambda: nv.vproj_quant_nvfp4(x, x3[0, :, :], None, 1, 16),
+                 attention=lambda: nv.nvfp4_flash_attention(y, x4, x4, 0.1),
+                 train=lambda: nv.nvfp4_flash_attn_func(y, x4, x4, 0.1),
+                 decode=lambda: nv.nvfp4_flash_decode_prequant(y, packed, 0.1))
+    with pytest.raises(ValueError):
+        calls[call]()
