@@ -811,7 +811,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   }
   tc_fence_before();
   __syncthreads();
-  report_error(&err, p.status);
+  report_error_call(&err, p.status);
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 

@@ -28,7 +28,7 @@ def test_every_kernel_with_waits_reports_and_drains_before_it_gives_up_its_memor
         for m in re.finditer(r"__shared__ int err\b", text):
             body = text[m.start():re.compile(r"^}", re.M).search(text, m.start()).start()]
             tail = body[body.rindex("__syncthreads();"):]
-            assert "report_error(&err, " in tail, name
+            assert re.search(r"report_error(_call)?\(&err, ", tail), name
             assert "tmem_dealloc" not in body or tail.index("report_error") < tail.index("tmem_dealloc"), name
             seen += 1
     assert seen == 8
