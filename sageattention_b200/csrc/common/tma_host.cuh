@@ -25,7 +25,8 @@ inline TensorMapEncodeTiledFn tensor_map_encoder() {
   return fn;
 }
 
-// Encoded by every call: 60 ns a map, a tenth of an allocation, and nothing is kept by a buffer's address.
+// Encoded by every call: nothing is kept by a buffer's address.  A map is 0.06 us in a loop and 0.15 within a call, a
+// quarter of an allocation: a decode step has four, the bf16 backward nine.
 struct TmapArgs {
   const void* base;
   uint64_t n0, n1, n2, s1, s2;
