@@ -6,8 +6,8 @@
 // eight torch.empty calls, the stream and device look-ups); a decode step of three launches spent 68 us
 // on the host for 14 us of GPU work.  Here an operator costs its launches (2.1 us each, its C entry included), its
 // allocations (0.55 us each, release included), 0.3 to 1.6 us of guards, checks and views, and 1.2 to 1.6 us of argument
-// parsing in the interpreter: a decode step 6.3 + 1.1 + 1.8 + 4.5 = 13.7 us, a short prompt with its cache
-// 5.8 + 3.9 + 1.9 + 3.7 = 15.3.  The GIL is released for the whole of a call.
+// parsing in the interpreter: a decode step 6.5 + 1.1 + 1.7 + 4.3 = 13.6 us, a short prompt with its cache
+// 5.9 + 3.9 + 1.9 + 3.4 = 15.1.  The GIL is released for the whole of a call.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContextLight.h>
 #include <ATen/cuda/EmptyTensor.h>
