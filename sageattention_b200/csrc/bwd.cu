@@ -451,7 +451,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int jt = blockIdx.y;           // key tile (low tiles have the most visible queries: first)
   const int unit = blockIdx.x;         // z * hk + kh
   const int split = kSplit ? p.split : 1;   // CTAs (of one cluster) that share the tile's steps
@@ -855,7 +855,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int shift = p.s_kv - p.s_q;
   const bool varlen = p.seq_start != nullptr;
   if (warp == 0) {

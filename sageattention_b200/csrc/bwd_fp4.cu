@@ -235,7 +235,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   __shared__ int err;
   __shared__ float gs_s;      // the power-of-two pre-scale of dO
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int shift = p.s_kv - p.s_q;
   const bool varlen = p.seq_start != nullptr;
 

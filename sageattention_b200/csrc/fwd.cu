@@ -164,7 +164,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   __shared__ float xm[2][128];                       // running maximum of the other group
   __shared__ float inv_tab[128];                     // reciprocal of every (non-negative) e4m3 byte
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int shift = p.s_kv - p.s_q;  // bottom-right aligned causal offset
 
   if (warp == 0) {

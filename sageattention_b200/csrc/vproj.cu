@@ -89,7 +89,7 @@ vproj_pack_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   __shared__ uint64_t full[kVpStages], empty[kVpStages], acc_done;
   __shared__ uint32_t tmem_base_s;
   __shared__ int err;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int f0 = blockIdx.x * 128, t0 = blockIdx.y * kNT, zi = blockIdx.z;
   const int nstage = (p.hidden + 63) / 64;
   if (tid == 0) {
