@@ -520,15 +520,18 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ S and dP issuer
-    if (elect_one() && nstep > 0) {
+    if (nstep > 0) {
+      const bool leader = elect_one();
       const uint32_t id_n64 = make_idesc_nvfp4(128, 64);
       mbar_wait(&x_full, 0, &err, 3);
       mbar_wait(&xsf_full, 0, &err, 4);
       tc_fence_after();
+      if (leader) {
 #pragma unroll
-      for (int c = 0; c < C::KB; ++c) {
-        tmem_cp_32x128b_warpx4(tmem + C::T_SFX1 + 4 * c, smem_u32(s_res + C::O_XSF + c * 512));
-        if constexpr (kDs) tmem_cp_32x128b_warpx4(tmem + C::T_SFX2 + 4 * c, smem_u32(s_res + C::O_XSF + (C::KB + c) * 512));
+        for (int c = 0; c < C::KB; ++c) {
+          tmem_cp_32x128b_warpx4(tmem + C::T_SFX1 + 4 * c, smem_u32(s_res + C::O_XSF + c * 512));
+          if constexpr (kDs) tmem_cp_32x128b_warpx4(tmem + C::T_SFX2 + 4 * c, smem_u32(s_res + C::O_XSF + (C::KB + c) * 512));
+        }
       }
       const uint64_t d_x1 = desc_sw64(s_res + C::O_X1, 0), d_x2 = desc_sw64(s_res + C::O_X2, 0);
       const uint64_t d_y1 = desc_sw64(s_stage + C::S_Y1, 0), d_y2 = desc_sw64(s_stage + C::S_Y2, 0);
@@ -543,25 +546,28 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
         else if (st >= 2) mbar_wait(&s_free[pp], ((st >> 1) - 1) & 1, &err, 7);
         tc_fence_after();
         const uint64_t so = (uint64_t)(s * (C::STAGE >> 4)) + (uint64_t)(pp * 256);   // 64 rows x 64 bytes further
-        // S (or S^T): rows x this step's 64 columns
-#pragma unroll
-        for (int c = 0; c < C::KB; ++c)
-          tmem_cp_32x128b_warpx4(tmem + C::T_SFY + 4 * c, smem_u32(sb + C::S_YSF + (pp * C::KB + c) * 512));
-#pragma unroll
-        for (int k = 0; k < C::KB; ++k)
-          umma_nvfp4(tmem + C::T_S + pp * 64, d_x1 + (k >> 1) * 512 + (k & 1) * 2, d_y1 + so + (k >> 1) * 512 + (k & 1) * 2,
-                     id_n64, tmem + C::T_SFX1 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
-        if constexpr (kDs) {
-          // dP (or dP^T)
+        if (leader) {
+          // S (or S^T): rows x this step's 64 columns
 #pragma unroll
           for (int c = 0; c < C::KB; ++c)
-            tmem_cp_32x128b_warpx4(tmem + C::T_SFY + 4 * c, smem_u32(sb + C::S_YSF + ((2 + pp) * C::KB + c) * 512));
+            tmem_cp_32x128b_warpx4(tmem + C::T_SFY + 4 * c, smem_u32(sb + C::S_YSF + (pp * C::KB + c) * 512));
 #pragma unroll
           for (int k = 0; k < C::KB; ++k)
-            umma_nvfp4(tmem + C::T_G, d_x2 + (k >> 1) * 512 + (k & 1) * 2, d_y2 + so + (k >> 1) * 512 + (k & 1) * 2,
-                       id_n64, tmem + C::T_SFX2 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
+            umma_nvfp4(tmem + C::T_S + pp * 64, d_x1 + (k >> 1) * 512 + (k & 1) * 2, d_y1 + so + (k >> 1) * 512 + (k & 1) * 2,
+                       id_n64, tmem + C::T_SFX1 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
+          if constexpr (kDs) {
+            // dP (or dP^T)
+#pragma unroll
+            for (int c = 0; c < C::KB; ++c)
+              tmem_cp_32x128b_warpx4(tmem + C::T_SFY + 4 * c, smem_u32(sb + C::S_YSF + ((2 + pp) * C::KB + c) * 512));
+#pragma unroll
+            for (int k = 0; k < C::KB; ++k)
+              umma_nvfp4(tmem + C::T_G, d_x2 + (k >> 1) * 512 + (k & 1) * 2, d_y2 + so + (k >> 1) * 512 + (k & 1) * 2,
+                         id_n64, tmem + C::T_SFX2 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
+          }
+          umma_commit(&s_full[pp]);
         }
-        umma_commit(&s_full[pp]);
+        __syncwarp();
       }
     }
     __syncwarp();
@@ -569,7 +575,8 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
     // ------------------------------------------------------------------ issuer of the gradient GEMMs
     // A thread of its own: one thread for all products paid its waits and commits one after the other, about 1100
     // clocks a step, and S and dP of the next step stood behind the wait for this one's operands.
-    if (elect_one() && nstep > 0) {
+    if (nstep > 0) {
+      const bool leader = elect_one();
       const uint32_t id_acc = make_idesc_nvfp4(128, D);
       const uint64_t d_a1 = kFp8 ? desc_sw128(s_res + C::O_A1, 0) : desc_sw64(s_res + C::O_A1, 0);
       const uint64_t d_a2 = kFp8 ? desc_sw128(s_res + C::O_A2, 0) : desc_sw64(s_res + C::O_A2, 0);
@@ -603,14 +610,17 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
         mbar_wait(&a_full[pp], (t >> 1) & 1, &err, 8);
         tc_fence_after();
         const uint32_t acc = t > 0 ? 1u : 0u;
-        if constexpr (kP) one_grad(pp, s, sb, acc, C::T_ACC1, d_a1, d_t1, C::O_ASF, C::S_TSF1, C::T_SFA1, C::T_SFT1);
-        if constexpr (kDs) one_grad(pp, s, sb, acc, C::T_ACC2, d_a2, d_t2, C::O_ASF2, C::S_TSF2, C::T_SFA2, C::T_SFT2);
-        umma_commit(&a_free[pp]);
-        if (pp == 1) umma_commit(&empty[s]);
+        if (leader) {
+          if constexpr (kP) one_grad(pp, s, sb, acc, C::T_ACC1, d_a1, d_t1, C::O_ASF, C::S_TSF1, C::T_SFA1, C::T_SFT1);
+          if constexpr (kDs) one_grad(pp, s, sb, acc, C::T_ACC2, d_a2, d_t2, C::O_ASF2, C::S_TSF2, C::T_SFA2, C::T_SFT2);
+          umma_commit(&a_free[pp]);
+          if (pp == 1) umma_commit(&empty[s]);
+        }
+        __syncwarp();
       };
 #pragma unroll 1
       for (int t = 0; t < nstep; ++t) grad_gemms(t);
-      umma_commit(&acc_done);
+      if (leader) umma_commit(&acc_done);
     }
     __syncwarp();
   } else if (warp >= 4) {

@@ -365,36 +365,38 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       }
       int unit, t0, t1;
       item_at(wi, unit, t0, t1);
+      uint32_t it = it_w, su = su_w;        // running counters of this item
+      const int qb = item_idx & 1;
+      mbar_wait(&q_full[qb], (item_idx >> 1) & 1, &err, 6);
+      tc_fence_after();
       if (leader) {
-        uint32_t it = it_w, su = su_w;      // the leader's running counters for this item
-        const int qb = item_idx & 1;
-        mbar_wait(&q_full[qb], (item_idx >> 1) & 1, &err, 6);
-        tc_fence_after();
 #pragma unroll
         for (int k = 0; k < C::KB; ++k)
           tmem_cp_32x128b_warpx4(tmem + C::T_SFQ + qb * C::KB * 4 + k * 4,
                                  smem_u32(s_qsf + qb * C::QSF_BYTES + k * 512));
-        for (int ts0 = t0; ts0 < t1; ts0 += ST, ++su) {
-          const int b = su & 1;
-          const int nt = min(ST, t1 - ts0);
-          if (su >= 2) {
-            mbar_spin_wait(&s_free[b], ((su >> 1) & 1) ^ 1, &err, 5);
-            // the V-scale TMEM slots of buffer b are rewritten below: the PV of round su - 2 must be done
-            mbar_spin_wait(&o_full[b], ((su >> 1) & 1) ^ 1, &err, 11);
-          }
-          for (int j = 0; j < nt; ++j, ++it) {
-            const int s = it % C::NSTAGE;
-            const uint32_t ph = (it / C::NSTAGE) & 1;
-            mbar_spin_wait(&full[s], ph, &err, 3);
-            tc_fence_after();
-            uint8_t* st = s_stage + s * C::STAGE_BYTES;
-            const uint32_t sfk = tmem + C::T_SFK + (b * C::STMAX + j) * C::KB * 4;
+      }
+      for (int ts0 = t0; ts0 < t1; ts0 += ST, ++su) {
+        const int b = su & 1;
+        const int nt = min(ST, t1 - ts0);
+        if (su >= 2) {
+          mbar_spin_wait(&s_free[b], ((su >> 1) & 1) ^ 1, &err, 5);
+          // the V-scale TMEM slots of buffer b are rewritten below: the PV of round su - 2 must be done
+          mbar_spin_wait(&o_full[b], ((su >> 1) & 1) ^ 1, &err, 11);
+        }
+        for (int j = 0; j < nt; ++j, ++it) {
+          const int s = it % C::NSTAGE;
+          const uint32_t ph = (it / C::NSTAGE) & 1;
+          mbar_spin_wait(&full[s], ph, &err, 3);
+          tc_fence_after();
+          uint8_t* st = s_stage + s * C::STAGE_BYTES;
+          const uint32_t sfk = tmem + C::T_SFK + (b * C::STMAX + j) * C::KB * 4;
+          // the V^T scales of this tile go to TMEM now as well, off the PV issuer's critical path
+          // (slot (b, j) was last read by the PV of round su - 2, complete before s_free fired)
+          const uint32_t sfv = tmem + C::T_SFV + (b * C::STMAX + j) * C::MT * 8;
+          if (leader) {
 #pragma unroll
             for (int k = 0; k < C::KB; ++k)
               tmem_cp_32x128b_warpx4(sfk + k * 4, smem_u32(st + C::K_BYTES + C::V_BYTES + k * 512));
-            // the V^T scales of this tile go to TMEM now as well, off the PV issuer's critical path
-            // (slot (b, j) was last read by the PV of round su - 2, complete before s_free fired)
-            const uint32_t sfv = tmem + C::T_SFV + (b * C::STMAX + j) * C::MT * 8;
 #pragma unroll
             for (int k = 0; k < C::MT * 2; ++k)
               tmem_cp_32x128b_warpx4(sfv + k * 4,
@@ -408,8 +410,9 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
                          tmem + C::T_SFQ + qb * C::KB * 4 + k * 4, k > 0);
             }
           }
-          umma_commit(&s_full[b]);
+          __syncwarp();
         }
+        if (leader) umma_commit(&s_full[b]);
       }
       it_w += (uint32_t)(t1 - t0);
       su_w += (uint32_t)((t1 - t0 + ST - 1) / ST);
@@ -417,21 +420,22 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     }
   } else if (warp == 3) {
     // ------------------------------------------------------------------ PV issuer
-    if (elect_one()) {
-      const uint32_t idesc = make_idesc_nvfp4(128, 16);
-      uint32_t it = 0, su = 0;
-      for (int wi = 0; wi < my_items; ++wi) {
-        int unit, t0, t1;
-        item_at(wi, unit, t0, t1);
-        for (int ts0 = t0; ts0 < t1; ts0 += ST, ++su) {
-          const int b = su & 1;
-          const int nt = min(ST, t1 - ts0);
-          mbar_spin_wait(&p_full[b], (su >> 1) & 1, &err, 7);
-          tc_fence_after();
-          for (int j = 0; j < nt; ++j, ++it) {
+    const bool leader = elect_one();
+    const uint32_t idesc = make_idesc_nvfp4(128, 16);
+    uint32_t it = 0, su = 0;
+    for (int wi = 0; wi < my_items; ++wi) {
+      int unit, t0, t1;
+      item_at(wi, unit, t0, t1);
+      for (int ts0 = t0; ts0 < t1; ts0 += ST, ++su) {
+        const int b = su & 1;
+        const int nt = min(ST, t1 - ts0);
+        mbar_spin_wait(&p_full[b], (su >> 1) & 1, &err, 7);
+        tc_fence_after();
+        if (leader) {
+          for (int j = 0; j < nt; ++j) {
             // V^T tile and scales of stage s were observed by the QK^T issuer before S^T of this
             // round was produced, and P arrived after the softmax warps saw that S^T
-            const int s = it % C::NSTAGE;
+            const int s = (it + j) % C::NSTAGE;
             uint8_t* st = s_stage + s * C::STAGE_BYTES;
             const uint32_t sfv = tmem + C::T_SFV + (b * C::STMAX + j) * C::MT * 8;
             const uint32_t sfp = tmem + C::T_SFP + (b * C::STMAX + j) * 8;
@@ -455,6 +459,8 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           }
           umma_commit(&o_full[b]);
         }
+        __syncwarp();
+        it += nt;
       }
     }
     __syncwarp();
