@@ -146,6 +146,45 @@ __device__ __forceinline__ uint8_t pack_group16(const float (&x)[16], uint32_t& 
   return sb;
 }
 
+// The same bytes for groups whose values come from a 16-bit type T (times a power of two), in half the instructions.
+// Such a value has at most 11 significant bits and a scale four, a rounding boundary t of e2m1 three: x / scale is either t
+// itself or 2^-12 or more away from it (relative), and so is amax / 6 from a boundary of e4m3.  A quotient that is off by far
+// less than that gives the same code, provided that it is t where x = t * scale, for ties go to the even neighbour.
+//   * amax * RN(1/6) is exactly the boundary for all of its 32 significands (checked one by one);
+//   * 1 / scale as hi + lo, hi below it and lo the rest (2^-22 of it): RN(x hi + RN(x lo)) is off by 2^-45 before its one
+//     rounding, hence t where the quotient is t.  lo is positive, so a zero keeps its sign.
+// Infinities end at the largest code as they do by division; nothing here can make a NaN of them.
+// Along D [128, 8192, 128] bf16 60.0 -> 52.3 us (6.6 TB/s, the copy rate), both ways at once [16, 8192, 256] 35.0 -> 27.8, V^T
+// [64, 8192, 128] 37.4 -> 34.3.  All 16-bit values under all scales are compared with the division in a test.
+template <typename T>
+__device__ __forceinline__ uint8_t pack_group16_of(const float (&x)[16], uint32_t& lo, uint32_t& hi) {
+  if constexpr (sizeof(T) != 2) {
+    return pack_group16(x, lo, hi);
+  } else {
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) amax = max3f(amax, fabsf(x[i]), fabsf(x[i + 1]));
+    const float s = fminf(fmaxf(amax * 0.16666667f, kScaleFloor), kScaleMax);
+    uint16_t sb;
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(sb) : "f"(0.0f), "f"(s));
+    const float sf = e4m3_to_f32((uint8_t)(sb & 0xFF));
+    float inv;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(sf));
+    const float ih = inv * 0.99999976f;                  // 1 - 2^-22: below 1 / sf by more than the approximation's error
+    const float il = fmaf(-sf, ih, 1.0f) * inv;
+    const float2 h2 = make_float2(ih, ih), l2 = make_float2(il, il);
+    float2 y[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float2 v = make_float2(x[2 * i], x[2 * i + 1]);
+      y[i] = __ffma2_rn(v, h2, __fmul2_rn(v, l2));
+    }
+    lo = e2m1x8(y[0].x, y[0].y, y[1].x, y[1].y, y[2].x, y[2].y, y[3].x, y[3].y);
+    hi = e2m1x8(y[4].x, y[4].y, y[5].x, y[5].y, y[6].x, y[6].y, y[7].x, y[7].y);
+    return (uint8_t)(sb & 0xFF);
+  }
+}
+
 // ---- MXFP8 (e4m3 values, one e8m0 power-of-two scale per 32): the gradient operands of the
 // fp8_rownorm backward.  Scale exponent e = the smallest integer with amax / 2^e <= 448 (the exact
 // form of ceil(log2(amax / 448)), flash.py:243-257), amax floored at 1e-30; stored as e + 127.

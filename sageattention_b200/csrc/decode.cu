@@ -229,7 +229,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
 #pragma unroll
       for (int e = 0; e < 16; ++e) v[e] = to_f32<TQ>(src[e]);
       uint32_t lo, hi;
-      const uint8_t sb = pack_group16(v, lo, hi);
+      const uint8_t sb = pack_group16_of<TQ>(v, lo, hi);
       *reinterpret_cast<uint2*>(dq + (gi >> 3) * 1024 + sw64_offset(qr, (gi & 7) * 8)) = make_uint2(lo, hi);
       dsf[(gi >> 2) * 512 + sf_atom_offset(qr, gi & 3)] = sb;
     }

@@ -33,7 +33,7 @@ __global__ void kv_append_kernel(const T* __restrict__ k_new, const T* __restric
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = to_f32<T>(kr[gi * 16 + i]);
     uint32_t lo, hi;
-    const uint8_t sb = pack_group16(v, lo, hi);
+    const uint8_t sb = pack_group16_of<T>(v, lo, hi);
     uint8_t* pn = knv + u * knv_unit + pos * (d / 2) + gi * 8;
     *reinterpret_cast<uint2*>(pn) = make_uint2(lo, hi);
     ksc[u * ksc_unit + pos * (d / 16) + gi] = sb;
@@ -57,7 +57,7 @@ __global__ void kv_append_kernel(const T* __restrict__ k_new, const T* __restric
     }
   }
   uint32_t lo, hi;
-  const uint8_t sb = pack_group16(v, lo, hi);
+  const uint8_t sb = pack_group16_of<T>(v, lo, hi);
   uint8_t* pv = vnv + u * vnv_unit + (int64_t)t * vnv_row + gidx * 8;
   *reinterpret_cast<uint2*>(pv) = make_uint2(lo, hi);
   vsc[u * vsc_unit + (int64_t)t * vsc_row + gidx] = sb;

@@ -78,7 +78,7 @@ __device__ __forceinline__ void pack_rows_group(
     for (int i = 0; i < 8; ++i) { v[i] = a[i]; v[8 + i] = c[i]; }
   }
   uint32_t lo, hi;
-  const uint8_t sb = pack_group16(v, lo, hi);
+  const uint8_t sb = pack_group16_of<T>(v, lo, hi);
   uint8_t* pn = nib + b * snb + r * snr + g * 8;
   if ((reinterpret_cast<uintptr_t>(pn) & 7) == 0) {
     *reinterpret_cast<uint2*>(pn) = make_uint2(lo, hi);
@@ -130,7 +130,7 @@ __device__ __forceinline__ void pack_rows_quad(const T* __restrict__ x, int ng_l
 #pragma unroll
     for (int j = 0; j < 16; ++j) v[j] = to_f32<T>(e[j]);
     uint32_t lo, hi;
-    const uint8_t sb = pack_group16(v, lo, hi);
+    const uint8_t sb = pack_group16_of<T>(v, lo, hi);
     if (first + i * 32 + lane < per_batch) {
       *reinterpret_cast<uint2*>(nib + b * snb + r[i] * snr + g[i] * 8) = make_uint2(lo, hi);
       sc[b * ssb + r[i] * ssr + g[i]] = sb;
@@ -236,9 +236,9 @@ __global__ void __launch_bounds__(256, 2) rope_pack_rows_kernel(
     uint32_t w0, w1;
     uint8_t* pn = nib + b * snb + r * snr + g * 8;
     uint8_t* ps = sc + b * ssb + r * ssr + g;
-    ps[0] = pack_group16(u, w0, w1);
+    ps[0] = pack_group16_of<T>(u, w0, w1);
     *reinterpret_cast<uint2*>(pn) = make_uint2(w0, w1);
-    ps[half >> 4] = pack_group16(v, w0, w1);
+    ps[half >> 4] = pack_group16_of<T>(v, w0, w1);
     *reinterpret_cast<uint2*>(pn + (half >> 1)) = make_uint2(w0, w1);
   }
 }
@@ -369,7 +369,7 @@ __device__ __forceinline__ void pack_cols_tile(
             const uint8_t sb = (sr_flags & 1)
                                    ? pack_group16_sr(v, w[2 * it], w[2 * it + 1], seed, (uint32_t)(b * k_read + k0 + key) * 2u,
                                                      (uint32_t)(r0 / 4 + g * 4))
-                                   : pack_group16(v, w[2 * it], w[2 * it + 1]);
+                                   : pack_group16_of<T>(v, w[2 * it], w[2 * it + 1]);
             sb2 |= (uint32_t)sb << (8 * it);
           }
           uint8_t* pn = dnib + b * dnb + (k0 + key) * dnr + rg / 2;
@@ -408,7 +408,7 @@ __device__ __forceinline__ void pack_cols_tile(
           const uint8_t sb = (kDual && (sr_flags & 2))
                                  ? pack_group16_sr(h ? v1 : v0, lo, hi, seed, (uint32_t)(b * R + r0 + row) * 2u + 1u,
                                                    (uint32_t)(k0 / 4 + g * 4))
-                                 : pack_group16(h ? v1 : v0, lo, hi);
+                                 : pack_group16_of<T>(h ? v1 : v0, lo, hi);
           *reinterpret_cast<uint2*>(&onib[row][g * 8]) = make_uint2(lo, hi);
           osc[row][g] = sb;
         }
@@ -451,7 +451,7 @@ __device__ __forceinline__ void pack_cols_tile(
           const uint8_t sb = (sr_flags & 1)
                                  ? pack_group16_sr(v, lo, hi, seed, (uint32_t)(b * k_read + k0 + key) * 2u,
                                                    (uint32_t)(r0 / 4 + g * 4))
-                                 : pack_group16(v, lo, hi);
+                                 : pack_group16_of<T>(v, lo, hi);
           *reinterpret_cast<uint2*>(dnib + b * dnb + (k0 + key) * dnr + (r0 + g * 16) / 2) = make_uint2(lo, hi);
           dsc[b * dsb + (k0 + key) * dsr + (r0 + g * 16) / 16] = sb;
         }
@@ -469,7 +469,7 @@ __device__ __forceinline__ void pack_cols_tile(
       const uint8_t sb = (kDual && (sr_flags & 2))
                              ? pack_group16_sr(v, lo, hi, seed, (uint32_t)(b * R + r0 + row) * 2u + 1u,
                                                (uint32_t)(k0 / 4 + g * 4))
-                             : pack_group16(v, lo, hi);
+                             : pack_group16_of<T>(v, lo, hi);
       *reinterpret_cast<uint2*>(&onib[row][g * 8]) = make_uint2(lo, hi);
       osc[row][g] = sb;
     }
@@ -768,7 +768,7 @@ __global__ void __launch_bounds__(256) pack_generic_kernel(
     v[i] = k < k_read ? to_f32<T>(x[b * sxb + r * sxr + k * sxk]) : 0.0f;
   }
   uint32_t lo, hi;
-  const uint8_t sb = pack_group16(v, lo, hi);
+  const uint8_t sb = pack_group16_of<T>(v, lo, hi);
   uint8_t* pn = nib + b * snb + r * snr + g * 8;
 #pragma unroll
   for (int i = 0; i < 4; ++i) { pn[i] = (lo >> (8 * i)) & 0xFF; pn[4 + i] = (hi >> (8 * i)) & 0xFF; }

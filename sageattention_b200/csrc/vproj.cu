@@ -61,7 +61,7 @@ __device__ __forceinline__ void vproj_store(const VprojParams& p, int zi, int f,
     if (vo != nullptr && tok + e < p.s) vo[(int64_t)(tok + e) * p.svs] = hv;
   }
   uint32_t lo, hi;
-  const uint8_t sb = pack_group16(v, lo, hi);
+  const uint8_t sb = pack_group16_of<T>(v, lo, hi);
   const int64_t row = ((int64_t)zi * p.hk + f / p.d) * p.d + f % p.d;
   *reinterpret_cast<uint2*>(p.vnv + row * (p.s_pad / 2) + tok / 2) = make_uint2(lo, hi);
   p.vsc[row * (p.s_pad / 16) + tok / 16] = sb;
