@@ -40,29 +40,53 @@ __device__ __forceinline__ void griddep_start(bool late) {
   if (!late) griddep_wait();
 }
 
-// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per kernel and device: a fixed open-addressing
-// table of kernel addresses (the library has fewer kernels than slots), lock-free, so that a launch
-// pays a look-up (~20 ns) instead of the driver call.  `bytes` must be the same in every call for a kernel.
-inline int allow_smem(const char* what, const void* kern, int bytes) {
-  constexpr int kSlots = 512;
-  static std::atomic<const void*> keys[kSlots];
-  static std::atomic<uint64_t> devices[kSlots];
+// What is done once per kernel and device: a fixed open-addressing table of kernel addresses (the library has fewer
+// kernels than slots), lock-free, so that a launch pays a look-up (~20 ns) instead of the driver call.  Two threads may
+// both be first; what they do is the same.
+struct KernelTable {
+  static constexpr int kSlots = 512;
+  std::atomic<const void*> keys[kSlots];
+  std::atomic<uint64_t> devices[kSlots];
+  // the slot's devices, or null where the table is full
+  std::atomic<uint64_t>* find(const void* kern) {
+    uint32_t i = (uint32_t)((reinterpret_cast<uintptr_t>(kern) >> 4) * 2654435761u) % kSlots;
+    for (int probe = 0; probe < kSlots; ++probe, i = (i + 1) % kSlots) {
+      const void* k = keys[i].load(std::memory_order_acquire);
+      if (k == nullptr && keys[i].compare_exchange_strong(k, kern, std::memory_order_acq_rel)) k = kern;
+      if (k == kern) return &devices[i];
+    }
+    return nullptr;
+  }
+};
+
+// cudaFuncSetAttribute(attr, value) of a kernel; `value` must be the same in every call for a kernel and attribute.
+template <cudaFuncAttribute kAttr>
+cudaError_t kernel_attribute(const void* kern, int value) {
+  static KernelTable table;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return fail((int)e, "%s: cudaGetDevice: %s", what, cudaGetErrorString(e));
+  if (e != cudaSuccess) return e;
   const uint64_t bit = dev < 64 ? 1ull << dev : 0;
-  uint32_t i = (uint32_t)((reinterpret_cast<uintptr_t>(kern) >> 4) * 2654435761u) % kSlots;
-  for (int probe = 0; probe < kSlots; ++probe, i = (i + 1) % kSlots) {
-    const void* k = keys[i].load(std::memory_order_acquire);
-    if (k == nullptr && keys[i].compare_exchange_strong(k, kern, std::memory_order_acq_rel)) k = kern;
-    if (k != kern) continue;
-    if (devices[i].load(std::memory_order_acquire) & bit) return 0;
-    break;
-  }
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  std::atomic<uint64_t>* seen = table.find(kern);
+  if (seen != nullptr && (seen->load(std::memory_order_acquire) & bit)) return cudaSuccess;
+  e = cudaFuncSetAttribute(kern, kAttr, value);
+  if (e == cudaSuccess && seen != nullptr) seen->fetch_or(bit, std::memory_order_acq_rel);
+  return e;
+}
+
+inline int allow_smem(const char* what, const void* kern, int bytes) {
+  const cudaError_t e = kernel_attribute<cudaFuncAttributeMaxDynamicSharedMemorySize>(kern, bytes);
   if (e != cudaSuccess) return fail((int)e, "%s: smem attribute: %s", what, cudaGetErrorString(e));
-  if (keys[i].load(std::memory_order_acquire) == kern) devices[i].fetch_or(bit, std::memory_order_acq_rel);
   return 0;
+}
+
+// For kernels that stream through L1: at most `kStreamSmem` percent of it as shared memory (three blocks of the V^T
+// packers).  A load in flight holds a line of L1, and an SM keeps the split that the kernel before it asked for: behind the
+// forward, whose 202 KB leave 28 of L1, the packs of a prompt Z4 S8192 took 119 us instead of 92 (prompt S12289 D256 in all
+// 675 -> 663).  A hint, not checked.
+constexpr int kStreamSmem = 45;
+inline void prefer_l1(const void* kern) {
+  if (kernel_attribute<cudaFuncAttributePreferredSharedMemoryCarveout>(kern, kStreamSmem) != cudaSuccess) cudaGetLastError();
 }
 
 // Clusters of 1, 2, 4 and 8 CTAs of a kernel that are resident at once, asked once per device: for kernels that leave
@@ -124,6 +148,13 @@ int launch_cluster(const char* what, void (*kern)(P...), dim3 grid, unsigned clu
 
 template <typename... P, typename... A>
 int launch(const char* what, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
+  return launch_cluster(what, kern, grid, 1, threads, smem, st, static_cast<A&&>(args)...);
+}
+
+// launch() of a kernel that streams through L1
+template <typename... P, typename... A>
+int launch_streaming(const char* what, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
+  prefer_l1(reinterpret_cast<const void*>(kern));
   return launch_cluster(what, kern, grid, 1, threads, smem, st, static_cast<A&&>(args)...);
 }
 

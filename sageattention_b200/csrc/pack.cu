@@ -796,23 +796,23 @@ int pack_dispatch(const T* x, int64_t B, int64_t R, int64_t k_read, int64_t k_pa
     if (lg >= 0 && k_read >= k_pad && (reinterpret_cast<uintptr_t>(x) & 31) == 0 && sxb % kVec32 == 0 &&
         sxr % kVec32 == 0 && (reinterpret_cast<uintptr_t>(nib) & 7) == 0 && snb % 8 == 0 && snr % 8 == 0) {
       dim3 qgrid((unsigned)((per_batch + 1023) / 1024), (unsigned)B);
-      return launch("nvfp4_pack(rows)", pack_rows_quad_kernel<T>, qgrid, 256, 0, st, x, lg, per_batch, sxb, sxr, nib, snb,
+      return launch_streaming("nvfp4_pack(rows)", pack_rows_quad_kernel<T>, qgrid, 256, 0, st, x, lg, per_batch, sxb, sxr, nib, snb,
                     snr, sc, ssb, ssr);
     }
     dim3 grid((unsigned)blocks, (unsigned)B);
-    return launch("nvfp4_pack(rows)", pack_rows_kernel<T>, grid, 256, 0, st, x, R, k_read, ngroups, lg, per_batch, sxb, sxr,
+    return launch_streaming("nvfp4_pack(rows)", pack_rows_kernel<T>, grid, 256, 0, st, x, R, k_read, ngroups, lg, per_batch, sxb, sxr,
                   nib, snb, snr, sc, ssb, ssr, vec);
   }
   if (sxr == 1 && B < 65536 && (R + kColsRows - 1) / kColsRows < 65536) {
     const int vec = base_ok && sxb % kVecElems == 0 && sxk % kVecElems == 0;
     dim3 grid((unsigned)((k_pad + kColsKeys * kColsRun - 1) / (kColsKeys * kColsRun)),
               (unsigned)((R + kColsRows - 1) / kColsRows), (unsigned)B);
-    return launch("nvfp4_pack(cols)", pack_cols_kernel<T, false>, grid, 256, 0, st, x, R, k_read, k_pad, sxb, sxk, nib, snb,
+    return launch_streaming("nvfp4_pack(cols)", pack_cols_kernel<T, false>, grid, 256, 0, st, x, R, k_read, k_pad, sxb, sxk, nib, snb,
                   snr, sc, ssb, ssr, vec, nullptr, 0, 0, nullptr, 0, 0, nullptr, 0, 0u);
   }
   const int64_t blocks = (total + 255) / 256;
   NVFP4_REQUIRE(blocks < (1LL << 31), "nvfp4_pack: tensor too large");
-  return launch("nvfp4_pack(generic)", pack_generic_kernel<T>, dim3((unsigned)blocks), 256, 0, st, x, R, k_read, ngroups,
+  return launch_streaming("nvfp4_pack(generic)", pack_generic_kernel<T>, dim3((unsigned)blocks), 256, 0, st, x, R, k_read, ngroups,
                 total, sxb, sxr, sxk, nib, snb, snr, sc, ssb, ssr);
 }
 
@@ -854,7 +854,7 @@ int pack_dual_launch(const void* x, int64_t B, int64_t S, int d, int64_t s_pad, 
   const int vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && sxb % kVecElems == 0 && sxs % kVecElems == 0;
   dim3 grid((unsigned)((s_pad + kColsKeys * kColsRun - 1) / (kColsKeys * kColsRun)),
             (unsigned)((d + kColsRows - 1) / kColsRows), (unsigned)B);
-  return launch(
+  return launch_streaming(
       "nvfp4_pack_dual", pack_cols_kernel<T, true>, grid, 256, 0, st, static_cast<const T*>(x), d, S, s_pad, sxb, sxs, tnib, (int64_t)d * (s_pad / 2), s_pad / 2, tsc,
       (int64_t)d * (s_pad / 16), s_pad / 16, vec, dnib, S * (int64_t)(d / 2), d / 2, dsc, S * (int64_t)(d / 16),
       d / 16, prescale_amax, sr_flags, seed);
@@ -883,7 +883,7 @@ int pack_qkv_launch(QkvArgs a, cudaStream_t st) {
   a.nbk = a.bpk * a.bk;
   const int64_t total = a.nbq + a.nbk + a.bk * ((a.tx + kColsRun - 1) / kColsRun) * a.ty;
   NVFP4_REQUIRE(total < (1LL << 31), "nvfp4_pack_qkv: tensors too large");
-  return launch("nvfp4_pack_qkv", pack_qkv_kernel<T>, dim3((unsigned)total), 256, 0, st, a);
+  return launch_streaming("nvfp4_pack_qkv", pack_qkv_kernel<T>, dim3((unsigned)total), 256, 0, st, a);
 }
 
 template <typename T>
@@ -907,7 +907,7 @@ int kv_prefill_launch(PrefillArgs a, cudaStream_t st) {
   a.bpc = (pieces + 256 * kPrefillCopyIters - 1) / (256 * kPrefillCopyIters);
   const int64_t total = a.nbk + a.nbv + a.bpc * a.zhk;
   NVFP4_REQUIRE(total < (1LL << 31), "nvfp4_kv_prefill: tensors too large");
-  return launch("nvfp4_kv_prefill", kv_prefill_kernel<T>, dim3((unsigned)total), 256, 0, st, a);
+  return launch_streaming("nvfp4_kv_prefill", kv_prefill_kernel<T>, dim3((unsigned)total), 256, 0, st, a);
 }
 
 }  // namespace nvfp4
@@ -977,7 +977,7 @@ extern "C" int nvfp4_pack_mx8_t(const void* x, int dtype, int64_t B, int64_t S, 
   {                                                                                                     \
     constexpr int64_t kVecElems = 16 / sizeof(T);                                                       \
     const int vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && sxb % kVecElems == 0 && sxs % kVecElems == 0; \
-    return launch("nvfp4_pack_mx8_t", pack_mx8_cols_kernel<T>, grid, 256, 0, st, static_cast<const T*>(x), d, S, s_pad, \
+    return launch_streaming("nvfp4_pack_mx8_t", pack_mx8_cols_kernel<T>, grid, 256, 0, st, static_cast<const T*>(x), d, S, s_pad, \
                   sxb, sxs, out, sc, vec, prescale_amax);                                               \
   }
   switch (dtype) {
@@ -1056,7 +1056,7 @@ extern "C" int nvfp4_rope_pack(const void* x, int dtype, int64_t B, int64_t R, i
   const int64_t bits = (int64_t)(uintptr_t)x | (sxb * es) | (sxr * es);
   const int align = bits % 32 == 0 ? 32 : (bits % 16 == 0 ? 16 : 1);
 #define NVFP4_ROPE(T)                                                                              \
-  return launch("nvfp4_rope_pack", rope_pack_rows_kernel<T>, grid, 256, 0, st, static_cast<const T*>(x), (int)B, d, lg, \
+  return launch_streaming("nvfp4_rope_pack", rope_pack_rows_kernel<T>, grid, 256, 0, st, static_cast<const T*>(x), (int)B, d, lg, \
                 npairs, nb, sxb, sxr, cos_tab, sin_tab, positions, pos0, nib, snb, snr, sc, ssb, ssr, align)
   switch (dtype) {
     case NVFP4_DT_BF16: NVFP4_ROPE(__nv_bfloat16);
