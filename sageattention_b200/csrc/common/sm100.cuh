@@ -284,6 +284,10 @@ __device__ __forceinline__ void cp_async_4_l2line(uint32_t saddr, const void* gp
                "r"(src_bytes)
                : "memory");
 }
+// This thread's copies so far arrive on `bar` (once, counted among its expected arrivals) when they have landed.
+__device__ __forceinline__ void cp_async_mbar_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {

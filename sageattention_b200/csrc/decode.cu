@@ -7,7 +7,7 @@
 // "keys on the M axis" orientation, so the cache layout is the operand layout:
 //     S^T[128 keys x 16] = K_tile[128 x D] . Q^T           (A = K tile, B = the G<=16 query rows)
 //     O^T[D x 16]       += V^T_tile[D x 128] . P^T          (A = V^T tile, B = P packed along keys)
-// Scale bytes are re-laid into the 32x16-byte form tcgen05.cp expects by two loader warps.
+// Scale bytes are re-laid into the 32x16-byte form tcgen05.cp expects by a loader warp.
 // Softmax runs with one thread per key (TMEM lane); P is packed to NVFP4 per 16 keys with the
 // same scale rule as the packer.  Each work item writes un-normalised (acc, m, l) partials; a
 // second small kernel combines them exactly and emits the output and its log-sum-exp.
@@ -15,6 +15,12 @@
 // Warp roles (384 threads): 0 TMA producer, 1 QK^T issuer, 2 scale loader, 3 PV issuer,
 // 4-11 softmax / accumulate / epilogue (two groups splitting each round's tiles).  Every barrier
 // wait is bounded.
+//
+// What bounds it: a long cache HBM (Z16 Hk8 S32768 D128, 604 MB: 104 us, 5.8 TB/s or 0.89 of the copy rate, where scale
+// bytes that were handed on three tiles late had it at 122), a short one a chain of cold steps: first loads, four
+// tiles' products, a softmax round, their P.V, the partials -- 7700 clocks for one round, 11700 with the L2 pulls in front of
+// the first load.  Graphs of append and decode: Z1 Hk8 S1021 13.9 -> 11.8 us, Z4 Hk4 S6007 D256 18.9 -> 16.0, Z16 Hk8
+// S32768 132 -> 113.7, with a window Z8 Hk8 S8190 41.5 -> 39.5-41.0.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
 #include "common/launch.cuh"
@@ -150,9 +156,9 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       t0 = (int)(max(bal_start, base) - base);
       t1 = (int)(min(bal_end, base + p.ntiles) - base);
     } else {
-      const int64_t w = blockIdx.x + (int64_t)i * nctas;
-      unit = (int)(w / p.nsplit);
-      const int split = (int)(w % p.nsplit);
+      const uint32_t w = blockIdx.x + (uint32_t)i * gridDim.x;      // below 2^31, as the number of items
+      unit = (int)(w / (uint32_t)p.nsplit);
+      const int split = (int)(w - (uint32_t)unit * (uint32_t)p.nsplit);
       t0 = split * p.chunk_tiles;
       t1 = min(t0 + p.chunk_tiles, p.ntiles);
     }
@@ -161,9 +167,26 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     return p.balanced ? (int64_t)blockIdx.x * p.maxseg + i : blockIdx.x + (int64_t)i * nctas;
   };
 
-  // Before anything else: ask L2 for the scale bytes of this CTA's first tiles.  They are the
-  // scattered first touches of the kernel (one 128-byte line per V^T row, a few KB of K scales), and
-  // their DRAM latency otherwise sits in front of the very first MMA.
+  // V^T rows are D separate strips in memory and a 128-key tile touches only 64 bytes of each; 1 KB per strip (16
+  // tiles) is pulled into L2 one 16-tile block ahead so DRAM sees long bursts.  8 strips (rows rows8 .. rows8+7 of every
+  // 128-row piece) of the block of <= 16 tiles that starts at tile tb and must not reach past tile te: 1 KB boxes
+  // for whole blocks, 256-byte boxes for a clipped tail, so nothing beyond the work item is read from DRAM.
+  auto pull = [&](int un, int tb, int te, int rows8) {
+    const int nt = min(16, te - tb);
+    if (nt <= 0) return;
+#pragma unroll
+    for (int mt = 0; mt < C::MT; ++mt) {
+      if (nt == 16) {
+        tma_prefetch_3d(&tm_vpf, tb * 16, mt * 128 + rows8, un);
+      } else {
+        for (int q4 = 0; q4 * 4 < nt; ++q4) tma_prefetch_3d(&tm_vpf4, (tb + q4 * 4) * 16, mt * 128 + rows8, un);
+      }
+    }
+  };
+  const TQ* qbase = static_cast<const TQ*>(p.q);
+  // Before anything else, and before the wait for the kernel in front (L2 is the point of coherence): ask L2 for the
+  // scale bytes of this CTA's first tiles, the scattered first touches of the kernel (one 128-byte line per V^T row, a few
+  // KB of K scales), and for the query rows.
   if (my_items > 0) {
     int unit, t0, t1;
     item_at(0, unit, t0, t1);
@@ -175,12 +198,15 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       const int64_t end = min((int64_t)min(t1, t0 + 8) * 128, p.s_kv) * (D / 16);
       if (off < end) prefetch_l2(p.ksc + (int64_t)unit * p.ksc_unit + off);
     }
+    if (warp == 1 && lane < p.g) prefetch_l2(qbase + (unit / p.hk) * p.s_qz + (int64_t)((unit % p.hk) * p.g + lane) * p.s_qh);
   }
 
+  if (tid == 32) tma_prefetch_map(&tm_k);
+  if (tid == 64) tma_prefetch_map(&tm_v);
   if (tid == 0) {
     err = 0;
     for (int i = 0; i < C::NSTAGE; ++i) {
-      mbar_init(&full[i], 2);          // TMA producer (and its bytes), scale loader
+      mbar_init(&full[i], 1 + 32);     // TMA producer (and its bytes), the scale loader's lanes
       mbar_init(&empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -193,29 +219,45 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     mbar_fence_init();
   }
   __syncthreads();
-  griddep_start(p.late_wait != 0);
   // The TMA producer (warp 0) and the scale loader (warp 2) need nothing but the barriers and the
-  // stage buffers: they start streaming now, while the other warps allocate TMEM and clear the
-  // operand buffers behind a barrier of their own.
+  // stage buffers: they are the first to wait for the kernel in front, while the other warps allocate TMEM and
+  // clear the operand buffers behind a barrier of their own.
   uint32_t tmem = 0;
   if (warp != 0 && warp != 2) {
     if (warp == 1) tmem_alloc(&tmem_base_s, C::T_COLS);
     // zero the operand buffers that are only partly rewritten (rows >= G stay zero)
     const int zt = warp == 1 ? lane : (warp == 3 ? 32 + lane : tid - 64);     // 0 .. 319
-    for (int i = zt; i < (2 * (C::Q_BYTES + C::QSF_BYTES) + 2 * C::STMAX * (C::P_BYTES + C::PSF_BYTES)) / 4;
+    for (int i = zt; i < (2 * (C::Q_BYTES + C::QSF_BYTES) + 2 * C::STMAX * (C::P_BYTES + C::PSF_BYTES)) / 16;
          i += kDecodeThreads - 64)
-      reinterpret_cast<uint32_t*>(s_q)[i] = 0u;
+      reinterpret_cast<uint4*>(s_q)[i] = make_uint4(0u, 0u, 0u, 0u);
     fence_proxy_async_smem();
     tc_fence_before();
     named_bar_sync(5, kDecodeThreads - 64);
     tc_fence_after();
-    griddep_launch();
     tmem = tmem_base_s;
+    // The first tiles' boxes, likewise in front of the wait, by the softmax warps, two strips of V^T and a tile of K
+    // each: a box takes the thread that asks ~260 clocks.  Asked for by the producer in front of its first load they held
+    // it up by 5200 (D = 256 8400) of the 11700 clocks that a CTA of one round took.
+    if (warp >= 4 && my_items > 0 && elect_one()) {
+      int unit, t0, t1;
+      item_at(0, unit, t0, t1);
+      const int w = warp - 4;
+      if (t0 + w < t1) {
+#pragma unroll
+        for (int ks = 0; ks < C::KSUB; ++ks) tma_prefetch_3d(&tm_k, ks * 64, (t0 + w) * 128, unit);
+      }
+      pull(unit, t0, t1, 16 * w);
+      pull(unit, t0, t1, 16 * w + 8);
+    }
+    __syncwarp();
   }
+  griddep_start(p.late_wait != 0);
+  if (warp != 0 && warp != 2) griddep_launch();
 
   // quantise the G query rows of item `wi`'s kv head into the B operand of QK^T, buffer `qb`
   // (called by the 32 lanes of the QK^T issuer's warp, one work item ahead of the MMAs)
-  const TQ* qbase = static_cast<const TQ*>(p.q);
+  const bool q_vec = ((reinterpret_cast<uintptr_t>(qbase) | (uintptr_t)(p.s_qz * (int64_t)sizeof(TQ)) |
+                       (uintptr_t)(p.s_qh * (int64_t)sizeof(TQ))) & 15) == 0;
   auto prep_q = [&](int wi, int qb) {
     int unit_q, t0q, t1q;
     item_at(wi, unit_q, t0q, t1q);
@@ -226,8 +268,18 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       const int qr = i / (D / 16), gi = i % (D / 16);
       const TQ* src = qbase + zq * p.s_qz + (int64_t)(khq * p.g + qr) * p.s_qh + gi * 16;
       float v[16];
+      if (q_vec) {
+        constexpr int kV = sizeof(TQ);      // 16-byte loads of a group
+        uint4 raw[kV];
 #pragma unroll
-      for (int e = 0; e < 16; ++e) v[e] = to_f32<TQ>(src[e]);
+        for (int e = 0; e < kV; ++e) raw[e] = reinterpret_cast<const uint4*>(src)[e];
+        const TQ* el = reinterpret_cast<const TQ*>(raw);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = to_f32<TQ>(el[e]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = to_f32<TQ>(src[e]);
+      }
       uint32_t lo, hi;
       const uint8_t sb = pack_group16_of<TQ>(v, lo, hi);
       *reinterpret_cast<uint2*>(dq + (gi >> 3) * 1024 + sw64_offset(qr, (gi & 7) * 8)) = make_uint2(lo, hi);
@@ -246,38 +298,6 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         int unit, t0, t1;
         item_at(wi, unit, t0, t1);
         for (int t = t0; t < t1; ++t, ++it) {
-          // V^T rows are D separate strips in memory and a 128-key tile touches only 64 bytes of
-          // each; 1 KB per strip (16 tiles) is pulled into L2 one 16-tile block ahead so DRAM sees
-          // long bursts.  The pull is spread over the tiles of the block before it (8 strips per
-          // tile): a whole block at once, from every CTA in step, stalls the demand loads behind it.
-          const int j = t - t0;
-          // 8 strips (rows rows8 .. rows8+7 of every 128-row piece) of the block of <= 16 tiles that
-          // starts at tile tb and must not reach past tile te: 1 KB boxes for whole blocks, 256-byte
-          // boxes for a clipped tail, so nothing beyond the work item is read from DRAM
-          auto pull = [&](int un, int tb, int te, int rows8) {
-            const int nt = min(16, te - tb);
-            if (nt <= 0) return;
-#pragma unroll
-            for (int mt = 0; mt < C::MT; ++mt) {
-              if (nt == 16) {
-                tma_prefetch_3d(&tm_vpf, tb * 16, mt * 128 + rows8, un);
-              } else {
-                for (int q4 = 0; q4 * 4 < nt; ++q4) tma_prefetch_3d(&tm_vpf4, (tb + q4 * 4) * 16, mt * 128 + rows8, un);
-              }
-            }
-          };
-          if (j == 0 && (wi == 0 || t1 - t0 < 16)) {
-#pragma unroll 1
-            for (int r = 0; r < 16; ++r) pull(unit, t0, t1, r * 8);
-          }
-          pull(unit, t0 + ((j >> 4) + 1) * 16, t1, (j & 15) * 8);      // the next block of this item
-          // the first block of this CTA's NEXT work item, a whole item ahead: its first tiles would
-          // otherwise be 128 scattered 64-byte first touches each, ~15k clocks of DRAM latency
-          if (j < 16 && wi + 1 < my_items) {
-            int unit_n, t0n, t1n;
-            item_at(wi + 1, unit_n, t0n, t1n);
-            pull(unit_n, t0n, t1n, j * 8);
-          }
           const int s = it % C::NSTAGE;
           if (it >= (uint32_t)C::NSTAGE) mbar_spin_wait(&empty[s], ((it / C::NSTAGE) & 1) ^ 1, &err, 1);
           uint8_t* st = s_stage + s * C::STAGE_BYTES;
@@ -288,6 +308,16 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
 #pragma unroll
           for (int mt = 0; mt < C::MT; ++mt)
             tma_load_3d(st + C::K_BYTES + mt * 8192, &tm_v, &full[s], t * 64, mt * 128, unit);
+          // The pulls are spread over the tiles (8 strips each): a whole block at once, from every CTA in step, stalls
+          // the demand loads behind it.  First the next block of this item; then the first block of this CTA's NEXT
+          // work item, which would otherwise be 128 scattered 64-byte first touches a tile, ~15k clocks of DRAM latency.
+          const int j = t - t0, n16 = min(16, t1 - t0);
+          pull(unit, t0 + ((j >> 4) + 1) * 16, t1, (j & 15) * 8);
+          if (j < n16 && wi + 1 < my_items) {
+            int unit_n, t0n, t1n;
+            item_at(wi + 1, unit_n, t0n, t1n);
+            for (int r = j * 16 / n16; r < (j + 1) * 16 / n16; ++r) pull(unit_n, t0n, t1n, r * 8);
+          }
         }
       }
     }
@@ -295,16 +325,10 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   } else if (warp == 2) {
     // ------------------------------------------------------------------ scale loader
     // K and V^T scale bytes go straight from global memory into the 32 x 16-byte atoms that
-    // tcgen05.cp copies, with per-thread 4-byte cp.async (no registers, no stall on the load):
-    // the copies of tile n are issued as soon as its stage is free, and the stage is published
-    // kLag tiles later, once cp.async.wait_group says they have landed.
-    constexpr int kLag = 3;
-    uint32_t it = 0, published = 0;   // tiles [published, it) have copies in flight
-    auto publish = [&](uint32_t n) {
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&full[n % C::NSTAGE]);
-    };
+    // tcgen05.cp copies, with per-thread 4-byte cp.async (no registers, no stall on the load).  A lane's copies arrive
+    // on the stage's barrier when they have landed; who waits for it brings them to the async proxy.  (Published by this
+    // warp, three tiles behind the copies, the first round of a CTA came 1300 clocks later.)
+    uint32_t it = 0;
     for (int wi = 0; wi < my_items; ++wi) {
       int unit, t0, t1;
       item_at(wi, unit, t0, t1);
@@ -312,15 +336,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       const uint8_t* vsrc = p.vsc + (int64_t)unit * p.vsc_unit;
       for (int t = t0; t < t1; ++t, ++it) {
         const int s = it % C::NSTAGE;
-        if (it >= (uint32_t)C::NSTAGE) {
-          const uint32_t par = ((it / C::NSTAGE) & 1) ^ 1;
-          if (!mbar_test_wait(&empty[s], par)) {
-            // about to block on a full ring: publish everything in flight first
-            cp_async_wait<0>();
-            for (; published < it; ++published) publish(published);
-            mbar_wait(&empty[s], par, &err, 2);
-          }
-        }
+        if (it >= (uint32_t)C::NSTAGE) mbar_wait(&empty[s], ((it / C::NSTAGE) & 1) ^ 1, &err, 2);
         const uint32_t st = smem_u32(s_stage + s * C::STAGE_BYTES + C::K_BYTES + C::V_BYTES);
 #pragma unroll
         for (int r4 = 0; r4 < 4; ++r4) {
@@ -340,16 +356,10 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           cp_async_4_l2line(st + C::KSF_BYTES + (mt * 2 + 0) * 512 + sf_atom_offset(r, 0), g, 4u);
           cp_async_4_l2line(st + C::KSF_BYTES + (mt * 2 + 1) * 512 + sf_atom_offset(r, 0), g + 4, 4u);
         }
-        cp_async_commit();
-        if (it + 1 - published > (uint32_t)kLag) {
-          cp_async_wait<kLag>();
-          publish(published++);
-        }
+        cp_async_mbar_arrive(&full[s]);
       }
     }
-    // drain
     cp_async_wait<0>();
-    for (; published < it; ++published) publish(published);
   } else if (warp == 1) {
     // ------------------------------------------------------------------ QK^T issuer (+ query prep)
     const bool leader = elect_one();
@@ -365,38 +375,37 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       }
       int unit, t0, t1;
       item_at(wi, unit, t0, t1);
-      uint32_t it = it_w, su = su_w;        // running counters of this item
-      const int qb = item_idx & 1;
-      mbar_wait(&q_full[qb], (item_idx >> 1) & 1, &err, 6);
-      tc_fence_after();
       if (leader) {
+        uint32_t it = it_w, su = su_w;      // the leader's running counters for this item
+        const int qb = item_idx & 1;
+        mbar_wait(&q_full[qb], (item_idx >> 1) & 1, &err, 6);
+        tc_fence_after();
 #pragma unroll
         for (int k = 0; k < C::KB; ++k)
           tmem_cp_32x128b_warpx4(tmem + C::T_SFQ + qb * C::KB * 4 + k * 4,
                                  smem_u32(s_qsf + qb * C::QSF_BYTES + k * 512));
-      }
-      for (int ts0 = t0; ts0 < t1; ts0 += ST, ++su) {
-        const int b = su & 1;
-        const int nt = min(ST, t1 - ts0);
-        if (su >= 2) {
-          mbar_spin_wait(&s_free[b], ((su >> 1) & 1) ^ 1, &err, 5);
-          // the V-scale TMEM slots of buffer b are rewritten below: the PV of round su - 2 must be done
-          mbar_spin_wait(&o_full[b], ((su >> 1) & 1) ^ 1, &err, 11);
-        }
-        for (int j = 0; j < nt; ++j, ++it) {
-          const int s = it % C::NSTAGE;
-          const uint32_t ph = (it / C::NSTAGE) & 1;
-          mbar_spin_wait(&full[s], ph, &err, 3);
-          tc_fence_after();
-          uint8_t* st = s_stage + s * C::STAGE_BYTES;
-          const uint32_t sfk = tmem + C::T_SFK + (b * C::STMAX + j) * C::KB * 4;
-          // the V^T scales of this tile go to TMEM now as well, off the PV issuer's critical path
-          // (slot (b, j) was last read by the PV of round su - 2, complete before s_free fired)
-          const uint32_t sfv = tmem + C::T_SFV + (b * C::STMAX + j) * C::MT * 8;
-          if (leader) {
+        for (int ts0 = t0; ts0 < t1; ts0 += ST, ++su) {
+          const int b = su & 1;
+          const int nt = min(ST, t1 - ts0);
+          if (su >= 2) {
+            mbar_spin_wait(&s_free[b], ((su >> 1) & 1) ^ 1, &err, 5);
+            // the V-scale TMEM slots of buffer b are rewritten below: the PV of round su - 2 must be done
+            mbar_spin_wait(&o_full[b], ((su >> 1) & 1) ^ 1, &err, 11);
+          }
+          for (int j = 0; j < nt; ++j, ++it) {
+            const int s = it % C::NSTAGE;
+            const uint32_t ph = (it / C::NSTAGE) & 1;
+            mbar_spin_wait(&full[s], ph, &err, 3);
+            fence_proxy_async_smem();        // the scale bytes: written by copies of the generic proxy
+            tc_fence_after();
+            uint8_t* st = s_stage + s * C::STAGE_BYTES;
+            const uint32_t sfk = tmem + C::T_SFK + (b * C::STMAX + j) * C::KB * 4;
 #pragma unroll
             for (int k = 0; k < C::KB; ++k)
               tmem_cp_32x128b_warpx4(sfk + k * 4, smem_u32(st + C::K_BYTES + C::V_BYTES + k * 512));
+            // the V^T scales of this tile go to TMEM now as well, off the PV issuer's critical path
+            // (slot (b, j) was last read by the PV of round su - 2, complete before s_free fired)
+            const uint32_t sfv = tmem + C::T_SFV + (b * C::STMAX + j) * C::MT * 8;
 #pragma unroll
             for (int k = 0; k < C::MT * 2; ++k)
               tmem_cp_32x128b_warpx4(sfv + k * 4,
@@ -410,9 +419,8 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
                          tmem + C::T_SFQ + qb * C::KB * 4 + k * 4, k > 0);
             }
           }
-          __syncwarp();
+          umma_commit(&s_full[b]);
         }
-        if (leader) umma_commit(&s_full[b]);
       }
       it_w += (uint32_t)(t1 - t0);
       su_w += (uint32_t)((t1 - t0 + ST - 1) / ST);
@@ -420,22 +428,21 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     }
   } else if (warp == 3) {
     // ------------------------------------------------------------------ PV issuer
-    const bool leader = elect_one();
-    const uint32_t idesc = make_idesc_nvfp4(128, 16);
-    uint32_t it = 0, su = 0;
-    for (int wi = 0; wi < my_items; ++wi) {
-      int unit, t0, t1;
-      item_at(wi, unit, t0, t1);
-      for (int ts0 = t0; ts0 < t1; ts0 += ST, ++su) {
-        const int b = su & 1;
-        const int nt = min(ST, t1 - ts0);
-        mbar_spin_wait(&p_full[b], (su >> 1) & 1, &err, 7);
-        tc_fence_after();
-        if (leader) {
-          for (int j = 0; j < nt; ++j) {
+    if (elect_one()) {
+      const uint32_t idesc = make_idesc_nvfp4(128, 16);
+      uint32_t it = 0, su = 0;
+      for (int wi = 0; wi < my_items; ++wi) {
+        int unit, t0, t1;
+        item_at(wi, unit, t0, t1);
+        for (int ts0 = t0; ts0 < t1; ts0 += ST, ++su) {
+          const int b = su & 1;
+          const int nt = min(ST, t1 - ts0);
+          mbar_spin_wait(&p_full[b], (su >> 1) & 1, &err, 7);
+          tc_fence_after();
+          for (int j = 0; j < nt; ++j, ++it) {
             // V^T tile and scales of stage s were observed by the QK^T issuer before S^T of this
             // round was produced, and P arrived after the softmax warps saw that S^T
-            const int s = (it + j) % C::NSTAGE;
+            const int s = it % C::NSTAGE;
             uint8_t* st = s_stage + s * C::STAGE_BYTES;
             const uint32_t sfv = tmem + C::T_SFV + (b * C::STMAX + j) * C::MT * 8;
             const uint32_t sfp = tmem + C::T_SFP + (b * C::STMAX + j) * 8;
@@ -459,8 +466,6 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           }
           umma_commit(&o_full[b]);
         }
-        __syncwarp();
-        it += nt;
       }
     }
     __syncwarp();
