@@ -134,16 +134,6 @@ struct StepCursor {
 // rank adds up 128 / n rows over the cluster, in rank order (results do not depend on timing).
 constexpr int kRedStride = 260;        // floats per row: 256 columns, padded so that 16-byte row accesses spread over the banks
 
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t saddr, uint32_t rank) {
-  uint32_t a;
-  float4 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
-}
 // 32 accumulator columns of one row into the reduction buffer
 __device__ __forceinline__ void red_store32(uint32_t buf, int row, int col, const uint32_t (&r)[32]) {
   const uint32_t a = buf + (uint32_t)(row * kRedStride + col) * 4u;

@@ -89,32 +89,34 @@ inline void prefer_l1(const void* kern) {
   if (kernel_attribute<cudaFuncAttributePreferredSharedMemoryCarveout>(kern, kStreamSmem) != cudaSuccess) cudaGetLastError();
 }
 
-// Clusters of 1, 2, 4 and 8 CTAs of a kernel that are resident at once, asked once per device: for kernels that leave
+// Clusters of `size` CTAs (1 to 8) of a kernel that are resident at once, asked once per device: for kernels that leave
 // room for one CTA per SM only (the answer depends on that alone).  allow_smem() has been called for `kern`.
-inline void cluster_slots(const void* kern, unsigned threads, int smem, int sms, int (&slots)[4]) {
-  static std::atomic<int> known[64][4];
+inline int cluster_slots(const void* kern, unsigned threads, int smem, int sms, int size) {
+  static std::atomic<int> known[64][9];
   int dev = 0;
   const bool keep = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
-  for (int i = 0; i < 4; ++i) {
-    slots[i] = keep ? known[dev][i].load(std::memory_order_relaxed) : 0;
-    if (slots[i] > 0) continue;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1u << i;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1, 1, 1u << i);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&slots[i], kern, &cfg) != cudaSuccess || slots[i] < 1) {
-      cudaGetLastError();
-      slots[i] = sms >> i;
-    } else if (keep) {
-      known[dev][i].store(slots[i], std::memory_order_relaxed);
-    }
+  int n = keep ? known[dev][size].load(std::memory_order_relaxed) : 0;
+  if (n > 0) return n;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = size;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, 1, size);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    return sms / size;
   }
+  if (keep) known[dev][size].store(n, std::memory_order_relaxed);
+  return n;
+}
+// the same for 1, 2, 4 and 8
+inline void cluster_slots(const void* kern, unsigned threads, int smem, int sms, int (&slots)[4]) {
+  for (int i = 0; i < 4; ++i) slots[i] = cluster_slots(kern, threads, smem, sms, 1 << i);
 }
 
 // Launch with programmatic stream serialisation; launch_cluster: clusters of `cluster` CTAs along z.

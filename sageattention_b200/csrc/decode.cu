@@ -9,8 +9,9 @@
 //     O^T[D x 16]       += V^T_tile[D x 128] . P^T          (A = V^T tile, B = P packed along keys)
 // Scale bytes are re-laid into the 32x16-byte form tcgen05.cp expects by a loader warp.
 // Softmax runs with one thread per key (TMEM lane); P is packed to NVFP4 per 16 keys with the
-// same scale rule as the packer.  Each work item writes un-normalised (acc, m, l) partials; a
-// second small kernel combines them exactly and emits the output and its log-sum-exp.
+// same scale rule as the packer.  Each work item leaves un-normalised (acc, m, l) partials; the cluster
+// that has all items of a unit, or a second small kernel, combines them exactly and emits the output and its
+// log-sum-exp.
 //
 // Warp roles (384 threads): 0 TMA producer, 1 QK^T issuer, 2 scale loader, 3 PV issuer,
 // 4-11 softmax / accumulate / epilogue (two groups splitting each round's tiles).  Every barrier
@@ -97,6 +98,8 @@ struct DecodeParams {
   float* ws_l;    // [nitems][16]
   int64_t extra_base;   // first of the partial slots appended by another kernel (n_extra per unit)
   int n_extra;
+  void* out;            // kMerge: the result itself, [units * g][D], and its log-sum-exp or null
+  float* lse;
   int late_wait;        // behind the window kernel: wait for it at the end, not at the start (launch.cuh)
   int* status;
 };
@@ -108,7 +111,10 @@ struct DecodeParams {
 // tile's P.V goes to a FRESH O^T accumulator in TMEM.  The softmax threads (one per head-dim
 // row in this role) fold those ST accumulators into registers one round later with the exact
 // weights exp(m_tile - m_now), so O is never rescaled in TMEM.
-template <int D, typename TQ, int NQ>
+//
+// kMerge: a CTA has one item, and the CTAs of a cluster (along z) have all items of one unit.  They merge their partials
+// through distributed shared memory, a share of the elements each, and write the result: no combine kernel.
+template <int D, typename TQ, int NQ, bool kMerge>
 __global__ void __launch_bounds__(kDecodeThreads, 1)
 decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
               const __grid_constant__ CUtensorMap tm_vpf, const __grid_constant__ CUtensorMap tm_vpf4,
@@ -134,29 +140,32 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   __shared__ int err;
   __shared__ float xch[C::STMAX][16];      // tile maxima of the current round, per head
   __shared__ float lred[C::STMAX][16];     // row sums at the end of an item, per tile slot and head
+  __shared__ __align__(16) float part_ml[kMerge ? 32 : 4];     // kMerge: maxima and sums of the item's heads
+  __shared__ float part_w[kMerge ? 9 : 1][kMerge ? 16 : 1];    // weights of the cluster's partials, and their common divisor
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
 
   // work items of this CTA: i = 0 .. my_items-1
-  const int64_t nctas = gridDim.x;
+  const uint32_t cta = kMerge ? blockIdx.z : blockIdx.x;
+  const int64_t nctas = kMerge ? gridDim.z : gridDim.x;
   int64_t bal_start = 0, bal_end = 0;
   int bal_u0 = 0, my_items = 0;
-  if (p.balanced) {
-    bal_start = (int64_t)blockIdx.x * p.total_tiles / nctas;
-    bal_end = (int64_t)(blockIdx.x + 1) * p.total_tiles / nctas;
+  if (!kMerge && p.balanced) {
+    bal_start = (int64_t)cta * p.total_tiles / nctas;
+    bal_end = (int64_t)(cta + 1) * p.total_tiles / nctas;
     bal_u0 = (int)(bal_start / p.ntiles);
     my_items = bal_end > bal_start ? (int)((bal_end - 1) / p.ntiles) - bal_u0 + 1 : 0;
-  } else if ((int64_t)blockIdx.x < p.nitems) {
-    my_items = (int)((p.nitems - blockIdx.x + nctas - 1) / nctas);
+  } else if ((int64_t)cta < p.nitems) {
+    my_items = (int)((p.nitems - cta + nctas - 1) / nctas);
   }
   auto item_at = [&](int i, int& unit, int& t0, int& t1) {
-    if (p.balanced) {
+    if (!kMerge && p.balanced) {
       unit = bal_u0 + i;
       const int64_t base = (int64_t)unit * p.ntiles;
       t0 = (int)(max(bal_start, base) - base);
       t1 = (int)(min(bal_end, base + p.ntiles) - base);
     } else {
-      const uint32_t w = blockIdx.x + (uint32_t)i * gridDim.x;      // below 2^31, as the number of items
+      const uint32_t w = cta + (uint32_t)i * (uint32_t)nctas;      // below 2^31, as the number of items
       unit = (int)(w / (uint32_t)p.nsplit);
       const int split = (int)(w - (uint32_t)unit * (uint32_t)p.nsplit);
       t0 = split * p.chunk_tiles;
@@ -164,7 +173,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     }
   };
   auto slot_at = [&](int i) -> int64_t {
-    return p.balanced ? (int64_t)blockIdx.x * p.maxseg + i : blockIdx.x + (int64_t)i * nctas;
+    return p.balanced ? (int64_t)cta * p.maxseg + i : cta + (int64_t)i * nctas;
   };
 
   // V^T rows are D separate strips in memory and a 128-key tile touches only 64 bytes of each; 1 KB per strip (16
@@ -699,8 +708,8 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         }
         named_bar_sync(1, 256);
         if (grp == 0) {
-          const int64_t w = slot_at(wi);
-          float* acc = p.ws_acc + w * 16 * D;
+          const int64_t w = kMerge ? 0 : slot_at(wi);
+          float* acc = kMerge ? s_merge : p.ws_acc + w * 16 * D;
 #pragma unroll
           for (int mt = 0; mt < C::MT; ++mt)
 #pragma unroll
@@ -715,8 +724,8 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
                 for (int ww = 0; ww < ST; ++ww) lsum += lred[ww][qi];
                 mfin = m_run[qi];
               }
-            p.ws_m[w * 16 + ts] = mfin;
-            p.ws_l[w * 16 + ts] = lsum;
+            (kMerge ? part_ml : p.ws_m + w * 16)[ts] = mfin;
+            (kMerge ? part_ml + 16 : p.ws_l + w * 16)[ts] = lsum;
           }
         }
         // no barrier here: the merge buffer (= the P tiles) and lred are next written after the
@@ -724,6 +733,57 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
         // program order; the kernel's final __syncthreads covers the last item
       }
     }
+  }
+  if constexpr (kMerge) {
+    tc_fence_before();
+    const uint32_t ncl = (uint32_t)p.nsplit, rank = cta % ncl;
+    const int unit = (int)(cta / ncl);
+    cluster_sync_all();                  // the partials of all CTAs are there
+    if (tid < p.g) {
+      float m[8], l[8], gm = -INFINITY, den = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        m[k] = (uint32_t)k < ncl ? ld_cluster_f32(smem_u32(&part_ml[tid]), k) : -INFINITY;
+        l[k] = (uint32_t)k < ncl ? ld_cluster_f32(smem_u32(&part_ml[16 + tid]), k) : 0.0f;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) gm = fmaxf(gm, m[k]);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float f = (m[k] == -INFINITY) ? 0.0f : expf(m[k] - gm);
+        part_w[k][tid] = f;
+        den += f * l[k];
+      }
+      if (den == 0.0f) den = 1.0f;
+      part_w[8][tid] = den;
+      if (p.lse != nullptr && rank == 0) p.lse[(int64_t)unit * p.g + tid] = gm + logf(den);
+    }
+    __syncthreads();
+    const uint32_t n4 = (uint32_t)p.g * (D / 4), acc0 = smem_u32(s_merge);
+    TQ* out = static_cast<TQ*>(p.out) + (int64_t)unit * p.g * D;
+    const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    for (uint32_t i = n4 * rank / ncl + tid; i < n4 * (rank + 1) / ncl; i += kDecodeThreads) {
+      const uint32_t qi = i / (D / 4);
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if ((uint32_t)k < ncl) {
+          const float4 x = ld_cluster_f4(acc0 + i * 16, k);
+          const float f = part_w[k][qi];
+          v.x = fmaf(f, x.x, v.x); v.y = fmaf(f, x.y, v.y); v.z = fmaf(f, x.z, v.z); v.w = fmaf(f, x.w, v.w);
+        }
+      const float den = part_w[8][qi];
+      v = make_float4(v.x / den, v.y / den, v.z / den, v.w / den);
+      if (!vec) {
+        out[4 * i] = from_f32<TQ>(v.x); out[4 * i + 1] = from_f32<TQ>(v.y);
+        out[4 * i + 2] = from_f32<TQ>(v.z); out[4 * i + 3] = from_f32<TQ>(v.w);
+      } else if constexpr (sizeof(TQ) == 2) {
+        *reinterpret_cast<uint2*>(out + 4 * i) = make_uint2(pack_16x2<TQ>(v.x, v.y), pack_16x2<TQ>(v.z, v.w));
+      } else {
+        *reinterpret_cast<float4*>(out + 4 * i) = v;
+      }
+    }
+    cluster_sync_all();                  // nobody's partials are read any more
   }
   tc_fence_before();
   __syncthreads();
@@ -857,15 +917,28 @@ int decode_launch(const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtens
     int ms;
     decode_balanced_geometry(zhk, p.ntiles, sm_count, &grid, &ms);
   }
-  auto launch = [&](auto kern) -> int {
+  // Up to eight items a unit, each with a CTA of its own: a cluster merges them (one item: a cluster of one), if all clusters
+  // are resident at once (74, 33 and 15 of two, four and eight; a second wave costs more than the combine's launch).
+  // A step of append and decode: 16.2 -> 14.0 us of host time at any of these sizes (one launch less); its graph, us: Z1 Hk8 S256
+  // (one item a unit) 9.4 -> 8.0, S1021 (two) 11.7 -> 11.1, S4000 (eight) 10.6 -> 9.9, Z8 S900 12.1 -> 10.8, D 256 Z1 Hk4
+  // S3000 (six) 13.2 -> 12.7.
+  bool merge = !p.balanced && p.n_extra == 0 && p.nsplit <= 8 && p.nitems == grid;
+  auto launch = [&](auto kern, auto kmerge) -> int {
+    if (merge) {
+      if (int rc = allow_smem("nvfp4_decode", reinterpret_cast<const void*>(kmerge), C::SMEM_BYTES)) return rc;
+      merge = zhk <= cluster_slots(reinterpret_cast<const void*>(kmerge), kDecodeThreads, C::SMEM_BYTES, sm_count, p.nsplit);
+    }
+    if (merge)
+      return nvfp4::launch_cluster("nvfp4_decode", kmerge, dim3(1, 1, grid), p.nsplit, kDecodeThreads, C::SMEM_BYTES, st, tm_k,
+                                   tm_v, tm_vpf, tm_vpf4, p);
     if (int rc = allow_smem("nvfp4_decode", reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return rc;
     return nvfp4::launch("nvfp4_decode", kern, dim3(grid), kDecodeThreads, C::SMEM_BYTES, st, tm_k, tm_v, tm_vpf, tm_vpf4, p);
   };
   int rc;
-  if (p.g <= 4) rc = launch(decode_kernel<D, TQ, 4>);
-  else if (p.g <= 8) rc = launch(decode_kernel<D, TQ, 8>);
-  else rc = launch(decode_kernel<D, TQ, 16>);
-  if (rc) return rc;
+  if (p.g <= 4) rc = launch(decode_kernel<D, TQ, 4, false>, decode_kernel<D, TQ, 4, true>);
+  else if (p.g <= 8) rc = launch(decode_kernel<D, TQ, 8, false>, decode_kernel<D, TQ, 8, true>);
+  else rc = launch(decode_kernel<D, TQ, 16, false>, decode_kernel<D, TQ, 16, true>);
+  if (rc || merge) return rc;
   CombineArgs c;
   c.ws_acc = p.ws_acc; c.ws_m = p.ws_m; c.ws_l = p.ws_l;
   c.nsplit = p.balanced ? 0 : p.nsplit;
@@ -1031,6 +1104,8 @@ static int decode_call(const void* q, int q_dtype, int64_t s_qz, int64_t s_qh, c
   p.ws_l = p.ws_m + slots * 16;
   p.extra_base = own_slots;
   p.n_extra = n_extra;
+  p.out = out;
+  p.lse = lse;
   p.late_wait = window != nullptr ? 1 : 0;
   p.status = status;
   if (window != nullptr) {
