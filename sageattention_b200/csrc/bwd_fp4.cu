@@ -75,8 +75,9 @@ struct B4Cfg {
   static constexpr int RES = ((O_ASF2 + (kDs ? 1024 : 0) + 1023) / 1024) * 1024;
   // one stage = 128 columns
   static constexpr int S_Y1 = 0, S_Y2 = X, S_T1 = S_Y2 + (kDs ? X : 0), S_T2 = S_T1 + (kP ? TB : 0);
-  static constexpr int S_YSF = S_T2 + (kDs ? TB : 0);     // Y1 atoms [2 steps][KB], then Y2 atoms [2][KB]
-  static constexpr int S_TSF1 = S_YSF + (kDs ? 4 : 2) * KB * 512;     // T1 atoms [2 parities][NW] (MXFP8: [NW])
+  // atoms [2 steps][KB]: rows 0-63 the 64 columns of the step of Y1, rows 64-127 those of Y2
+  static constexpr int S_YSF = S_T2 + (kDs ? TB : 0);
+  static constexpr int S_TSF1 = S_YSF + 2 * KB * 512;     // T1 atoms [2 parities][NW] (MXFP8: [NW])
   static constexpr int S_TSF2 = S_TSF1 + (kP ? 2 * NW * 512 : 0);
   static constexpr int S_AUX = S_TSF2 + (kDs ? 2 * NW * 512 : 0);     // two float[128]
   static constexpr int STAGE = ((S_AUX + 1024 + 1023) / 1024) * 1024;
@@ -490,8 +491,9 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
         for (int k = 0; k < C::KB; ++k)
 #pragma unroll
           for (int pp = 0; pp < 2; ++pp) {
-            sts_v2(at + C::S_YSF + (pp * C::KB + k) * 512, y1[2 * pp][k], y1[2 * pp + 1][k]);
-            if constexpr (kDs) sts_v2(at + C::S_YSF + ((2 + pp) * C::KB + k) * 512, y2[2 * pp][k], y2[2 * pp + 1][k]);
+            const uint32_t a = at + C::S_YSF + (pp * C::KB + k) * 512;
+            if constexpr (kDs) sts_v4(a, y1[2 * pp][k], y1[2 * pp + 1][k], y2[2 * pp][k], y2[2 * pp + 1][k]);
+            else sts_v2(a, y1[2 * pp][k], y1[2 * pp + 1][k]);
           }
 #pragma unroll
         for (int nw = 0; nw < C::NW; ++nw)
@@ -540,10 +542,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
         const int pp = st & 1, sg = st >> 1, s = sg % C::NSTAGE;
         uint8_t* sb = s_stage + s * C::STAGE;
         if (pp == 0) mbar_wait(&full[s], (sg / C::NSTAGE) & 1, &err, 5);
-        // S slot: read by the team of step st - 2; the one dP slot: by that of step st - 1
-        if (kDs && st >= 2) mbar_wait_all(&s_free[pp], ((st >> 1) - 1) & 1, &g_free, (st - 1) & 1, &err, 7);
-        else if (kDs && st > 0) mbar_wait(&g_free, (st - 1) & 1, &err, 9);
-        else if (st >= 2) mbar_wait(&s_free[pp], ((st >> 1) - 1) & 1, &err, 7);
+        if (st >= 2) mbar_wait(&s_free[pp], ((st >> 1) - 1) & 1, &err, 7);      // S slot: read by the team of step st - 2
         tc_fence_after();
         const uint64_t so = (uint64_t)(s * (C::STAGE >> 4)) + (uint64_t)(pp * 256);   // 64 rows x 64 bytes further
         if (leader) {
@@ -555,18 +554,25 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
           for (int k = 0; k < C::KB; ++k)
             umma_nvfp4(tmem + C::T_S + pp * 64, d_x1 + (k >> 1) * 512 + (k & 1) * 2, d_y1 + so + (k >> 1) * 512 + (k & 1) * 2,
                        id_n64, tmem + C::T_SFX1 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
-          if constexpr (kDs) {
+        }
+        if constexpr (kDs) {
+          // The one dP slot is read by the team of step st - 1.  Only dP waits for it: S and both scales are under way
+          // meanwhile.  With both behind this wait the slot's round trip was the step of the dQ pass at D = 256
+          // (1270 clocks of which 850 the next team's wait).  Both scales come with one copy a block of D: S8192 D128
+          // 1427 -> 1381 us in all, S4100 D256 385 -> 373, S8192 D256 1170 -> 1140.
+          if (st > 0) {
+            mbar_wait(&g_free, (st - 1) & 1, &err, 9);
+            tc_fence_after();
+          }
+          if (leader) {
             // dP (or dP^T)
-#pragma unroll
-            for (int c = 0; c < C::KB; ++c)
-              tmem_cp_32x128b_warpx4(tmem + C::T_SFY + 4 * c, smem_u32(sb + C::S_YSF + ((2 + pp) * C::KB + c) * 512));
 #pragma unroll
             for (int k = 0; k < C::KB; ++k)
               umma_nvfp4(tmem + C::T_G, d_x2 + (k >> 1) * 512 + (k & 1) * 2, d_y2 + so + (k >> 1) * 512 + (k & 1) * 2,
-                         id_n64, tmem + C::T_SFX2 + k * 4, tmem + C::T_SFY + k * 4, k > 0);
+                         id_n64, tmem + C::T_SFX2 + k * 4, tmem + C::T_SFY + k * 4 + 2, k > 0);
           }
-          umma_commit(&s_full[pp]);
         }
+        if (leader) umma_commit(&s_full[pp]);
         __syncwarp();
       }
     }
