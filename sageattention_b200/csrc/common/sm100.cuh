@@ -287,6 +287,10 @@ __device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* m, int c0, in
                "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
+// a run of bytes; address and size are multiples of 16
+__device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
