@@ -246,7 +246,17 @@ __global__ void __launch_bounds__(256, 2) rope_pack_rows_kernel(
 // ---------------------------------------------------------------- rows contiguous (V^T)
 constexpr int kColsKeys = 128;  // contraction extent of a tile
 constexpr int kColsRows = 64;   // row (head-dim) extent of a tile
-constexpr int kColsRun = 4;     // consecutive key tiles one block walks (the next tile's loads fly under the pack)
+// Consecutive key tiles one block walks, the next tile's loads under the present one's pack: four where that leaves two
+// rounds of three blocks an SM, fewer for smaller problems, whose time is that of one block.  V^T of [2, 777, 128] 3.7 -> 1.8 us,
+// [8, 4096, 128] 5.6 -> 3.5, [32, 2048, 128] 7.3 -> 5.4, [8, 16384, 128] (2048 tiles) 10.9 -> 10.5; one tile a block everywhere:
+// [32, 8192, 128] (4096 tiles) 18.7 -> 21.1.
+constexpr int kColsRun = 4;
+constexpr int kColsBlocks = 888;
+inline int cols_run(int64_t tiles) {
+  int run = kColsRun;
+  while (run > 1 && tiles < (int64_t)run * kColsBlocks) run >>= 1;
+  return run;
+}
 
 // The input tile: fp32 inputs as floats (one padding column); 16-bit inputs as loaded, two rows per
 // 32-bit word, 144-byte key rows (16-byte aligned, and a quarter warp's 16-byte accesses to
@@ -508,13 +518,13 @@ __global__ void __launch_bounds__(256, 3) pack_cols_kernel(
     uint8_t* __restrict__ nib, int64_t snb, int64_t snr, uint8_t* __restrict__ sc, int64_t ssb,
     int64_t ssr, int vec_in, uint8_t* __restrict__ dnib, int64_t dnb, int64_t dnr,
     uint8_t* __restrict__ dsc, int64_t dsb, int64_t dsr, const float* __restrict__ prescale_amax,
-    int sr_flags, uint32_t seed) {
+    int sr_flags, uint32_t seed, int run) {
   __shared__ ColsSmem<T> sm;
   griddep_launch();
   griddep_wait();
-  const int64_t tx = (k_pad + kColsKeys - 1) / kColsKeys, bx = (int64_t)blockIdx.x * kColsRun;
+  const int64_t tx = (k_pad + kColsKeys - 1) / kColsKeys, bx = (int64_t)blockIdx.x * run;
   pack_cols_tile<T, kDual>(sm, x, R, k_read, k_pad, sxb, sxk, nib, snb, snr, sc, ssb, ssr, vec_in, bx,
-                           (int)(tx - bx < kColsRun ? tx - bx : kColsRun), blockIdx.y, blockIdx.z, dnib, dnb, dnr,
+                           (int)(tx - bx < run ? tx - bx : run), blockIdx.y, blockIdx.z, dnib, dnb, dnr,
                            dsc, dsb, dsr, prescale_amax, sr_flags, seed);
 }
 
@@ -610,6 +620,7 @@ struct QkvArgs {
   int64_t bpq, bpk;          // 256-thread blocks per batch entry
   int64_t nbq, nbk;          // blocks of the Q and K parts
   int64_t s_kv, s_pad, tx, ty;            // V: keys, padded keys, tiles along keys / along D
+  int run;
   uint8_t *qnv, *qsc, *knv, *ksc, *vnv, *vsc;
 };
 
@@ -648,14 +659,14 @@ __global__ void __launch_bounds__(256, 3) pack_qkv_kernel(const QkvArgs a) {
     return;
   }
   const int64_t w = v - a.nbq - a.nbk;
-  const int64_t runs = (a.tx + kColsRun - 1) / kColsRun;      // runs of key tiles per row of tiles
+  const int64_t runs = (a.tx + a.run - 1) / a.run;            // runs of key tiles per row of tiles
   const int64_t per = runs * a.ty;
   const int64_t b = w / per;
   const int64_t rem = w - b * per;
-  const int64_t by = rem / runs, bx = (rem - by * runs) * kColsRun;
+  const int64_t by = rem / runs, bx = (rem - by * runs) * a.run;
   pack_cols_tile<T, false>(sm, static_cast<const T*>(a.v), a.d, a.s_kv, a.s_pad, a.svb, a.svk, a.vnv,
                            (int64_t)a.d * (a.s_pad / 2), a.s_pad / 2, a.vsc, (int64_t)a.d * (a.s_pad / 16),
-                           a.s_pad / 16, a.vec_v, bx, (int)(a.tx - bx < kColsRun ? a.tx - bx : kColsRun), by, b,
+                           a.s_pad / 16, a.vec_v, bx, (int)(a.tx - bx < a.run ? a.tx - bx : a.run), by, b,
                            nullptr, 0, 0, nullptr, 0, 0, nullptr);
 }
 
@@ -675,6 +686,7 @@ struct PrefillArgs {
   void *partial, *rk, *rv;          // [unit][16][d]; rings [unit][ring_cap][d] or null
   int64_t ring_cap, ring_n;         // the last ring_n tokens go to the rings
   int64_t bpk, nbk, s_pad, tx, ty, nbv, bpc;
+  int run;
 };
 
 constexpr int kPrefillCopyIters = 8;   // 16-byte pieces per thread of a copy block
@@ -704,11 +716,11 @@ __global__ void __launch_bounds__(256, 3) kv_prefill_kernel(const PrefillArgs a)
   }
   if (blk < a.nbk + a.nbv) {
     const int64_t w = blk - a.nbk;
-    const int64_t runs = (a.tx + kColsRun - 1) / kColsRun, per = runs * a.ty;
+    const int64_t runs = (a.tx + a.run - 1) / a.run, per = runs * a.ty;
     const int64_t b = w / per, rem = w - b * per;
-    const int64_t by = rem / runs, bx = (rem - by * runs) * kColsRun;
+    const int64_t by = rem / runs, bx = (rem - by * runs) * a.run;
     pack_cols_tile<T, false>(sm, static_cast<const T*>(a.v), a.d, a.s, a.s_pad, a.svb, a.svr, a.vnv, a.vnv_unit, a.vnv_row,
-                             a.vsc, a.vsc_unit, a.vsc_row, a.vec_v, bx, (int)(a.tx - bx < kColsRun ? a.tx - bx : kColsRun),
+                             a.vsc, a.vsc_unit, a.vsc_row, a.vec_v, bx, (int)(a.tx - bx < a.run ? a.tx - bx : a.run),
                              by, b, nullptr, 0, 0, nullptr, 0, 0, nullptr);
     return;
   }
@@ -805,10 +817,11 @@ int pack_dispatch(const T* x, int64_t B, int64_t R, int64_t k_read, int64_t k_pa
   }
   if (sxr == 1 && B < 65536 && (R + kColsRows - 1) / kColsRows < 65536) {
     const int vec = base_ok && sxb % kVecElems == 0 && sxk % kVecElems == 0;
-    dim3 grid((unsigned)((k_pad + kColsKeys * kColsRun - 1) / (kColsKeys * kColsRun)),
-              (unsigned)((R + kColsRows - 1) / kColsRows), (unsigned)B);
+    const int64_t tx = (k_pad + kColsKeys - 1) / kColsKeys, ty = (R + kColsRows - 1) / kColsRows;
+    const int run = cols_run(tx * ty * B);
+    dim3 grid((unsigned)((tx + run - 1) / run), (unsigned)ty, (unsigned)B);
     return launch_streaming("nvfp4_pack(cols)", pack_cols_kernel<T, false>, grid, 256, 0, st, x, R, k_read, k_pad, sxb, sxk, nib, snb,
-                  snr, sc, ssb, ssr, vec, nullptr, 0, 0, nullptr, 0, 0, nullptr, 0, 0u);
+                  snr, sc, ssb, ssr, vec, nullptr, 0, 0, nullptr, 0, 0, nullptr, 0, 0u, run);
   }
   const int64_t blocks = (total + 255) / 256;
   NVFP4_REQUIRE(blocks < (1LL << 31), "nvfp4_pack: tensor too large");
@@ -852,12 +865,13 @@ int pack_dual_launch(const void* x, int64_t B, int64_t S, int d, int64_t s_pad, 
                      uint8_t* tnib, uint8_t* tsc, cudaStream_t st) {
   constexpr int64_t kVecElems = 16 / sizeof(T);
   const int vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && sxb % kVecElems == 0 && sxs % kVecElems == 0;
-  dim3 grid((unsigned)((s_pad + kColsKeys * kColsRun - 1) / (kColsKeys * kColsRun)),
-            (unsigned)((d + kColsRows - 1) / kColsRows), (unsigned)B);
+  const int64_t tx = (s_pad + kColsKeys - 1) / kColsKeys, ty = (d + kColsRows - 1) / kColsRows;
+  const int run = cols_run(tx * ty * B);
+  dim3 grid((unsigned)((tx + run - 1) / run), (unsigned)ty, (unsigned)B);
   return launch_streaming(
       "nvfp4_pack_dual", pack_cols_kernel<T, true>, grid, 256, 0, st, static_cast<const T*>(x), d, S, s_pad, sxb, sxs, tnib, (int64_t)d * (s_pad / 2), s_pad / 2, tsc,
       (int64_t)d * (s_pad / 16), s_pad / 16, vec, dnib, S * (int64_t)(d / 2), d / 2, dsc, S * (int64_t)(d / 16),
-      d / 16, prescale_amax, sr_flags, seed);
+      d / 16, prescale_amax, sr_flags, seed, run);
 }
 
 template <typename T>
@@ -881,7 +895,8 @@ int pack_qkv_launch(QkvArgs a, cudaStream_t st) {
   a.bpk = (a.rk * ng + (a.quad_k ? 1023 : 255)) / (a.quad_k ? 1024 : 256);
   a.nbq = a.bpq * a.bq;
   a.nbk = a.bpk * a.bk;
-  const int64_t total = a.nbq + a.nbk + a.bk * ((a.tx + kColsRun - 1) / kColsRun) * a.ty;
+  a.run = cols_run(a.bk * a.tx * a.ty);
+  const int64_t total = a.nbq + a.nbk + a.bk * ((a.tx + a.run - 1) / a.run) * a.ty;
   NVFP4_REQUIRE(total < (1LL << 31), "nvfp4_pack_qkv: tensors too large");
   return launch_streaming("nvfp4_pack_qkv", pack_qkv_kernel<T>, dim3((unsigned)total), 256, 0, st, a);
 }
@@ -902,7 +917,8 @@ int kv_prefill_launch(PrefillArgs a, cudaStream_t st) {
   a.nbk = a.bpk * a.zhk;
   a.tx = (a.s_pad + kColsKeys - 1) / kColsKeys;
   a.ty = (a.d + kColsRows - 1) / kColsRows;
-  a.nbv = a.zhk * ((a.tx + kColsRun - 1) / kColsRun) * a.ty;
+  a.run = cols_run(a.zhk * a.tx * a.ty);
+  a.nbv = a.zhk * ((a.tx + a.run - 1) / a.run) * a.ty;
   const int64_t pieces = (16 + (a.rk != nullptr ? 2 * a.ring_n : 0)) * (a.d / kVecElems);
   a.bpc = (pieces + 256 * kPrefillCopyIters - 1) / (256 * kPrefillCopyIters);
   const int64_t total = a.nbk + a.nbv + a.bpc * a.zhk;
