@@ -32,9 +32,9 @@
 // one for the P buffer stands behind the first exponentials; at D = 128 the 32 columns read last for the
 // maxima are the first to be exponentiated, without another read; reciprocal scales come from a table in
 // shared memory, not from the pipe that ex2 needs; P leaves in 16-byte stores.
-// Measured on a B200, kernel alone, causal bf16, against one CTA per query tile: Z4 H32 Hk8 S8192 D128 2033 -> 1695 us
-// (1.30 PFLOP/s), Z1 S4096 150 -> 119, S2048 51.6 -> 37.7, eight samples in 16384 tokens 403 -> 271; H16 Hk4 D256
-// S8192 334 -> 297, S2048 33.2 -> 28.5.
+// Measured on a B200, kernel alone, causal bf16, against one CTA per query tile and, the last figure, with uniform registers
+// for addresses, six stages and whole scale rows: Z4 H32 Hk8 S8192 D128 2033 -> 1695 -> 1576 us (1.40 PFLOP/s), Z1 S2048
+// 51.6 -> 37.7 -> 34.0; H16 Hk4 D256 S8192 334 -> 297 -> 270, S2048 33.2 -> 28.5 -> 25.7.
 // Masks: only tiles at an edge of what a row may see -- diagonal, ragged end, ends of a packed sample -- and
 // tiles whose bias has a value other than zero (added already divided by the scaling) are edited, in tensor memory
 // before the maxima are taken, by bits of a 32-column word formed from the row's range; the loop over the others holds
@@ -107,6 +107,7 @@ struct FwdParams {
   float scaling;
   int causal;
   int tma_out;         // tm_o describes out
+  int vec_sc;          // scale rows of Q and K are aligned to their size
   int* status;
 };
 
@@ -363,37 +364,40 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       uint32_t qx[4][C::KB], kx[4][C::KB];
       float nb[4];
       uint2 vx[D / 32];
+      // The D / 16 scale bytes of a row: one load where rows are aligned to them, else words.  This warp's instructions are
+      // taken from the softmax warps of its scheduler, which the others wait for (a fifth longer in their exponentials): one
+      // load a row and one store of four rows an atom, S8192 H16 D256 278 -> 270 us, Z4 S8192 D128 1582 -> 1576.
+      auto row_scales = [&](const uint8_t* src, uint32_t (&x)[C::KB]) {
+        if (!p.vec_sc) {
+#pragma unroll
+          for (int k = 0; k < C::KB; ++k) x[k] = __ldg(reinterpret_cast<const uint32_t*>(src) + k);
+        } else if constexpr (C::KB == 2) {
+          const uint2 v = __ldg(reinterpret_cast<const uint2*>(src));
+          x[0] = v.x; x[1] = v.y;
+        } else {
+          const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+          x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+        }
+      };
+      // Keys behind the last one take its scales: their scores are masked.
       auto fetch = [&](int first) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int key = first + lane + 32 * j;
-#pragma unroll
-          for (int k = 0; k < C::KB; ++k) kx[j][k] = 0u;
-          nb[j] = 0.0f;
-          if (key < p.s_kv) {
-            const uint32_t* gsrc = reinterpret_cast<const uint32_t*>(ksrc + (int64_t)key * (D / 16));
-#pragma unroll
-            for (int k = 0; k < C::KB; ++k) kx[j][k] = __ldg(gsrc + k);
-            if (kBias) nb[j] = __ldg(p.bias + (int64_t)zi * p.s_kv + key) * inv_scaling;
-          }
+          const int key = min(first + lane + 32 * j, p.s_kv - 1);
+          row_scales(ksrc + (int64_t)key * (D / 16), kx[j]);
+          if (kBias) nb[j] = first + lane + 32 * j < p.s_kv ? __ldg(p.bias + (int64_t)zi * p.s_kv + key) * inv_scaling : 0.0f;
         }
 #pragma unroll
         for (int j = 0; j < D / 32; ++j)
           vx[j] = __ldg(reinterpret_cast<const uint2*>(vsrc + (int64_t)(lane + 32 * j) * (p.s_pad / 16) + (first >> 4)));
       };
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int row = m0 + lane + 32 * j;
-#pragma unroll
-        for (int k = 0; k < C::KB; ++k)
-          qx[j][k] = row < p.s_q ? __ldg(reinterpret_cast<const uint32_t*>(qsrc + (int64_t)row * (D / 16)) + k) : 0u;
-      }
+      for (int j = 0; j < 4; ++j) row_scales(qsrc + (int64_t)min(m0 + lane + 32 * j, p.s_q - 1) * (D / 16), qx[j]);
       if (r1 > r0) fetch(key0);
+      // rows lane, lane + 32, .. of an atom are neighbours
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int k = 0; k < C::KB; ++k)
-          *reinterpret_cast<uint32_t*>(s_qsf + sl * C::QSF_BYTES + k * 512 + sf_atom_offset(lane + 32 * j, 0)) = qx[j][k];
+      for (int k = 0; k < C::KB; ++k)
+        fwd_sts_v4(smem_u32(s_qsf + sl * C::QSF_BYTES + k * 512) + lane * 16, qx[0][k], qx[1][k], qx[2][k], qx[3][k]);
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&qsf_full[sl]);
@@ -402,25 +406,21 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         const int s = r % C::NSTAGE;
         if (r >= C::NSTAGE) mbar_wait(&empty[s], ((r / C::NSTAGE) & 1) ^ 1, &err, 4);
         uint8_t* st = s_stage + s * C::STAGE_BYTES + C::K_BYTES + C::V_BYTES;
+        const uint32_t at = smem_u32(st) + lane * 16;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int row = lane + 32 * j;
+        for (int k = 0; k < C::KB; ++k) fwd_sts_v4(at + k * 512, kx[0][k], kx[1][k], kx[2][k], kx[3][k]);
+        if (kBias) {
 #pragma unroll
-          for (int k = 0; k < C::KB; ++k)
-            *reinterpret_cast<uint32_t*>(st + k * 512 + sf_atom_offset(row, 0)) = kx[j][k];
-          if (kBias) reinterpret_cast<float*>(st + C::KSF_BYTES + C::VSF_BYTES)[row] = nb[j];
+          for (int j = 0; j < 4; ++j) reinterpret_cast<float*>(st + C::KSF_BYTES + C::VSF_BYTES)[lane + 32 * j] = nb[j];
         }
         if (kBias) {
           const int any = __any_sync(0xffffffffu, nb[0] != 0.0f || nb[1] != 0.0f || nb[2] != 0.0f || nb[3] != 0.0f);
           if (lane == 0) s_biased[s] = any;
         }
-        uint8_t* dst = st + C::KSF_BYTES;
 #pragma unroll
-        for (int j = 0; j < D / 32; ++j) {
-          const int dr = lane + 32 * j;
-          const int nt = dr >> 7, row = dr & 127;
-          *reinterpret_cast<uint32_t*>(dst + (0 * C::NT + nt) * 512 + sf_atom_offset(row, 0)) = vx[j].x;
-          *reinterpret_cast<uint32_t*>(dst + (1 * C::NT + nt) * 512 + sf_atom_offset(row, 0)) = vx[j].y;
+        for (int nt = 0; nt < C::NT; ++nt) {
+          fwd_sts_v4(at + C::KSF_BYTES + nt * 512, vx[4 * nt].x, vx[4 * nt + 1].x, vx[4 * nt + 2].x, vx[4 * nt + 3].x);
+          fwd_sts_v4(at + C::KSF_BYTES + (C::NT + nt) * 512, vx[4 * nt].y, vx[4 * nt + 1].y, vx[4 * nt + 2].y, vx[4 * nt + 3].y);
         }
         if (r + 1 < r1) fetch(key0 + (r + 1 - r0) * 128);
         fence_proxy_async_smem();
@@ -458,7 +458,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         mbar_wait(&full[s], ph, &err, 5);
         if (r >= C::NSBUF) {      // the S buffer's last tile has been read into registers
           const int u = r - C::NSBUF;
-          mbar_spin_wait(&s_free[u & 1], (u >> 1) & 1, &err, 7);
+          mbar_wait(&s_free[u & 1], (u >> 1) & 1, &err, 7);
         }
         tc_fence_after();
         uint8_t* st = s_stage + s * C::STAGE_BYTES;
@@ -513,7 +513,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             tmem_cp_32x128b_warpx4(sfv + k * 4,
                                    smem_u32(st + C::K_BYTES + C::V_BYTES + C::KSF_BYTES + k * 512));
         }
-        mbar_spin_wait(&p_full[b], (r >> 1) & 1, &err, 8);
+        mbar_wait(&p_full[b], (r >> 1) & 1, &err, 8);
         tc_fence_after();
         if (leader) {
 #pragma unroll
@@ -877,6 +877,7 @@ extern "C" int nvfp4_fwd(const uint8_t* qnv, const uint8_t* qsc, const uint8_t* 
   p.out = out; p.so_z = so_z; p.so_h = so_h; p.so_s = so_s; p.lse = lse;
   p.h = (int)h; p.hk = (int)hk; p.g = (int)(h / hk);
   p.s_q = (int)s_q; p.s_kv = (int)s_kv; p.s_pad = (int)s_pad;
+  p.vec_sc = (((uintptr_t)qsc | (uintptr_t)ksc) % (d / 16)) == 0;
   p.scaling = scaling; p.causal = (flags & NVFP4_FWD_CAUSAL) ? 1 : 0; p.status = status;
   // Rows leave through a tensor map; strides that a map cannot express (zero, negative, beyond 2^40 bytes) are stored
   // row by row.  A stride that is never taken is replaced by one that a map accepts.
