@@ -153,10 +153,10 @@ int launch(const char* what, void (*kern)(P...), dim3 grid, unsigned threads, si
   return launch_cluster(what, kern, grid, 1, threads, smem, st, static_cast<A&&>(args)...);
 }
 
-// launch() of a kernel that streams through L1
-template <typename... P, typename... A>
+// launch() of a kernel that streams through L1, if its blocks' shared memory leaves three of them room within the hint
+template <bool kFits = true, typename... P, typename... A>
 int launch_streaming(const char* what, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
-  prefer_l1(reinterpret_cast<const void*>(kern));
+  if constexpr (kFits) prefer_l1(reinterpret_cast<const void*>(kern));
   return launch_cluster(what, kern, grid, 1, threads, smem, st, static_cast<A&&>(args)...);
 }
 

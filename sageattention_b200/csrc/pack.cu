@@ -820,7 +820,7 @@ int pack_dispatch(const T* x, int64_t B, int64_t R, int64_t k_read, int64_t k_pa
     const int64_t tx = (k_pad + kColsKeys - 1) / kColsKeys, ty = (R + kColsRows - 1) / kColsRows;
     const int run = cols_run(tx * ty * B);
     dim3 grid((unsigned)((tx + run - 1) / run), (unsigned)ty, (unsigned)B);
-    return launch_streaming("nvfp4_pack(cols)", pack_cols_kernel<T, false>, grid, 256, 0, st, x, R, k_read, k_pad, sxb, sxk, nib, snb,
+    return launch_streaming<sizeof(T) == 2>("nvfp4_pack(cols)", pack_cols_kernel<T, false>, grid, 256, 0, st, x, R, k_read, k_pad, sxb, sxk, nib, snb,
                   snr, sc, ssb, ssr, vec, nullptr, 0, 0, nullptr, 0, 0, nullptr, 0, 0u, run);
   }
   const int64_t blocks = (total + 255) / 256;
@@ -868,7 +868,7 @@ int pack_dual_launch(const void* x, int64_t B, int64_t S, int d, int64_t s_pad, 
   const int64_t tx = (s_pad + kColsKeys - 1) / kColsKeys, ty = (d + kColsRows - 1) / kColsRows;
   const int run = cols_run(tx * ty * B);
   dim3 grid((unsigned)((tx + run - 1) / run), (unsigned)ty, (unsigned)B);
-  return launch_streaming(
+  return launch_streaming<sizeof(T) == 2>(
       "nvfp4_pack_dual", pack_cols_kernel<T, true>, grid, 256, 0, st, static_cast<const T*>(x), d, S, s_pad, sxb, sxs, tnib, (int64_t)d * (s_pad / 2), s_pad / 2, tsc,
       (int64_t)d * (s_pad / 16), s_pad / 16, vec, dnib, S * (int64_t)(d / 2), d / 2, dsc, S * (int64_t)(d / 16),
       d / 16, prescale_amax, sr_flags, seed, run);
@@ -898,7 +898,7 @@ int pack_qkv_launch(QkvArgs a, cudaStream_t st) {
   a.run = cols_run(a.bk * a.tx * a.ty);
   const int64_t total = a.nbq + a.nbk + a.bk * ((a.tx + a.run - 1) / a.run) * a.ty;
   NVFP4_REQUIRE(total < (1LL << 31), "nvfp4_pack_qkv: tensors too large");
-  return launch_streaming("nvfp4_pack_qkv", pack_qkv_kernel<T>, dim3((unsigned)total), 256, 0, st, a);
+  return launch_streaming<sizeof(T) == 2>("nvfp4_pack_qkv", pack_qkv_kernel<T>, dim3((unsigned)total), 256, 0, st, a);
 }
 
 template <typename T>
@@ -923,7 +923,7 @@ int kv_prefill_launch(PrefillArgs a, cudaStream_t st) {
   a.bpc = (pieces + 256 * kPrefillCopyIters - 1) / (256 * kPrefillCopyIters);
   const int64_t total = a.nbk + a.nbv + a.bpc * a.zhk;
   NVFP4_REQUIRE(total < (1LL << 31), "nvfp4_kv_prefill: tensors too large");
-  return launch_streaming("nvfp4_kv_prefill", kv_prefill_kernel<T>, dim3((unsigned)total), 256, 0, st, a);
+  return launch_streaming<sizeof(T) == 2>("nvfp4_kv_prefill", kv_prefill_kernel<T>, dim3((unsigned)total), 256, 0, st, a);
 }
 
 }  // namespace nvfp4
@@ -993,7 +993,7 @@ extern "C" int nvfp4_pack_mx8_t(const void* x, int dtype, int64_t B, int64_t S, 
   {                                                                                                     \
     constexpr int64_t kVecElems = 16 / sizeof(T);                                                       \
     const int vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && sxb % kVecElems == 0 && sxs % kVecElems == 0; \
-    return launch_streaming("nvfp4_pack_mx8_t", pack_mx8_cols_kernel<T>, grid, 256, 0, st, static_cast<const T*>(x), d, S, s_pad, \
+    return launch("nvfp4_pack_mx8_t", pack_mx8_cols_kernel<T>, grid, 256, 0, st, static_cast<const T*>(x), d, S, s_pad, \
                   sxb, sxs, out, sc, vec, prescale_amax);                                               \
   }
   switch (dtype) {
