@@ -113,7 +113,9 @@ struct DecodeParams {
 // weights exp(m_tile - m_now), so O is never rescaled in TMEM.
 //
 // kMerge: a CTA has one item, and the CTAs of a cluster (along z) have all items of one unit.  They merge their partials
-// through distributed shared memory, a share of the elements each, and write the result: no combine kernel.
+// through distributed shared memory, a share of the elements each, and write the result: no combine kernel.  Products and
+// sums are those of the combine kernel in its order -- pieces k and k + 4 are its warp k's, sums of exponentials go through a
+// butterfly of lanes -- so that a unit's result is the same to the bit whichever of the two its call takes.
 template <int D, typename TQ, int NQ, bool kMerge>
 __global__ void __launch_bounds__(kDecodeThreads, 1)
 decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -740,7 +742,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     const int unit = (int)(cta / ncl);
     cluster_sync_all();                  // the partials of all CTAs are there
     if (tid < p.g) {
-      float m[8], l[8], gm = -INFINITY, den = 0.0f;
+      float m[8], l[8], gm = -INFINITY;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         m[k] = (uint32_t)k < ncl ? ld_cluster_f32(smem_u32(&part_ml[tid]), k) : -INFINITY;
@@ -752,8 +754,9 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       for (int k = 0; k < 8; ++k) {
         const float f = (m[k] == -INFINITY) ? 0.0f : expf(m[k] - gm);
         part_w[k][tid] = f;
-        den += f * l[k];
+        l[k] = __fmul_rn(f, l[k]);       // no FMA with the sum
       }
+      float den = ((l[0] + l[4]) + (l[2] + l[6])) + ((l[1] + l[5]) + (l[3] + l[7]));
       if (den == 0.0f) den = 1.0f;
       part_w[8][tid] = den;
       if (p.lse != nullptr && rank == 0) p.lse[(int64_t)unit * p.g + tid] = gm + logf(den);
@@ -764,14 +767,20 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     for (uint32_t i = n4 * rank / ncl + tid; i < n4 * (rank + 1) / ncl; i += kDecodeThreads) {
       const uint32_t qi = i / (D / 4);
-      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      float4 s[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) s[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
       for (int k = 0; k < 8; ++k)
         if ((uint32_t)k < ncl) {
           const float4 x = ld_cluster_f4(acc0 + i * 16, k);
           const float f = part_w[k][qi];
-          v.x = fmaf(f, x.x, v.x); v.y = fmaf(f, x.y, v.y); v.z = fmaf(f, x.z, v.z); v.w = fmaf(f, x.w, v.w);
+          float4& a = s[k & 3];
+          a.x = fmaf(f, x.x, a.x); a.y = fmaf(f, x.y, a.y); a.z = fmaf(f, x.z, a.z); a.w = fmaf(f, x.w, a.w);
         }
+      float4 v = s[0];
+#pragma unroll
+      for (int k = 1; k < 4; ++k) { v.x += s[k].x; v.y += s[k].y; v.z += s[k].z; v.w += s[k].w; }
       const float den = part_w[8][qi];
       v = make_float4(v.x / den, v.y / den, v.z / den, v.w / den);
       if (!vec) {
@@ -949,6 +958,7 @@ int decode_launch(const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtens
   // with 64 / 128 / 256 threads: one piece 12.45 / 12.6 / 12.8 (Z1 S600), 14.5 / 14.8 / 14.9 (Z16 S1024); 2 to 8 pieces
   // at 128 up to 0.8 less than at 64 (0.1 more at worst) and up to 0.5 less than at 256 (0.3 more at worst); 16 pieces
   // 13.3 / 12.6 / 12.9, at D 256 15.3 / 14.0 / 13.75; 36 pieces 16.6 / 15.3 / 14.9; 64 pieces 17.0 / 14.9 / 14.2.
+  // The order of the sums follows from the warps: a cluster merges two to eight pieces as the four warps here would.
   const int64_t pieces = (p.balanced ? ((int64_t)p.ntiles * grid + p.total_tiles - 1) / p.total_tiles + 1 : p.nsplit) + p.n_extra;
   const unsigned threads = pieces * (D / 128) > 16 ? 256 : (pieces > 1 ? 128 : 64);
   return nvfp4::launch("nvfp4_decode(combine)", decode_combine_kernel<D, TQ>, dim3((unsigned)(zhk * p.g)), threads, 0, st, c);
