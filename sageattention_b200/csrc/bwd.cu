@@ -788,7 +788,6 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
     }
   }
   if (kSplit) {
-    __syncwarp();
     cluster_sync_all();
     TG* base_k = static_cast<TG*>(p.dk) + ((int64_t)unit * p.s_kv + n0) * D + half * 128;
     TG* base_v = static_cast<TG*>(p.dv) + ((int64_t)unit * p.s_kv + n0) * D + half * 128;

@@ -851,7 +851,6 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
   }
   if constexpr (kKeys) {
     if (p.split > 1) {
-      __syncwarp();
       cluster_sync_all();
       const int64_t first = ((int64_t)rb * R + row0) * D;
       red_sum_store<TG>(smem_u32(smem), rank, p.split, tid, C::THREADS, R - row0, kP ? static_cast<TG*>(p.out1) + first : nullptr,

@@ -208,7 +208,9 @@ __device__ __forceinline__ bool clc_answer(const void* resp, int& x, int& y, int
   return got != 0;
 }
 
+// All threads of the cluster; `.aligned` wants the lanes of a warp together, whatever branches and loops lie behind them.
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t saddr, uint32_t rank) {
