@@ -89,12 +89,15 @@ inline void prefer_l1(const void* kern) {
   if (kernel_attribute<cudaFuncAttributePreferredSharedMemoryCarveout>(kern, kStreamSmem) != cudaSuccess) cudaGetLastError();
 }
 
-// Clusters of `size` CTAs (1 to 8) of a kernel that are resident at once, asked once per device: for kernels that leave
-// room for one CTA per SM only (the answer depends on that alone).  allow_smem() has been called for `kern`.
+// Clusters of `size` CTAs (1 to 8, else 0) of a kernel that are resident at once.  Of kernels whose shared memory leaves room
+// for one CTA per SM the answer depends on the size alone and is asked once per device; of others on every call.
+// allow_smem() has been called for `kern`.
+constexpr int kSmemPerSm = 228 * 1024;
 inline int cluster_slots(const void* kern, unsigned threads, int smem, int sms, int size) {
   static std::atomic<int> known[64][9];
+  if (size < 1 || size > 8) return 0;
   int dev = 0;
-  const bool keep = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
+  const bool keep = 2 * smem > kSmemPerSm && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
   int n = keep ? known[dev][size].load(std::memory_order_relaxed) : 0;
   if (n > 0) return n;
   cudaLaunchAttribute attr;
