@@ -129,6 +129,18 @@ __device__ __forceinline__ void mbar_wait_all(uint64_t* a, uint32_t pa, uint64_t
   mbar_wait(b, pb, err, site);
 }
 
+// The same by a whole warp of which one thread acts on it (issues products or copies).  No lane is left behind: what that
+// thread does lets the barrier go on, and by its next phase the parity that a late lane looks for would be gone again.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* err, int site) {
+  const bool ok = mbar_wait(bar, parity, err, site);
+  __syncwarp();
+  return ok;
+}
+__device__ __forceinline__ void mbar_wait_all_warp(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb, volatile int* err, int site) {
+  mbar_wait_all(a, pa, b, pb, err, site);
+  __syncwarp();
+}
+
 // Bounded wait that polls without parking the thread: lowest wake-up latency, meant for a lone
 // elected thread (an MMA issuer) whose reaction time is on the critical path.
 __device__ __forceinline__ bool mbar_spin_wait(uint64_t* bar, uint32_t parity, volatile int* err,

@@ -381,7 +381,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       // the whole warp quantises the NEXT item's query rows into the other buffer; that buffer's
       // last readers are the QK^T MMAs of the previous item, complete once its last s_full fired
       if (wi + 1 < my_items) {
-        if (item_idx > 0) mbar_wait(&s_full[(su_w - 1) & 1], ((su_w - 1) >> 1) & 1, &err, 12);
+        if (item_idx > 0) mbar_wait_warp(&s_full[(su_w - 1) & 1], ((su_w - 1) >> 1) & 1, &err, 12);
         prep_q(wi + 1, (int)((item_idx + 1) & 1));
       }
       int unit, t0, t1;

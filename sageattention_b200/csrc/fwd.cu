@@ -316,7 +316,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll 1
       for (int r = r0; r < r1; ++r) {
         const int s = r % C::NSTAGE, t = t0 + r;
-        if (r >= C::NSTAGE) mbar_wait(&empty[s], ((r / C::NSTAGE) & 1) ^ 1, &err, 1);
+        if (r >= C::NSTAGE) mbar_wait_warp(&empty[s], ((r / C::NSTAGE) & 1) ^ 1, &err, 1);
         if (leader) {
           uint8_t* st = s_stage + s * C::STAGE_BYTES;
           mbar_expect_tx(&full[s], C::K_BYTES + C::V_BYTES);
@@ -441,8 +441,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       if (!mbar_wait_item_warp(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
       const int r1 = __shfl_sync(0xffffffffu, s_item[sl].r1, 0);
       if (r1 < 0) break;
-      mbar_wait(&q_full[sl], (it >> 1) & 1, &err, 3);
-      mbar_wait(&qsf_full[sl], (it >> 1) & 1, &err, 6);
+      mbar_wait_warp(&q_full[sl], (it >> 1) & 1, &err, 3);
+      mbar_wait_warp(&qsf_full[sl], (it >> 1) & 1, &err, 6);
       tc_fence_after();
       const uint32_t sfq = tmem + C::T_SFQ + sl * C::KB * 4;
       uint8_t* q = s_q + sl * C::Q_BYTES;
@@ -455,10 +455,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       for (; r < r1; ++r) {
         const int s = r % C::NSTAGE, b = r % C::NSBUF;
         const uint32_t ph = (r / C::NSTAGE) & 1;
-        mbar_wait(&full[s], ph, &err, 5);
+        mbar_wait_warp(&full[s], ph, &err, 5);
         if (r >= C::NSBUF) {      // the S buffer's last tile has been read into registers
           const int u = r - C::NSBUF;
-          mbar_wait(&s_free[u & 1], (u >> 1) & 1, &err, 7);
+          mbar_wait_warp(&s_free[u & 1], (u >> 1) & 1, &err, 7);
         }
         tc_fence_after();
         uint8_t* st = s_stage + s * C::STAGE_BYTES;
@@ -493,7 +493,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       const int r1 = __shfl_sync(0xffffffffu, s_item[sl].r1, 0);
       if (r1 < 0) break;
       if (r1 > r && r > 0) {          // O of the last item that had tiles has been read
-        mbar_wait(&o_free, o_phase, &err, 2);
+        mbar_wait_warp(&o_free, o_phase, &err, 2);
         o_phase ^= 1u;
       }
       const int r0 = r;
@@ -502,7 +502,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         const int s = r % C::NSTAGE, b = r & 1;
         // the V tile and V scales of stage s landed before this tile's QK^T was issued, but this
         // thread has to observe them itself; it does so while P is still being written
-        mbar_wait(&full[s], (r / C::NSTAGE) & 1, &err, 15);
+        mbar_wait_warp(&full[s], (r / C::NSTAGE) & 1, &err, 15);
         tc_fence_after();
         uint8_t* st = s_stage + s * C::STAGE_BYTES;
         const uint32_t sfp = tmem + C::T_SFP + b * 8;
@@ -513,7 +513,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             tmem_cp_32x128b_warpx4(sfv + k * 4,
                                    smem_u32(st + C::K_BYTES + C::V_BYTES + C::KSF_BYTES + k * 512));
         }
-        mbar_wait(&p_full[b], (r >> 1) & 1, &err, 8);
+        mbar_wait_warp(&p_full[b], (r >> 1) & 1, &err, 8);
         tc_fence_after();
         if (leader) {
 #pragma unroll
