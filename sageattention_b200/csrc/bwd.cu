@@ -768,7 +768,9 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
     }
     if (nstep > 0 || kSplit) {
       uint32_t r[32];
-#pragma unroll
+      // One after the other at D = 256 where a cluster shares the tile: unrolled, the kernel spills 8 bytes stored and 20 loaded.
+      // Backward H8 Hk2 D256 S384 18.33 -> 17.94 us, S512 23.95 -> 23.41 (before the spills grew 18.42 and 23.80).
+#pragma unroll(kSplit && D == 256 ? 1 : 2)
       for (int o = 0; o < 2; ++o) {         // dV, dK
         if (nstep > 0) {
           tmem_ld32(tmem + lane_addr + (o ? T_DK : T_DV) + part * 32, r);
