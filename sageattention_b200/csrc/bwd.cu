@@ -602,9 +602,9 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
       const bool leader = elect_one();
       const uint32_t id_s = make_idesc_nvfp4(128, 64);
       const uint32_t id_dp = make_idesc_bf16(128, 64, false);
-      mbar_wait_warp(&kv_full, 0, &err, 3);
-      mbar_wait_warp(&ksf_full, 0, &err, 4);
-      if (KT > 0) mbar_wait_warp(&a_full, 0, &err, 15);
+      mbar_wait(&kv_full, 0, &err, 3);
+      mbar_wait(&ksf_full, 0, &err, 4);
+      if (KT > 0) mbar_wait(&a_full, 0, &err, 15);
       tc_fence_after();
       if (leader) {
 #pragma unroll
@@ -616,7 +616,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
 #pragma unroll 1
       for (int st = 0; st < nstep; ++st) {
         const int s = st % L::NSTAGE, b = st & 1;
-        mbar_wait_warp(&full[s], (st / L::NSTAGE) & 1, &err, 5);
+        mbar_wait(&full[s], (st / L::NSTAGE) & 1, &err, 5);
         tc_fence_after();
         const uint32_t qsf = smem_u32(s_stage + L::O_QSF) + s * L::STAGE;
         if (leader) {
@@ -626,9 +626,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
         const uint64_t so = (uint64_t)(s * (L::STAGE >> 4));
         const uint64_t x_qp = b_qp + so, x_do = b_do + so;
         if (st > 0) {
-          mbar_wait_warp(&s_free, (st - 1) & 1, &err, 7);
+          mbar_wait(&s_free, (st - 1) & 1, &err, 7);
           tc_fence_after();
         }
+        __syncwarp();
         if (leader) {
 #pragma unroll
           for (int k = 0; k < L::KB; ++k)
@@ -666,7 +667,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kp, const __grid_constant
         const int s = st % L::NSTAGE, b = st & 1;
         // dO and Q of the stage landed before S^T and dP^T of the step were issued, but this thread has to observe them
         // itself; it does so while P^T and dS^T are still being written
-        mbar_wait_warp(&full[s], (st / L::NSTAGE) & 1, &err, 6);
+        mbar_wait(&full[s], (st / L::NSTAGE) & 1, &err, 6);
         mbar_wait_warp(&pds_full[b], (st >> 1) & 1, &err, 8);
         tc_fence_after();
         // dV += P^T dO and dK += dS^T Q; slot columns: [P^T q0-31 | dS^T q0-31 | P^T q32-63 | dS^T q32-63], 16 each
@@ -1076,9 +1077,10 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
       if (!mbar_wait_item_warp(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
       const int r1 = __shfl_sync(0xffffffffu, s_item[sl].r1, 0);
       if (r1 < 0) break;
-      mbar_wait_warp(&q_full[sl], (it >> 1) & 1, &err, 3);
-      mbar_wait_warp(&qsf_full[sl], (it >> 1) & 1, &err, 4);
-      if (r1 > r) mbar_wait_warp(&a_full[sl], (it >> 1) & 1, &err, 15);
+      mbar_wait(&q_full[sl], (it >> 1) & 1, &err, 3);
+      mbar_wait(&qsf_full[sl], (it >> 1) & 1, &err, 4);
+      if (r1 > r) mbar_wait(&a_full[sl], (it >> 1) & 1, &err, 15);
+      __syncwarp();
       tc_fence_after();
       const uint64_t b_qp = desc_sw64(s_qp + si * L::QP, 0);
       const uint32_t sfq = tmem + T_SFQ + si * SF;
@@ -1091,9 +1093,9 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
         const int s = r % L::NSTAGE, b = r & 1;
         // the operands of the step; what its dP slot held, dS of step r - NG, has been consumed
         if (r >= L::NG)
-          mbar_wait_all_warp(&full[s], (r / L::NSTAGE) & 1, &empty[(r - L::NG) % L::NSTAGE], ((r - L::NG) / L::NSTAGE) & 1, &err, 5);
+          mbar_wait_all(&full[s], (r / L::NSTAGE) & 1, &empty[(r - L::NG) % L::NSTAGE], ((r - L::NG) / L::NSTAGE) & 1, &err, 5);
         else
-          mbar_wait_warp(&full[s], (r / L::NSTAGE) & 1, &err, 5);
+          mbar_wait(&full[s], (r / L::NSTAGE) & 1, &err, 5);
         tc_fence_after();
         const uint64_t so = (uint64_t)(s * (L::STAGE >> 4));
         const uint64_t x_kp = b_kp + so, x_v = b_v + so;
@@ -1106,9 +1108,10 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
           for (int c = 0; c < L::KB; ++c) tmem_cp_32x128b_warpx4(tmem + T_SFK + b * SF + 4 * c, ksf + c * 512);
         }
         if (r > 0) {
-          mbar_wait_warp(&s_free, (r - 1) & 1, &err, 7);
+          mbar_wait(&s_free, (r - 1) & 1, &err, 7);
           tc_fence_after();
         }
+        __syncwarp();
         if (leader) {
 #pragma unroll
           for (int k = 0; k < L::KB; ++k)
@@ -1138,8 +1141,8 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qp, const __grid_constant__
       for (; r < r1; ++r) {
         // K of the stage landed before S and dP of the step were issued, but this thread has to observe it itself;
         // it does so while dS is still being written
-        mbar_wait_warp(&full[r % L::NSTAGE], (r / L::NSTAGE) & 1, &err, 6);
-        if (r == first && n > 0) mbar_wait_warp(&dq_free, (n - 1) & 1, &err, 16);
+        mbar_wait(&full[r % L::NSTAGE], (r / L::NSTAGE) & 1, &err, 6);
+        if (r == first && n > 0) mbar_wait(&dq_free, (n - 1) & 1, &err, 16);
         mbar_wait_warp(&ds_full[r & 1], (r >> 1) & 1, &err, 8);
         tc_fence_after();
         const uint32_t a_ds = tmem + T_DP + (r % L::NG) * 64;

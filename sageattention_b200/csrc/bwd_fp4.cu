@@ -14,7 +14,7 @@
 //               group in turn (dV / dK are reduced over the group in TMEM and written once); one pass
 //               for both at D = 128, one each at D = 256;
 //   dQ pass     rows = queries of a head, columns = keys.
-// Per step one issuer thread queues S (or S^T) and dP as N=64 block-scaled MMAs, another the gradient GEMMs; a
+// Per step one issuer warp queues S (or S^T) and dP as N=64 block-scaled MMAs, another the gradient GEMMs; a
 // softmax thread owns one row and 16-column chunks of the step's 64 columns, so the per-16 packs of
 // P and dS along the columns are thread-local: nibbles and scale bytes go to shared memory in the
 // operand layout and feed one MMA (M128, N = head dim, K64) per gradient and step.  FP4 MMAs replace
@@ -525,8 +525,8 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
     if (nstep > 0) {
       const bool leader = elect_one();
       const uint32_t id_n64 = make_idesc_nvfp4(128, 64);
-      mbar_wait_warp(&x_full, 0, &err, 3);
-      mbar_wait_warp(&xsf_full, 0, &err, 4);
+      mbar_wait(&x_full, 0, &err, 3);
+      mbar_wait(&xsf_full, 0, &err, 4);
       tc_fence_after();
       if (leader) {
 #pragma unroll
@@ -541,8 +541,8 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
       for (int st = 0; st < nstep; ++st) {
         const int pp = st & 1, sg = st >> 1, s = sg % C::NSTAGE;
         uint8_t* sb = s_stage + s * C::STAGE;
-        if (pp == 0) mbar_wait_warp(&full[s], (sg / C::NSTAGE) & 1, &err, 5);
-        if (st >= 2) mbar_wait_warp(&s_free[pp], ((st >> 1) - 1) & 1, &err, 7);      // S slot: read by the team of step st - 2
+        if (pp == 0) mbar_wait(&full[s], (sg / C::NSTAGE) & 1, &err, 5);
+        if (st >= 2) mbar_wait(&s_free[pp], ((st >> 1) - 1) & 1, &err, 7);      // S slot: read by the team of step st - 2
         tc_fence_after();
         const uint64_t so = (uint64_t)(s * (C::STAGE >> 4)) + (uint64_t)(pp * 256);   // 64 rows x 64 bytes further
         if (leader) {
@@ -561,9 +561,10 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
           // (1270 clocks of which 850 the next team's wait).  Both scales come with one copy a block of D: S8192 D128
           // 1427 -> 1381 us in all, S4100 D256 385 -> 373, S8192 D256 1170 -> 1140.
           if (st > 0) {
-            mbar_wait_warp(&g_free, (st - 1) & 1, &err, 9);
+            mbar_wait(&g_free, (st - 1) & 1, &err, 9);
             tc_fence_after();
           }
+          __syncwarp();
           if (leader) {
             // dP (or dP^T)
 #pragma unroll
@@ -572,6 +573,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
                          id_n64, tmem + C::T_SFX2 + k * 4, tmem + C::T_SFY + k * 4 + 2, k > 0);
           }
         }
+        if constexpr (!kDs) __syncwarp();
         if (leader) umma_commit(&s_full[pp]);
         __syncwarp();
       }
@@ -579,7 +581,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
     __syncwarp();
   } else if (warp == 3) {
     // ------------------------------------------------------------------ issuer of the gradient GEMMs
-    // A thread of its own: one thread for all products paid its waits and commits one after the other, about 1100
+    // A warp of its own: one issuer for all products paid its waits and commits one after the other, about 1100
     // clocks a step, and S and dP of the next step stood behind the wait for this one's operands.
     if (nstep > 0) {
       const bool leader = elect_one();
@@ -612,7 +614,7 @@ bwd4_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ C
       auto grad_gemms = [&](int t) {
         const int pp = t & 1, s = (t >> 1) % C::NSTAGE;
         uint8_t* sb = s_stage + s * C::STAGE;
-        if (pp == 0) mbar_wait_warp(&full[s], ((t >> 1) / C::NSTAGE) & 1, &err, 6);   // the transposed tiles, seen by this thread
+        if (pp == 0) mbar_wait(&full[s], ((t >> 1) / C::NSTAGE) & 1, &err, 6);   // the transposed tiles, seen by this thread
         mbar_wait_warp(&a_full[pp], (t >> 1) & 1, &err, 8);
         tc_fence_after();
         const uint32_t acc = t > 0 ? 1u : 0u;

@@ -441,7 +441,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       if (!mbar_wait_item_warp(&item_full[sl], (it >> 1) & 1, &err, 22)) break;
       const int r1 = __shfl_sync(0xffffffffu, s_item[sl].r1, 0);
       if (r1 < 0) break;
-      mbar_wait_warp(&q_full[sl], (it >> 1) & 1, &err, 3);
+      mbar_wait(&q_full[sl], (it >> 1) & 1, &err, 3);
       mbar_wait_warp(&qsf_full[sl], (it >> 1) & 1, &err, 6);
       tc_fence_after();
       const uint32_t sfq = tmem + C::T_SFQ + sl * C::KB * 4;
@@ -455,14 +455,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       for (; r < r1; ++r) {
         const int s = r % C::NSTAGE, b = r % C::NSBUF;
         const uint32_t ph = (r / C::NSTAGE) & 1;
-        mbar_wait_warp(&full[s], ph, &err, 5);
+        mbar_wait(&full[s], ph, &err, 5);
         if (r >= C::NSBUF) {      // the S buffer's last tile has been read into registers
           const int u = r - C::NSBUF;
-          mbar_wait_warp(&s_free[u & 1], (u >> 1) & 1, &err, 7);
+          mbar_wait(&s_free[u & 1], (u >> 1) & 1, &err, 7);
         }
         tc_fence_after();
         uint8_t* st = s_stage + s * C::STAGE_BYTES;
         const uint32_t sfk = tmem + C::T_SFK + (r & 1) * C::KB * 4;
+        __syncwarp();
         if (leader) {
 #pragma unroll
           for (int k = 0; k < C::KB; ++k)
@@ -493,7 +494,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       const int r1 = __shfl_sync(0xffffffffu, s_item[sl].r1, 0);
       if (r1 < 0) break;
       if (r1 > r && r > 0) {          // O of the last item that had tiles has been read
-        mbar_wait_warp(&o_free, o_phase, &err, 2);
+        mbar_wait(&o_free, o_phase, &err, 2);
         o_phase ^= 1u;
       }
       const int r0 = r;
@@ -502,7 +503,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         const int s = r % C::NSTAGE, b = r & 1;
         // the V tile and V scales of stage s landed before this tile's QK^T was issued, but this
         // thread has to observe them itself; it does so while P is still being written
-        mbar_wait_warp(&full[s], (r / C::NSTAGE) & 1, &err, 15);
+        mbar_wait(&full[s], (r / C::NSTAGE) & 1, &err, 15);
         tc_fence_after();
         uint8_t* st = s_stage + s * C::STAGE_BYTES;
         const uint32_t sfp = tmem + C::T_SFP + b * 8;
