@@ -154,8 +154,9 @@ __device__ __forceinline__ uint8_t pack_group16(const float (&x)[16], uint32_t& 
 //   * 1 / scale as hi + lo, hi below it and lo the rest (2^-22 of it): RN(x hi + RN(x lo)) is off by 2^-45 before its one
 //     rounding, hence t where the quotient is t.  lo is positive, so a zero keeps its sign.
 // Infinities end at the largest code as they do by division; nothing here can make a NaN of them.
-// Along D [128, 8192, 128] bf16 60.0 -> 52.3 us (6.6 TB/s, the copy rate), both ways at once [16, 8192, 256] 35.0 -> 27.8, V^T
-// [64, 8192, 128] 37.4 -> 34.3.  All 16-bit values under all scales are compared with the division in a test.
+// Along D [64, 8192, 128] bf16 31.5 -> 27.4 us, [128, 8192, 128] on changing clocks 62 -> 54.4 (6.3 TB/s, 0.96 of the copy
+// rate), both ways at once [16, 8192, 256] 34.7 -> 27.7, V^T [64, 8192, 128] 37.1 -> 34.0.  All 16-bit values under all scales,
+// and boundary values behind a power of two, are compared with the division in tests.
 template <typename T>
 __device__ __forceinline__ uint8_t pack_group16_of(const float (&x)[16], uint32_t& lo, uint32_t& hi) {
   if constexpr (sizeof(T) != 2) {

@@ -20,8 +20,8 @@
 // What bounds it: a long cache HBM (Z16 Hk8 S32768 D128, 604 MB: 104 us, 5.8 TB/s or 0.89 of the copy rate, where scale
 // bytes that were handed on three tiles late had it at 122), a short one a chain of cold steps: first loads, four
 // tiles' products, a softmax round, their P.V, the partials -- 7700 clocks for one round, 11700 with the L2 pulls in front of
-// the first load.  Graphs of append and decode: Z1 Hk8 S1021 13.9 -> 11.8 us, Z4 Hk4 S6007 D256 18.9 -> 16.0, Z16 Hk8
-// S32768 132 -> 113.7, with a window Z8 Hk8 S8190 41.5 -> 39.5-41.0.
+// the first load.  Graphs of append and decode, with the cluster merge: Z1 Hk8 S1021 14.1 -> 11.3 us, Z4 Hk4 S6007 D256
+// 19.1 -> 16.2, Z16 Hk8 S32768 132 -> 112.3, with a window Z8 Hk8 S8190 41.2 -> 37.5.
 #include "common/abi.cuh"
 #include "common/fp4.cuh"
 #include "common/launch.cuh"
@@ -929,8 +929,8 @@ int decode_launch(const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtens
   // Up to eight items a unit, each with a CTA of its own: a cluster merges them (one item: a cluster of one), if all clusters
   // are resident at once (74, 33 and 15 of two, four and eight; a second wave costs more than the combine's launch).
   // A step of append and decode: 16.2 -> 14.0 us of host time at any of these sizes (one launch less); its graph, us: Z1 Hk8 S256
-  // (one item a unit) 9.4 -> 8.0, S1021 (two) 11.7 -> 11.1, S4000 (eight) 10.6 -> 9.9, Z8 S900 12.1 -> 10.8, D 256 Z1 Hk4
-  // S3000 (six) 13.2 -> 12.7.
+  // (one item a unit) 9.7 -> 8.25, S1021 (two) 11.95 -> 11.3, S4000 (eight) 10.85 -> 10.2, Z8 S900 12.4 -> 11.2, D 256 Z1 Hk4
+  // S3000 (six) 13.4 -> 12.9.
   bool merge = !p.balanced && p.n_extra == 0 && p.nsplit <= 8 && p.nitems == grid;
   auto launch = [&](auto kern, auto kmerge) -> int {
     if (merge) {

@@ -33,8 +33,8 @@
 // maxima are the first to be exponentiated, without another read; reciprocal scales come from a table in
 // shared memory, not from the pipe that ex2 needs; P leaves in 16-byte stores.
 // Measured on a B200, kernel alone, causal bf16, against one CTA per query tile and, the last figure, with uniform registers
-// for addresses, six stages and whole scale rows: Z4 H32 Hk8 S8192 D128 2033 -> 1695 -> 1576 us (1.40 PFLOP/s), Z1 S2048
-// 51.6 -> 37.7 -> 34.0; H16 Hk4 D256 S8192 334 -> 297 -> 270, S2048 33.2 -> 28.5 -> 25.7.
+// for addresses, six stages and whole scale rows: Z4 H32 Hk8 S8192 D128 2033 -> 1693 -> 1579 us (1.39 PFLOP/s), Z1 S2048
+// 51.6 -> 37.7 -> 34.5; H16 Hk4 D256 S8192 334 -> 296 -> 269, S2048 33.2 -> 28.4 -> 26.2.
 // Masks: only tiles at an edge of what a row may see -- diagonal, ragged end, ends of a packed sample -- and
 // tiles whose bias has a value other than zero (added already divided by the scaling) are edited, in tensor memory
 // before the maxima are taken, by bits of a 32-column word formed from the row's range; the loop over the others holds

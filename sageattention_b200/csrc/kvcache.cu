@@ -27,8 +27,8 @@ __global__ void kv_append_kernel(const T* __restrict__ k_new, const T* __restric
   const T* kr = k_new + u * s_new;
   const T* vr = v_new + u * s_new;
   {
-    // In front of the wait, while the kernel before drains: the open group and the new rows into L2.  Step of a cache with
-    // a window Z8 Hk8 S8190 43.8 -> 41.2 us; graph of Z1 S1021 11.08 -> 10.9.
+    // In front of the wait, while the kernel before drains: the open group and the new rows into L2.  Step of a cache with a
+    // window Z8 Hk8 S8190 on changing inputs 42.35 -> 39.9 us, its graph 39.05 -> 37.5; without a window -0.1 to 0.
     constexpr int kLine = 128 / sizeof(T);
     const int slots = (int)(pos % 16), lines = d / kLine;
     for (int i = t; i < slots * lines; i += blockDim.x) prefetch_l2(partial + (u * 16 * d + (int64_t)i * kLine));
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(kWinThreads, D == 128 ? 2 : 1) window_mma_kern
   const int cap = (int)ring_cap, first = (int)((first_pos_all + k0) % ring_cap);
   if (tid < 2 && count > 0) {
     // In front of the wait: the piece's K (thread 0) and V rows into L2, while the append writes the newest of them; one
-    // run of memory, or two where the ring wraps.  Step Z8 Hk8 S8190 window 512: 41.2 -> 40.2 us.
+    // run of memory, or two where the ring wraps.  Step Z8 Hk8 S8190 window 512 on changing inputs: 40.5 -> 39.7 us.
     const T* base = (tid ? rv : rk) + (int64_t)blockIdx.x * ring_cap * D;
     const int n = min(count, cap - first);
     bulk_prefetch_l2(base + (int64_t)first * D, (uint32_t)n * kRowB);
